@@ -23,34 +23,39 @@
 #include "mcb_gemm.h"
 #include "mcb_launch.h"
 #include "mcb_route.cuh"
+#include "mcb_tmap.h"
 
 namespace mcb {
 
-__global__ void __launch_bounds__(kFfnThreads, 1) expert_ffn_kernel(const __grid_constant__ McbFfnArgs a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1) expert_ffn_kernel(const __grid_constant__ McbFfnArgs a) {
+  ffn_setup(a);
   pdl_wait();
   pdl_launch_dependents();
   ffn_device(a);
+  ffn_teardown();
 }
 
 template <bool EMU>
-__global__ void __launch_bounds__(kFfnThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1)
 moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* eargs) {
   const McbLayerArgs& p = EMU ? eargs[blockIdx.y] : p_;
   const McbCtx& c = p.ctx;
   uint32_t ll_launch = 0;
   const bool tracing = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
   if (tracing) p.trace[0] = globaltimer_ns();
+  ffn_setup(p.ffn);
   agv_device<MCB_SITE_FC1_FUSED>(c, p.agv, ll_launch);      // waits for the previous kernel first
   if (tracing) p.trace[1] = globaltimer_ns();
   // The arrival counter is back at zero whenever a launch has ended (its last block resets it).
   uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 1);
   grid_sync(c, arrivals, gridDim.x);
   if (tracing) p.trace[2] = globaltimer_ns();
-  route_device(p.route);
+  route_device(p.route, reinterpret_cast<int*>(FfnSmem().pipe));     // the pipeline is not in use yet
   if (tracing) p.trace[3] = globaltimer_ns();
   grid_sync(c, arrivals, 2u * gridDim.x);
   if (tracing) p.trace[4] = globaltimer_ns();
   ffn_device(p.ffn);
+  ffn_teardown();
   if (tracing) p.trace[5] = globaltimer_ns();
   grid_sync(c, arrivals, 3u * gridDim.x);                   // every y row is written before any is summed
   if (tracing) p.trace[6] = globaltimer_ns();
@@ -82,11 +87,33 @@ static bool configure_ffn_kernels() {
 }
 
 static int check_ffn_args(const McbFfnArgs* a) {
-  if (!a || !a->x || !a->pair_token || !a->expert_offset || !a->max_rows || !a->act || !a->y || !a->ffn_done) return 1;
+  if (!a || !a->x || !a->pair_token || !a->expert_offset || !a->max_rows || !a->act || !a->y || !a->ffn_done || !a->sync) return 1;
   if (!a->w1 || !a->w2 || (reinterpret_cast<uintptr_t>(a->w1) & 15) || (reinterpret_cast<uintptr_t>(a->w2) & 15)) return 1;
-  if (a->num_local_experts < 1 || a->num_local_experts > kFfnMaxExperts || a->hidden < 128 || a->hidden % 128 || a->intermediate < 128 || a->intermediate % 128) return 1;
-  if (a->x_row_bytes & 15) return 1;
+  if (a->num_local_experts < 1 || a->num_local_experts > kFfnMaxExperts || a->hidden < 256 || a->hidden % 256 || a->intermediate < 128 || a->intermediate % 128) return 1;
+  if (!a->tmaps || (reinterpret_cast<uintptr_t>(a->tmaps) & 63)) return 1;
   return 0;
+}
+
+// The kernels run in CTA pairs: an odd grid is rounded down, one CTA is rounded up.
+static int pair_grid(int grid) { return grid < 2 ? 2 : grid & ~1; }
+
+// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory; the caller
+// copies them to the device.  x: token rows; act, y: activations and expert outputs; w1, w2: the packed weights.
+int mcb_make_ffn_tmaps(void* out, const void* x, uint64_t x_rows, const void* act, const void* y, uint64_t pair_rows, const void* w1,
+                       const void* w2, int experts, int hidden, int intermediate) {
+  uint8_t* o = reinterpret_cast<uint8_t*>(out);
+  const uint64_t E = experts, H = hidden, I = intermediate;
+  if (!out || experts < 1 || hidden % 256 || intermediate % 128) return (int)cudaErrorInvalidValue;
+  int err = make_tmap_bf16(o + MCB_FFN_MAP_X * 128, x, x_rows, H, 1);
+  for (int b = 0; b < 8 && !err; ++b) {
+    err = make_tmap_bf16(o + (MCB_FFN_MAP_ACT + b) * 128, act, pair_rows, I, 8 * (b + 1));
+    if (!err) err = make_tmap_bf16(o + (MCB_FFN_MAP_XP + b) * 128, y, pair_rows, H, 8 * (b + 1));
+  }
+  for (int d = 0; d < 2 && !err; ++d) {
+    err = make_tmap_flat(o + (MCB_FFN_MAP_W1 + 2 * d) * 128, w1, E * 2 * I * H * 2, 8 * (d + 1));
+    if (!err) err = make_tmap_flat(o + (MCB_FFN_MAP_W2 + 2 * d) * 128, w2, E * H * I * 2, 8 * (d + 1));
+  }
+  return err;
 }
 
 // Gate/up + SwiGLU + down over the pair lists of a routing, as one persistent launch.
@@ -94,7 +121,7 @@ int mcb_launch_expert_ffn(const McbFfnArgs* args, int grid, int pdl, cudaStream_
   if (grid < 1 || check_ffn_args(args)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
   // A down block waits for gate/up blocks that other CTAs compute: all CTAs must be resident.
-  return launch_kernel(expert_ffn_kernel, dim3(grid), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *args);
+  return launch_kernel(expert_ffn_kernel, dim3(pair_grid(grid)), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *args);
 }
 
 static int check_layer_args(const McbLayerArgs* p, int grid) {
@@ -108,7 +135,7 @@ static int check_layer_args(const McbLayerArgs* p, int grid) {
 int mcb_launch_moe_layer(const McbLayerArgs* p, int grid, int pdl, cudaStream_t stream) {
   if (check_layer_args(p, grid)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
-  return launch_kernel(moe_layer_kernel<false>, dim3(grid), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *p,
+  return launch_kernel(moe_layer_kernel<false>, dim3(pair_grid(grid)), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *p,
                        (const McbLayerArgs*)nullptr);
 }
 
@@ -129,7 +156,7 @@ int mcb_emu_moe_layer(const McbLayerArgs* d_args, const McbLayerArgs* h_args0, i
   if (!d_args || world < 1 || check_layer_args(h_args0, grid)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
   McbLayerArgs dummy{};
-  return launch_kernel(moe_layer_kernel<true>, dim3(grid, world), dim3(kFfnThreads), kFfnSmemBytes, stream, 0, true,
+  return launch_kernel(moe_layer_kernel<true>, dim3(pair_grid(grid), world), dim3(kFfnThreads), kFfnSmemBytes, stream, 0, true,
                        dummy, d_args);
 }
 

@@ -29,6 +29,7 @@
 #include "mcb_dense.cuh"
 #include "mcb_gemm.h"
 #include "mcb_launch.h"
+#include "mcb_tmap.h"
 #include "mcb_route.cuh"
 #include "mcb_tc.cuh"
 
@@ -253,7 +254,8 @@ dispatch_route_fc1_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
   // The arrival counter is back at zero whenever a launch has ended (its last block resets it).
   uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 1);
   grid_sync(c, arrivals, gridDim.x);
-  route_device(r);
+  __shared__ int s_route[2 * kMaxLocalExperts];
+  route_device(r, s_route);
   grid_sync(c, arrivals, 2u * gridDim.x);
   gemm_device<MCB_GEMM_FC1>(w_map, a);
   launch_end(c, MCB_SITE_FC1_FUSED, ll_launch, arrivals);
@@ -285,31 +287,10 @@ extern "C" {
 int mcb_sizeof_gemm_args() { return (int)sizeof(McbGemmArgs); }
 int mcb_gemm_smem_bytes() { return kSmemBytes; }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Fills `out` (128 bytes, 64-byte aligned host memory) with a tensor map over a row-major bf16
-// matrix [rows, cols]: boxes of 128 rows x 64 columns, 128-byte swizzle.
+// Tensor map of the weights for the tokens-as-rows kernels: boxes of 128 rows x 64 columns, 128-byte swizzle.
 int mcb_make_weight_tmap(void* out, const void* base, uint64_t rows, uint64_t cols) {
-  static EncodeTiledFn encode = nullptr;
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
-    if (err != cudaSuccess) return (int)err;
-    if (qres != cudaDriverEntryPointSuccess || !fn) return (int)cudaErrorNotSupported;
-    encode = reinterpret_cast<EncodeTiledFn>(fn);
-  }
-  if (cols % kBlockK || rows % 128 || (reinterpret_cast<uintptr_t>(base) & 15)) return (int)cudaErrorInvalidValue;
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {cols * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)kBlockK, 128};
-  const cuuint32_t estr[2] = {1, 1};
-  CUresult r = encode(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
-                      dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+  if (rows % 128) return (int)cudaErrorInvalidValue;
+  return make_tmap_bf16(out, base, rows, cols, 128);
 }
 
 static bool configure_gemm_kernels() {

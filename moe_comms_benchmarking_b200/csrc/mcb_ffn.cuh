@@ -1,407 +1,592 @@
-// Grouped SwiGLU expert FFN for decode-size batches on the 5th-generation tensor cores, with the
-// operands swapped: the WEIGHTS are the M = 128 operand and the tokens of one expert are the small N.
+// Grouped SwiGLU expert FFN on the 5th-generation tensor cores, from decode to prefill sizes, with the
+// WEIGHTS as the M operand and the tokens of one expert as N.
 //
-// The reference has no expert computation at all (identity expert, bench_nvls.py:109-112).  At
-// decode sizes an expert sees a handful of tokens (3 at a global batch of 64, 170 at 4096 with 512
-// experts / top-22), and a layer is bound by streaming 6 MB of weights per expert.  With tokens as
-// the M operand every expert costs a full 128-row MMA and experts with more than 128 tokens read
-// their weights once per 128 tokens; here
-//   * a work unit is 128 weight rows x the whole reduction length (256 KB of bf16 at K = 1024) of
-//     one expert, multiplied with ALL tokens of that expert in one pass: D[128, N] += W[128, K] X[N, K]^T
-//     with N = the expert's token count rounded up to 16 (up to 256 per pass, accumulators double
-//     buffered in TMEM), so an MMA costs N / 256 of the padded one and every weight byte is read once;
-//   * both projections run in ONE persistent kernel: units 0 .. E * 2I/128 are the gate/up blocks,
-//     the rest the down blocks, dealt round-robin over the CTAs, so the weight stream does not stop
-//     at a kernel boundary.  A down block of expert e waits until all gate/up blocks of e have
-//     stored their activations (a counter per expert; every CTA meets all its gate/up blocks before
-//     its first down block, so the wait cannot deadlock);
-//   * the gate/up matrix is stored interleaved (row 2i = gate row i, row 2i + 1 = up row i), so a
-//     128-row block yields 64 finished activations: the two values meet in neighbouring TMEM lanes
-//     and are exchanged with one shuffle;
-//   * the weights are PRE-PACKED, once, into the image their tiles have in shared memory: tile
-//     (128-row block, 64-column block) is 16 KB of contiguous memory holding the 128 x 64 bf16 values
-//     in the K-major layout with 128-byte swizzle that the MMA descriptor expects, and the 16 tiles of
-//     a work unit follow one another.  A stage is then filled by ONE bulk copy (cp.async.bulk, no
-//     tensor map, no multicast) of a contiguous 16 KB range, so DRAM sees long sequential reads
-//     instead of 128 strided 128-byte pieces per tile;
-//   * token rows arrive by asynchronous 16-byte copies through the pair -> token list (the routing
-//     permute fused into the operand load) into the same swizzled K-major layout, eight neighbouring
-//     threads reading the 128 bytes of one row; a pipeline stage holds two 64-column blocks (one 32 KB
-//     bulk copy: with 16 KB stages the per-stage work of the single MMA-issuing thread - barrier wait,
-//     proxy fence, descriptors, commit - limited the weight stream), and the number of stages grows as
-//     the token tile shrinks (5 stages of 36 KB at N = 16; tiles of more than 64 tokens go back to one
-//     block per stage, 4 stages of 48 KB at N = 256);
-//   * nothing at a unit boundary goes to global memory: the experts' pair offsets sit in shared memory, and
-//     the gather indices of the next unit's first pass (and, for a down block, its expert's "gate/up blocks
-//     done" counter) are requested while the current unit is still being copied; the routing weights of a
-//     pass are fetched once per pass and handed to the epilogue's stores by shuffles.  (With these trips to
-//     L2 on the critical path the pipeline drained at every unit: 147.7 -> 128.6 us at 4096 gathered tokens.)
-//   * the epilogue reads the accumulators with tcgen05.ld (a lane holds ONE output feature of 16 tokens),
-//     turns them through a small shared-memory tile and stores 16 bytes per lane, feature-contiguous as
-//     the next GEMM and the combine want them (2-byte stores made the epilogue the slowest role from a
-//     few thousand tokens on: 128.4 -> 111.7 us at 4096 gathered tokens);
-//   * one elected thread issues tcgen05.mma; every mbarrier wait is bounded and reports through the
-//     status words.
+// The reference has no expert computation at all (identity expert, bench_nvls.py:109-112).  A layer is
+// bound by streaming 6 MB of weights per expert while experts see a handful of tokens, and by the tensor
+// pipe once they see a few hundred; in between the limit is what the SMs can take from L2, because every
+// weight block needs the rows of all tokens of its expert.  Hence:
+//   * a CTA PAIR (cluster of two, cta_group::2) works on one M = 256 tile: each CTA streams 128 weight rows
+//     and HALF of the token rows, so a token row enters the SMs once per 256 weight rows, and one thread of
+//     the pair issues the MMAs of both SMs.  A work unit is 256 weight rows x the whole reduction length x
+//     one chunk of up to 256 tokens of one expert; an expert's tokens are cut into equal chunks, rounded up
+//     to 32, and the accumulators are double buffered in TMEM;
+//   * every operand arrives by TMA: weights as 16 or 32 KB tiles (pre-packed once into the swizzled K-major
+//     image of their shared-memory tile, so a tile is contiguous in memory), activations as boxes of rows.
+//     Token rows come four at a time through the pair -> token list (tile::gather4, the routing permute fused
+//     into the load) while an expert has at most kFfnGatherN tokens.  One gather costs its issuing thread about
+//     100 cycles whatever it moves, which at more tokens is slower than the MMAs it feeds, so there the
+//     rows are first copied into pair order (into the memory of the expert outputs, which an expert's down
+//     units overwrite only after all its gate/up units have read it) and come as boxes too;
+//   * work units are listed per CTA pair in shared memory before the roles start: experts without tokens are
+//     left out of the numbering, so the pairs get equally many units whatever the routing, and a
+//     popular expert's chunks spread over the chip;
+//   * both projections run in one persistent stream.  While the activations of all experts fit in L2 the gate/up
+//     units of every expert come first, then the down units; above that a down unit follows its gate/up
+//     units at a distance of two rounds of the grid, while its activations are still in L2.  A down
+//     unit waits for a counter of its expert's finished gate/up units; units are taken in list order, so the
+//     wait cannot deadlock;
+//   * the gate/up matrix is stored interleaved (row 2i = gate row i, row 2i + 1 = up row i): the two values
+//     of an activation meet in neighbouring TMEM lanes and are exchanged with one shuffle;
+//   * weights and tokens have producer warps of their own, so the weight stream runs on while a down unit
+//     waits; eight epilogue warps read the accumulators with tcgen05.ld (a lane holds one output feature),
+//     turn them through a small shared-memory tile and store 16 bytes per lane, feature-contiguous;
+//   * every mbarrier wait is bounded and reports through the status words.
+// Measured on one B200 with 64 experts of 1024 x 1024 (402.7 MB of weights), against one CTA per unit of 128 weight rows
+// with token rows copied by cp.async and units numbered over all experts: 67 us (66 before) at 3 tokens per expert,
+// where the weight stream is the limit; 97 (113) at 173 and 150 (204) at 350 tokens per expert, where the SMs' reads from
+// L2 are; with skewed routing (8191 tokens, Zipf 1.2) 222 (536).  With 22 of 512 experts in use 36 (52).
 #pragma once
 #include "mcb_tc.cuh"
 
 namespace mcb {
 
-constexpr int kFfnThreads = 320;            // 10 warps: TMA, MMA, 4 epilogue, 4 token-row producers
-constexpr int kFfnRowsM = 128;              // weight rows per unit
+constexpr int kFfnEpiWarps = 8;
+constexpr int kFfnTokWarps = 2;
+constexpr int kFfnThreads = 32 * (2 + kFfnEpiWarps + kFfnTokWarps);      // weight TMA, MMA, epilogue, token TMA
+constexpr int kFfnRowsM = 256;              // weight rows per unit (128 in each CTA of the pair)
 constexpr int kFfnBlockK = 64;              // 128 bytes of bf16
-constexpr int kFfnMaxN = 256;               // tokens per pass
-constexpr int kFfnMaxStages = 12;
-constexpr int kFfnMaxSub = 2;               // 64-column blocks per pipeline stage at small token tiles (one 32 KB bulk copy)
-constexpr int kFfnABytes = kFfnRowsM * kFfnBlockK * 2;           // 16 KiB per 64-column block
-constexpr int kFfnPipeBytes = 196 * 1024;
-constexpr int kFfnMaxExperts = 1024;        // local experts (their pair offsets are kept in shared memory)
-constexpr int kFfnOffBytes = (kFfnMaxExperts + 1) * 4 + 124;     // rounded to 128
-constexpr int kFfnEpiBytes = 4 * 1024;      // one 16 column x 32 feature bf16 transposition tile per epilogue warp
-constexpr int kFfnSmemBytes = kFfnPipeBytes + 1024 /*align*/ + 512 /*barriers*/ + kFfnOffBytes + kFfnEpiBytes;
+constexpr int kFfnMaxN = 256;               // tokens per chunk
+constexpr int kFfnGatherN = 64;             // largest chunk whose token rows are gathered by TMA
+constexpr int kFfnDoubleN = 128;            // up to this many tokens per chunk a stage holds two 64-column blocks
+constexpr int kFfnMaxStages = 10;
+constexpr int kFfnABytes = 128 * kFfnBlockK * 2;                 // 16 KiB of weights per CTA and 64-column block
+constexpr int kFfnPipeBytes = 192 * 1024;   // 6 stages at 256 tokens, 5 of two blocks at 32
+constexpr int kFfnMaxExperts = 1024;        // local experts
+constexpr int kFfnListUnits = 256;          // units listed at a time
+// Shared memory behind the pipeline: barriers, unit list, epilogue tiles, expert offsets, chunk prefix, active experts.
+constexpr int kFfnBarBytes = 512;
+constexpr int kFfnListBytes = kFfnListUnits * 16;
+constexpr int kFfnTileBytes = 2048;         // one 32 column x 32 feature bf16 tile per epilogue warp
+constexpr int kFfnEpiBytes = kFfnEpiWarps * kFfnTileBytes;
+constexpr int kFfnOffBytes = (kFfnMaxExperts + 1) * 4 + 28;      // rounded to 32
+constexpr int kFfnCumBytes = kFfnOffBytes;
+constexpr int kFfnIdBytes = kFfnMaxExperts * 2;
+constexpr int kFfnSmemBytes = kFfnPipeBytes + 1024 /*align*/ + kFfnBarBytes + kFfnListBytes + kFfnEpiBytes + kFfnOffBytes +
+                              kFfnCumBytes + kFfnIdBytes;
 
 __device__ __forceinline__ int ld_acquire_gpu_i32(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_bf16(void* p, float v) {
-  *reinterpret_cast<__nv_bfloat16*>(p) = __float2bfloat16_rn(v);
+// Shared memory by its 32-bit address (the generic pointers of the carved-up buffer hide the address space).
+__device__ __forceinline__ void sts_bf16(uint32_t addr, float v) {
+  asm volatile("st.shared.b16 [%0], %1;" :: "r"(addr), "h"(__bfloat16_as_ushort(__float2bfloat16_rn(v))) : "memory");
+}
+__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
 }
 
+// Equal chunks of an expert's `rows` tokens, at most kFfnMaxN each; all but the last are a multiple of 32.
+__device__ __forceinline__ int ffn_chunks(int rows) { return (rows + kFfnMaxN - 1) / kFfnMaxN; }
+__device__ __forceinline__ int ffn_chunk_rows(int rows, int chunks) { return ((rows + chunks - 1) / chunks + 31) & ~31; }
+
+// One entry of the unit list.
 struct FfnUnit {
-  int fc;          // 0 = gate/up block, 1 = down block
-  int e;           // local expert
-  int j;           // 128-row block inside the expert's matrix
-  int row0;        // first pair row of the expert
-  int rows;        // pair rows of the expert
+  uint32_t e_fc;       // local expert | 1 << 31 for a down unit
+  uint32_t j_ch;       // 256-row block of the expert's matrix | chunks of the expert << 12
+  int row0;            // first pair row of the chunk
+  int n;               // pair rows of the chunk
+  __device__ __forceinline__ int fc() const { return (int)(e_fc >> 31); }
+  __device__ __forceinline__ int e() const { return (int)(e_fc & 0x7fffffffu); }
+  __device__ __forceinline__ int j() const { return (int)(j_ch & 0xfffu); }
+  __device__ __forceinline__ int chunks() const { return (int)(j_ch >> 12); }
+  __device__ __forceinline__ int half() const { return ((n + 31) & ~31) >> 1; }      // token rows per CTA
+};
+// What the unit numbering needs, the same in every CTA.  Slots are the experts that have tokens, in order;
+// slot s contributes its gate/up units and the down units of slot s - lag.
+struct FfnPlanS {
+  const int* off;            // [E + 1] first pair row of each expert
+  const int* cum;            // [active + 1] chunks of the slots before
+  const uint16_t* ids;       // [active] expert of a slot
+  int active, lag;
+  int n1, n2;                // 256-row blocks of the gate/up and of the down matrix
+  __device__ __forceinline__ int total() const { return (n1 + n2) * cum[active]; }
+  // units before slot s
+  __device__ __forceinline__ int before(int s) const {
+    return n1 * cum[s < active ? s : active] + n2 * cum[s > lag ? s - lag : 0];
+  }
+  __device__ __forceinline__ FfnUnit unit(int u) const {
+    int lo = 0, hi = active + lag;                 // before(lo) <= u < before(hi)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (before(mid) <= u) lo = mid; else hi = mid;
+    }
+    int o = u - before(lo), slot = lo, fc = 0;
+    const int u1 = lo < active ? n1 * (cum[lo + 1] - cum[lo]) : 0;
+    if (o >= u1) { o -= u1; slot = lo - lag; fc = 1; }
+    const int e = ids[slot], ch = cum[slot + 1] - cum[slot];
+    const int j = o / ch, c = o - j * ch;          // the chunks of a weight block are neighbours: they share it in L2
+    const int rows = off[e + 1] - off[e], cr = ffn_chunk_rows(rows, ch);
+    FfnUnit r;
+    r.e_fc = (uint32_t)e | ((uint32_t)fc << 31);
+    r.j_ch = (uint32_t)j | ((uint32_t)ch << 12);
+    r.row0 = off[e] + c * cr;
+    r.n = rows - c * cr < cr ? rows - c * cr : cr;
+    return r;
+  }
 };
 
-// `off` = the expert offsets (a.expert_offset) in shared memory: a unit boundary must not cost a trip to L2.
-__device__ __forceinline__ FfnUnit ffn_unit(const McbFfnArgs& a, const int* off, int u, int n1, int n2) {
-  FfnUnit r;
-  const int u1 = a.num_local_experts * n1;
-  r.fc = u >= u1;
-  const int v = r.fc ? u - u1 : u;
-  const int per = r.fc ? n2 : n1;
-  r.e = v / per;
-  r.j = v - r.e * per;
-  r.row0 = off[r.e];
-  r.rows = off[r.e + 1] - r.row0;
-  return r;
-}
-// First unit at or after u (stepping by the grid) whose expert has tokens; >= total when there is none.
-__device__ __forceinline__ int ffn_next_unit(const McbFfnArgs& a, const int* off, int u, int total, int n1, int n2) {
-  while (u < total && ffn_unit(a, off, u, n1, n2).rows <= 0) u += gridDim.x;
-  return u;
-}
-
-// Call from all kFfnThreads threads of every CTA of the grid; dynamic shared memory of at least
-// kFfnSmemBytes.  a.w1 is the packed interleaved gate/up matrix (E * 2I rows, H columns), a.w2 the
-// packed down matrix (E * H rows, I columns): tile (row block v, column block kb) of a matrix with
-// KB column blocks starts at byte (v * KB + kb) * 16384.
-template <int NSUB>
-__device__ __forceinline__ void ffn_device_impl(const McbFfnArgs& a, const int n_slot) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kFfnPipeBytes);
-  uint64_t* full = bars;                             // [kFfnMaxStages]
-  uint64_t* empty = bars + kFfnMaxStages;            // [kFfnMaxStages]
-  uint64_t* tfull = bars + 2 * kFfnMaxStages;        // [2]
-  uint64_t* tempty = bars + 2 * kFfnMaxStages + 2;   // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kFfnMaxStages + 4);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* s_off = reinterpret_cast<int*>(smem + kFfnPipeBytes + 512);
-
+// Fills cum / ids from the expert offsets; returns the number of experts with tokens.  All threads of the CTA.
+__device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16_t* ids, int* scratch) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int per = (E + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int e0 = threadIdx.x * per, e1 = e0 + per < E ? e0 + per : E;
+  int act = 0, chunks = 0;
+  for (int e = e0; e < e1; ++e) {
+    const int rows = off[e + 1] - off[e];
+    act += rows > 0;
+    chunks += ffn_chunks(rows);
+  }
+  int a_inc = act, c_inc = chunks;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, a_inc, o), c = __shfl_up_sync(0xffffffffu, c_inc, o);
+    if (lane >= o) { a_inc += a; c_inc += c; }
+  }
+  if (lane == 31) { scratch[warp] = a_inc; scratch[32 + warp] = c_inc; }
+  __syncthreads();
+  int a_base = a_inc - act, c_base = c_inc - chunks, total = 0, total_c = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+    if (w < warp) { a_base += scratch[w]; c_base += scratch[32 + w]; }
+    total += scratch[w];
+    total_c += scratch[32 + w];
+  }
+  for (int e = e0; e < e1; ++e) {
+    const int rows = off[e + 1] - off[e];
+    if (rows <= 0) continue;
+    ids[a_base] = (uint16_t)e;
+    cum[a_base] = c_base;
+    ++a_base;
+    c_base += ffn_chunks(rows);
+  }
+  if (threadIdx.x == 0) cum[total] = total_c;
+  __syncthreads();
+  return total;
+}
+
+// Down units follow their gate/up units at once-per-expert order only while the activations between them fit
+// comfortably in L2 (126 MB, shared with the weight stream, the tokens and the expert outputs).
+constexpr long long kFfnActL2Bytes = 24ll << 20;
+
+
+// Shared memory of the FFN, carved out of the dynamic buffer.
+struct FfnSmem {
+  uint8_t* pipe;             // [stages][weights x NSUB][token half x NSUB]
+  uint64_t* full;            // [kFfnMaxStages], used in the leading CTA
+  uint64_t* empty;           // [kFfnMaxStages]
+  uint64_t* tfull;           // [2]
+  uint64_t* tempty;          // [2], used in the leading CTA
+  uint32_t* tmem_slot;
+  volatile int* abort_flag;
+  uint4* list;
+  uint8_t* epi;
+  int* off;
+  int* cum;
+  uint16_t* ids;
+  __device__ __forceinline__ FfnSmem() {
+    extern __shared__ uint8_t smem_raw[];
+    pipe = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    full = reinterpret_cast<uint64_t*>(pipe + kFfnPipeBytes);
+    empty = full + kFfnMaxStages;
+    tfull = empty + kFfnMaxStages;
+    tempty = tfull + 2;
+    tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint8_t* p = pipe + kFfnPipeBytes + kFfnBarBytes;
+    list = reinterpret_cast<uint4*>(p);
+    epi = p + kFfnListBytes;
+    off = reinterpret_cast<int*>(epi + kFfnEpiBytes);
+    cum = off + kFfnOffBytes / 4;
+    ids = reinterpret_cast<uint16_t*>(cum + kFfnCumBytes / 4);
+  }
+};
+
+// Before the FFN, once per kernel: barriers, TMEM, tensor maps.  All threads of both CTAs of the pair; touches nothing
+// that another kernel writes, so a kernel with other work to do first calls it at its very start.
+__device__ __forceinline__ void ffn_setup(const McbFfnArgs& a) {
+  const FfnSmem sm;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kFfnMaxStages; ++s) { mbar_init(&full[s], 1 + 128); mbar_init(&empty[s], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&tfull[i], 1); mbar_init(&tempty[i], 4); }
-    *abort_flag = 0;
+    // full: the weight producer and the first token producer of the leading CTA announce the bytes of both CTAs
+    for (int s = 0; s < kFfnMaxStages; ++s) { mbar_init(&sm.full[s], 2); mbar_init(&sm.empty[s], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sm.tfull[i], 1); mbar_init(&sm.tempty[i], 2 * kFfnEpiWarps); }
+    *sm.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (int e = threadIdx.x; e <= a.num_local_experts; e += blockDim.x) s_off[e] = a.expert_offset[e];
-  if (warp == 1) tmem_alloc(tmem_slot, 512);
+  if (threadIdx.x >= 32 && threadIdx.x < 64) tmem_alloc_pair(sm.tmem_slot, 512);
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + MCB_FFN_TMAPS)
+    tma_prefetch_map(reinterpret_cast<const uint8_t*>(a.tmaps) + (threadIdx.x - 64) * 128);
   tc_fence_before();
   __syncthreads();
+  cluster_sync();                                    // barriers initialised and TMEM allocated in both CTAs
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const Abort ab{abort_flag, a.status, a.timeout_ns};
+}
 
+// After it: TMEM back.  Nobody leaves before the other CTA of the pair is done with this one's shared memory.
+__device__ __forceinline__ void ffn_teardown() {
+  const FfnSmem sm;
+  tc_fence_before();
+  __syncthreads();
+  if (*sm.abort_flag) __nanosleep(50000);            // let any copy still in flight land before the CTA goes away
+  cluster_sync();
+  if (threadIdx.x >= 32 && threadIdx.x < 64) {
+    tc_fence_after();
+    tmem_dealloc_pair(*sm.tmem_slot, 512);
+  }
+}
+
+// Bounded wait for a counter in global memory to reach `want` (acquire); gives up like mbar_wait.
+__device__ __forceinline__ void ffn_wait_count(const int* word, int want, const Abort& ab, uint32_t where, uint32_t what) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0; ld_acquire_gpu_i32(word) < want; ++i) {
+    if (*ab.flag) return;
+    if ((i & 31u) != 31u) continue;
+    if (t0 == 0) t0 = now_ns();
+    if (ab.status && *reinterpret_cast<volatile uint32_t*>(ab.status) != 0u) { *ab.flag = 1; return; }
+    if (now_ns() - t0 > ab.timeout_ns) {
+      *ab.flag = 1;
+      if (ab.status && atomicCAS(ab.status, 0u, (uint32_t)MCB_GEMM_ERR_TIMEOUT) == 0u) {
+        ab.status[1] = where; ab.status[2] = blockIdx.x; ab.status[3] = what;
+      }
+      return;
+    }
+  }
+}
+
+// Token rows into pair order: row p of y = row pair_token[p] of x, for all `pairs` rows, over the warps that call it.
+// Eight 512-byte pieces per warp in flight; a.hidden is a multiple of 256, so a piece lies inside one row.
+__device__ __forceinline__ void ffn_permute_rows(const McbFfnArgs& a, int pairs, int wid, int nwarps) {
+  const int lane = threadIdx.x & 31, per_row = a.hidden / 256;
+  const long long pieces = (long long)pairs * per_row;
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x) + lane * 16;
+  uint8_t* xp = reinterpret_cast<uint8_t*>(a.y) + lane * 16;
+  for (long long i0 = (long long)wid * 8; i0 < pieces; i0 += (long long)nwarps * 8) {
+    long long src[8];
+    uint4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const long long i = i0 + k < pieces ? i0 + k : pieces - 1;
+      const int row = (int)(i / per_row);
+      src[k] = (long long)a.pair_token[row] * a.hidden * 2 + (i - (long long)row * per_row) * 512;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = ld_v4(x + src[k]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (i0 + k < pieces) st_v4(xp + (i0 + k) * 512, v[k]);
+  }
+}
+
+// a.w1 is the packed interleaved gate/up matrix (E * 2I rows, H columns), a.w2 the packed down matrix (E * H rows,
+// I columns): tile (128-row block v, column block kb) of a matrix with KB column blocks is the 16 KB at byte
+// (v * KB + kb) * 16384.
+template <int NSUB>
+__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& plan, const int n_slot) {
+  const FfnSmem sm;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank();           // 0 = the CTA that issues the MMAs of the pair
   const int H = a.hidden, I = a.intermediate;
-  const int n1 = 2 * I / kFfnRowsM, n2 = H / kFfnRowsM;
-  const int total_units = a.num_local_experts * (n1 + n2);
-  constexpr int nsub = NSUB;                                    // 64-column blocks per pipeline stage
-  const int b_sub_bytes = n_slot * 128;                         // token tile of one 64-column block
-  const int stage_bytes = nsub * (kFfnABytes + b_sub_bytes);    // [A block 0][A block 1][B block 0][B block 1]
+  const int npairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
+  const int total = plan.total();
+  const uint32_t tmem_base = *sm.tmem_slot;
+  const Abort ab{sm.abort_flag, a.status, a.timeout_ns};
+  const uint8_t* maps = reinterpret_cast<const uint8_t*>(a.tmaps);
+  const bool gather = n_slot <= kFfnGatherN;
+
+  const int b_sub_bytes = (n_slot >> 1) * 128;                    // token half of one 64-column block
+  const int stage_bytes = NSUB * (kFfnABytes + b_sub_bytes);
   int stages = kFfnPipeBytes / stage_bytes;
   if (stages > kFfnMaxStages) stages = kFfnMaxStages;
 
-  constexpr uint32_t kStageA = (uint32_t)(nsub * kFfnABytes);     // weight bytes per stage: one bulk copy
+  // Pipeline position of this warp's role, kept from one batch of the list to the next.
+  int s = 0; uint32_t ph = 0;
+  int acc = 0; uint32_t acc_ph = 0;
+  bool ok = true;
 
-  if (warp == 0) {
-    // ---------------- TMA producer: 128 weight rows x 64 columns per stage ----------------
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
-        const FfnUnit un = ffn_unit(a, s_off, u, n1, n2);
-        if (un.rows <= 0) continue;
-        const int k_blocks = (un.fc ? I : H) / kFfnBlockK;
-        const long long v = (long long)un.e * (un.fc ? n2 : n1) + un.j;       // 128-row block of the matrix
-        const uint8_t* tiles = reinterpret_cast<const uint8_t*>(un.fc ? a.w2 : a.w1) + v * k_blocks * (long long)kFfnABytes;
-        for (int c0 = 0; c0 < un.rows && ok; c0 += kFfnMaxN) {
-          for (int kb = 0; kb < k_blocks; kb += nsub) {
-            if (!(ok = mbar_wait(&empty[s], ph ^ 1u, ab, 11))) break;
-            mbar_arrive_expect_tx(&full[s], kStageA);
-            bulk_load(smem + s * stage_bytes, tiles + (long long)kb * kFfnABytes, kStageA, &full[s]);
+  auto fill = [&](int first) {             // the units first, first + npairs, ... of this pair
+    for (int i = threadIdx.x; i < kFfnListUnits; i += blockDim.x) {
+      const long long u = first + (long long)i * npairs;
+      if (u < total) {
+        const FfnUnit un = plan.unit((int)u);
+        sm.list[i] = make_uint4(un.e_fc, un.j_ch, (uint32_t)un.row0, (uint32_t)un.n);
+      }
+    }
+    __syncthreads();
+  };
+  auto listed = [&](int i) {
+    const uint4 v = sm.list[i];
+    return FfnUnit{v.x, v.y, (int)v.z, (int)v.w};
+  };
+  fill(pair);
+  if (!gather && warp >= 2) {
+    // every warp but the weight producer and the MMA issuer takes a share of the copy into pair order
+    ffn_permute_rows(a, plan.off[a.num_local_experts], (int)blockIdx.x + (warp - 2) * (int)gridDim.x,
+                     (kFfnEpiWarps + kFfnTokWarps) * (int)gridDim.x);
+    fence_proxy_async_global();
+    __threadfence();
+    asm volatile("bar.sync 1, %0;" :: "n"(32 * (kFfnEpiWarps + kFfnTokWarps)) : "memory");
+    if (warp == 2 && lane == 0) atomicAdd(&a.sync[0], 1);
+  }
+
+  for (int first = pair; first < total; first += kFfnListUnits * npairs) {
+    int count = (total - first + npairs - 1) / npairs;
+    if (count > kFfnListUnits) count = kFfnListUnits;
+    if (warp == 0) {
+      // ---------------- weights: 128 rows x 64 NSUB columns per CTA and stage ----------------
+      if (elect_one()) {
+        for (int i = 0; i < count && ok; ++i) {
+          const FfnUnit un = listed(i);
+          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
+          const uint8_t* map = maps + ((un.fc() ? MCB_FFN_MAP_W2 : MCB_FFN_MAP_W1) + (NSUB - 1) * 2) * 128;
+          const int v = (un.e() * (un.fc() ? plan.n2 : plan.n1) + un.j()) * 2 + rank;     // 128-row block of the matrix
+          int row = v * k_blocks * (kFfnABytes / 2048);
+          for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
+            if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 11))) break;
+            if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * NSUB * kFfnABytes);
+            tma_load_2d_pair(sm.pipe + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row);
             if (++s == stages) { s = 0; ph ^= 1u; }
           }
         }
       }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      int acc = 0; uint32_t acc_ph = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
-        const FfnUnit un = ffn_unit(a, s_off, u, n1, n2);
-        if (un.rows <= 0) continue;
-        const int k_blocks = (un.fc ? I : H) / kFfnBlockK;
-        for (int c0 = 0; c0 < un.rows && ok; c0 += kFfnMaxN) {
-          const int n = un.rows - c0 < kFfnMaxN ? un.rows - c0 : kFfnMaxN;
-          const uint32_t idesc = umma_idesc_bf16(kFfnRowsM, (uint32_t)((n + 15) & ~15));
-          if (!(ok = mbar_wait(&tempty[acc], acc_ph ^ 1u, ab, 12))) break;
+    } else if (warp == 1) {
+      // ---------------- MMA: one thread of the leading CTA drives the tensor cores of both ----------------
+      if (rank == 0 && elect_one()) {
+        for (int i = 0; i < count && ok; ++i) {
+          const FfnUnit un = listed(i);
+          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
+          const uint32_t idesc = umma_idesc_bf16(kFfnRowsM, (uint32_t)(un.half() * 2));
+          if (!(ok = mbar_wait(&sm.tempty[acc], acc_ph ^ 1u, ab, 12))) break;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kFfnMaxN);
-          for (int kb = 0; kb < k_blocks; kb += nsub) {
-            if (!(ok = mbar_wait(&full[s], ph, ab, 13))) break;
-            fence_proxy_async_smem();           // the token rows were written by cp.async, not by TMA
+          for (int kb = 0; kb < k_blocks; kb += NSUB) {
+            if (!(ok = mbar_wait(&sm.full[s], ph, ab, 13))) break;
             tc_fence_after();
-            const uint32_t sa = smem_u32(smem + s * stage_bytes);
+            const uint32_t sa = smem_u32(sm.pipe + s * stage_bytes);
 #pragma unroll
-            for (int sub = 0; sub < nsub; ++sub) {
+            for (int sub = 0; sub < NSUB; ++sub) {
               const uint64_t da = make_sw128_desc(sa + sub * kFfnABytes);
-              const uint64_t db = make_sw128_desc(sa + nsub * kFfnABytes + sub * b_sub_bytes);
+              const uint64_t db = make_sw128_desc(sa + NSUB * kFfnABytes + sub * b_sub_bytes);
 #pragma unroll
               for (int kk = 0; kk < kFfnBlockK / 16; ++kk)
-                umma_bf16(d_tmem, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (kb | sub | kk) != 0);
+                umma_bf16_pair(d_tmem, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (kb | sub | kk) != 0);
             }
-            umma_commit(&empty[s]);
+            umma_commit_pair(&sm.empty[s]);
             if (++s == stages) { s = 0; ph ^= 1u; }
           }
           if (!ok) break;
-          umma_commit(&tfull[acc]);
+          umma_commit_pair(&sm.tfull[acc]);
           if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
         }
       }
-    }
-  } else if (warp < 6) {
-    // ---------------- epilogue: TMEM (lane = weight row, column = token) -> global ----------------
-    const int q = warp & 3;                  // TMEM lane quarter this warp may read
-    // A lane holds ONE feature of 16 tokens, memory wants the features of a token side by side: the values
-    // cross a small tile in shared memory ([column][feature], 64 or 32 bytes per row) and leave as 16-byte
-    // stores, two (down) or one (gate/up) per 16 columns instead of sixteen or eight 2-byte ones.
-    uint8_t* tile = smem + kFfnPipeBytes + 512 + kFfnOffBytes + q * 1024;
-    int acc = 0; uint32_t acc_ph = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < total_units && ok; u += gridDim.x) {
-      const FfnUnit un = ffn_unit(a, s_off, u, n1, n2);
-      if (un.rows <= 0) continue;
-      for (int c0 = 0; c0 < un.rows && ok; c0 += kFfnMaxN) {
-        const int n = un.rows - c0 < kFfnMaxN ? un.rows - c0 : kFfnMaxN;
-        if (!(ok = mbar_wait(&tfull[acc], acc_ph, ab, 14))) break;
+    } else if (warp < 2 + kFfnEpiWarps) {
+      // ---------------- epilogue: TMEM (lane = weight row, column = token) -> global ----------------
+      const int q = warp & 3;                  // TMEM lane quarter this warp may read
+      const int hw = (warp - 2) >> 2;          // it takes the even or the odd 32-column groups
+      // A lane holds ONE feature of 32 tokens, memory wants the features of a token side by side: the values
+      // cross a small tile in shared memory ([column][feature], 64 or 32 bytes per row) and leave as 16-byte stores.
+      const uint32_t tile = smem_u32(sm.epi + (warp - 2) * kFfnTileBytes);
+      const uint32_t tempty_addr = cluster_map(sm.tempty, 0);
+      for (int i = 0; i < count && ok; ++i) {
+        const FfnUnit un = listed(i);
+        const int n = un.n;
+        if (!(ok = mbar_wait(&sm.tfull[acc], acc_ph, ab, 14))) break;
         tc_fence_after();
-        const long long prow0 = (long long)un.row0 + c0;
-        {
-          const int j = un.j;
-          const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kFfnMaxN);
-          if (!un.fc) {
-            // rows alternate gate / up: lane pairs (2i, 2i + 1) hold the two halves of activation i
-            const int feat = j * (kFfnRowsM / 2) + q * 16 + (lane >> 1);
-            const bool odd = lane & 1;
-            uint8_t* obase0 = reinterpret_cast<uint8_t*>(a.act) + (long long)(feat - (lane >> 1)) * 2;   // first feature of the warp
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kFfnMaxN);
+        const int wrow = un.j() * kFfnRowsM + rank * 128 + q * 32;       // first weight row of the warp
+        auto release = [&] {                   // the accumulator has been read: hand it back before the stores
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(tempty_addr + acc * 8);
+        };
+        if (hw * 32 >= n) release();
+        if (!un.fc()) {
+          // rows alternate gate / up: lane pairs (2i, 2i + 1) hold the two halves of activation i; the even lane
+          // finishes the even columns, the odd lane the odd ones
+          const bool odd = lane & 1;
+          uint8_t* obase = reinterpret_cast<uint8_t*>(a.act) + (long long)un.row0 * I * 2 + wrow + (lane & 1) * 16;
 #pragma unroll 1
-            for (int cc = 0; cc < n; cc += 16) {
-              uint32_t v[16];
-              tmem_ld16(t_row + cc, v);
-              tmem_ld_wait();
+          for (int cc = hw * 32; cc < n; cc += 64) {
+            uint32_t v[32];
+            tmem_ld32(t_row + cc, v);
+            tmem_ld_wait();
+            if (cc + 64 >= n) release();
+            // Each step over all columns before the next one: the stores keep their order with everything
+            // volatile, so a loop over columns would run one column's whole chain after the other.
+            uint32_t recv[16];
+            float r[16];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                // the even lane finishes columns cc .. cc+7, the odd lane columns cc+8 .. cc+15
-                const uint32_t send = odd ? v[i] : v[8 + i];
-                const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                const float g = __uint_as_float(odd ? recv : v[i]);
-                const float up = __uint_as_float(odd ? v[8 + i] : recv);
-                st_bf16(tile + ((odd ? 8 : 0) + i) * 32 + (lane >> 1) * 2, silu(g) * up);
-              }
-              __syncwarp();
-              {   // 16 columns x 16 features: lane l stores half (l & 1) of column l >> 1
-                const int col = cc + (lane >> 1);
-                const uint4 w = *reinterpret_cast<const uint4*>(tile + (lane >> 1) * 32 + (lane & 1) * 16);
-                if (col < n) st_v4(obase0 + (prow0 + col) * (long long)I * 2 + (lane & 1) * 16, w);
-              }
-              __syncwarp();
-            }
-          } else {
-            const int feat = j * kFfnRowsM + q * 32 + lane;
-            uint8_t* obase0 = reinterpret_cast<uint8_t*>(a.y) + (long long)(feat - lane) * 2;             // first feature of the warp
-            // routing weights of the pass: lane l keeps those of columns l, l + 32, ... (one trip to L2 for the
-            // whole pass instead of one per 16 columns), handed out by shuffles below
-            float pp[kFfnMaxN / 32];
+            for (int k = 0; k < 16; ++k) recv[k] = __shfl_xor_sync(0xffffffffu, odd ? v[2 * k] : v[2 * k + 1], 1);
 #pragma unroll
-            for (int i = 0; i < kFfnMaxN / 32; ++i) {
-              const int col = lane + 32 * i;
-              pp[i] = (a.pair_prob && col < n) ? a.pair_prob[prow0 + col] : 1.0f;
+            for (int k = 0; k < 16; ++k) {
+              const float g = __uint_as_float(odd ? recv[k] : v[2 * k]);
+              const float up = __uint_as_float(odd ? v[2 * k + 1] : recv[k]);
+              r[k] = silu(g) * up;
             }
+#pragma unroll
+            for (int k = 0; k < 16; ++k) sts_bf16(tile + (2 * k + (lane & 1)) * 32 + (lane >> 1) * 2, r[k]);
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {      // 32 columns x 16 features: lane l stores half (l & 1) of column 16h + (l >> 1)
+              const int cl = 16 * h + (lane >> 1);
+              const uint4 w = lds_v4(tile + cl * 32 + (lane & 1) * 16);
+              if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * I * 2, w);
+            }
+            __syncwarp();
+          }
+          // This warp's share of the gate/up unit is stored: make it visible to TMA loads of other CTAs and count
+          // it for the expert's down units (no barrier between the warps, so nothing can wait for a warp that
+          // has given up).
+          fence_proxy_async_global();
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) atomicAdd(&a.ffn_done[un.e()], 1);
+        } else {
+          uint8_t* obase = reinterpret_cast<uint8_t*>(a.y) + ((long long)un.row0 * H + wrow) * 2 + (lane & 3) * 16;
 #pragma unroll 1
-            for (int cc = 0; cc < n; cc += 16) {
-              uint32_t v[16];
-              tmem_ld16(t_row + cc, v);
-              float mine = pp[0];
+          for (int cc = hw * 32; cc < n; cc += 64) {
+            const float mine = (a.pair_prob && cc + lane < n) ? a.pair_prob[un.row0 + cc + lane] : 1.0f;
+            uint32_t v[32];
+            tmem_ld32(t_row + cc, v);
+            tmem_ld_wait();
+            if (cc + 64 >= n) release();
+            float r[32];
 #pragma unroll
-              for (int i = 1; i < kFfnMaxN / 32; ++i)
-                if ((cc >> 5) == i) mine = pp[i];
-              tmem_ld_wait();
+            for (int k = 0; k < 32; ++k) r[k] = __uint_as_float(v[k]) * __shfl_sync(0xffffffffu, mine, k);
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const int col = cc + i;
-                const float p = __shfl_sync(0xffffffffu, mine, col & 31);
-                st_bf16(tile + i * 64 + lane * 2, __uint_as_float(v[i]) * p);
-              }
-              __syncwarp();
+            for (int k = 0; k < 32; ++k) sts_bf16(tile + k * 64 + lane * 2, r[k]);
+            __syncwarp();
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {   // 16 columns x 32 features: lane l stores quarter (l & 3) of column 8h + (l >> 2)
-                const int cl = 8 * h + (lane >> 2);
-                const uint4 w = *reinterpret_cast<const uint4*>(tile + cl * 64 + (lane & 3) * 16);
-                if (cc + cl < n) st_v4(obase0 + (prow0 + cc + cl) * (long long)H * 2 + (lane & 3) * 16, w);
-              }
-              __syncwarp();
+            for (int h = 0; h < 4; ++h) {      // 32 columns x 32 features: lane l stores quarter (l & 3) of column 8h + (l >> 2)
+              const int cl = 8 * h + (lane >> 2);
+              const uint4 w = lds_v4(tile + cl * 64 + (lane & 3) * 16);
+              if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * H * 2, w);
             }
+            __syncwarp();
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty[acc]);
         if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
       }
-      if (!un.fc && ok) {
-        // This warp's quarter of the gate/up block is stored: count it for the expert's down blocks
-        // (four counts per block; no barrier between the warps, so nothing can wait for a warp that
-        // has given up).
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) atomicAdd(&a.ffn_done[un.e], 1);
+    } else {
+      // ---------------- tokens: this CTA's half of the chunk into the swizzled K-major B tile ----------------
+      // Each of the two warps fetches half of the half, from one thread: four rows per gather, or one box.  Rows past
+      // the end of the chunk (they feed columns nobody reads) are fetched too, so that BOTH warps of both CTAs
+      // contribute bytes to every stage: one that the stage did not wait for could fall a whole ring behind and
+      // misread the parity of `empty`.  The gather indices of the next unit are requested while the current
+      // one is still being copied.
+      if (elect_one()) {
+        const int t = warp - 2 - kFfnEpiWarps;
+        constexpr int kOps = kFfnGatherN / 8 / kFfnTokWarps;
+        int nxt[kOps][4];
+        auto fetch_idx = [&](const FfnUnit& un) {
+          if (un.fc() || !gather) return;
+          const int rows = un.half() / kFfnTokWarps, base = rank * un.half() + t * rows;
+#pragma unroll
+          for (int k = 0; k < kOps; ++k) {
+            if (k * 4 >= rows) break;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+              int r = base + k * 4 + m;
+              if (r >= un.n) r %= un.n;              // spread over the chunk's rows, not all on one
+              nxt[k][m] = a.pair_token[un.row0 + r];
+            }
+          }
+        };
+        fence_proxy_async_global();          // token rows written by ordinary stores before this point
+        fetch_idx(listed(0));
+        if (!gather && first == pair) {
+          ffn_wait_count(&a.sync[0], (int)gridDim.x, ab, 18, 0);
+          fence_proxy_async_global();
+        }
+        for (int i = 0; i < count && ok; ++i) {
+          const FfnUnit un = listed(i);
+          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
+          const int rows = un.half() / kFfnTokWarps;           // 8, 16, ... 64
+          const uint32_t bytes = (uint32_t)un.half() * 256u * NSUB;
+          const int row = un.row0 + rank * un.half() + t * rows;
+          const uint8_t* map = maps + ((un.fc() ? MCB_FFN_MAP_ACT : MCB_FFN_MAP_XP) + (rows >> 3) - 1) * 128;
+          int cur[kOps][4];
+#pragma unroll
+          for (int k = 0; k < kOps; ++k)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) cur[k][m] = nxt[k][m];
+          if (i + 1 < count) fetch_idx(listed(i + 1));
+          if (un.fc()) {
+            // the activations of this expert are complete once every epilogue warp of every gate/up unit has been counted
+            ffn_wait_count(&a.ffn_done[un.e()], 2 * kFfnEpiWarps * plan.n1 * un.chunks(), ab, 15, (uint32_t)un.e());
+            fence_proxy_async_global();
+          }
+          const bool box = un.fc() || !gather;
+          for (int kb = 0; kb < k_blocks; kb += NSUB) {
+            if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 16))) break;
+            uint8_t* dst = sm.pipe + s * stage_bytes + NSUB * kFfnABytes + t * rows * 128;
+            const uint32_t bar = cluster_map(&sm.full[s], 0);
+            if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[s], bytes);
+            if (box) {
+#pragma unroll
+              for (int sub = 0; sub < NSUB; ++sub)
+                tma_load_2d_pair(dst + sub * b_sub_bytes, map, bar, (kb + sub) * kFfnBlockK, row);
+            } else {
+#pragma unroll
+              for (int k = 0; k < kOps; ++k) {
+                if (k * 4 >= rows) break;
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub)
+                  tma_gather4_pair(dst + sub * b_sub_bytes + k * 512, maps + MCB_FFN_MAP_X * 128, bar,
+                                   (kb + sub) * kFfnBlockK, cur[k][0], cur[k][1], cur[k][2], cur[k][3]);
+              }
+            }
+            if (++s == stages) { s = 0; ph ^= 1u; }
+          }
+        }
       }
     }
-  } else {
-    // ---------------- token-row producers: gather rows into the swizzled K-major B tile ----------------
-    // Thread t copies 16-byte chunk (t & 7) of rows (t >> 3), (t >> 3) + 16, ...: the eight threads of a
-    // row read its 128 bytes as one line, and a warp's 32 chunks fill four whole shared-memory rows.
-    const int t = threadIdx.x - 6 * 32;      // 0..127
-    const int chunk = t & 7, rbase = t >> 3;
-    int s = 0; uint32_t ph = 0;
-    bool ok = true;
-    // Everything a unit needs from global memory before its first copy can be issued (the gather indices of
-    // its first pass, the "gate/up blocks done" counter of a down block) is requested while the previous
-    // unit is still being copied: a unit boundary must not drain the pipeline.
-    int srow_n[kFfnMaxN / 16];
-    int done_n = 0;
-    auto prefetch = [&](const FfnUnit& un) {
-      const int n = un.rows < kFfnMaxN ? un.rows : kFfnMaxN;
-#pragma unroll
-      for (int i = 0; i < kFfnMaxN / 16; ++i) {
-        const int r = rbase + 16 * i;
-        srow_n[i] = 0;
-        if (r < n) srow_n[i] = un.fc ? un.row0 + r : a.pair_token[un.row0 + r];
-      }
-      if (un.fc && lane == 0) done_n = ld_acquire_gpu_i32(&a.ffn_done[un.e]);
-    };
-    int u = ffn_next_unit(a, s_off, blockIdx.x, total_units, n1, n2);
-    if (u < total_units) prefetch(ffn_unit(a, s_off, u, n1, n2));
-    while (u < total_units && ok) {
-      const FfnUnit un = ffn_unit(a, s_off, u, n1, n2);
-      const int u_next = ffn_next_unit(a, s_off, u + (int)gridDim.x, total_units, n1, n2);
-      const int k_blocks = (un.fc ? I : H) / kFfnBlockK;
-      if (un.fc) {
-        // the activations of this expert are complete once all its gate/up blocks have been counted
-        // (four epilogue warps each); one lane per producer warp polls, bounded
-        if (lane == 0 && done_n < 4 * n1) {
-          const uint64_t t0 = now_ns();
-          while (ld_acquire_gpu_i32(&a.ffn_done[un.e]) < 4 * n1) {
-            if (*ab.flag) break;
-            if (ab.status && *reinterpret_cast<volatile uint32_t*>(ab.status) != 0u) { *ab.flag = 1; break; }
-            if (now_ns() - t0 > ab.timeout_ns) {
-              *ab.flag = 1;
-              if (ab.status && atomicCAS(ab.status, 0u, (uint32_t)MCB_GEMM_ERR_TIMEOUT) == 0u) {
-                ab.status[1] = 15; ab.status[2] = blockIdx.x; ab.status[3] = (uint32_t)un.e;
-              }
-              break;
-            }
-          }
-        }
-        __syncwarp();
-      }
-      const uint64_t src_row_bytes = un.fc ? (uint64_t)I * 2 : a.x_row_bytes;
-      const uint8_t* src_base = reinterpret_cast<const uint8_t*>(un.fc ? a.act : a.x) + chunk * 16;
-      bool prefetched = false;
-      for (int c0 = 0; c0 < un.rows && ok; c0 += kFfnMaxN) {
-        const int n = un.rows - c0 < kFfnMaxN ? un.rows - c0 : kFfnMaxN;
-        // source rows of this thread's rows of the tile (up to 16 of them)
-        int srow[kFfnMaxN / 16];
-#pragma unroll
-        for (int i = 0; i < kFfnMaxN / 16; ++i) {
-          const int r = rbase + 16 * i;
-          srow[i] = srow_n[i];
-          if (c0 > 0) srow[i] = r < n ? (un.fc ? un.row0 + c0 + r : a.pair_token[un.row0 + c0 + r]) : 0;
-        }
-        for (int kb = 0; kb < k_blocks; kb += nsub) {
-          if (!(ok = mbar_wait(&empty[s], ph ^ 1u, ab, 16))) break;
-          uint8_t* sb = smem + s * stage_bytes + nsub * kFfnABytes;
-          const uint8_t* g = src_base + (long long)kb * (kFfnBlockK * 2);
-#pragma unroll
-          for (int i = 0; i < kFfnMaxN / 16; ++i) {
-            const int r = rbase + 16 * i;
-            if (r < n) {
-              const uint8_t* gr = g + (long long)srow[i] * (long long)src_row_bytes;
-              uint8_t* dst = sb + r * 128 + ((chunk ^ (r & 7)) << 4);
-#pragma unroll
-              for (int sub = 0; sub < nsub; ++sub) cp_async_16(dst + sub * b_sub_bytes, gr + sub * (kFfnBlockK * 2));
-            }
-          }
-          cp_async_arrive_noinc(&full[s]);     // arrives when this thread's copies have landed
-          if (++s == stages) { s = 0; ph ^= 1u; }
-          if (!prefetched && c0 + kFfnMaxN >= un.rows) {       // last pass under way: srow_n is free again
-            prefetched = true;
-            if (u_next < total_units) prefetch(ffn_unit(a, s_off, u_next, n1, n2));
-          }
-        }
-      }
-      u = u_next;
+    if (count == kFfnListUnits) {
+      __syncthreads();                     // the list is free for the next batch
+      fill(first + kFfnListUnits * npairs);
     }
   }
-
-  // ---------------- teardown ----------------
-  tc_fence_before();
-  __syncthreads();
-  if (*abort_flag) __nanosleep(50000);        // let any copy still in flight land before the CTA goes away
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+  if (warp == 0 && elect_one()) {
+    // The last commits still arrive on both CTAs' `empty` barriers: nobody leaves before they have.
+    for (int i = 0; i < stages && ok; ++i) {
+      ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 17);
+      if (++s == stages) { s = 0; ph ^= 1u; }
+    }
+  }
+  if (!gather && threadIdx.x == 0) {       // the last CTA out leaves the copy's counters at zero for the next launch
+    __threadfence();
+    if (atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1) {
+      a.sync[0] = 0;
+      a.sync[1] = 0;
+      __threadfence();
+    }
   }
 }
 
-// Token tile of this launch: the largest expert, rounded up to 16, at most kFfnMaxN per pass.  Two
-// 64-column blocks per pipeline stage while the tile is small (the weight stream is then the limit and
-// the per-stage work of the MMA-issuing thread must be amortised), one when it is large.
+// Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
+// ffn_teardown, once the pair lists are visible; dynamic shared memory of at least kFfnSmemBytes.
 __device__ __forceinline__ void ffn_device(const McbFfnArgs& a) {
+  const FfnSmem sm;
+  const int E = a.num_local_experts;
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) sm.off[e] = a.expert_offset[e];
   int max_rows = *a.max_rows;
   if (max_rows < 1) max_rows = 1;
-  const int n_slot = max_rows >= kFfnMaxN ? kFfnMaxN : ((max_rows + 15) & ~15);
-  if (n_slot <= 128) ffn_device_impl<kFfnMaxSub>(a, n_slot);
-  else ffn_device_impl<1>(a, n_slot);
+  fence_proxy_async_smem();                // the pipeline's memory may have been in ordinary use until here
+  __syncthreads();
+  FfnPlanS plan;
+  plan.off = sm.off; plan.cum = sm.cum; plan.ids = sm.ids;
+  plan.n1 = 2 * a.intermediate / kFfnRowsM; plan.n2 = a.hidden / kFfnRowsM;
+  plan.active = ffn_slots(sm.off, E, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi));
+  plan.lag = plan.active;
+  if ((long long)sm.off[E] * a.intermediate * 2 > kFfnActL2Bytes) {      // two rounds of the grid, in slots of average size
+    const int lag = (int)((long long)gridDim.x * plan.active / plan.total()) + 2;
+    if (lag < plan.lag) plan.lag = lag;
+  }
+  // Token tile of this launch: the largest expert, rounded up to 32, at most kFfnMaxN per chunk.
+  const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 31) & ~31);
+  if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, plan, n_slot);
+  else ffn_roles<1>(a, plan, n_slot);
 }
 
 }  // namespace mcb

@@ -7,6 +7,14 @@
 
 #define MCB_GEMM_FC1 0          // gate/up projection + SwiGLU epilogue
 #define MCB_GEMM_FC2 1          // down projection + per-row scale epilogue
+// Tensor maps of the fused FFN: token rows (gathered four at a time), gate/up and down tiles (16 KB, then 32 KB), and
+// activations and token rows in pair order in boxes of 8, 16, ... 64 rows.
+#define MCB_FFN_MAP_X 0
+#define MCB_FFN_MAP_W1 1
+#define MCB_FFN_MAP_W2 2
+#define MCB_FFN_MAP_ACT 5
+#define MCB_FFN_MAP_XP 13
+#define MCB_FFN_TMAPS 21
 #define MCB_GEMM_ERR_TIMEOUT 5  // status code: a bounded mbarrier wait ran out
 
 #ifdef __cplusplus
@@ -41,16 +49,18 @@ typedef struct {
   const int32_t* expert_offset;  // [E_loc + 1] first pair row of each local expert
   const int32_t* max_rows;     // device scalar: largest pair count of one expert
   void* act;                   // [P, intermediate] bf16 (written by the gate/up blocks, read by the down blocks)
-  void* y;                     // [P, hidden] bf16 = prob * (act . Wd^T)
-  int32_t* ffn_done;           // [E_loc] quarter-blocks of gate/up finished (zeroed by the routing)
+  void* y;                     // [P, hidden] bf16 = prob * (act . Wd^T); holds the token rows in pair order before
+  int32_t* ffn_done;           // [E_loc] warp shares of gate/up blocks finished (zeroed by the routing)
   int32_t num_local_experts;
-  int32_t hidden;              // multiple of 128
+  int32_t hidden;              // multiple of 256
   int32_t intermediate;        // multiple of 128
   int32_t reserved0;
   uint32_t* status;
   uint64_t timeout_ns;
   const void* w1;              // packed interleaved gate/up matrix (E * 2I rows, hidden columns), see mcb_ffn.cuh
   const void* w2;              // packed down matrix (E * hidden rows, I columns)
+  const void* tmaps;           // device memory, MCB_FFN_TMAPS tensor maps of 128 bytes, 64-byte aligned (mcb_make_ffn_tmaps)
+  int32_t* sync;               // [2] zero between launches: CTAs that have copied their token rows, CTAs that have left
 } McbFfnArgs;
 
 // Routing of the gathered tokens to this rank's experts.

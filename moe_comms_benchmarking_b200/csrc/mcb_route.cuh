@@ -77,9 +77,9 @@ __device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const int* s
 
 // One launch, two phases separated by a "last block computes the offsets" hand-over; blocks of
 // the same launch wait for it on a local counter, so the grid must be co-resident (<= #SMs).
-// Call from all threads of every block of the grid.
-__device__ __forceinline__ void route_device(const McbRouteArgs& a) {
-  __shared__ int s_hist[kMaxLocalExperts];
+// Call from all threads of every block of the grid; `s_hist` is shared memory for 2 * kMaxLocalExperts words.
+__device__ __forceinline__ void route_device(const McbRouteArgs& a, int* s_hist) {
+  int* s_cursor = s_hist + kMaxLocalExperts;
   __shared__ int s_flag;
   const int tid = threadIdx.x;
   const int E = a.num_local_experts;
@@ -94,7 +94,6 @@ __device__ __forceinline__ void route_device(const McbRouteArgs& a) {
     // per thread and round.  On a 320-thread block: 3.7 us for 352 entries, 7.6 us for 2816 (the
     // multi-block form with its hand-over takes 11.7 us there), 21 us for 11264 (multi-block: about 13).
     if (blockIdx.x != 0) return;
-    __shared__ int s_cursor[kMaxLocalExperts];
     for (int e = tid; e < E; e += blockDim.x) { s_hist[e] = 0; s_cursor[e] = 0; }
     __syncthreads();
     for (int i0 = tid; i0 < (int)entries; i0 += blockDim.x * 4) {

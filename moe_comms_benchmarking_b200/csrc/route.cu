@@ -19,7 +19,8 @@ namespace mcb {
 __global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __grid_constant__ McbRouteArgs a) {
   pdl_wait();
   pdl_launch_dependents();
-  route_device(a);
+  __shared__ int s_route[2 * kMaxLocalExperts];
+  route_device(a, s_route);
 }
 
 // ------------------------------------------------------------------------------------------------

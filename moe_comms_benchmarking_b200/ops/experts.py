@@ -122,6 +122,23 @@ def make_weight_tmap(w2d: torch.Tensor):
     return (raw, addr)     # keep `raw` alive; `addr` is what launches take
 
 
+def make_ffn_tmaps(weights: "ExpertWeights", x: torch.Tensor, act: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+    """The tensor maps of one FFN launch (token rows, activations, expert outputs, packed weights) as a device tensor."""
+    raw = torch.zeros(_ext.FFN_TMAPS * 128 + 64, dtype=torch.uint8)
+    addr = (raw.data_ptr() + 63) & ~63
+    lib = _ext.require()
+    _ext.check(lib.mcb_make_ffn_tmaps(C.c_void_p(addr), C.c_void_p(x.data_ptr()), C.c_uint64(x.shape[0]),
+                                      C.c_void_p(act.data_ptr()), C.c_void_p(y.data_ptr()),
+                                      C.c_uint64(min(act.shape[0], y.shape[0])),
+                                      C.c_void_p(weights.w1.data_ptr()), C.c_void_p(weights.w2.data_ptr()),
+                                      weights.num_local_experts, weights.hidden, weights.intermediate), "make_ffn_tmaps")
+    off = addr - raw.data_ptr()
+    maps = raw[off:off + _ext.FFN_TMAPS * 128].to(act.device, non_blocking=True)    # pageable source: read before the call returns
+    if maps.data_ptr() % 64:
+        raise RuntimeError("device allocation is not 64-byte aligned")
+    return maps
+
+
 class RouteBuffers:
     """Device buffers written by the routing kernel and read by the GEMMs and the combine."""
 
@@ -285,7 +302,8 @@ def _aligned_layer_args(count: int):
 
 class ExpertFfnPlan:
     """Gate/up + SwiGLU + down over the pair lists of ``route`` as ONE persistent launch
-    (``expert_ffn_kernel``): weights are the M = 128 operand, an expert's tokens the small N."""
+    (``expert_ffn_kernel``): weights are the M operand, an expert's tokens the N.  The kernel runs in pairs of
+    CTAs, so an odd ``grid`` is rounded down (and 1 up to 2)."""
 
     def __init__(self, weights: ExpertWeights, route: RouteBuffers, x: torch.Tensor, act: torch.Tensor, y: torch.Tensor,
                  status: torch.Tensor | None = None, grid: int = NUM_SMS, timeout_s: float = 2.0):
@@ -300,8 +318,11 @@ class ExpertFfnPlan:
         if not (1 <= grid <= NUM_SMS):
             raise ValueError("down blocks wait for gate/up blocks of other CTAs: grid <= number of SMs")
         self.weights, self.grid = weights, grid
-        self._keep = (route, x, act, y, status)
+        tmaps = make_ffn_tmaps(weights, x, act, y)
+        sync = torch.zeros(2, dtype=torch.int32, device=y.device)
+        self._keep = (route, x, act, y, status, tmaps, sync)
         a = _ext.McbFfnArgs()
+        a.tmaps, a.sync = tmaps.data_ptr(), sync.data_ptr()
         a.x, a.x_row_bytes = x.data_ptr(), H * 2
         a.pair_token, a.pair_prob = route.pair_token.data_ptr(), route.pair_prob.data_ptr()
         a.expert_offset, a.max_rows = route.expert_offset.data_ptr(), route.max_rows.data_ptr()

@@ -189,9 +189,11 @@ class EmuWorld:
         (ExpertWeights), ``route`` (RouteBuffers), ``src`` = (hidden, routing, probs) local inputs,
         ``dst`` = (hidden, routing, probs) gathered HeapTensors, ``partial`` (HeapTensor), ``n_local``,
         ``step_meta``, ``act``, ``y``, ``out``, ``expert_begin`` and optionally ``ll_stage``."""
+        from ..ops.experts import make_ffn_tmaps
         stride = _ext.layer_args_size()
         blob = bytearray(stride * self.world)
         first = None
+        keep = []
         for r, d in enumerate(ranks):
             p = _ext.McbLayerArgs()
             w, route = d["weights"], d["route"]
@@ -221,6 +223,8 @@ class EmuWorld:
             ff.num_local_experts, ff.hidden, ff.intermediate = w.num_local_experts, w.hidden, w.intermediate
             ff.status, ff.timeout_ns = self.status[r].data_ptr(), int(timeout_s * 1e9)
             ff.w1, ff.w2 = w.w1.data_ptr(), w.w2.data_ptr()
+            keep += [make_ffn_tmaps(w, d["dst"][0].tensor, d["act"], d["y"]), torch.zeros(2, dtype=torch.int32, device=self.device)]
+            ff.tmaps, ff.sync = keep[-2].data_ptr(), keep[-1].data_ptr()
             cm = p.cmb
             cm.y, cm.pair_pos, cm.partial_off, cm.out = d["y"].data_ptr(), route.pair_pos.data_ptr(), d["partial"].offset, d["out"].data_ptr()
             cm.n_local, cm.step_meta = d["n_local"].data_ptr(), d["step_meta"].data_ptr()

@@ -288,3 +288,49 @@ def test_layer_kernel_phase_trace_world1(world1):
     ref = d.reference_output(h, i, w, layer=0)
     assert float((d.out.float().cpu() - ref).abs().max()) < 0.05 * float(ref.abs().max())
     d.destroy()
+
+
+@pytest.mark.parametrize("rows,H,I,grid", [
+    ([1, 31, 32, 33, 0, 64], 256, 128, 148),             # gathered token rows: below, at and above a multiple of 32, an idle expert
+    ([65, 0, 3], 512, 256, 6),                           # token rows copied into pair order, two column blocks per stage
+    ([129, 1], 256, 128, 148),                           # one column block per stage; more CTAs than units
+    ([256, 257, 0, 513, 5], 256, 384, 148),              # one, two and three chunks of an expert
+    ([40] * 200, 512, 256, 2),                           # more units than one list holds
+    ([2600, 300, 1, 900, 2400, 700], 256, 2048, 148),    # activations beyond the L2 bound: down units follow at a distance
+])
+def test_expert_ffn_chunk_edges(world1, rows, H, I, grid):
+    """expert_ffn_kernel where the token count of an expert meets the edges of its chunks, its token path and
+    its unit list.  Tokens are routed to one expert each, so `rows` sets the counts exactly.  bf16 inputs with fp32
+    sums: the error of an activation is its rounding to bf16 (2^-9 relative) plus that of its inputs' sum order."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, T = len(rows), sum(rows)
+    g = torch.Generator(device=DEV).manual_seed(29)
+    x = torch.randn(T, H, device=DEV, generator=g).to(torch.bfloat16)
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(rows, device=DEV))
+    idx = idx[torch.randperm(T, device=DEV, generator=g)].view(T, 1).contiguous()
+    w = torch.rand(T, 1, device=DEV, generator=g) + 0.1
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    ntok = torch.tensor([T], dtype=torch.int32, device=DEV)
+    route = RouteBuffers(T, 1, E, DEV)
+    weights = ExpertWeights(E, H, I, DEV, seed=6, std=0.05)
+    act = torch.zeros(T, I, dtype=torch.bfloat16, device=DEV)
+    y = torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)
+    rp = RoutePlan(route, idx, w, ntok, expert_begin=0, status=heap.status)
+    ffn = ExpertFfnPlan(weights, route, x, act, y, heap.status, grid=grid)
+    for rep in range(2):
+        act.fill_(float("nan")); y.fill_(float("nan"))
+        rp.launch(); ffn.launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        off, tok = route.expert_offset.tolist(), route.pair_token[:T].long()
+        wgu, wd = weights.w_gate_up.float(), weights.w_down.float()
+        for e in range(E):
+            if not rows[e]:
+                continue
+            sl = slice(off[e], off[e + 1])
+            gu = x.float()[tok[sl]] @ wgu[e].t()
+            want = torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]
+            assert float((act[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} gate/up"
+            want = act[sl].float() @ wd[e].t() * route.pair_prob[sl].unsqueeze(1)
+            assert float((y[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} down"
