@@ -215,3 +215,19 @@ def test_step_kernel_check_payload_depends_on_the_layer(lib):
     assert par2 != par and not torch.equal(rig.dst_h[1].tensor[par2, :8].view(torch.int16), first)
     assert [int(e.item()) for e in errs] == [0, 0]
     rig.w.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("K,grid,threads", [(22, 148, 512), (5, 2, 64), (3, 1, 32)])
+def test_world_of_one_copies(lib, dtype, K, grid, threads):
+    """A world of one: the layers of a step are flat copies of all ranges of a layer at once.  Rows of 8, 12, 20,
+    24 or 40 bytes leave words behind the last whole 16-byte pack, and the small grids reach both sides of the line
+    between the packs a thread keeps for all layers and those it works out layer by layer."""
+    cap, H = 132, 264
+    rig = _Rig(1, cap, H, K, 0, dtype)
+    for step, (n, layers) in enumerate([(1, 3), (3, 2), (132, 2), (0, 1), (7, 4)]):
+        rig.new_inputs()
+        rig.step([n], layers, grid, threads)
+        rig.check([n], expect_mode=0)
+        assert torch.equal(rig.outs[0][:n], rig.rsv[0].tensor[:n])
+    rig.w.check_status()
