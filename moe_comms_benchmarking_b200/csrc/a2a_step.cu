@@ -44,11 +44,12 @@ __device__ __forceinline__ DestMask dest_mask(const McbCtx& c, const McbA2AStepA
       report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)t, (uint32_t)e);
       continue;
     }
-    const int d = (int)(e / epr);
+    const uint32_t d = (uint32_t)e / (uint32_t)epr;
     m.w[d >> 5] |= 1u << (d & 31);
   }
 #pragma unroll
-  for (int i = 0; i < 3; ++i) m.w[i] = __reduce_or_sync(0xffffffffu, m.w[i]);
+  for (int i = 0; i < 3; ++i)
+    if (i * 32 < c.world) m.w[i] = __reduce_or_sync(0xffffffffu, m.w[i]);
   return m;
 }
 
@@ -246,161 +247,215 @@ __device__ __noinline__ void packet_layers(const McbCtx& c, const McbA2AStepArgs
   if (tid == 0) *epoch_ptr(c, MCB_SITE_A2A_STEP_CREDIT, bid) = cb + (uint32_t)L;
 }
 
+// ---- barrier mode -----------------------------------------------------------------------------------
+// A warp serves one slice of a token's row: kSlicePacks 16-byte packs, four per lane, so a wide row (hidden 7168: seven
+// slices) has as many loads in flight as seven narrow ones and a step of a few hundred wide tokens fills the chip.  Alone
+// on one B200, 58 layers of 333 rows of 7168 values with e4m3 dispatch: 265 us, against 1767 with one warp per token
+// packed into as few blocks as possible and the pull as a pass of its own.
+constexpr int kSlicePacks = 128;
+
+struct RowSlice {
+  int t, p0;            // token, first pack
+  uint64_t row;         // row of the token in the receive layout
+};
+
+struct BarrierShape {
+  int slices, row_packs, nblk, meta_chunks, epr;
+  uint64_t row_bytes, xrow_bytes;
+};
+
+__device__ __forceinline__ void load_packs(uint4 (&v)[4], const uint8_t* row, int p0, int row_packs, int lane) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int p = p0 + u * 32 + lane;
+    v[u] = p < row_packs ? ld_v4_stream(row + (uint64_t)p * 16) : make_uint4(0, 0, 0, 0);
+  }
+}
+
+// Chunk j of the metadata row: 0 = {stamp, token, id 0, weight 0}, j = {id 2j-1, weight 2j-1, id 2j, weight 2j}.
+__device__ __forceinline__ uint4 meta_chunk(const McbA2AStepArgs& a, int t, int j, uint32_t stamp) {
+  const int k0 = j == 0 ? 0 : 2 * j - 1, k1 = 2 * j;
+  const long long tb = (long long)t * a.topk;
+  const uint32_t id0 = k0 < a.topk ? (uint32_t)a.topk_idx[tb + k0] : 0xffffffffu;
+  const uint32_t w0 = k0 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k0] : 1.0f) : 0u;
+  if (j == 0) return make_uint4(stamp, (uint32_t)t, id0, w0);
+  const uint32_t id1 = k1 < a.topk ? (uint32_t)a.topk_idx[tb + k1] : 0xffffffffu;
+  const uint32_t w1 = k1 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k1] : 1.0f) : 0u;
+  return make_uint4(id0, w0, id1, w1);
+}
+
+// Slice of a row (and, with the first slice, the metadata row) to every destination in the mask.
+__device__ __forceinline__ void push_slice(const McbCtx& c, const McbA2AStepArgs& a, const BarrierShape& s, const RowSlice& r,
+                                           const DestMask& m, const uint4 (&v)[4], uint4 meta, uint32_t par, uint32_t stamp,
+                                           int lane) {
+  uint2 q[4];
+  float scale[4];
+  if (a.fp8) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float amax = pack_absmax(v[u]);          // 16 lanes hold one 128-value block
+#pragma unroll
+      for (int sh = 8; sh >= 1; sh >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
+      scale[u] = e4m3_scale(amax);
+      q[u] = quant_pack_e4m3(v[u], scale[u]);
+    }
+  }
+#pragma unroll 1
+  for (int wi = 0; wi < 3; ++wi) {
+    uint32_t bits = m.w[wi];
+    while (bits) {
+      const int d = wi * 32 + __ffs(bits) - 1;
+      bits &= bits - 1;
+      uint8_t* peer = c.heap_peer[d];
+      uint8_t* dst = peer + a.recv_x_off + (uint64_t)par * a.x_par_stride + r.row * s.xrow_bytes;
+      uint8_t* sc = peer + a.recv_scale_off + (uint64_t)par * a.scale_par_stride + r.row * s.nblk * 4;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int p = r.p0 + u * 32 + lane;
+        if (p >= s.row_packs) continue;
+        if (a.fp8) {
+          st_v2(dst + (uint64_t)p * 8, q[u]);
+          if ((lane & 15) == 0) st_b32(sc + (p >> 4) * 4, __float_as_uint(scale[u]));
+        } else {
+          st_v4(dst + (uint64_t)p * 16, v[u]);
+        }
+      }
+      if (r.p0 == 0) {
+        uint8_t* md = peer + a.recv_meta_off + (uint64_t)par * a.meta_par_stride + r.row * a.meta_row_bytes;
+        if (lane < s.meta_chunks) st_v4(md + lane * 16, meta);
+        for (int j = lane + 32; j < s.meta_chunks; j += 32) st_v4(md + (uint64_t)j * 16, meta_chunk(a, r.t, j, stamp));
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void add_packs(float (&acc)[4][8], const uint4 (&v)[4]) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc_bf16x8(acc[u], v[u]);
+}
+
+__device__ __forceinline__ void store_out(const McbA2AStepArgs& a, const BarrierShape& s, const RowSlice& r,
+                                          const float (&acc)[4][8], int lane) {
+  uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + (uint64_t)r.t * s.row_bytes;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int p = r.p0 + u * 32 + lane;
+    if (p < s.row_packs)
+      st_v4(out + (uint64_t)p * 16, make_uint4(pack_bf16x2(acc[u][0], acc[u][1]), pack_bf16x2(acc[u][2], acc[u][3]),
+                                               pack_bf16x2(acc[u][4], acc[u][5]), pack_bf16x2(acc[u][6], acc[u][7])));
+  }
+}
+
 // Barrier-mode layers of a step: push -> one block-matched barrier -> pull + fp32 sum.  Out of line, as above.
 __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, int ep_max, uint32_t layer_base) {
   const int tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   const int W = c.world, L = a.num_layers;
-  // One warp per token; as many blocks as the largest rank needs, the same on every rank.
-  int nact = (ep_max + nwarps - 1) / nwarps;
-  nact = nact > (int)gridDim.x ? (int)gridDim.x : nact;
-  const int epr = a.num_experts / W;
-  const int row_packs = a.hidden / 8;
-  const uint64_t row_bytes = (uint64_t)a.hidden * 2;
-  const uint64_t xrow_bytes = a.fp8 ? (uint64_t)a.hidden : row_bytes;     // bytes of a dispatched row
-  const int nblk = a.hidden / 128;
-  const int meta_chunks = (int)(a.meta_row_bytes >> 4);
+  BarrierShape s;
+  s.row_packs = a.hidden / 8;
+  s.slices = (s.row_packs + kSlicePacks - 1) / kSlicePacks;
+  s.nblk = a.hidden / 128;
+  s.meta_chunks = (int)(a.meta_row_bytes >> 4);
+  s.epr = a.num_experts / W;
+  s.row_bytes = (uint64_t)a.hidden * 2;
+  s.xrow_bytes = a.fp8 ? (uint64_t)a.hidden : s.row_bytes;     // bytes of a dispatched row
   const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
-  uint8_t* out = reinterpret_cast<uint8_t*>(a.out);
+  const uint64_t slot0 = (uint64_t)c.rank * a.cap;             // first row of this source on a destination
+  // As many blocks as the largest rank needs, the same on every rank: with peers full blocks (each costs a flag per
+  // rank and layer), alone one warp per block first, so that the smallest steps spread over the chip.
+  const long long items = (long long)ep_max * s.slices;
+  const long long want = W == 1 ? items : (items + nwarps - 1) / nwarps;
+  const int nact = (int)(want > (long long)gridDim.x ? (long long)gridDim.x : want);
+  if (bid >= nact) return;
+  const long long mine = (long long)n * s.slices;
+  const long long first = W == 1 ? bid + (long long)warp * nact : (long long)bid * nwarps + warp;
+  const long long step = (long long)nact * nwarps;
+  auto slice_of = [&](long long i) {
+    RowSlice r;
+    r.t = (int)(i / s.slices);
+    r.p0 = (int)(i - (long long)r.t * s.slices) * kSlicePacks;
+    r.row = slot0 + r.t;
+    return r;
+  };
 
-  if (bid < nact) {
-    uint32_t ep = *epoch_ptr(c, MCB_SITE_A2A_STEP, bid);
+  if (W == 1) {
+    // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.
+    // The identity expert on bf16 rows returns the row just delivered, which is still in registers.
+    const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
     for (int l = 0; l < L; ++l) {
       const uint32_t par = (layer_base + (uint32_t)l) & 1u;
       const uint32_t stamp = layer_base + (uint32_t)l + 1u;
-      const uint64_t slot0 = (uint64_t)c.rank * a.cap;            // first row of this source on a destination
-      // ---- push: row (+ scales) and metadata to every distinct destination rank ----
-      for (int t = bid * nwarps + warp; t < n; t += nact * nwarps) {
-        const DestMask m = dest_mask(c, a, t, epr, lane);
-        const uint8_t* xrow = x + (uint64_t)t * row_bytes;
-        const uint64_t row = slot0 + t;
-        for (int p0 = 0; p0 < row_packs; p0 += 128) {
-          uint4 v[4];
-          uint2 q[4];
-          float scale[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int p = p0 + u * 32 + lane;
-            v[u] = p < row_packs ? ld_v4(xrow + (uint64_t)p * 16) : make_uint4(0, 0, 0, 0);
-          }
-          if (a.fp8) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              float amax = pack_absmax(v[u]);          // 16 lanes hold one 128-value block
-#pragma unroll
-              for (int sh = 8; sh >= 1; sh >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
-              scale[u] = e4m3_scale(amax);
-              q[u] = quant_pack_e4m3(v[u], scale[u]);
-            }
-          }
-#pragma unroll 1
-          for (int wi = 0; wi < 3; ++wi) {
-            uint32_t bits = m.w[wi];
-            while (bits) {
-              const int d = wi * 32 + __ffs(bits) - 1;
-              bits &= bits - 1;
-              uint8_t* peer = c.heap_peer[d];
-              uint8_t* dst = peer + a.recv_x_off + (uint64_t)par * a.x_par_stride + row * xrow_bytes;
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int p = p0 + u * 32 + lane;
-                if (p >= row_packs) continue;
-                if (a.fp8) {
-                  st_v2(dst + (uint64_t)p * 8, q[u]);
-                  if ((lane & 15) == 0)
-                    st_b32(peer + a.recv_scale_off + (uint64_t)par * a.scale_par_stride + (row * nblk + (p >> 4)) * 4,
-                           __float_as_uint(scale[u]));
-                } else {
-                  st_v4(dst + (uint64_t)p * 16, v[u]);
-                }
-              }
-            }
-          }
+      for (long long i = first; i < mine; i += step) {
+        const RowSlice r = slice_of(i);
+        uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
+        load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
+        if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
+        if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
+        const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
+        push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
+        float acc[4][8] = {};
+        if (m.w[0]) {
+          if (echo) add_packs(acc, v);
+          else add_packs(acc, y);
         }
-        // metadata row: chunk 0 = {stamp, token, id 0, weight 0}, chunk j = {id 2j-1, weight 2j-1, id 2j, weight 2j}
-        for (int j = lane; j < meta_chunks; j += 32) {
-          uint4 ch;
-          const int k0 = j == 0 ? 0 : 2 * j - 1, k1 = 2 * j;
-          const long long tb = (long long)t * a.topk;
-          const uint32_t id0 = k0 < a.topk ? (uint32_t)a.topk_idx[tb + k0] : 0xffffffffu;
-          const uint32_t w0 = k0 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k0] : 1.0f) : 0u;
-          if (j == 0) {
-            ch = make_uint4(stamp, (uint32_t)t, id0, w0);
-          } else {
-            const uint32_t id1 = k1 < a.topk ? (uint32_t)a.topk_idx[tb + k1] : 0xffffffffu;
-            const uint32_t w1 = k1 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k1] : 1.0f) : 0u;
-            ch = make_uint4(id0, w0, id1, w1);
-          }
-#pragma unroll 1
-          for (int wi = 0; wi < 3; ++wi) {
-            uint32_t bits = m.w[wi];
-            while (bits) {
-              const int d = wi * 32 + __ffs(bits) - 1;
-              bits &= bits - 1;
-              st_v4(c.heap_peer[d] + a.recv_meta_off + (uint64_t)par * a.meta_par_stride + row * a.meta_row_bytes +
-                        (uint64_t)j * 16, ch);
-            }
-          }
-        }
-      }
-      // ---- one barrier: the matching block of every rank has pushed its tokens of this layer ----
-      if (W > 1) {
-        __syncthreads();
-        signal_all<true>(c, MCB_SITE_A2A_STEP, bid);
-        if (tid == 0) wait_flag(c, MCB_SITE_A2A_STEP, bid, (ep + 1u) * (uint32_t)W);
-        ++ep;
-        __syncthreads();
-      }
-      // ---- pull: one expert-output row per destination rank, summed in fp32 ----
-      for (int t = bid * nwarps + warp; t < n; t += nact * nwarps) {
-        const DestMask m = dest_mask(c, a, t, epr, lane);
-        const uint64_t yoff = a.y_off + (uint64_t)par * a.y_par_stride + (slot0 + t) * row_bytes;
-        for (int p0 = 0; p0 < row_packs; p0 += 128) {
-          float acc[4][8];
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
-#pragma unroll 1
-          for (int wi = 0; wi < 3; ++wi) {
-            uint32_t bits = m.w[wi];
-            while (bits) {
-              // two destinations per round: 8 independent 16-byte peer loads in flight per lane
-              const int d0 = wi * 32 + __ffs(bits) - 1;
-              bits &= bits - 1;
-              int d1 = -1;
-              if (bits) { d1 = wi * 32 + __ffs(bits) - 1; bits &= bits - 1; }
-              uint4 v0[4], v1[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const int p = p0 + u * 32 + lane;
-                const bool in = p < row_packs;
-                v0[u] = in ? ld_v4_stream(c.heap_peer[d0] + yoff + (uint64_t)p * 16) : make_uint4(0, 0, 0, 0);
-                v1[u] = in && d1 >= 0 ? ld_v4_stream(c.heap_peer[d1] + yoff + (uint64_t)p * 16) : make_uint4(0, 0, 0, 0);
-              }
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                acc[u][0] += bf16_lo(v0[u].x) + bf16_lo(v1[u].x); acc[u][1] += bf16_hi(v0[u].x) + bf16_hi(v1[u].x);
-                acc[u][2] += bf16_lo(v0[u].y) + bf16_lo(v1[u].y); acc[u][3] += bf16_hi(v0[u].y) + bf16_hi(v1[u].y);
-                acc[u][4] += bf16_lo(v0[u].z) + bf16_lo(v1[u].z); acc[u][5] += bf16_hi(v0[u].z) + bf16_hi(v1[u].z);
-                acc[u][6] += bf16_lo(v0[u].w) + bf16_lo(v1[u].w); acc[u][7] += bf16_hi(v0[u].w) + bf16_hi(v1[u].w);
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int p = p0 + u * 32 + lane;
-            if (p < row_packs)
-              st_v4(out + (uint64_t)t * row_bytes + (uint64_t)p * 16,
-                    make_uint4(pack_bf16x2(acc[u][0], acc[u][1]), pack_bf16x2(acc[u][2], acc[u][3]),
-                               pack_bf16x2(acc[u][4], acc[u][5]), pack_bf16x2(acc[u][6], acc[u][7])));
-          }
-        }
+        store_out(a, s, r, acc, lane);
       }
     }
-    if (tid == 0) *epoch_ptr(c, MCB_SITE_A2A_STEP, bid) = ep;
+    return;
   }
 
+  uint32_t ep = *epoch_ptr(c, MCB_SITE_A2A_STEP, bid);
+  for (int l = 0; l < L; ++l) {
+    const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+    const uint32_t stamp = layer_base + (uint32_t)l + 1u;
+    // ---- push: row (+ scales) and metadata to every distinct destination rank ----
+    DestMask m = {{0u, 0u, 0u}};
+    for (long long i = first; i < mine; i += step) {
+      const RowSlice r = slice_of(i);
+      uint4 v[4], meta = make_uint4(0, 0, 0, 0);
+      load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
+      if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
+      m = dest_mask(c, a, r.t, s.epr, lane);
+      push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
+    }
+    // ---- one barrier: the matching block of every rank has pushed its tokens of this layer ----
+    __syncthreads();
+    signal_all<true>(c, MCB_SITE_A2A_STEP, bid);
+    if (tid == 0) wait_flag(c, MCB_SITE_A2A_STEP, bid, (ep + 1u) * (uint32_t)W);
+    ++ep;
+    __syncthreads();
+    // ---- pull: one expert-output row per destination rank, summed in fp32 ----
+    for (long long i = first; i < mine; i += step) {
+      const RowSlice r = slice_of(i);
+      if (mine > step) m = dest_mask(c, a, r.t, s.epr, lane);      // else the warp's only slice: the mask of its push
+      const uint64_t yoff = a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes;
+      float acc[4][8] = {};
+#pragma unroll 1
+      for (int wi = 0; wi < 3; ++wi) {
+        uint32_t bits = m.w[wi];
+        while (bits) {
+          // two destinations per round: 8 independent 16-byte peer loads in flight per lane
+          const int d0 = wi * 32 + __ffs(bits) - 1;
+          bits &= bits - 1;
+          int d1 = -1;
+          if (bits) { d1 = wi * 32 + __ffs(bits) - 1; bits &= bits - 1; }
+          uint4 v0[4], v1[4];
+          load_packs(v0, c.heap_peer[d0] + yoff, r.p0, s.row_packs, lane);
+          if (d1 >= 0) load_packs(v1, c.heap_peer[d1] + yoff, r.p0, s.row_packs, lane);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (d1 < 0) v1[u] = make_uint4(0, 0, 0, 0);
+            acc[u][0] += bf16_lo(v0[u].x) + bf16_lo(v1[u].x); acc[u][1] += bf16_hi(v0[u].x) + bf16_hi(v1[u].x);
+            acc[u][2] += bf16_lo(v0[u].y) + bf16_lo(v1[u].y); acc[u][3] += bf16_hi(v0[u].y) + bf16_hi(v1[u].y);
+            acc[u][4] += bf16_lo(v0[u].z) + bf16_lo(v1[u].z); acc[u][5] += bf16_hi(v0[u].z) + bf16_hi(v1[u].z);
+            acc[u][6] += bf16_lo(v0[u].w) + bf16_lo(v1[u].w); acc[u][7] += bf16_hi(v0[u].w) + bf16_hi(v1[u].w);
+          }
+        }
+      }
+      store_out(a, s, r, acc, lane);
+    }
+  }
+  if (tid == 0) *epoch_ptr(c, MCB_SITE_A2A_STEP, bid) = ep;
 }
 
 template <bool EMU>

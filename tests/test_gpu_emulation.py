@@ -273,6 +273,50 @@ def test_a2a_step_kernel(lib, fp8, grid, threads, ll_rows):
     w.check_status()
 
 
+@pytest.mark.parametrize("W", [1, 2])
+@pytest.mark.parametrize("fp8,H", [(False, 2056), (True, 1152), (False, 1024)])
+@pytest.mark.parametrize("grid,threads", [(2, 64), (37, 512)])
+def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
+    """Rows served slice by slice (128 packs of 16 bytes per warp): one pack and 16 packs in the last slice, more slices
+    than warps and fewer, alone and with a peer."""
+    E, K, cap = 16, 5, 9
+    w = EmuWorld(W, 16 << 20, DEV)
+    b = w.a2a_step_buffers(cap, H, K, fp8)
+    g = torch.Generator(device=DEV).manual_seed(31)
+    metas = [torch.zeros(8, dtype=torch.int32, device=DEV) for _ in range(W)]
+    outs = [torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV) for _ in range(W)]
+    if fp8:
+        for r in range(W):
+            b["y"][r].tensor.copy_(torch.randn(2, W, cap, H, device=DEV, generator=g))
+    for counts, layers in (([9, 4], 3), ([1, 2], 2)):
+        counts = counts[:W]
+        xs = [torch.randn(cap, H, device=DEV, generator=g).to(torch.bfloat16) for _ in range(W)]
+        idxs = [torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(cap)]) for _ in range(W)]
+        ws = [torch.rand(cap, K, device=DEV, generator=g) for _ in range(W)]
+        w.a2a_step(b, xs, idxs, ws, outs, _scalars(counts), metas, E, layers, grid=grid, threads=threads)
+        par, stamp = int(metas[0][5]), int(metas[0][7])
+        for s in range(W):
+            c = counts[s]
+            ref = torch.zeros(c, H)
+            for d in range(W):
+                here = ((idxs[s][:c] // (E // W)) == d).any(dim=1)
+                words = b["recv_meta"][d].tensor[par, s, :c].view(torch.int32).view(c, -1)
+                assert torch.equal(words[:, 0] == stamp, here)
+                sel = here.nonzero().flatten()
+                assert torch.equal(words[sel][:, 2:2 + 2 * K:2].long(), idxs[s][sel])
+                if fp8:
+                    q, s_ref = oracle.quant_e4m3_1x128(xs[s][sel].float().cpu())
+                    assert torch.equal(b["recv_scale"][d].tensor[par, s][sel].cpu(), s_ref)
+                    assert torch.equal(b["recv_x"][d].tensor[par, s][sel].cpu(), q.view(torch.uint8))
+                    ref += b["y"][d].tensor[par, s, :c].float().cpu() * here.cpu()[:, None]
+                else:
+                    assert torch.equal(b["recv_x"][d].tensor[par, s][sel], xs[s][sel])
+                    ref += xs[s][:c].float().cpu() * here.cpu()[:, None]
+            # at most two bf16 rows are summed in fp32 and rounded once
+            assert torch.allclose(outs[s][:c].float().cpu(), ref, rtol=2 ** -8, atol=1e-6)
+    w.check_status()
+
+
 def test_a2a_fp8_dispatch(lib):
     W, E, K, H, counts = 2, 16, 4, 512, [6, 3]
     w, b, xs, idxs, ws, n_locals, cap = _a2a_case(W, E, K, H, counts, True, 13)
