@@ -80,6 +80,16 @@ typedef struct {
   int32_t reserved0;
 } McbMetaArgs;
 
+// One step's inputs (hidden rows, routing, weights) into persistent buffers, and the token count.
+typedef struct {
+  const void* src[3];          // device memory or pinned host memory, 4-byte aligned
+  void* dst[3];                // 16-byte aligned
+  uint64_t bytes[3];           // multiples of 4
+  int32_t* n_local;            // device scalar, set to n
+  int32_t n;
+  int32_t reserved0;
+} McbLoadArgs;
+
 #define MCB_MAX_TENSORS 4
 
 // Variable all-gather of up to MCB_MAX_TENSORS row-major tensors into packed

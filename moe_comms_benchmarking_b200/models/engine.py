@@ -72,20 +72,11 @@ class MoEDecodeEngine:
         this call returns: it synchronises)."""
         d = self.dispatcher
         n = hidden_pinned.shape[0]
-        if n > d.cap:
-            raise ValueError(f"{n} tokens exceed the per-rank capacity {d.cap}")
+        d._load_rows(hidden_pinned, idx_pinned, w_pinned, pinned=True)
         if self._pinned is None:
-            self._pinned = {"n": torch.zeros(1, dtype=torch.int32).pin_memory(),
-                            "out": torch.empty(d.cap, self.cfg.hidden, dtype=d.out_buf.dtype).pin_memory()}
-        self._pinned["n"][0] = n
-        if n:
-            d.in_hidden[:n].copy_(hidden_pinned, non_blocking=True)
-            d.in_routing[:n].copy_(idx_pinned, non_blocking=True)
-            d.in_probs[:n].copy_(w_pinned, non_blocking=True)
-        d.n_local.copy_(self._pinned["n"], non_blocking=True)
-        d.local_tokens = n
+            self._pinned = torch.empty(d.cap, self.cfg.hidden, dtype=d.out_buf.dtype).pin_memory()
         self.run()
-        out = out_pinned if out_pinned is not None else self._pinned["out"]
+        out = out_pinned if out_pinned is not None else self._pinned
         if n:
             out[:n].copy_(d.out_buf[:n], non_blocking=True)
         torch.cuda.current_stream().synchronize()

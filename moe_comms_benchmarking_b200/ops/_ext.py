@@ -54,6 +54,10 @@ class McbMetaArgs(C.Structure):
                 ("reserved0", _i32)]
 
 
+class McbLoadArgs(C.Structure):
+    _fields_ = [("src", _vp * 3), ("dst", _vp * 3), ("bytes", _u64 * 3), ("n_local", _vp), ("n", _i32), ("reserved0", _i32)]
+
+
 class McbAgvArgs(C.Structure):
     _fields_ = [
         ("src", _vp * MAX_TENSORS), ("dst_off", _u64 * MAX_TENSORS), ("row_bytes", _u32 * MAX_TENSORS),
@@ -172,9 +176,19 @@ GEMM_FC1, GEMM_FC2 = 0, 1
 FFN_TMAPS = 21
 
 _STRUCTS = {
-    "ctx": McbCtx, "meta_args": McbMetaArgs, "agv_args": McbAgvArgs, "rsv_args": McbRsvArgs,
+    "ctx": McbCtx, "load_args": McbLoadArgs, "meta_args": McbMetaArgs, "agv_args": McbAgvArgs, "rsv_args": McbRsvArgs,
     "a2a_dispatch_args": McbA2ADispatchArgs, "a2a_combine_args": McbA2ACombineArgs, "a2a_step_args": McbA2AStepArgs, "norm_args": McbNormArgs,
     "dense_step_args": McbDenseStepArgs, "gemm_args": McbGemmArgs, "ffn_args": McbFfnArgs, "route_args": McbRouteArgs, "combine_args": McbCombineArgs,
+}
+
+# Argument types of the launchers that are called once per operation or step (p = pointer, i = int): ctypes then converts
+# by table instead of asking each value what it is.
+_ARG = {"p": C.c_void_p, "i": C.c_int}
+_LAUNCHERS = {
+    "mcb_launch_load_batch": "pip", "mcb_launch_metadata": "ppip", "mcb_launch_agv": "ppiiip", "mcb_launch_rsv": "ppiiip",
+    "mcb_launch_dense_step": "ppiiip", "mcb_launch_a2a_dispatch": "ppiiip", "mcb_launch_a2a_combine": "ppiiip",
+    "mcb_launch_a2a_step": "ppiiip", "mcb_launch_route": "piip", "mcb_launch_expert_ffn": "piip",
+    "mcb_launch_combine": "ppiiip", "mcb_launch_moe_layer": "piip",
 }
 
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libmcb.so"
@@ -226,6 +240,8 @@ def load():
                                f"{layer_args_size()} in ctypes")
     lib.mcb_error_string.restype = C.c_char_p
     lib.mcb_error_string.argtypes = [C.c_int]
+    for name, sig in _LAUNCHERS.items():
+        getattr(lib, name).argtypes = [_ARG[c] for c in sig]
     _lib = lib
     return lib
 
@@ -246,7 +262,22 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def stream_handle(stream=None) -> C.c_void_p:
+def _raw_stream_getter():
+    """The current stream's handle without building a ``torch.cuda.Stream`` (3 us of a launch's 4 us of host time)."""
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or dev is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(dev())
+
+
+_current_raw_stream = None
+
+
+def stream_handle(stream=None) -> C.c_void_p:
+    global _current_raw_stream
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    if _current_raw_stream is None:
+        _current_raw_stream = _raw_stream_getter()
+    return C.c_void_p(_current_raw_stream())

@@ -80,11 +80,11 @@ class A2ADispatchPlan:
         a.n_local = n_local.data_ptr()
         a.hidden, a.topk, a.num_experts, a.cap = bufs.hidden, bufs.topk, int(num_experts), bufs.cap
         a.fp8 = 1 if bufs.fp8 else 0
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_a2a_dispatch(C.byref(self.heap.ctx()), C.byref(self.args), self.grid,
+        _ext.check(lib.mcb_launch_a2a_dispatch(self.heap.ctx_ref(), self._ref, self.grid,
                                                self.threads, int(pdl), _ext.stream_handle(stream)),
                    "a2a_dispatch")
 
@@ -102,12 +102,12 @@ class A2ACombinePlan:
         a.out, a.y_off = out.data_ptr(), bufs.y.offset
         a.slot_map, a.n_local = bufs.slot_map.data_ptr(), n_local.data_ptr()
         a.hidden, a.cap = bufs.hidden, bufs.cap
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_A2A_COMBINE, self.grid)
-        _ext.check(lib.mcb_launch_a2a_combine(C.byref(self.heap.ctx()), C.byref(self.args), self.grid,
+        _ext.check(lib.mcb_launch_a2a_combine(self.heap.ctx_ref(), self._ref, self.grid,
                                               self.threads, int(pdl), _ext.stream_handle(stream)),
                    "a2a_combine")
 
@@ -229,18 +229,18 @@ class A2AStepPlan:
                 _check_heap_tensor(heap, getattr(bufs, name), name)
             a.ll_rows, a.ll_src_rows = bufs.ll_rows, min(bufs.cap, bufs.ll_rows)
             a.ll_x_off, a.ll_y_off, a.credit_off = bufs.ll_x.offset, bufs.ll_y.offset, bufs.credits.offset
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_a2a_step(C.byref(self.heap.ctx()), C.byref(self.args), self.grid, self.threads,
+        _ext.check(lib.mcb_launch_a2a_step(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
                                            int(pdl), _ext.stream_handle(stream)), "a2a_step")
 
 
 def a2a_decode_step(heap, d: A2ADispatchPlan, c: A2ACombinePlan, num_layers: int, pdl: bool = False, stream=None):
     lib = _ext.require()
     heap.level_launch_counters(_ext.SITE_A2A_COMBINE, d.grid)
-    _ext.check(lib.mcb_a2a_decode_step(C.byref(heap.ctx()), C.byref(d.args), C.byref(c.args), int(num_layers),
+    _ext.check(lib.mcb_a2a_decode_step(heap.ctx_ref(), C.byref(d.args), C.byref(c.args), int(num_layers),
                                        d.grid, d.threads, int(pdl), _ext.stream_handle(stream)),
                "a2a_decode_step")
 

@@ -74,11 +74,11 @@ class MetadataPlan:
         a.counts_off = heap.counts_off
         a.step_meta = step_meta.data_ptr()
         a.cap = int(cap)
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_metadata(C.byref(self.heap.ctx()), C.byref(self.args), int(pdl),
+        _ext.check(lib.mcb_launch_metadata(self.heap.ctx_ref(), self._ref, int(pdl),
                                            _ext.stream_handle(stream)), "metadata")
 
 
@@ -122,12 +122,12 @@ class AllGatherVPlan:
                 raise ValueError(f"low-latency staging holds {ll_stage.nbytes} bytes, {need} needed")
             a.ll_off, a.ll_rows = ll_stage.offset, int(ll_rows)
             self._keep += (ll_stage,)
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_AGV_LL, self.grid)
-        _ext.check(lib.mcb_launch_agv(C.byref(self.heap.ctx()), C.byref(self.args), self.grid, self.threads,
+        _ext.check(lib.mcb_launch_agv(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
                                       int(pdl), _ext.stream_handle(stream)), "all_gather_v")
 
 
@@ -164,12 +164,12 @@ class ReduceScatterVPlan:
             a.ll_off, a.ll_rows, a.counts_off = ll_stage.offset, int(ll_rows), heap.counts_off
             a.ll_src_rows = min(int(cap), int(ll_rows))
             self._keep += (ll_stage,)
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_RSV_LL, self.grid)
-        _ext.check(lib.mcb_launch_rsv(C.byref(self.heap.ctx()), C.byref(self.args), self.grid, self.threads,
+        _ext.check(lib.mcb_launch_rsv(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
                                       int(pdl), _ext.stream_handle(stream)), "reduce_scatter_v")
 
 
@@ -180,7 +180,7 @@ def dense_decode_step(heap, meta: MetadataPlan, agv: AllGatherVPlan, rsv: Reduce
     lib = _ext.require()
     heap.level_launch_counters(_ext.SITE_AGV_LL, agv.grid)
     heap.level_launch_counters(_ext.SITE_RSV_LL, agv.grid)
-    _ext.check(lib.mcb_dense_decode_step(C.byref(heap.ctx()), C.byref(meta.args), C.byref(agv.args),
+    _ext.check(lib.mcb_dense_decode_step(heap.ctx_ref(), C.byref(meta.args), C.byref(agv.args),
                                          C.byref(rsv.args), int(num_layers), agv.grid, agv.threads, int(pdl),
                                          _ext.stream_handle(stream)), "dense_decode_step")
 
@@ -291,11 +291,11 @@ class DenseStepPlan:
             a.check_errors, a.check = check_errors.data_ptr(), 1
             a.delay_ns, a.delay_every = int(delay_ns), max(1, int(delay_every))
             self._keep += (check_errors,)
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_dense_step(C.byref(self.heap.ctx()), C.byref(self.args), self.grid, self.threads,
+        _ext.check(lib.mcb_launch_dense_step(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
                                              int(pdl), _ext.stream_handle(stream)), "dense_step")
 
 

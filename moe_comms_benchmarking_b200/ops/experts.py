@@ -183,11 +183,11 @@ class RoutePlan:
             setattr(a, f, getattr(bufs, f).data_ptr())
         a.max_pairs, a.max_tiles = bufs.max_pairs, bufs.max_tiles
         a.status, a.timeout_ns = _ext.ptr(status), int(timeout_s * 1e9)
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_route(C.byref(self.args), self.grid, int(pdl), _ext.stream_handle(stream)), "route")
+        _ext.check(lib.mcb_launch_route(self._ref, self.grid, int(pdl), _ext.stream_handle(stream)), "route")
 
 
 class GroupedGemmPlan:
@@ -217,11 +217,11 @@ class GroupedGemmPlan:
         g.tile_rows, g.num_m_tiles = route.tile_rows.data_ptr(), route.num_m_tiles.data_ptr()
         g.n_total, g.k_total = int(n_total), int(k_total)
         g.status, g.timeout_ns = _ext.ptr(status), int(timeout_s * 1e9)
-        self.args = g
+        self.args, self._ref = g, C.byref(g)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_grouped_gemm(C.c_void_p(self.tmap[1]), C.byref(self.args), self.mode, self.grid,
+        _ext.check(lib.mcb_launch_grouped_gemm(C.c_void_p(self.tmap[1]), self._ref, self.mode, self.grid,
                                                int(pdl), _ext.stream_handle(stream)), "grouped_gemm")
 
 
@@ -244,11 +244,11 @@ class ExpertCombinePlan:
         a.n_local, a.step_meta = n_local.data_ptr(), step_meta.data_ptr()
         a.hidden, a.topk, a.cap, a.site = hidden, route.topk, int(cap), int(site)
         a.partial_par_stride = partial.nbytes // 2 if two else 0
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_combine(C.byref(self.heap.ctx()), C.byref(self.args), self.grid, self.threads,
+        _ext.check(lib.mcb_launch_combine(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
                                           int(pdl), _ext.stream_handle(stream)), "expert_combine")
 
 
@@ -267,7 +267,7 @@ class Fc2CombinePlan:
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
         _ext.check(lib.mcb_launch_fc2_combine(C.c_void_p(self.fc2.tmap[1]), C.byref(self.fc2.args),
-                                              C.byref(self.heap.ctx()), C.byref(self.combine.args), self.grid,
+                                              self.heap.ctx_ref(), C.byref(self.combine.args), self.grid,
                                               int(pdl), _ext.stream_handle(stream)), "fc2_combine")
 
 
@@ -287,7 +287,7 @@ class DispatchRouteFc1Plan:
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
         _ext.check(lib.mcb_launch_dispatch_route_fc1(C.c_void_p(self.fc1.tmap[1]), C.byref(self.fc1.args),
-                                                     C.byref(self.heap.ctx()), C.byref(self.agv.args),
+                                                     self.heap.ctx_ref(), C.byref(self.agv.args),
                                                      C.byref(self.route.args), self.grid, int(pdl),
                                                      _ext.stream_handle(stream)), "dispatch_route_fc1")
 
@@ -330,11 +330,11 @@ class ExpertFfnPlan:
         a.num_local_experts, a.hidden, a.intermediate = weights.num_local_experts, H, I
         a.status, a.timeout_ns = _ext.ptr(status), int(timeout_s * 1e9)
         a.w1, a.w2 = weights.w1.data_ptr(), weights.w2.data_ptr()
-        self.args = a
+        self.args, self._ref = a, C.byref(a)
 
     def launch(self, pdl: bool = False, stream=None):
         lib = _ext.require()
-        _ext.check(lib.mcb_launch_expert_ffn(C.byref(self.args), self.grid, int(pdl), _ext.stream_handle(stream)),
+        _ext.check(lib.mcb_launch_expert_ffn(self._ref, self.grid, int(pdl), _ext.stream_handle(stream)),
                    "expert_ffn")
 
 
@@ -392,6 +392,6 @@ class MoeLayerPlan:
     def decode_step(self, num_layers: int, pdl: bool = False, stream=None):
         lib = _ext.require()
         self._sync_ctx()
-        _ext.check(lib.mcb_moe_decode_step(C.byref(self.heap.ctx()), C.byref(self.meta.args), C.c_void_p(self._addr),
+        _ext.check(lib.mcb_moe_decode_step(self.heap.ctx_ref(), C.byref(self.meta.args), C.c_void_p(self._addr),
                                            len(self.ffns), int(num_layers), self.grid, int(pdl),
                                            _ext.stream_handle(stream)), "moe_decode_step")

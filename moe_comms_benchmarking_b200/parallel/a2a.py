@@ -113,15 +113,7 @@ class A2ADispatcher(Dispatcher):
             self._make_plans()
 
     def setup_batch(self, hidden, topk_idx, topk_weights):
-        n = hidden.shape[0]
-        if n > self.cap:
-            raise ValueError(f"{n} local tokens exceed the per-rank capacity {self.cap}")
-        self.local_tokens = n
-        if n:
-            self.in_hidden[:n].copy_(hidden, non_blocking=True)
-            self.in_routing[:n].copy_(topk_idx, non_blocking=True)
-            self.in_probs[:n].copy_(topk_weights, non_blocking=True)
-        self.n_local.fill_(n)
+        self._load_rows(hidden, topk_idx, topk_weights)
 
     @property
     def out(self):

@@ -8,9 +8,12 @@ inputs), ``dispatch`` / ``combine`` / ``step`` / ``decode_step`` (the timed oper
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
 from ..config import Config
+from ..ops import _ext
 
 
 class Dispatcher:
@@ -58,6 +61,42 @@ class Dispatcher:
 
     def destroy(self):
         pass
+
+    # loading one step's inputs into in_hidden / in_routing / in_probs / n_local ------------------------------------
+    def _load_rows(self, hidden, topk_idx, topk_weights, pinned: bool = False):
+        """This rank's rows for the next step, stream-ordered: one kernel launch when the three tensors have the
+        buffers' types, are contiguous and lie on this GPU (or, with ``pinned``, in pinned host memory); copies
+        otherwise (other types, strides or devices, which ``copy_`` converts)."""
+        n = hidden.shape[0]
+        if n > self.cap:
+            raise ValueError(f"{n} local tokens exceed the per-rank capacity {self.cap}")
+        self.local_tokens = n
+        bufs = (self.in_hidden, self.in_routing, self.in_probs)
+        if getattr(self, "_load_for", None) is not self.in_hidden:       # first call since build()
+            self._load_for = self.in_hidden
+            a = _ext.McbLoadArgs()
+            for t, b in enumerate(bufs):
+                a.dst[t] = b.data_ptr()
+            a.n_local = self.n_local.data_ptr()
+            self._load_args, self._load_ref = a, C.byref(a)
+            self._load_row = [(b.dtype, b.device, b.shape[1], b.shape[1] * b.element_size()) for b in bufs]
+        a = self._load_args
+        for t, s in enumerate((hidden, topk_idx, topk_weights)):
+            dtype, device, cols, row_bytes = self._load_row[t]
+            ptr = s.data_ptr()
+            if (s.dtype is not dtype or s.shape != (n, cols) or ptr & 3 or not s.is_contiguous()
+                    or not (s.is_pinned() if pinned else s.device == device)):
+                break
+            a.src[t], a.bytes[t] = ptr, n * row_bytes
+        else:
+            a.n = n
+            err = _ext.require().mcb_launch_load_batch(self._load_ref, int(self.pdl), _ext.stream_handle())
+            _ext.check(err, "load_batch")
+            return
+        if n:
+            for b, s in zip(bufs, (hidden, topk_idx, topk_weights)):
+                b[:n].copy_(s, non_blocking=True)
+        self.n_local.fill_(n)
 
     # helpers -----------------------------------------------------------------------------------
     def _validation_counts(self, global_b: int):

@@ -250,8 +250,14 @@ class SymmetricHeap:
             c.status = self.status.data_ptr()
             for p in range(self.world):
                 c.heap_peer[p] = self.peer_ptrs[p]
-            self._ctx = c
+            self._ctx, self._ctx_ref = c, C.byref(c)
         return self._ctx
+
+    def ctx_ref(self):
+        """The context as launches take it (a pointer to ``ctx()``)."""
+        if self._ctx is None:
+            self.ctx()
+        return self._ctx_ref
 
     def set_timeout(self, seconds: float):
         self.timeout_s = seconds
