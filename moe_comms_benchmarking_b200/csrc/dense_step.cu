@@ -281,52 +281,21 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
 }
 
 // ---- a world of one: the layers of a step are local copies ------------------------------------------------------
-// The byte ranges one layer copies: the gathered tensors (by parity) and the combine's rows, laid end to end as 16-byte
-// packs, so that a thread asks for all its packs of a layer, whatever tensor they belong to, before it stores any: a
-// layer costs one trip to memory instead of one per tensor.  Measured on one B200, 88 layers of hidden 1024 and top-22:
-// 54 us (244 before) with one token, 778 (1186) with 8192, where 71 MB a layer move within L2.
-struct LocalRanges {
-  const uint8_t* src[MCB_MAX_TENSORS + 1];
-  uint8_t* dst[MCB_MAX_TENSORS + 1];          // parity 0
-  uint64_t par[MCB_MAX_TENSORS + 1];          // bytes from parity 0 to parity 1
-  int words[MCB_MAX_TENSORS + 1];             // 4-byte words behind the last whole pack (0 .. 3)
-  long long end[MCB_MAX_TENSORS + 1];         // packs up to and including this range
-};
-
 template <bool FP8>
 __device__ __noinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
   __shared__ LocalRanges r;
-  constexpr int R = MCB_MAX_TENSORS + 1;
+  constexpr int R = LocalRanges::R;
   const int tid = threadIdx.x;
   if (tid == 0) {
-    long long run = 0;
-    for (int t = 0; t < R; ++t) {
-      const bool combine = t == R - 1;
-      // quantised values and scales are pushed on their own
-      const bool used = combine || (t < a.num_tensors && !(FP8 && (t == 0 || t == 3)));
-      const long long bytes = used ? (long long)n * (combine ? a.rsv_row_bytes : a.row_bytes[t]) : 0;
-      r.src[t] = combine ? c.heap_local + a.rsv_off : reinterpret_cast<const uint8_t*>(a.src[t]);
-      r.dst[t] = combine ? reinterpret_cast<uint8_t*>(a.out) : c.heap_local + a.dst_off[t];
-      r.par[t] = combine ? 0 : a.dst_par_stride[t];
-      r.words[t] = (int)(bytes & 15) >> 2;
-      run += bytes >> 4;
-      r.end[t] = run;
+    for (int t = 0; t < R - 1; ++t) {       // quantised values and scales are pushed on their own
+      const bool used = t < a.num_tensors && !(FP8 && (t == 0 || t == 3));
+      r.set(t, a.src[t], c.heap_local + a.dst_off[t], a.dst_par_stride[t], used ? (long long)n * a.row_bytes[t] : 0);
     }
+    r.set(R - 1, c.heap_local + a.rsv_off, reinterpret_cast<uint8_t*>(a.out), 0, (long long)n * a.rsv_row_bytes);
   }
   __syncthreads();
   const long long start = (long long)blockIdx.x * blockDim.x + tid, stride = (long long)nact * blockDim.x;
   const long long total = r.end[R - 1];
-  auto range_of = [&](long long i, long long& off) {
-    int t = 0;
-#pragma unroll
-    for (int k = 0; k < R - 1; ++k) t += i >= r.end[k];
-    off = (i - (t ? r.end[t - 1] : 0)) * 16;
-    return t;
-  };
-  // the words behind the last whole pack of a range: one thread each, in block 0
-  const int wt = tid >> 2, ww = tid & 3;
-  const bool word = blockIdx.x == 0 && wt < R && ww < r.words[wt < R ? wt : 0];
-  const long long wpos = word ? (r.end[wt] - (wt ? r.end[wt - 1] : 0)) * 16 + ww * 4 : 0;
 
   constexpr int S = 4;
   if (total <= stride * S) {
@@ -340,7 +309,7 @@ __device__ __noinline__ void local_layers(const McbCtx& c, const McbDenseStepArg
       const long long i = start + u * stride;
       live[u] = i < total;
       long long off = 0;
-      const int t = live[u] ? range_of(i, off) : 0;
+      const int t = live[u] ? r.find(i, off) : 0;
       src[u] = r.src[t] + off;
       dst[u] = r.dst[t] + off;
       par_off[u] = r.par[t];
@@ -348,42 +317,22 @@ __device__ __noinline__ void local_layers(const McbCtx& c, const McbDenseStepArg
     for (int l = 0; l < a.num_layers; ++l) {
       const uint32_t par = (layer_base + (uint32_t)l) & 1u;
       uint4 v[S];
-      uint32_t w = 0;
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) v[u] = ld_v4_stream(src[u]);
-      if (word) w = ld_b32(r.src[wt] + wpos);
+      const uint32_t w = r.load_word();
       if (FP8) fp8_push(c, a, par, 0, 0, n, start, stride);
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) st_v4(dst[u] + (par ? par_off[u] : 0), v[u]);
-      if (word) st_b32(r.dst[wt] + (par ? r.par[wt] : 0) + wpos, w);
+      r.store_word(par, w);
     }
     return;
   }
-  constexpr int U = 8;
   for (int l = 0; l < a.num_layers; ++l) {
     const uint32_t par = (layer_base + (uint32_t)l) & 1u;
     if (FP8) fp8_push(c, a, par, 0, 0, n, start, stride);
-    if (word) st_b32(r.dst[wt] + (par ? r.par[wt] : 0) + wpos, ld_b32(r.src[wt] + wpos));
-    for (long long i0 = start; i0 < total; i0 += stride * U) {
-      uint4 v[U];
-      uint8_t* dst[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const long long i = i0 + u * stride;
-        dst[u] = nullptr;
-        if (i < total) {
-          long long off;
-          const int t = range_of(i, off);
-          v[u] = ld_v4_stream(r.src[t] + off);
-          dst[u] = r.dst[t] + (par ? r.par[t] : 0) + off;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (dst[u]) st_v4(dst[u], v[u]);
-    }
+    copy_ranges(r, par, start, stride);
   }
 }
 

@@ -3,12 +3,13 @@
 //
 //   dispatch    every CTA pushes its share of the local tokens to all ranks (multimem.st + cross-GPU
 //               barrier, or flagged packets for small steps)                          mcb_dense.cuh
-//   routing     histogram -> offsets -> pair lists for this rank's experts               mcb_route.cuh
+//   routing     counts -> offsets -> pair lists for this rank's experts                  mcb_route.cuh
 //   experts     gate/up blocks, then down blocks, one persistent weight stream            mcb_ffn.cuh
 //   combine     per-token pre-sum of the local expert outputs into the symmetric buffer, block-matched
 //               cross-GPU barrier, multimem.ld_reduce of the rows this rank owns       mcb_combine.cuh
 //
-// separated by grid-wide barriers (the launch is cooperative: all CTAs are resident).  The reference
+// separated by grid-wide barriers (the launch is cooperative: all CTAs are resident), except that every CTA works out
+// the experts' offsets itself and starts its weight stream before the others have placed their pairs.  The reference
 // stops at the identity expert (bench_nvls.py:109-121); its dispatch and combine are the first and the
 // last phase here.  EMU = true runs several ranks inside one launch (gridDim.y = world, each y-slice
 // with its own argument block in device memory), which is how the cross-rank protocol of this kernel
@@ -42,25 +43,54 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* ea
   const McbCtx& c = p.ctx;
   uint32_t ll_launch = 0;
   const bool tracing = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
-  if (tracing) p.trace[0] = globaltimer_ns();
+  auto stamp = [&](int i) { if (tracing) p.trace[i] = globaltimer_ns(); };
+  // Grid-wide barriers count up a word that is back at zero whenever a launch has ended (its last block resets it).
+  uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 1);
+  uint32_t target = 0;
+  auto meet = [&] { grid_sync(c, arrivals, target += gridDim.x); };
+  stamp(0);
   ffn_setup(p.ffn);
   agv_device<MCB_SITE_FC1_FUSED>(c, p.agv, ll_launch);      // waits for the previous kernel first
-  if (tracing) p.trace[1] = globaltimer_ns();
-  // The arrival counter is back at zero whenever a launch has ended (its last block resets it).
-  uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 1);
-  grid_sync(c, arrivals, gridDim.x);
-  if (tracing) p.trace[2] = globaltimer_ns();
-  route_device(p.route, reinterpret_cast<int*>(FfnSmem().pipe));     // the pipeline is not in use yet
-  if (tracing) p.trace[3] = globaltimer_ns();
-  grid_sync(c, arrivals, 2u * gridDim.x);
-  if (tracing) p.trace[4] = globaltimer_ns();
-  ffn_device(p.ffn);
+  stamp(1);
+  // Routing needs the gathered ids of all tokens; a world of one has them in its own inputs and need not wait for the copy.
+  const bool alone = c.world == 1;
+  const int64_t* ids = alone ? reinterpret_cast<const int64_t*>(p.agv.src[1]) : p.route.topk_idx;
+  const float* probs = alone ? reinterpret_cast<const float*>(p.agv.src[2]) : p.route.topk_w;
+  if (!alone) meet();
+  stamp(2);
+  const FfnSmem sm;
+  RouteSmem m(reinterpret_cast<int*>(sm.pipe));              // the pipeline is not in use yet
+  m.off = sm.off;
+  const RouteShare share = route_share(p.route, (int)blockIdx.x, (int)gridDim.x);
+  if (route_counts_all(share)) {
+    route_count(p.route, ids, m, 0, share.entries, share.lo);
+  } else {
+    route_count(p.route, ids, m, share.lo, share.hi, 0);
+    route_publish(p.route, m);
+    meet();
+    route_collect(p.route, m);
+  }
+  const int max_rows = route_offsets(p.route, m, blockIdx.x == 0);
+  route_place(p.route, ids, probs, m, share);
+  // This block's pair rows (and gathered rows, when alone) are there.  Nobody waits here: the weight stream starts at
+  // once, the roles that read rows or lists wait for all blocks.
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrivals, 1u);
+  }
+  target += gridDim.x;
+  stamp(3);
+  stamp(4);
+  ffn_run(p.ffn, max_rows, FfnReady{arrivals, (int)target});
   ffn_teardown();
-  if (tracing) p.trace[5] = globaltimer_ns();
-  grid_sync(c, arrivals, 3u * gridDim.x);                   // every y row is written before any is summed
-  if (tracing) p.trace[6] = globaltimer_ns();
+  stamp(5);
+  meet();                                                   // every y row is written before any is summed
+  stamp(6);
+  if (blockIdx.x == gridDim.x - 1)                          // every block has read the counters of the routing
+    for (int e = threadIdx.x; e < p.route.num_local_experts; e += blockDim.x) p.route.expert_count[e] = 0;
   combine_body(c, p.cmb, ll_launch);      // partial sums alternate between two buffers, layer by layer
-  if (tracing) p.trace[7] = globaltimer_ns();
+  stamp(7);
   launch_end(c, MCB_SITE_FC1_FUSED, ll_launch, arrivals);
 }
 

@@ -254,7 +254,7 @@ dispatch_route_fc1_kernel(const __grid_constant__ CUtensorMap w_map, const __gri
   // The arrival counter is back at zero whenever a launch has ended (its last block resets it).
   uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 1);
   grid_sync(c, arrivals, gridDim.x);
-  __shared__ int s_route[2 * kMaxLocalExperts];
+  __shared__ int s_route[kRouteSmemWords];
   route_device(r, s_route);
   grid_sync(c, arrivals, 2u * gridDim.x);
   gemm_device<MCB_GEMM_FC1>(w_map, a);

@@ -70,6 +70,78 @@ __device__ __forceinline__ void broadcast_flat(const McbCtx& c, const uint8_t* s
 }
 
 // ------------------------------------------------------------------------------------------
+// A world of one: dispatch and combine are local copies.  The byte ranges to copy (in shared memory) are laid end to end
+// as 16-byte packs, so that a thread asks for all its packs, whatever tensor they belong to, before it stores any: one
+// trip to memory instead of one per tensor.  Measured on one B200, 88 layers of hidden 1024 and top-22 in one launch:
+// 54 us (244 before) with one token, 778 (1186) with 8192, where 71 MB a layer move within L2.
+// ------------------------------------------------------------------------------------------
+struct LocalRanges {
+  static constexpr int R = MCB_MAX_TENSORS + 1;
+  const uint8_t* src[R];
+  uint8_t* dst[R];          // parity 0
+  uint64_t par[R];          // bytes from parity 0 to parity 1
+  int words[R];             // 4-byte words behind the last whole pack (0 .. 3)
+  long long end[R];         // packs up to and including this range
+  // one thread, ranges in order
+  __device__ __forceinline__ void set(int t, const void* s, uint8_t* d, uint64_t par_stride, long long bytes) {
+    src[t] = reinterpret_cast<const uint8_t*>(s);
+    dst[t] = d;
+    par[t] = par_stride;
+    words[t] = (int)(bytes & 15) >> 2;
+    end[t] = (t ? end[t - 1] : 0) + (bytes >> 4);
+  }
+  // range of pack i and its byte offset in there
+  __device__ __forceinline__ int find(long long i, long long& off) const {
+    int t = 0;
+#pragma unroll
+    for (int k = 0; k < R - 1; ++k) t += i >= end[k];
+    off = (i - (t ? end[t - 1] : 0)) * 16;
+    return t;
+  }
+  // The words behind the last whole pack of a range: one thread each, in block 0.
+  __device__ __forceinline__ bool word_of(int& t, long long& off) const {
+    t = threadIdx.x >> 2;
+    const int w = threadIdx.x & 3;
+    if (blockIdx.x != 0 || t >= R || w >= words[t]) return false;
+    off = (end[t] - (t ? end[t - 1] : 0)) * 16 + w * 4;
+    return true;
+  }
+  __device__ __forceinline__ uint32_t load_word() const {
+    int t; long long off;
+    return word_of(t, off) ? ld_b32(src[t] + off) : 0u;
+  }
+  __device__ __forceinline__ void store_word(uint32_t parity, uint32_t v) const {
+    int t; long long off;
+    if (word_of(t, off)) st_b32(dst[t] + (parity ? par[t] : 0) + off, v);
+  }
+};
+
+__device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parity, long long start, long long stride) {
+  constexpr int U = 8;
+  const long long total = r.end[LocalRanges::R - 1];
+  const uint32_t word = r.load_word();
+  for (long long i0 = start; i0 < total; i0 += stride * U) {
+    uint4 v[U];
+    uint8_t* dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const long long i = i0 + u * stride;
+      dst[u] = nullptr;
+      if (i < total) {
+        long long off;
+        const int t = r.find(i, off);
+        v[u] = ld_v4_stream(r.src[t] + off);
+        dst[u] = r.dst[t] + (parity ? r.par[t] : 0) + off;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (dst[u]) st_v4(dst[u], v[u]);
+  }
+  r.store_word(parity, word);
+}
+
+// ------------------------------------------------------------------------------------------
 // Flat cross-rank reduction: out[i] = sum over ranks of heap[base + 16 * i], 16 bytes at a time.
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ void acc_bf16x8(float (&acc)[8], uint4 v) {
@@ -331,6 +403,18 @@ __device__ __forceinline__ void agv_device(const McbCtx& c, const McbAgvArgs& a,
   }
   const long long start = (long long)bid * blockDim.x + threadIdx.x;
   const long long stride = (long long)nact * blockDim.x;
+  if (c.world == 1) {        // no peer to meet either
+    __shared__ LocalRanges r;
+    if (threadIdx.x == 0)
+      for (int t = 0; t < LocalRanges::R; ++t) {
+        const bool used = t < a.num_tensors;
+        r.set(t, used ? a.src[t] : nullptr, used ? c.heap_local + a.dst_off[t] + (uint64_t)offset * a.row_bytes[t] : nullptr, 0,
+              used ? (long long)n * a.row_bytes[t] : 0);
+      }
+    __syncthreads();
+    copy_ranges(r, 0, start, stride);
+    return;
+  }
 #pragma unroll
   for (int t = 0; t < MCB_MAX_TENSORS; ++t) {
     if (t >= a.num_tensors) break;

@@ -22,7 +22,7 @@
 //     popular expert's chunks spread over the chip;
 //   * both projections run in one persistent stream.  While the activations of all experts fit in L2 the gate/up
 //     units of every expert come first, then the down units; above that a down unit follows its gate/up
-//     units at a distance of two rounds of the grid, while its activations are still in L2.  A down
+//     units at a distance of three rounds of the grid, while its activations are still in L2.  A down
 //     unit waits for a counter of its expert's finished gate/up units; units are taken in list order, so the
 //     wait cannot deadlock;
 //   * the gate/up matrix is stored interleaved (row 2i = gate row i, row 2i + 1 = up row i): the two values
@@ -282,8 +282,15 @@ __device__ __forceinline__ void ffn_permute_rows(const McbFfnArgs& a, int pairs,
 // a.w1 is the packed interleaved gate/up matrix (E * 2I rows, H columns), a.w2 the packed down matrix (E * H rows,
 // I columns): tile (128-row block v, column block kb) of a matrix with KB column blocks is the 16 KB at byte
 // (v * KB + kb) * 16384.
+// What the token rows and pair lists still have to wait for: a counter that other CTAs of this launch raise (null:
+// nothing).  The weight stream does not wait for it.
+struct FfnReady {
+  const uint32_t* word;
+  int want;
+};
+
 template <int NSUB>
-__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& plan, const int n_slot) {
+__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
   const FfnSmem sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();           // 0 = the CTA that issues the MMAs of the pair
@@ -320,6 +327,10 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
     return FfnUnit{v.x, v.y, (int)v.z, (int)v.w};
   };
   fill(pair);
+  if (ready.word && warp >= 2) {
+    if (lane == 0) ffn_wait_count(reinterpret_cast<const int*>(ready.word), ready.want, ab, 19, 0);
+    __syncwarp();
+  }
   if (!gather && warp >= 2) {
     // every warp but the weight producer and the MMA issuer takes a share of the copy into pair order
     ffn_permute_rows(a, plan.off[a.num_local_experts], (int)blockIdx.x + (warp - 2) * (int)gridDim.x,
@@ -565,12 +576,11 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
 }
 
 // Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
-// ffn_teardown, once the pair lists are visible; dynamic shared memory of at least kFfnSmemBytes.
-__device__ __forceinline__ void ffn_device(const McbFfnArgs& a) {
+// ffn_teardown, with the experts' offsets in the shared memory of FfnSmem::off (visible to all threads) and the largest
+// number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.
+__device__ __forceinline__ void ffn_run(const McbFfnArgs& a, int max_rows, const FfnReady ready) {
   const FfnSmem sm;
   const int E = a.num_local_experts;
-  for (int e = threadIdx.x; e <= E; e += blockDim.x) sm.off[e] = a.expert_offset[e];
-  int max_rows = *a.max_rows;
   if (max_rows < 1) max_rows = 1;
   fence_proxy_async_smem();                // the pipeline's memory may have been in ordinary use until here
   __syncthreads();
@@ -579,14 +589,21 @@ __device__ __forceinline__ void ffn_device(const McbFfnArgs& a) {
   plan.n1 = 2 * a.intermediate / kFfnRowsM; plan.n2 = a.hidden / kFfnRowsM;
   plan.active = ffn_slots(sm.off, E, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi));
   plan.lag = plan.active;
-  if ((long long)sm.off[E] * a.intermediate * 2 > kFfnActL2Bytes) {      // two rounds of the grid, in slots of average size
-    const int lag = (int)((long long)gridDim.x * plan.active / plan.total()) + 2;
+  if ((long long)sm.off[E] * a.intermediate * 2 > kFfnActL2Bytes) {      // three rounds of the grid, in slots of average size
+    const int lag = (int)((long long)gridDim.x * 3 / 2 * plan.active / plan.total()) + 2;
     if (lag < plan.lag) plan.lag = lag;
   }
   // Token tile of this launch: the largest expert, rounded up to 32, at most kFfnMaxN per chunk.
   const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 31) & ~31);
-  if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, plan, n_slot);
-  else ffn_roles<1>(a, plan, n_slot);
+  if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, plan, n_slot, ready);
+  else ffn_roles<1>(a, plan, n_slot, ready);
+}
+
+// The same after a routing of its own launch, whose results are in global memory.
+__device__ __forceinline__ void ffn_device(const McbFfnArgs& a) {
+  const FfnSmem sm;
+  for (int e = threadIdx.x; e <= a.num_local_experts; e += blockDim.x) sm.off[e] = a.expert_offset[e];
+  ffn_run(a, *a.max_rows, FfnReady{nullptr, 0});
 }
 
 }  // namespace mcb

@@ -1,6 +1,17 @@
-// Routing of the gathered tokens to this rank's experts as a device function (histogram ->
-// offsets -> pair lists -> row-tile table), shared by the stand-alone routing kernel and the
-// fused dispatch + routing + FC1 kernel.
+// Routing of the gathered tokens to this rank's experts as device functions (histogram -> offsets -> pair lists ->
+// row-tile table), shared by the stand-alone routing kernel, the fused dispatch + routing + FC1 kernel and the
+// whole-layer kernel.
+//
+// The (token, k) entries are shared out over the blocks in order.  A block needs two things beyond its own entries: how
+// many entries each expert has in all (the offsets follow from these) and where its own entries of an expert begin.
+//   few entries   every block counts ALL entries itself, and those before its share once more: no block waits for
+//                 another, and every block has the offsets in shared memory at once;
+//   many entries  a block counts its share and adds it to a counter per expert, which returns where its entries
+//                 begin; after a barrier over the blocks everybody reads the counters.
+// Either way every block then works out the offsets for itself (a block-wide scan over the experts) and places its own
+// entries with cursors in shared memory.  Against counters handed over through one last block that scanned alone and one
+// global atomic per entry: 28 -> 10 us inside the layer kernel at 90112 entries and 512 experts, and with one token the
+// experts' weights start 8 us earlier.
 #pragma once
 #include "mcb_barrier.cuh"
 #include "mcb_gemm.h"
@@ -9,208 +20,155 @@ namespace mcb {
 
 constexpr int kRouteThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
-constexpr int kSingleBlockPerThread = 20;    // (token, k) entries per thread up to which ONE block routes alone
+// Shared memory of a routing block: counts, own begins (later cursors), offsets, scan scratch.
+constexpr int kRouteSmemWords = 3 * kMaxLocalExperts + 1 + 3 * 32;
+// Entries per thread up to which every block counts all of them.
+constexpr int kRouteAllPerThread = 16;
 
-__device__ __forceinline__ bool spin_until_ge(const volatile int* p, int target, uint64_t timeout_ns) {
-  if (*p - target >= 0) return true;
-  uint64_t t0 = globaltimer_ns();
-  for (;;) {
-    for (int i = 0; i < 64; ++i)
-      if (*p - target >= 0) return true;
-    if (globaltimer_ns() - t0 > timeout_ns) return false;
-  }
-}
+struct RouteSmem {
+  int *cnt, *begin, *off, *scan;
+  __device__ __forceinline__ explicit RouteSmem(int* base)
+      : cnt(base), begin(base + kMaxLocalExperts), off(base + 2 * kMaxLocalExperts), scan(base + 3 * kMaxLocalExperts + 1) {}
+};
 
-// Exclusive prefix of the per-expert pair counts s_cnt[0..E) into a.expert_offset[0..E], the
-// 128-row tile table of the tokens-as-rows GEMMs, the largest count, and the per-expert "gate/up
-// blocks done" counters of the fused FFN back at zero.  One warp: every lane owns a contiguous
-// run of experts, the runs are joined with a shuffle scan (E <= 1024 means at most 32 experts per
-// lane, instead of a serial walk over all of them on one thread).  Call from the 32 threads of
-// ONE warp; s_cnt must be visible to them.  Returns the total in every lane.
-__device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const int* s_cnt, int* s_off, int E) {
-  const int lane = threadIdx.x & 31;
-  const int per = (E + 31) / 32;
-  const int e0 = lane * per, e1 = e0 + per < E ? e0 + per : E;
-  int rows = 0, tiles = 0, mx = 0;
-  for (int e = e0; e < e1; ++e) {
-    const int c = s_cnt[e];
-    rows += c;
-    tiles += (c + 127) >> 7;
-    mx = c > mx ? c : mx;
-  }
-  int row_pre = rows, tile_pre = tiles;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int r = __shfl_up_sync(0xffffffffu, row_pre, o), t = __shfl_up_sync(0xffffffffu, tile_pre, o);
-    if (lane >= o) { row_pre += r; tile_pre += t; }
-  }
-  const int total = __shfl_sync(0xffffffffu, row_pre, 31), total_tiles = __shfl_sync(0xffffffffu, tile_pre, 31);
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  int run = row_pre - rows, tile = tile_pre - tiles;
-  for (int e = e0; e < e1; ++e) {
-    const int c = s_cnt[e];
-    if (s_off) s_off[e] = run;
-    a.expert_offset[e] = run;
-    if (a.ffn_done) a.ffn_done[e] = 0;
-    for (int r0 = 0; r0 < c; r0 += 128, ++tile) {
-      if (tile < a.max_tiles) {
-        a.tile_expert[tile] = e;
-        a.tile_row0[tile] = run + r0;
-        a.tile_rows[tile] = c - r0 < 128 ? c - r0 : 128;
-      }
-    }
-    run += c;
-  }
-  if (lane == 0) {
-    a.expert_offset[E] = total;
-    if (a.max_rows) *a.max_rows = mx;
-    if (total_tiles > a.max_tiles || total > a.max_pairs) {
-      if (a.status && atomicCAS(a.status, 0u, (uint32_t)MCB_ERR_CAPACITY) == 0u) {
-        a.status[1] = 100; a.status[2] = (uint32_t)total_tiles; a.status[3] = (uint32_t)total;
-      }
-    }
-    *a.num_m_tiles = total_tiles < a.max_tiles ? total_tiles : a.max_tiles;
-  }
-  return total;
-}
-
-// One launch, two phases separated by a "last block computes the offsets" hand-over; blocks of
-// the same launch wait for it on a local counter, so the grid must be co-resident (<= #SMs).
-// Call from all threads of every block of the grid; `s_hist` is shared memory for 2 * kMaxLocalExperts words.
-__device__ __forceinline__ void route_device(const McbRouteArgs& a, int* s_hist) {
-  int* s_cursor = s_hist + kMaxLocalExperts;
-  __shared__ int s_flag;
-  const int tid = threadIdx.x;
-  const int E = a.num_local_experts;
+// This block's share of the entries.
+struct RouteShare {
+  long long entries, lo, hi;
+};
+__device__ __forceinline__ RouteShare route_share(const McbRouteArgs& a, int block, int blocks) {
   int T = *a.num_tokens;
   if (T < 0) T = 0;
   if (T > a.max_tokens) T = a.max_tokens;
-  const int ready_base = *reinterpret_cast<volatile int*>(&a.sync[2]);   // stable until this launch's hand-over
-  const long long entries = (long long)T * a.topk;
-  if (entries <= (long long)kSingleBlockPerThread * blockDim.x) {
-    // Small step: block 0 does everything in shared memory (no hand-over between blocks, no
-    // global atomics), the other blocks leave at once.  Two passes of dependent loads, four entries
-    // per thread and round.  On a 320-thread block: 3.7 us for 352 entries, 7.6 us for 2816 (the
-    // multi-block form with its hand-over takes 11.7 us there), 21 us for 11264 (multi-block: about 13).
-    if (blockIdx.x != 0) return;
-    for (int e = tid; e < E; e += blockDim.x) { s_hist[e] = 0; s_cursor[e] = 0; }
-    __syncthreads();
-    for (int i0 = tid; i0 < (int)entries; i0 += blockDim.x * 4) {
-      long long e[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
-        e[u] = i < (int)entries ? a.topk_idx[i] - a.expert_begin : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (e[u] >= 0 && e[u] < E) atomicAdd(&s_hist[(int)e[u]], 1);
-    }
-    __syncthreads();
-    if (tid < 32) route_offsets(a, s_hist, s_cursor, E);     // offsets land in s_cursor ...
-    __syncthreads();
-    for (int e = tid; e < E; e += blockDim.x) { s_hist[e] = s_cursor[e]; s_cursor[e] = 0; }   // ... and move over
-    __syncthreads();
-    for (int i0 = tid; i0 < (int)entries; i0 += blockDim.x * 4) {
-      long long e[4];
-      float w[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
-        const bool in = i < (int)entries;
-        e[u] = in ? a.topk_idx[i] - a.expert_begin : -1;
-        w[u] = in && a.topk_w ? a.topk_w[i] : 1.0f;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = i0 + u * blockDim.x;
-        if (i >= (int)entries) break;
-        int pos = -1;
-        if (e[u] >= 0 && e[u] < E) {
-          pos = s_hist[(int)e[u]] + atomicAdd(&s_cursor[(int)e[u]], 1);
-          if (pos < a.max_pairs) {
-            a.pair_token[pos] = i / a.topk;
-            a.pair_prob[pos] = w[u];
-          } else {
-            pos = -1;
-          }
-        }
-        a.pair_pos[i] = pos;
-      }
-    }
-    return;
-  }
-  const long long per_block = (entries + gridDim.x - 1) / gridDim.x;
-  const long long lo = per_block * blockIdx.x;
-  const long long hi = lo + per_block < entries ? lo + per_block : entries;
+  RouteShare s;
+  s.entries = (long long)T * a.topk;
+  const long long per = (s.entries + blocks - 1) / blocks;
+  s.lo = per * block < s.entries ? per * block : s.entries;
+  s.hi = s.lo + per < s.entries ? s.lo + per : s.entries;
+  return s;
+}
+__device__ __forceinline__ bool route_counts_all(const RouteShare& s) {
+  return s.entries <= (long long)kRouteAllPerThread * blockDim.x;
+}
 
-  // ---- phase 1: histogram of the entries owned by this block ----
-  for (int e = tid; e < E; e += blockDim.x) s_hist[e] = 0;
+// Counts the entries [lo, hi) into m.cnt, those before `split` into m.begin too.  All threads of the block.
+__device__ __forceinline__ void route_count(const McbRouteArgs& a, const int64_t* topk_idx, const RouteSmem& m, long long lo,
+                                            long long hi, long long split) {
+  const int tid = threadIdx.x, E = a.num_local_experts;
+  for (int e = tid; e < E; e += blockDim.x) { m.cnt[e] = 0; m.begin[e] = 0; }
   __syncthreads();
   for (long long i0 = lo + tid; i0 < hi; i0 += blockDim.x * 4) {
     long long e[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * blockDim.x;
-      e[u] = i < hi ? a.topk_idx[i] - a.expert_begin : -1;
+      e[u] = i < hi ? topk_idx[i] - a.expert_begin : -1;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (e[u] >= 0 && e[u] < E) atomicAdd(&s_hist[(int)e[u]], 1);
+      if (e[u] >= 0 && e[u] < E) {
+        atomicAdd(&m.cnt[(int)e[u]], 1);
+        if (i0 + u * blockDim.x < split) atomicAdd(&m.begin[(int)e[u]], 1);
+      }
   }
   __syncthreads();
-  for (int e = tid; e < E; e += blockDim.x)
-    if (s_hist[e]) atomicAdd(&a.expert_count[e], s_hist[e]);
+}
+
+// Many entries, before the barrier: this block's counts into the counters; m.begin = where its entries begin.
+__device__ __forceinline__ void route_publish(const McbRouteArgs& a, const RouteSmem& m) {
+  for (int e = threadIdx.x; e < a.num_local_experts; e += blockDim.x)
+    m.begin[e] = m.cnt[e] ? atomicAdd(&a.expert_count[e], m.cnt[e]) : 0;
+}
+// ... and after it: the counts of all blocks.
+__device__ __forceinline__ void route_collect(const McbRouteArgs& a, const RouteSmem& m) {
+  for (int e = threadIdx.x; e < a.num_local_experts; e += blockDim.x)
+    m.cnt[e] = *reinterpret_cast<volatile int*>(&a.expert_count[e]);
   __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_flag = (atomicAdd(&a.sync[0], 1) == (int)gridDim.x - 1);
-    __threadfence();
+}
+
+// Offsets of the experts (exclusive prefix of m.cnt) into m.off[0 .. E] by a block-wide scan; the block that `writes` puts
+// them, the 128-row tile table of the tokens-as-rows GEMMs, the largest count and the zeroed "gate/up done" counters of
+// the fused FFN into global memory.  Returns the largest count in every thread.  All threads of the block.
+__device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteSmem& m, bool writes) {
+  const int E = a.num_local_experts, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
+  const int per = (E + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int e0 = threadIdx.x * per, e1 = e0 + per < E ? e0 + per : E;
+  int rows = 0, tiles = 0, mx = 0;
+  for (int e = e0; e < e1; ++e) {
+    const int c = m.cnt[e];
+    rows += c;
+    tiles += (c + 127) >> 7;
+    mx = c > mx ? c : mx;
   }
+  int r_inc = rows, t_inc = tiles;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int r = __shfl_up_sync(0xffffffffu, r_inc, o), t = __shfl_up_sync(0xffffffffu, t_inc, o);
+    if (lane >= o) { r_inc += r; t_inc += t; }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 31) { m.scan[warp] = r_inc; m.scan[32 + warp] = t_inc; m.scan[64 + warp] = mx; }
   __syncthreads();
-  if (s_flag) {
-    // Last block: exclusive prefix over experts, row-tile table, then release the others.
-    for (int e = tid; e < E; e += blockDim.x) s_hist[e] = *reinterpret_cast<volatile int*>(&a.expert_count[e]);
-    __syncthreads();
-    if (tid < 32) {
-      route_offsets(a, s_hist, nullptr, E);
-      __threadfence();                   // every lane's table entries before the hand-over below
-      __syncwarp();
-      if (tid == 0) {
-        a.sync[0] = 0;
-        __threadfence();
-        atomicAdd(&a.sync[2], 1);
+  int run = r_inc - rows, tile = t_inc - tiles, total = 0, total_tiles = 0;
+  for (int w = 0; w < nw; ++w) {
+    if (w < warp) { run += m.scan[w]; tile += m.scan[32 + w]; }
+    total += m.scan[w];
+    total_tiles += m.scan[32 + w];
+    mx = m.scan[64 + w] > mx ? m.scan[64 + w] : mx;
+  }
+  for (int e = e0; e < e1; ++e) {
+    const int c = m.cnt[e];
+    m.off[e] = run;
+    if (writes) {
+      a.expert_offset[e] = run;
+      if (a.ffn_done) a.ffn_done[e] = 0;
+      for (int r0 = 0; r0 < c; r0 += 128, ++tile) {
+        if (tile < a.max_tiles) {
+          a.tile_expert[tile] = e;
+          a.tile_row0[tile] = run + r0;
+          a.tile_rows[tile] = c - r0 < 128 ? c - r0 : 128;
+        }
       }
     }
+    run += c;
   }
-  if (tid == 0) {
-    if (!spin_until_ge(reinterpret_cast<volatile int*>(&a.sync[2]), ready_base + 1, a.timeout_ns)) {
-      if (a.status && atomicCAS(a.status, 0u, (uint32_t)MCB_ERR_TIMEOUT) == 0u) { a.status[1] = 101; a.status[2] = blockIdx.x; }
+  if (threadIdx.x == 0) {
+    m.off[E] = total;
+    if (writes) {
+      a.expert_offset[E] = total;
+      if (a.max_rows) *a.max_rows = mx;
+      if (total_tiles > a.max_tiles || total > a.max_pairs) {
+        if (a.status && atomicCAS(a.status, 0u, (uint32_t)MCB_ERR_CAPACITY) == 0u) {
+          a.status[1] = 100; a.status[2] = (uint32_t)total_tiles; a.status[3] = (uint32_t)total;
+        }
+      }
+      *a.num_m_tiles = total_tiles < a.max_tiles ? total_tiles : a.max_tiles;
     }
-    __threadfence();
   }
   __syncthreads();
+  return mx;
+}
 
-  // ---- phase 2: place every local (token, k) entry into its expert's segment ----
-  for (int e = tid; e < E; e += blockDim.x) s_hist[e] = *reinterpret_cast<volatile int*>(&a.expert_offset[e]);
-  __syncthreads();
-  for (long long i0 = lo + tid; i0 < hi; i0 += blockDim.x * 4) {
+// Places this block's entries: pair row = offset of the expert + where the block's entries of it begin + a cursor (m.begin
+// is used up).  All threads of the block.
+__device__ __forceinline__ void route_place(const McbRouteArgs& a, const int64_t* topk_idx, const float* topk_w,
+                                            const RouteSmem& m, const RouteShare& s) {
+  const int E = a.num_local_experts;
+  for (long long i0 = s.lo + threadIdx.x; i0 < s.hi; i0 += blockDim.x * 4) {
     long long e[4];
     float w[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * blockDim.x;
-      e[u] = i < hi ? a.topk_idx[i] - a.expert_begin : -1;
-      w[u] = i < hi && a.topk_w ? a.topk_w[i] : 1.0f;
+      e[u] = i < s.hi ? topk_idx[i] - a.expert_begin : -1;
+      w[u] = i < s.hi && topk_w ? topk_w[i] : 1.0f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const long long i = i0 + u * blockDim.x;
-      if (i >= hi) break;
+      if (i >= s.hi) break;
       int pos = -1;
       if (e[u] >= 0 && e[u] < E) {
-        pos = s_hist[(int)e[u]] + atomicAdd(&a.expert_cursor[(int)e[u]], 1);
+        pos = m.off[(int)e[u]] + atomicAdd(&m.begin[(int)e[u]], 1);
         if (pos < a.max_pairs) {
           a.pair_token[pos] = (int)(i / a.topk);
           a.pair_prob[pos] = w[u];
@@ -221,16 +179,55 @@ __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* s_hist)
       a.pair_pos[i] = pos;
     }
   }
+}
+
+// The whole routing by the blocks of a launch that has nothing else to share a barrier with: few entries by block 0
+// alone, many by all blocks, which wait for one another on a counter that only grows (the grid must be co-resident).
+// Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.
+__device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
+  const RouteSmem m(smem);
+  const int tid = threadIdx.x;
+  RouteShare s = route_share(a, 0, 1);
+  if (route_counts_all(s)) {
+    if (blockIdx.x != 0) return;
+    route_count(a, a.topk_idx, m, 0, s.entries, 0);
+    route_offsets(a, m, true);
+    route_place(a, a.topk_idx, a.topk_w, m, s);
+    return;
+  }
+  s = route_share(a, (int)blockIdx.x, (int)gridDim.x);
+  volatile int* arrived = a.sync;                            // back at zero when the last block has left
+  route_count(a, a.topk_idx, m, s.lo, s.hi, 0);
+  route_publish(a, m);
   __syncthreads();
   if (tid == 0) {
     __threadfence();
-    s_flag = (atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1);
+    atomicAdd(&a.sync[0], 1);
+    uint64_t t0 = 0;
+    for (uint32_t i = 0; *arrived < (int)gridDim.x; ++i) {
+      if ((i & 63u) != 63u) continue;
+      if (t0 == 0) t0 = globaltimer_ns();
+      if (globaltimer_ns() - t0 > a.timeout_ns) {
+        if (a.status && atomicCAS(a.status, 0u, (uint32_t)MCB_ERR_TIMEOUT) == 0u) { a.status[1] = 101; a.status[2] = blockIdx.x; }
+        break;
+      }
+    }
+    __threadfence();
   }
   __syncthreads();
-  if (s_flag) {
-    // Last block out: scratch back to zero for the next launch.
-    for (int e = tid; e < E; e += blockDim.x) { a.expert_count[e] = 0; a.expert_cursor[e] = 0; }
-    if (tid == 0) a.sync[1] = 0;
+  route_collect(a, m);
+  route_offsets(a, m, blockIdx.x == 0);
+  route_place(a, a.topk_idx, a.topk_w, m, s);
+  __shared__ int s_last;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (s_last) {      // last block out: the counters back to zero for the next launch
+    for (int e = tid; e < a.num_local_experts; e += blockDim.x) a.expert_count[e] = 0;
+    if (tid == 0) { a.sync[0] = 0; a.sync[1] = 0; }
   }
 }
 

@@ -19,7 +19,7 @@ namespace mcb {
 __global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __grid_constant__ McbRouteArgs a) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ int s_route[2 * kMaxLocalExperts];
+  __shared__ int s_route[kRouteSmemWords];
   route_device(a, s_route);
 }
 

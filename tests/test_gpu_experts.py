@@ -334,3 +334,35 @@ def test_expert_ffn_chunk_edges(world1, rows, H, I, grid):
             assert float((act[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} gate/up"
             want = act[sl].float() @ wd[e].t() * route.pair_prob[sl].unsqueeze(1)
             assert float((y[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} down"
+
+
+@pytest.mark.parametrize("W,B", [(2, 900), (2, 2200), (1, 1), (1, 2100)])
+def test_moe_layer_kernel_routing_and_combine_branches(lib, W, B):
+    """The whole-layer kernel where its routing and combine change form: four packs per lane in the combine (900 tokens),
+    counts shared through global counters instead of taken by every block (from about 2050 tokens of top-3), with a
+    peer and alone (ids read from the inputs, sums written straight to the output)."""
+    test_moe_layer_kernel_emulated_ranks(lib, W, B, 0)
+
+
+@pytest.mark.parametrize("T,K,H", [(1, 22, 1024), (3, 40, 264), (500, 5, 1032), (40, 8, 7168), (2600, 3, 256)])
+def test_expert_combine_slices(world1, T, K, H):
+    """One, two and four packs per lane, a ragged last slice, more than 32 routing slots, entries of other ranks (-1)."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertCombinePlan, RouteBuffers
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    heap = SymmetricHeap(world1, T * H * 2 + (1 << 20), DEV)
+    partial = heap.alloc("partial", [T, H], torch.bfloat16)
+    route = RouteBuffers(T, K, K, DEV)
+    y = torch.randn(route.max_pairs, H, device=DEV, generator=g).to(torch.bfloat16)
+    pos = torch.randint(0, route.max_pairs, (T, K), device=DEV, generator=g, dtype=torch.int32)
+    pos[torch.rand(T, K, device=DEV, generator=g) < 0.4] = -1
+    route.pair_pos.copy_(pos)
+    out = torch.full((T, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+    n = torch.tensor([T], dtype=torch.int32, device=DEV)
+    meta = torch.tensor([T, 0, T, 1], dtype=torch.int32, device=DEV)
+    ExpertCombinePlan(heap, y, route, partial, out, n, meta, T).launch()
+    torch.cuda.synchronize()
+    heap.check_status()
+    live = (pos >= 0).unsqueeze(-1)
+    ref = torch.stack([(y[pos[t].clamp(min=0).long()].float() * live[t]).sum(0) for t in range(T)])
+    assert torch.allclose(out.float(), ref, rtol=2 ** -8, atol=1e-5)      # fp32 sums in another order, rounded once
