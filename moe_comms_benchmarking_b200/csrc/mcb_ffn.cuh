@@ -27,6 +27,11 @@
 //     wait cannot deadlock;
 //   * the gate/up matrix is stored interleaved (row 2i = gate row i, row 2i + 1 = up row i): the two values
 //     of an activation meet in neighbouring TMEM lanes and are exchanged with one shuffle;
+//   * weights are loaded with an evict-first policy: a layer reads each of its weights once (the chunks of a weight block
+//     are neighbours in time), and without it 138 MB of them threw the kernel's own code, its inputs, the pair lists and the
+//     activations out of L2, so that every phase of the next layer began with trips to HBM.  88 layers of one token
+//     4595 -> 3757 us (dispatch 6.8 -> 3.8, experts 30.0 -> 27.2, combine 5.8 -> 3.1 us a layer), a layer of 37 tokens
+//     406 -> 384 us, of 190 wide tokens 454 -> 435 us, no difference at 4096;
 //   * weights and tokens have producer warps of their own, so the weight stream runs on while a down unit
 //     waits; eight epilogue warps read the accumulators with tcgen05.ld (a lane holds one output feature),
 //     turn them through a small shared-memory tile and store 16 bytes per lane, feature-contiguous;
@@ -347,6 +352,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
     if (warp == 0) {
       // ---------------- weights: 128 rows x 64 NSUB columns per CTA and stage ----------------
       if (elect_one()) {
+        const uint64_t stream = l2_evict_first();
         for (int i = 0; i < count && ok; ++i) {
           const FfnUnit un = listed(i);
           const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
@@ -356,7 +362,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
           for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
             if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 11))) break;
             if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * NSUB * kFfnABytes);
-            tma_load_2d_pair(sm.pipe + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row);
+            tma_load_2d_pair_hint(sm.pipe + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row, stream);
             if (++s == stages) { s = 0; ph ^= 1u; }
           }
         }
