@@ -138,13 +138,13 @@ __global__ void __launch_bounds__(512) a2a_dispatch_kernel(const __grid_constant
           v[u] = p < row_packs ? ld_v4(xrow + p * 16) : make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          // amax over the 16 lanes that hold one 128-element block
-          float amax = pack_absmax(v[u]);
+        for (int u = 0; u < 4; u += 2) {
+          block_absmax_pair(v[u], v[u + 1], scale[u], scale[u + 1]);
 #pragma unroll
-          for (int sh = 8; sh >= 1; sh >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
-          scale[u] = amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f;
-          q[u] = quant_pack_e4m3(v[u], scale[u]);
+          for (int k = u; k < u + 2; ++k) {
+            scale[k] = e4m3_scale(scale[k]);
+            q[k] = quant_pack_e4m3(v[k], scale[k]);
+          }
         }
         for (int j = 0; j < m; ++j) {
           const uint64_t row = (uint64_t)c.rank * a.cap + L.slot[j];

@@ -252,16 +252,16 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
       const long long i = base + u * stride + (threadIdx.x & 31);
       v[u] = i < total ? ld_v4_stream(src + i * 16) : make_uint4(0, 0, 0, 0);
     }
+    float amax[U];
+#pragma unroll
+    for (int u = 0; u < U; u += 2) block_absmax_pair(v[u], v[u + 1], amax[u], amax[u + 1]);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long i = base + u * stride + (threadIdx.x & 31);
-      float amax = pack_absmax(v[u]);
-#pragma unroll
-      for (int sh = 8; sh >= 1; sh >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, sh));
       if (i >= total) continue;
-      const float scale = e4m3_scale(amax);
+      const float scale = e4m3_scale(amax[u]);
       const uint2 q = quant_pack_e4m3(v[u], scale);
-      const long long row = i / ppr;
+      const long long row = total >> 32 ? i / ppr : (long long)((uint32_t)i / (uint32_t)ppr);
       const int pk = (int)(i - row * ppr);
       const uint64_t qo = q_off + (uint64_t)row * H + (uint64_t)pk * 8;
       const uint64_t so = s_off + ((uint64_t)row * nblk + (pk >> 4)) * 4;

@@ -8,29 +8,72 @@
 
 namespace mcb {
 
+// The quotients below are v / scale and amax / 448 rounded to fp32, as an fp32 reference has them.  For ordinary scales
+// they are a product with the reciprocal and one correction by its residual (Markstein, IBM J. Res. Dev. 34(1), 1990):
+// three instructions where a division takes about twelve and a branch, and the quantisation is most of what a dispatching
+// warp issues.  That the results are the same follows by exhaustion, with the reciprocal up to three units in the last
+// place off (the hardware's approximation is within one): a scale is (bf16 value) / 448, so there are 128 x 128 pairs of
+// significands and some twenty exponents apart before everything rounds to zero.  The range of scales keeps the residuals
+// out of underflow, the order of the signs keeps negative zeros.
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float div_corrected(float v, float d, float rcp) {
+  const float q = __fmul_rn(v, rcp);
+  return __fmaf_rn(__fmaf_rn(q, d, -v), -rcp, q);
+}
+__device__ __forceinline__ bool e4m3_ordinary(float scale) { return scale > 0x1p-80f && scale < 0x1p80f; }
+
 // Quantise 8 bf16 values (one 16-byte pack) to 8 e4m3 bytes: saturating RNE of v / scale.
 __device__ __forceinline__ uint2 quant_pack_e4m3(uint4 v, float scale) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  uint16_t q[4];
+  uint32_t q[4];
+  if (e4m3_ordinary(scale)) {
+    const float r = rcp_approx(scale);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    // true division (not a reciprocal multiply) so results match an fp32 reference bit for bit
-    const float2 f = make_float2(__fdiv_rn(bf16_lo(w[i]), scale), __fdiv_rn(bf16_hi(w[i]), scale));
-    q[i] = (uint16_t)__nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E4M3);
+    for (int i = 0; i < 4; ++i)
+      q[i] = __nv_cvt_float2_to_fp8x2(make_float2(div_corrected(bf16_lo(w[i]), scale, r), div_corrected(bf16_hi(w[i]), scale, r)),
+                                      __NV_SATFINITE, __NV_E4M3);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      q[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(bf16_lo(w[i]), scale), __fdiv_rn(bf16_hi(w[i]), scale)), __NV_SATFINITE,
+                                      __NV_E4M3);
   }
-  return make_uint2((uint32_t)q[0] | ((uint32_t)q[1] << 16), (uint32_t)q[2] | ((uint32_t)q[3] << 16));
+  return make_uint2(__byte_perm(q[0], q[1], 0x5410), __byte_perm(q[2], q[3], 0x5410));
 }
 
+// Largest magnitudes of the even and of the odd values of a pack, as bf16x2 (NaNs are passed over).
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t pack_absmax2(uint4 v) {
+  constexpr uint32_t kAbs = 0x7fff7fffu;
+  return max_bf16x2(max_bf16x2(v.x & kAbs, v.y & kAbs), max_bf16x2(v.z & kAbs, v.w & kAbs));
+}
 __device__ __forceinline__ float pack_absmax(uint4 v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-  float m = 0.f;
+  const uint32_t m = pack_absmax2(v);
+  return fmaxf(0.f, fmaxf(bf16_lo(m), bf16_hi(m)));
+}
+// Largest magnitudes of the 128-value blocks of two packs per lane, 16 neighbouring lanes holding a block; all 32 lanes.
+__device__ __forceinline__ void block_absmax_pair(uint4 v0, uint4 v1, float& m0, float& m1) {
+  const uint32_t a = pack_absmax2(v0), b = pack_absmax2(v1);
+  uint32_t m = max_bf16x2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));     // pack 0 in the low half, pack 1 in the high
 #pragma unroll
-  for (int i = 0; i < 4; ++i) m = fmaxf(m, fmaxf(fabsf(bf16_lo(w[i])), fabsf(bf16_hi(w[i]))));
-  return m;
+  for (int sh = 8; sh >= 1; sh >>= 1) m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, sh));
+  m0 = bf16_lo(m);
+  m1 = bf16_hi(m);
 }
 
-// Scale of a 128-value block from its largest magnitude.
-__device__ __forceinline__ float e4m3_scale(float amax) { return amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f; }
+// Scale of a 128-value block from its largest magnitude (1 if that is zero or the block has only NaNs).
+__device__ __forceinline__ float e4m3_scale(float amax) {
+  if (e4m3_ordinary(amax)) return div_corrected(amax, 448.0f, 1.0f / 448.0f);
+  return amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f;
+}
 
 // Largest magnitude of the 128-value block that starts at `block` (16 packs of 16 bytes), read by
 // ONE thread (for the packet mode, where the threads that share a block are not neighbours).

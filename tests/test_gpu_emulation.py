@@ -317,6 +317,34 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
     w.check_status()
 
 
+def _all_quotients(exponent):
+    """Blocks of 128 values whose largest has each of the 128 bf16 significands, the others every significand at
+    distances of 0 .. 23 binades with alternating signs, and both zeros: every quotient the quantisation can meet."""
+    sig = 1 + torch.arange(128, dtype=torch.float64) / 128
+    d = torch.arange(24, dtype=torch.float64)
+    v = sig.view(1, 1, 128) * 2.0 ** -d.view(1, 24, 1)
+    v = torch.minimum(v, sig.view(128, 1, 1)) * (1 - 2 * (torch.arange(128) % 2))
+    v[..., 0] = sig.view(128, 1)
+    v[..., 1], v[..., 2] = -0.0, 0.0
+    return (v * 2.0 ** exponent).to(torch.bfloat16).view(-1, 1024)
+
+
+@pytest.mark.parametrize("exponent", [0, -70, -73, -126, 85, 90, 127])     # scales on both sides of the short division's range
+def test_fp8_quantisation_bytes(lib, exponent):
+    x = _all_quotients(exponent)
+    cap, H = x.shape
+    w = EmuWorld(1, 32 << 20, DEV)
+    b = w.a2a_step_buffers(cap, H, 1, True)
+    meta, out = torch.zeros(8, dtype=torch.int32, device=DEV), torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV)
+    idx, wt = torch.zeros(cap, 1, dtype=torch.int64, device=DEV), torch.ones(cap, 1, device=DEV)
+    w.a2a_step(b, [x.to(DEV)], [idx], [wt], [out], _scalars([cap]), [meta], 4, 1)
+    q, scale = oracle.quant_e4m3_1x128(x.float())
+    par = int(meta[5])
+    assert torch.equal(b["recv_scale"][0].tensor[par, 0].cpu(), scale)
+    assert torch.equal(b["recv_x"][0].tensor[par, 0].cpu(), q.view(torch.uint8))
+    w.check_status()
+
+
 def test_a2a_fp8_dispatch(lib):
     W, E, K, H, counts = 2, 16, 4, 512, [6, 3]
     w, b, xs, idxs, ws, n_locals, cap = _a2a_case(W, E, K, H, counts, True, 13)
