@@ -330,6 +330,11 @@ __device__ __forceinline__ void push_slice(const McbCtx& c, const McbA2AStepArgs
   }
 }
 
+__device__ __forceinline__ void add_packs(float (&acc)[4][8], const uint4 (&v)[4]) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) acc_bf16x8(acc[u], v[u]);
+}
+
 __device__ __forceinline__ void store_out(const McbA2AStepArgs& a, const BarrierShape& s, const RowSlice& r,
                                           const float (&acc)[4][8], int lane) {
   uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + (uint64_t)r.t * s.row_bytes;
@@ -339,75 +344,6 @@ __device__ __forceinline__ void store_out(const McbA2AStepArgs& a, const Barrier
     if (p < s.row_packs)
       st_v4(out + (uint64_t)p * 16, make_uint4(pack_bf16x2(acc[u][0], acc[u][1]), pack_bf16x2(acc[u][2], acc[u][3]),
                                                pack_bf16x2(acc[u][4], acc[u][5]), pack_bf16x2(acc[u][6], acc[u][7])));
-  }
-}
-
-// A world of one: nobody to wait for, so a slice is delivered and combined in one go.  The loads of a warp's next slice
-// (mostly the same slice of the next layer) are in flight while the current one is quantised and stored.  What bounds it
-// is the chain of instructions of a slice (four warps share a scheduler): 58 layers of 333 rows of 7168 values, e4m3
-// dispatch, 253 -> 224 us with the next slice's loads in flight and the quantisation without divisions.
-struct AloneSlice {
-  RowSlice r;
-  uint32_t par, stamp;
-  uint4 v[4], y[4], meta;
-  long long id;             // expert id of this lane's routing slot (the first 32 slots)
-};
-
-__device__ __noinline__ void alone_layers(const McbCtx& c, const McbA2AStepArgs& a, const BarrierShape& s, const uint8_t* x,
-                                          uint64_t slot0, long long first, long long step, long long mine,
-                                          uint32_t layer_base) {
-  const int lane = threadIdx.x & 31, L = a.num_layers;
-  // The identity expert on bf16 rows returns the row just delivered, which is still in registers.
-  const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
-  RowSlice r;
-  auto locate = [&](long long i) {
-    r.t = (int)(i / s.slices);
-    r.p0 = (int)(i - (long long)r.t * s.slices) * kSlicePacks;
-    r.row = slot0 + r.t;
-  };
-  auto load = [&](AloneSlice& w, int l) {
-    w.r = r;
-    w.par = (layer_base + (uint32_t)l) & 1u;
-    w.stamp = layer_base + (uint32_t)l + 1u;
-    load_packs(w.v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
-    if (!echo)
-      load_packs(w.y, c.heap_local + a.y_off + (uint64_t)w.par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
-    w.meta = make_uint4(0, 0, 0, 0);
-    if (r.p0 == 0 && lane < s.meta_chunks) w.meta = meta_chunk(a, r.t, lane, w.stamp);
-    w.id = lane < a.topk ? a.topk_idx[(long long)r.t * a.topk + lane] : -1;
-  };
-  int l = 0;
-  long long i = first;
-  if (L <= 0) return;
-  locate(i);
-  AloneSlice cur;
-  load(cur, l);
-  for (;;) {
-    if ((i += step) >= mine) { i = first; ++l; }
-    const bool more = l < L;
-    AloneSlice nxt;
-    if (more) {
-      if (mine > step) locate(i);
-      load(nxt, l);
-    }
-    bool any = false;
-    for (int k = lane; k < a.topk; k += 32) {
-      const long long e = k == lane ? cur.id : a.topk_idx[(long long)cur.r.t * a.topk + k];
-      if (e >= 0 && e < a.num_experts) any = true;
-      else report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)cur.r.t, (uint32_t)e);
-    }
-    const DestMask m = {{__any_sync(0xffffffffu, any) ? 1u : 0u, 0u, 0u}};
-    push_slice(c, a, s, cur.r, m, cur.v, cur.meta, cur.par, cur.stamp, lane);
-    // The sum over the one destination's row: 0 + row, exact in bf16.
-    uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + (uint64_t)cur.r.t * s.row_bytes;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int p = cur.r.p0 + u * 32 + lane;
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      if (p < s.row_packs) st_v4(out + (uint64_t)p * 16, m.w[0] ? add_bf16x8(echo ? cur.v[u] : cur.y[u], zero) : zero);
-    }
-    if (!more) break;
-    cur = nxt;
   }
 }
 
@@ -444,7 +380,28 @@ __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArg
   };
 
   if (W == 1) {
-    if (first < mine) alone_layers(c, a, s, x, slot0, first, step, mine, layer_base);
+    // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.
+    // The identity expert on bf16 rows returns the row just delivered, which is still in registers.
+    const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
+    for (int l = 0; l < L; ++l) {
+      const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+      const uint32_t stamp = layer_base + (uint32_t)l + 1u;
+      for (long long i = first; i < mine; i += step) {
+        const RowSlice r = slice_of(i);
+        uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
+        load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
+        if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
+        if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
+        const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
+        push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
+        float acc[4][8] = {};
+        if (m.w[0]) {
+          if (echo) add_packs(acc, v);
+          else add_packs(acc, y);
+        }
+        store_out(a, s, r, acc, lane);
+      }
+    }
     return;
   }
 
