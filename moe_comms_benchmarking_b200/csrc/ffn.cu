@@ -63,9 +63,9 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* ea
   m.off = sm.off;
   const RouteShare share = route_share(p.route, (int)blockIdx.x, (int)gridDim.x);
   if (route_counts_all(share)) {
-    route_count(p.route, ids, m, 0, share.entries, share.lo);
+    route_count<true>(p.route, ids, m, 0, share.entries, share.lo);
   } else {
-    route_count(p.route, ids, m, share.lo, share.hi, 0);
+    route_count<false>(p.route, ids, m, share.lo, share.hi, 0);
     route_publish(p.route, m);
     meet();
     route_collect(p.route, m);
