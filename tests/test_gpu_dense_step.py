@@ -231,3 +231,17 @@ def test_world_of_one_copies(lib, dtype, K, grid, threads):
         rig.check([n], expect_mode=0)
         assert torch.equal(rig.outs[0][:n], rig.rsv[0].tensor[:n])
     rig.w.check_status()
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 9, 16])          # 17.5 packs a row on 64 threads: up to 1, 2, 4 packs per thread and more
+@pytest.mark.parametrize("layers", [1, 2, 7, 8, 9, 17])     # on both sides of the layers whose loads go out together
+def test_world_of_one_layers_in_flight(lib, n, layers):
+    rig = _Rig(1, 16, 64, 2, 0)
+    rig.new_inputs()
+    rig.step([n], layers, 1, 64)
+    rig.check([n], expect_mode=0)
+    par = int(rig.metas[0][5])
+    for p in {par, (par + layers - 1) % 2}:                 # the last two layers, where there are two
+        for dst, src in ((rig.dst_h, rig.src_h), (rig.dst_r, rig.src_r), (rig.dst_p, rig.src_p)):
+            assert torch.equal(dst[0].tensor[p, :n], src[0][:n])
+    rig.w.check_status()
