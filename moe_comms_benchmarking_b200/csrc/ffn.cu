@@ -50,12 +50,13 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* ea
   auto meet = [&] { grid_sync(c, arrivals, target += gridDim.x); };
   stamp(0);
   ffn_setup(p.ffn);
-  agv_device<MCB_SITE_FC1_FUSED>(c, p.agv, ll_launch);      // waits for the previous kernel first
+  const GatheredRows got = agv_device<MCB_SITE_FC1_FUSED>(c, p.agv, ll_launch);      // waits for the previous kernel first
   stamp(1);
-  // Routing needs the gathered ids of all tokens; a world of one has them in its own inputs and need not wait for the copy.
-  const bool alone = c.world == 1;
-  const int64_t* ids = alone ? reinterpret_cast<const int64_t*>(p.agv.src[1]) : p.route.topk_idx;
-  const float* probs = alone ? reinterpret_cast<const float*>(p.agv.src[2]) : p.route.topk_w;
+  // Routing needs the ids and weights that its arguments name, of all gathered tokens.  In a world of one these are usually
+  // rows that this all-gather copies: then they are read where they come from, and nobody waits for the copy.
+  const bool alone = c.world == 1 && p.local_ids && got.offset == 0 && got.valid <= got.n;
+  const int64_t* ids = alone ? p.local_ids : p.route.topk_idx;
+  const float* probs = alone ? p.local_probs : p.route.topk_w;
   if (!alone) meet();
   stamp(2);
   const FfnSmem sm;

@@ -354,13 +354,17 @@ __device__ __forceinline__ void agv_ll(const McbCtx& c, const McbAgvArgs& a, int
   }
 }
 
+// What an all-gather has moved.
+struct GatheredRows {
+  int n, offset, valid;       // rows of this rank (0 if the counts were refused), its first row, rows of all ranks
+};
 // Body of the variable all-gather, shared by the stand-alone kernel and the fused
 // dispatch + routing + FC1 kernel.  Call from all threads of the block.  The launch number (the
 // packet flag) is returned in `ll_launch`: FUSED_SITE < 0 takes it from the per-block counters of
 // MCB_SITE_AGV_LL; otherwise from launch_begin(FUSED_SITE), and the calling kernel must end with
 // launch_end(FUSED_SITE, ll_launch).
 template <int FUSED_SITE>
-__device__ __forceinline__ void agv_device(const McbCtx& c, const McbAgvArgs& a, uint32_t& ll_launch) {
+__device__ __forceinline__ GatheredRows agv_device(const McbCtx& c, const McbAgvArgs& a, uint32_t& ll_launch) {
   const int bid = blockIdx.x;
   int n = 0, valid_pre = 0, offset = 0, ep_max = 0;
   if (a.meta_stable) {
@@ -380,19 +384,20 @@ __device__ __forceinline__ void agv_device(const McbCtx& c, const McbAgvArgs& a,
   const int nact = active_blocks((int)gridDim.x, ep_max, bytes_per_row, (int)blockDim.x);
   pdl_launch_dependents();
   const bool bad = n < 0 || n > a.cap || offset < 0 || (long long)offset + n > (long long)a.cap * c.world;
+  const GatheredRows got{bad ? 0 : n, offset, valid_pre};
   if (a.ll_rows > 0 && c.world > 1) {
     const uint32_t flag = ll_launch;      // changes with every launch, in either mode
     if (agv_ll_eligible(c, a, valid_pre)) {
       const int valid = valid_pre;
       if (bad) {
         if (threadIdx.x == 0) report_error(c, MCB_ERR_BOUNDS, (uint32_t)a.site, (uint32_t)bid, (uint32_t)n, (uint32_t)valid);
-        return;
+        return got;
       }
       agv_ll(c, a, n, offset, valid, flag);
-      return;
+      return got;
     }
   }
-  if (bid >= nact) return;
+  if (bid >= nact) return got;
   const uint32_t ep = *epoch_ptr(c, a.site, bid);
   if (n < 0) n = 0;
   if (bad) {
@@ -413,7 +418,7 @@ __device__ __forceinline__ void agv_device(const McbCtx& c, const McbAgvArgs& a,
       }
     __syncthreads();
     copy_ranges(r, 0, start, stride);
-    return;
+    return got;
   }
 #pragma unroll
   for (int t = 0; t < MCB_MAX_TENSORS; ++t) {
@@ -428,6 +433,7 @@ __device__ __forceinline__ void agv_device(const McbCtx& c, const McbAgvArgs& a,
   }
   // Trailing barrier: when this kernel has finished on a rank, every peer's rows are there.
   block_barrier_all(c, a.site, bid, ep);
+  return got;
 }
 
 }  // namespace mcb

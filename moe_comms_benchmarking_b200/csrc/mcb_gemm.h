@@ -120,6 +120,10 @@ typedef struct {
 typedef struct alignas(64) {
   McbCtx ctx;
   McbAgvArgs agv;
+  // World of one only: where the rows of route.topk_idx and route.topk_w (null: weight 1) come from, if agv is what gathers
+  // them and agv.step_meta is what counts them; local_ids null: the routing reads the gathered rows.
+  const int64_t* local_ids;
+  const float* local_probs;
   McbRouteArgs route;
   McbFfnArgs ffn;
   McbCombineArgs cmb;

@@ -162,7 +162,8 @@ class McbLayerArgs(C.Structure):
     """One MoE layer as one kernel parameter: the context and the argument blocks of the four
     phases (64-byte aligned as a whole)."""
     _fields_ = [
-        ("ctx", McbCtx), ("agv", McbAgvArgs), ("route", McbRouteArgs), ("ffn", McbFfnArgs), ("cmb", McbCombineArgs),
+        ("ctx", McbCtx), ("agv", McbAgvArgs), ("local_ids", _vp), ("local_probs", _vp), ("route", McbRouteArgs),
+        ("ffn", McbFfnArgs), ("cmb", McbCombineArgs),
         ("trace", _vp), ("reserved0", _u64),
     ]
 

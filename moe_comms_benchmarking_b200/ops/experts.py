@@ -338,6 +338,18 @@ class ExpertFfnPlan:
                    "expert_ffn")
 
 
+def local_routing(heap: SymmetricHeap, agv: "_ext.McbAgvArgs", route: "_ext.McbRouteArgs"):
+    """(ids, weights): where a world of one finds the rows of ``route.topk_idx`` and ``route.topk_w`` before ``agv`` has
+    copied them; (None, None) unless ``agv`` gathers and counts exactly these rows."""
+    if heap.world != 1 or route.num_tokens != agv.step_meta:
+        return None, None
+    base = heap.ctx().heap_local
+    source = {(base + agv.dst_off[t], agv.row_bytes[t]): agv.src[t] for t in range(agv.num_tensors)}
+    ids = source.get((route.topk_idx, 8 * route.topk))
+    probs = source.get((route.topk_w, 4 * route.topk))
+    return (ids, probs) if ids and (probs or not route.topk_w) else (None, None)
+
+
 class MoeLayerPlan:
     """One whole MoE layer per launch (``moe_layer_kernel``: dispatch, routing, experts, combine), for
     one or several weight sets; ``launch(s)`` runs the layer with set ``s``, ``decode_step(n)`` issues the
@@ -364,6 +376,7 @@ class MoeLayerPlan:
             C.memmove(C.addressof(p.ffn), C.addressof(f.args), C.sizeof(_ext.McbFfnArgs))
             C.memmove(C.addressof(p.cmb), C.addressof(self.combine.args), C.sizeof(_ext.McbCombineArgs))
             p.trace = self.trace.data_ptr() if self.trace is not None else None
+            p.local_ids, p.local_probs = local_routing(self.heap, self.agv.args, self.route.args)
         self._ctx_version = id(ctx)
 
     def _sync_ctx(self):

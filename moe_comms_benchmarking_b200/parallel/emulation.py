@@ -206,6 +206,8 @@ class EmuWorld:
             a.n_local, a.step_meta = d["n_local"].data_ptr(), d["step_meta"].data_ptr()
             if ll_rows > 0:
                 a.ll_off, a.ll_rows = d["ll_stage"].offset, ll_rows
+            if self.world == 1:
+                p.local_ids, p.local_probs = d["src"][1].data_ptr(), d["src"][2].data_ptr()
             ro = p.route
             ro.topk_idx, ro.topk_w = d["dst"][1].tensor.data_ptr(), d["dst"][2].tensor.data_ptr()
             ro.num_tokens = d["step_meta"].data_ptr()

@@ -176,6 +176,30 @@ def test_expert_plans_validate_arguments(lib):
         DispatchRouteFc1Plan(h, agv, rp, fc2)
 
 
+def test_layer_reads_ids_at_their_source_only_if_gathered():
+    """The short cut of the layer kernel in a world of one: taken for the rows that the all-gather copies and counts, by
+    address and row size, in any order of the tensors; refused for everything else."""
+    from moe_comms_benchmarking_b200.ops.experts import RouteBuffers, RoutePlan, local_routing
+    h = _heap(2 << 20)
+    T, K, H = 8, 4, 256
+    x, idx, w = torch.zeros(T, H, dtype=torch.bfloat16), torch.zeros(T, K, dtype=torch.int64), torch.zeros(T, K)
+    gx, gi, gw = h.alloc("gx", [T, H], torch.bfloat16), h.alloc("gi", [T, K], torch.int64), h.alloc("gw", [T, K], torch.float32)
+    n, meta = torch.zeros(1, dtype=torch.int32), torch.zeros(4, dtype=torch.int32)
+    route = RouteBuffers(T, K, 8, "cpu")
+
+    def found(dsts, srcs, ids, weights, count=meta):
+        agv = AllGatherVPlan(h, dsts, srcs, n, meta, T)
+        return local_routing(h, agv.args, RoutePlan(route, ids, weights, count, expert_begin=0).args)
+
+    here = (idx.data_ptr(), w.data_ptr())
+    assert found([gx, gi, gw], [x, idx, w], gi.tensor, gw.tensor, meta[0:1]) == here
+    assert found([gw, gx, gi], [w, x, idx], gi.tensor, gw.tensor) == here
+    assert found([gx, gi], [x, idx], gi.tensor, None) == (idx.data_ptr(), None)
+    for ids, weights, count in ((idx.clone(), gw.tensor, meta), (gi.tensor, w.clone(), meta), (gi.tensor, gw.tensor, n)):
+        assert found([gx, gi, gw], [x, idx, w], ids, weights, count) == (None, None)
+    assert found([gx], [x], idx, w) == (None, None) and found([gx, gi], [x, idx], gi.tensor, gw.tensor) == (None, None)
+
+
 def test_capability_checks():
     from moe_comms_benchmarking_b200 import ops
     assert not ops.is_device_multimem_capable("cpu") and not ops.is_device_tcgen05_capable("cpu")

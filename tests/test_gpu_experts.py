@@ -366,3 +366,45 @@ def test_expert_combine_slices(world1, T, K, H):
     live = (pos >= 0).unsqueeze(-1)
     ref = torch.stack([(y[pos[t].clamp(min=0).long()].float() * live[t]).sum(0) for t in range(T)])
     assert torch.allclose(out.float(), ref, rtol=2 ** -8, atol=1e-5)      # fp32 sums in another order, rounded once
+
+
+@pytest.mark.parametrize("form", ["gathered", "no_weights", "own", "own_weights", "hidden_only", "order"])
+def test_layer_plan_follows_its_routing_plan(world1, form):
+    """The layer kernel of a world of one routes by the ids and weights of its RoutePlan: the gathered ones, tensors of
+    the caller's own, or weight 1, whatever tensors the all-gather carries and in whatever order."""
+    from moe_comms_benchmarking_b200.ops import oracle
+    from moe_comms_benchmarking_b200.ops.dense import AllGatherVPlan, MetadataPlan
+    from moe_comms_benchmarking_b200.ops.experts import (ExpertCombinePlan, ExpertFfnPlan, ExpertWeights, MoeLayerPlan,
+                                                         RouteBuffers, RoutePlan)
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, cap, E, K, H, I = 40, 44, 6, 3, 256, 128
+    pad = lambda t: torch.cat([t, t[:cap - T]]).contiguous()
+    x, idx, w = (pad(t) for t in _case(T, E, K, H, I, 17))
+    _, own_idx, own_w = (pad(t) for t in _case(T, E, K, H, I, 18))
+    heap = SymmetricHeap(world1, 2 << 20, DEV)
+    gx, gi, gw = heap.alloc("gx", [cap, H], torch.bfloat16), heap.alloc("gi", [cap, K], torch.int64), heap.alloc("gw", [cap, K], torch.float32)
+    pairs = {"hidden_only": [(gx, x)], "order": [(gw, w), (gx, x), (gi, idx)]}.get(form, [(gx, x), (gi, idx), (gw, w)])
+    r_idx = own_idx if form in ("own", "hidden_only") else gi.tensor
+    r_w = {"no_weights": None, "own": own_w, "own_weights": own_w, "hidden_only": own_w}.get(form, gw.tensor)
+    n = torch.tensor([T], dtype=torch.int32, device=DEV)
+    meta = torch.zeros(4, dtype=torch.int32, device=DEV)
+    route = RouteBuffers(cap, K, E, DEV)
+    weights = ExpertWeights(E, H, I, DEV, seed=19, std=0.05)
+    act = torch.zeros(route.max_pairs, I, dtype=torch.bfloat16, device=DEV)
+    y = torch.zeros(route.max_pairs, H, dtype=torch.bfloat16, device=DEV)
+    out = torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV)
+    partial = heap.alloc("partial", [2, cap, H], torch.bfloat16)
+    plan = MoeLayerPlan(heap, AllGatherVPlan(heap, [d for d, _ in pairs], [s for _, s in pairs], n, meta, cap),
+                        RoutePlan(route, r_idx, r_w, meta[0:1], expert_begin=0, status=heap.status),
+                        [ExpertFfnPlan(weights, route, gx.tensor, act, y, heap.status)],
+                        ExpertCombinePlan(heap, y, route, partial, out, n, meta, cap), MetadataPlan(heap, n, meta, cap))
+    used_idx = own_idx if form in ("own", "hidden_only") else idx
+    used_w = {"no_weights": torch.ones_like(w), "own": own_w, "own_weights": own_w, "hidden_only": own_w}.get(form, w)
+    ref = oracle.moe_layer(x[:T].cpu(), used_idx[:T].cpu(), used_w[:T].cpu(), weights.w_gate_up.cpu(), weights.w_down.cpu())
+    for rep in range(2):        # twice: counters must come back clean
+        out.fill_(float("nan"))
+        plan.decode_step(1)
+        torch.cuda.synchronize()
+        heap.check_status()
+        s = float(ref.abs().max())
+        assert float((out[:T].float().cpu() - ref).abs().max()) < 0.03 * s + 1e-3, f"rep {rep}"
