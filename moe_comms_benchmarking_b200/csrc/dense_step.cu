@@ -282,8 +282,9 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
 
 // ---- a world of one: the layers of a step are local copies ------------------------------------------------------
 // Up to S packs per thread and layer: where they come from and go to is worked out once for all layers.  Nothing that a
-// layer reads is written in the step, so the loads of D layers go out together and are stored layer by layer: with one
-// layer at a time each layer was a trip to L2.  88 layers of hidden 1024 and top-22, one B200: 57 -> 37 us with one
+// layer reads is written in the step (else: a.in_order), so the loads of D layers go out together and are stored layer
+// by layer; the layers of such a step run into each other.  With one layer at a time each layer was a trip to L2: 88 layers
+// of hidden 1024 and top-22, one B200: 57 -> 37 us with one
 // token, 47 -> 34 with 200, 62 -> 55 with 333, where the second pack per thread begins.
 template <bool FP8, int S, int D>
 __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, long long start,
@@ -342,6 +343,14 @@ __device__ __noinline__ void local_layers(const McbCtx& c, const McbDenseStepArg
   __syncthreads();
   const long long start = (long long)blockIdx.x * blockDim.x + tid, stride = (long long)nact * blockDim.x;
   const long long total = r.end[R - 1];
+  if (a.in_order) {
+    for (int l = 0; l < a.num_layers; ++l) {
+      const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+      if (FP8) fp8_push(c, a, par, 0, 0, n, start, stride);
+      copy_ranges_in_order(r, par, start, stride);
+    }
+    return;
+  }
 
   // Few packs: eight of them in flight per thread, those of several layers where a layer has fewer.
   if (FP8) {
@@ -553,20 +562,42 @@ static int check_step_args(const McbDenseStepArgs* a, int grid, int threads) {
   return 0;
 }
 
+// Whether a step in a world of one writes rows that it reads, or writes rows twice: an output on a source (a step in
+// place), partial sums that are gathered rows (the identity expert).  Its copies then keep the order of the layers.
+int mcb_dense_step_in_order(const McbCtx* ctx, const McbDenseStepArgs* a) {
+  if (ctx->world != 1) return 0;
+  struct Range { uint64_t at, bytes; };
+  auto meet = [](Range x, Range y) { return x.at && y.at && x.at < y.at + y.bytes && y.at < x.at + x.bytes; };
+  const uint64_t heap = reinterpret_cast<uint64_t>(ctx->heap_local), cap = (uint64_t)a->cap;
+  const Range out{reinterpret_cast<uint64_t>(a->out), cap * a->rsv_row_bytes}, sums{heap + a->rsv_off, cap * a->rsv_row_bytes};
+  bool hit = meet(out, sums);
+  for (int t = 0; t < a->num_tensors; ++t) {
+    const Range rows{heap + a->dst_off[t], a->dst_par_stride[t] + cap * a->row_bytes[t]};
+    hit = hit || meet(rows, sums) || meet(rows, out);
+    for (int u = 0; u < a->num_tensors; ++u) {
+      const Range src{reinterpret_cast<uint64_t>(a->src[u]), cap * (a->fp8_hidden && u == 0 ? 2u * a->fp8_hidden : a->row_bytes[u])};
+      hit = hit || meet(src, rows) || meet(src, out);
+    }
+  }
+  return hit;
+}
+
 // The pipeline groups wait on one another inside the launch, so with groups > 1 all blocks must be
 // resident at once: the launch is cooperative.
 int mcb_launch_dense_step(const McbCtx* ctx, const McbDenseStepArgs* args, int grid, int threads, int pdl,
                           cudaStream_t stream) {
   if (!ctx || check_step_args(args, grid, threads)) return cudaErrorInvalidValue;
   const bool coop = args->groups > 1;
+  McbDenseStepArgs a = *args;
+  a.in_order = mcb_dense_step_in_order(ctx, args);
   if (args->check)
     return launch_kernel(dense_step_kernel<false, true, false>, dim3(grid), dim3(threads), 0, stream, pdl, coop, *ctx,
-                         *args, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
+                         a, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
   if (args->fp8_hidden)
     return launch_kernel(dense_step_kernel<false, false, true>, dim3(grid), dim3(threads), 0, stream, pdl, coop, *ctx,
-                         *args, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
+                         a, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
   return launch_kernel(dense_step_kernel<false, false, false>, dim3(grid), dim3(threads), 0, stream, pdl, coop, *ctx,
-                       *args, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
+                       a, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);
 }
 
 int mcb_emu_dense_step(const McbCtx* d_ctx, const McbDenseStepArgs* d_args, const McbDenseStepArgs* h_args0,

@@ -183,6 +183,8 @@ typedef struct {
   // Non-zero: tensor 0's source is bf16 [cap, fp8_hidden] and is dispatched as 1 x 128 block-scaled e4m3
   // (row_bytes[0] = fp8_hidden bytes), with the fp32 scales as gathered tensor 3 (src[3] unused).
   uint32_t fp8_hidden;
+  int32_t in_order;             // world of one: the step reads rows that it writes (mcb_launch_dense_step sets it)
+  int32_t reserved0;
 } McbDenseStepArgs;
 
 // All-to-all-V dispatch (one copy of a token per distinct destination rank).

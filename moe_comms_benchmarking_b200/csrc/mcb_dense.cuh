@@ -141,6 +141,28 @@ __device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parit
   r.store_word(parity, word);
 }
 
+// The same range by range, each dealt from the first thread on: pack i of every range belongs to the same thread, so what
+// a range reads of an earlier one's rows, in the same place, it reads after that one's store.
+__device__ __forceinline__ void copy_ranges_in_order(const LocalRanges& r, uint32_t parity, long long start, long long stride) {
+  constexpr int U = 8;
+  const uint32_t word = r.load_word();
+  for (int t = 0; t < LocalRanges::R; ++t) {
+    const uint8_t* src = r.src[t];
+    uint8_t* dst = r.dst[t] + (parity ? r.par[t] : 0);
+    const long long packs = r.end[t] - (t ? r.end[t - 1] : 0);
+    for (long long i0 = start; i0 < packs; i0 += stride * U) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * stride < packs) v[u] = ld_v4_stream(src + (i0 + u * stride) * 16);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (i0 + u * stride < packs) st_v4(dst + (i0 + u * stride) * 16, v[u]);
+    }
+  }
+  r.store_word(parity, word);
+}
+
 // ------------------------------------------------------------------------------------------
 // Flat cross-rank reduction: out[i] = sum over ranks of heap[base + 16 * i], 16 bytes at a time.
 // ------------------------------------------------------------------------------------------

@@ -85,6 +85,7 @@ class McbDenseStepArgs(C.Structure):
         ("agv_ll_off", _u64), ("rsv_ll_off", _u64), ("ll_src_rows", _i32), ("groups", _i32),
         ("group_min_bytes", _u64), ("n_local", _vp), ("step_meta", _vp), ("counts_off", _u64), ("credit_off", _u64), ("state", _vp),
         ("check_errors", _vp), ("check", _i32), ("delay_every", _i32), ("delay_ns", _u32), ("fp8_hidden", _u32),
+        ("in_order", _i32), ("reserved0", _i32),
     ]
 
 

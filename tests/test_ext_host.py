@@ -273,6 +273,30 @@ def test_step_plans_validate_arguments():
     assert st.shape == (3,) and ids.shape == (3, K) and wts.dtype == torch.float32
 
 
+def test_step_on_its_own_rows_keeps_its_order(lib):
+    """A step of a world of one whose output lies on a source, or whose partial sums lie on gathered rows, is marked to keep
+    the order of its layers; one on buffers of its own, next to one another even, is not."""
+    from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
+    h = _heap(4 << 20)
+    cap, H, K = 8, 256, 6
+    n_local, meta = torch.zeros(1, dtype=torch.int32), torch.zeros(8, dtype=torch.int32)
+    gh, gr = h.alloc("gh", [2, cap, H], torch.bfloat16), h.alloc("gr", [2, cap, K], torch.int64)
+    q, gp, sc = h.alloc("q", [2, cap, H], torch.uint8), h.alloc("gp", [2, cap, K], torch.float32), h.alloc("sc", [2, cap, 2], torch.float32)
+    rsv = h.alloc("rsv", [cap, H], torch.bfloat16)
+    both = torch.zeros(2 * cap, H, dtype=torch.bfloat16)
+    x, ids, p = both[:cap], torch.zeros(cap, K, dtype=torch.int64), torch.zeros(cap, K)
+
+    def marked(out, sums=rsv, fp8=False):
+        dsts, srcs = ([q, gr, gp, sc], [x, ids, p, None]) if fp8 else ([gh, gr], [x, ids])
+        plan = DenseStepPlan(h, dsts, srcs, out, sums, n_local, meta, cap, 4, fp8_hidden=H if fp8 else 0)
+        return lib.mcb_dense_step_in_order(C.byref(h.ctx()), C.byref(plan.args))
+
+    assert marked(both[cap:]) == 0 and marked(both[cap:], fp8=True) == 0
+    assert marked(x) == 1 and marked(both[1:cap + 1]) == 1 and marked(x, fp8=True) == 1      # all rows, all but one, fp8
+    assert marked(both[cap - 1:2 * cap - 1], fp8=True) == 1                                  # the last bf16 row of an fp8 source
+    assert marked(both[cap:], gh) == 1 and marked(gh.tensor[1]) == 1 and marked(rsv.tensor) == 1
+
+
 def test_weight_tile_packing_round_trip():
     """The pre-packed weight layout: tile (row block, column block) is 16 KB of contiguous memory in the
     swizzled K-major shared-memory image; packing and unpacking are inverse, and chunk c of row r of a

@@ -245,3 +245,54 @@ def test_world_of_one_layers_in_flight(lib, n, layers):
         for dst, src in ((rig.dst_h, rig.src_h), (rig.dst_r, rig.src_r), (rig.dst_p, rig.src_p)):
             assert torch.equal(dst[0].tensor[p, :n], src[0][:n])
     rig.w.check_status()
+
+
+@pytest.mark.parametrize("form", ["in_place", "in_place_fp8", "identity"])
+@pytest.mark.parametrize("n,layers", [(1, 1), (1, 9), (5, 2), (5, 3), (40, 4), (130, 3)])      # 1 to 140 packs a thread and more on 2 x 64 threads
+def test_world_of_one_step_on_its_own_rows(lib, form, n, layers):
+    """A step whose output is its source (each layer dispatches what the layer before combined), and one whose partial
+    sums are the gathered rows of parity 0 (the identity expert): layer by layer, as with peers."""
+    from moe_comms_benchmarking_b200.ops.a2a import dequant_e4m3_1x128
+    from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    cap, H, K, fp8 = 132, 256, 4, form == "in_place_fp8"
+    g = torch.Generator(device=DEV).manual_seed(n + layers)
+    heap = SymmetricHeap(None, 4 << 20, DEV)
+    x = torch.randn(cap, H, device=DEV, generator=g).to(torch.bfloat16)
+    ids, w = torch.randint(0, 64, (cap, K), device=DEV, generator=g), torch.rand(cap, K, device=DEV, generator=g)
+    gh = heap.alloc("gh", [2, cap, H], torch.uint8 if fp8 else torch.bfloat16)
+    gi, gw = heap.alloc("gi", [2, cap, K], torch.int64), heap.alloc("gw", [2, cap, K], torch.float32)
+    gs = heap.alloc("gs", [2, cap, H // 128], torch.float32)
+    rsv = heap.alloc("rsv", [cap, H], torch.bfloat16)
+    rsv.tensor.normal_()
+    if form == "identity":
+        gh.tensor.normal_()
+        rsv, out = gh, torch.zeros_like(x)
+    else:
+        out = x
+    meta = torch.zeros(8, dtype=torch.int32, device=DEV)
+    plan = DenseStepPlan(heap, [gh, gi, gw] + [gs] * fp8, [x, ids, w] + [None] * fp8, out, rsv,
+                         torch.tensor([n], dtype=torch.int32, device=DEV), meta, cap, layers, grid=2, threads=64,
+                         fp8_hidden=H if fp8 else 0)
+    for step in range(2):
+        src, rows = x[:n].clone(), [gh.tensor[p, :n].clone() for p in (0, 1)]
+        first = 0 if step == 0 else layers % 2
+        for l in range(layers):                     # the step, one layer after the other
+            par = (first + l) % 2
+            rows[par] = src
+            res = (rows[0] if form == "identity" else rsv.tensor[:n]).clone()
+            if form != "identity":
+                src = res
+        plan.launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        assert int(meta[5]) == par
+        assert torch.equal(out[:n], res)
+        for p in {par, (par + layers - 1) % 2}:
+            if fp8:     # e4m3 has three bits behind the leading one: half a unit of the last is 2^-4 of the value, 2^-10 of the scale
+                got, want = dequant_e4m3_1x128(gh.tensor[p, :n], gs.tensor[p, :n]).float(), rows[p].float()
+                lim = want.abs() * (2 ** -4 + 2 ** -8) + gs.tensor[p, :n].repeat_interleave(128, 1) * 2 ** -9
+                assert bool(((got - want).abs() <= lim).all())
+            else:
+                assert torch.equal(gh.tensor[p, :n], rows[p])
+            assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
