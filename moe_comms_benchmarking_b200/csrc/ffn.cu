@@ -28,18 +28,20 @@
 
 namespace mcb {
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1) expert_ffn_kernel(const __grid_constant__ McbFfnArgs a) {
-  ffn_setup(a);
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1) expert_ffn_kernel(const __grid_constant__ McbFfnArgs a,
+                                                                                              const __grid_constant__ FfnMaps maps) {
+  ffn_setup<false>(maps.map);
   pdl_wait();
   pdl_launch_dependents();
-  ffn_device(a);
+  ffn_device(a, maps.map);
   ffn_teardown();
 }
 
 template <bool EMU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1)
-moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* eargs) {
+moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant__ FfnMaps maps_, const McbLayerArgs* eargs) {
   const McbLayerArgs& p = EMU ? eargs[blockIdx.y] : p_;
+  const CUtensorMap* maps = EMU ? reinterpret_cast<const CUtensorMap*>(p.ffn.tmaps) : maps_.map;
   const McbCtx& c = p.ctx;
   uint32_t ll_launch = 0;
   const bool tracing = p.trace != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
@@ -49,7 +51,7 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* ea
   uint32_t target = 0;
   auto meet = [&] { grid_sync(c, arrivals, target += gridDim.x); };
   stamp(0);
-  ffn_setup(p.ffn);
+  ffn_setup<EMU>(maps);
   const GatheredRows got = agv_device<MCB_SITE_FC1_FUSED>(c, p.agv, ll_launch);      // waits for the previous kernel first
   stamp(1);
   // Routing needs the ids and weights that its arguments name, of all gathered tokens.  In a world of one these are usually
@@ -83,7 +85,7 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const McbLayerArgs* ea
   target += gridDim.x;
   stamp(3);
   stamp(4);
-  ffn_run(p.ffn, max_rows, FfnReady{arrivals, (int)target});
+  ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
   ffn_teardown();
   stamp(5);
   meet();                                                   // every y row is written before any is summed
@@ -128,8 +130,7 @@ static int check_ffn_args(const McbFfnArgs* a) {
 // The kernels run in CTA pairs: an odd grid is rounded down, one CTA is rounded up.
 static int pair_grid(int grid) { return grid < 2 ? 2 : grid & ~1; }
 
-// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory; the caller
-// copies them to the device.  x: token rows; act, y: activations and expert outputs; w1, w2: the packed weights.
+// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory.  x: token rows; act, y: activations and expert outputs; w1, w2: the packed weights.
 int mcb_make_ffn_tmaps(void* out, const void* x, uint64_t x_rows, const void* act, const void* y, uint64_t pair_rows, const void* w1,
                        const void* w2, int experts, int hidden, int intermediate) {
   uint8_t* o = reinterpret_cast<uint8_t*>(out);
@@ -152,7 +153,8 @@ int mcb_launch_expert_ffn(const McbFfnArgs* args, int grid, int pdl, cudaStream_
   if (grid < 1 || check_ffn_args(args)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
   // A down block waits for gate/up blocks that other CTAs compute: all CTAs must be resident.
-  return launch_kernel(expert_ffn_kernel, dim3(pair_grid(grid)), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *args);
+  return launch_kernel(expert_ffn_kernel, dim3(pair_grid(grid)), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *args,
+                       *reinterpret_cast<const FfnMaps*>(args->tmaps));
 }
 
 static int check_layer_args(const McbLayerArgs* p, int grid) {
@@ -167,7 +169,7 @@ int mcb_launch_moe_layer(const McbLayerArgs* p, int grid, int pdl, cudaStream_t 
   if (check_layer_args(p, grid)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
   return launch_kernel(moe_layer_kernel<false>, dim3(pair_grid(grid)), dim3(kFfnThreads), kFfnSmemBytes, stream, pdl, true, *p,
-                       (const McbLayerArgs*)nullptr);
+                       *reinterpret_cast<const FfnMaps*>(p->ffn.tmaps), (const McbLayerArgs*)nullptr);
 }
 
 // One decode step with real experts, issued natively: the count exchange, then num_layers layer
@@ -187,8 +189,9 @@ int mcb_emu_moe_layer(const McbLayerArgs* d_args, const McbLayerArgs* h_args0, i
   if (!d_args || world < 1 || check_layer_args(h_args0, grid)) return cudaErrorInvalidValue;
   if (!configure_ffn_kernels()) return cudaErrorUnknown;
   McbLayerArgs dummy{};
+  FfnMaps no_maps{};
   return launch_kernel(moe_layer_kernel<true>, dim3(pair_grid(grid), world), dim3(kFfnThreads), kFfnSmemBytes, stream, 0, true,
-                       dummy, d_args);
+                       dummy, no_maps, d_args);
 }
 
 }  // extern "C"

@@ -209,9 +209,15 @@ struct FfnSmem {
   }
 };
 
-// Before the FFN, once per kernel: barriers, TMEM, tensor maps.  All threads of both CTAs of the pair; touches nothing
+// The tensor maps of a launch, as a kernel parameter.
+struct FfnMaps {
+  CUtensorMap map[MCB_FFN_TMAPS];
+};
+
+// Before the FFN, once per kernel: barriers, TMEM, tensor maps (GLOBAL: in global memory).  All threads of both CTAs of the pair; touches nothing
 // that another kernel writes, so a kernel with other work to do first calls it at its very start.
-__device__ __forceinline__ void ffn_setup(const McbFfnArgs& a) {
+template <bool GLOBAL>
+__device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
   const FfnSmem sm;
   if (threadIdx.x == 0) {
     // full: the weight producer and the first token producer of the leading CTA announce the bytes of both CTAs
@@ -221,8 +227,10 @@ __device__ __forceinline__ void ffn_setup(const McbFfnArgs& a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x >= 32 && threadIdx.x < 64) tmem_alloc_pair(sm.tmem_slot, 512);
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + MCB_FFN_TMAPS)
-    tma_prefetch_map(reinterpret_cast<const uint8_t*>(a.tmaps) + (threadIdx.x - 64) * 128);
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + MCB_FFN_TMAPS) {
+    if (GLOBAL) tma_acquire_map(maps + (threadIdx.x - 64));
+    tma_prefetch_map(maps + (threadIdx.x - 64));
+  }
   tc_fence_before();
   __syncthreads();
   cluster_sync();                                    // barriers initialised and TMEM allocated in both CTAs
@@ -295,7 +303,7 @@ struct FfnReady {
 };
 
 template <int NSUB>
-__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
+__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap* maps, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
   const FfnSmem sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();           // 0 = the CTA that issues the MMAs of the pair
@@ -304,7 +312,6 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
   const int total = plan.total();
   const uint32_t tmem_base = *sm.tmem_slot;
   const Abort ab{sm.abort_flag, a.status, a.timeout_ns};
-  const uint8_t* maps = reinterpret_cast<const uint8_t*>(a.tmaps);
   const bool gather = n_slot <= kFfnGatherN;
 
   const int b_sub_bytes = (n_slot >> 1) * 128;                    // token half of one 64-column block
@@ -356,7 +363,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
         for (int i = 0; i < count && ok; ++i) {
           const FfnUnit un = listed(i);
           const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
-          const uint8_t* map = maps + ((un.fc() ? MCB_FFN_MAP_W2 : MCB_FFN_MAP_W1) + (NSUB - 1) * 2) * 128;
+          const CUtensorMap* map = maps + (un.fc() ? MCB_FFN_MAP_W2 : MCB_FFN_MAP_W1) + (NSUB - 1) * 2;
           const int v = (un.e() * (un.fc() ? plan.n2 : plan.n1) + un.j()) * 2 + rank;     // 128-row block of the matrix
           int row = v * k_blocks * (kFfnABytes / 2048);
           for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
@@ -522,7 +529,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
           const int rows = un.half() / kFfnTokWarps;           // 8, 16, ... 64
           const uint32_t bytes = (uint32_t)un.half() * 256u * NSUB;
           const int row = un.row0 + rank * un.half() + t * rows;
-          const uint8_t* map = maps + ((un.fc() ? MCB_FFN_MAP_ACT : MCB_FFN_MAP_XP) + (rows >> 3) - 1) * 128;
+          const CUtensorMap* map = maps + (un.fc() ? MCB_FFN_MAP_ACT : MCB_FFN_MAP_XP) + (rows >> 3) - 1;
           int cur[kOps][4];
 #pragma unroll
           for (int k = 0; k < kOps; ++k)
@@ -550,7 +557,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
                 if (k * 4 >= rows) break;
 #pragma unroll
                 for (int sub = 0; sub < NSUB; ++sub)
-                  tma_gather4_pair(dst + sub * b_sub_bytes + k * 512, maps + MCB_FFN_MAP_X * 128, bar,
+                  tma_gather4_pair(dst + sub * b_sub_bytes + k * 512, maps + MCB_FFN_MAP_X, bar,
                                    (kb + sub) * kFfnBlockK, cur[k][0], cur[k][1], cur[k][2], cur[k][3]);
               }
             }
@@ -584,7 +591,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const FfnPlanS& p
 // Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
 // ffn_teardown, with the experts' offsets in the shared memory of FfnSmem::off (visible to all threads) and the largest
 // number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.
-__device__ __forceinline__ void ffn_run(const McbFfnArgs& a, int max_rows, const FfnReady ready) {
+__device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
   const FfnSmem sm;
   const int E = a.num_local_experts;
   if (max_rows < 1) max_rows = 1;
@@ -601,15 +608,15 @@ __device__ __forceinline__ void ffn_run(const McbFfnArgs& a, int max_rows, const
   }
   // Token tile of this launch: the largest expert, rounded up to 32, at most kFfnMaxN per chunk.
   const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 31) & ~31);
-  if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, plan, n_slot, ready);
-  else ffn_roles<1>(a, plan, n_slot, ready);
+  if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, maps, plan, n_slot, ready);
+  else ffn_roles<1>(a, maps, plan, n_slot, ready);
 }
 
 // The same after a routing of its own launch, whose results are in global memory.
-__device__ __forceinline__ void ffn_device(const McbFfnArgs& a) {
+__device__ __forceinline__ void ffn_device(const McbFfnArgs& a, const CUtensorMap* maps) {
   const FfnSmem sm;
   for (int e = threadIdx.x; e <= a.num_local_experts; e += blockDim.x) sm.off[e] = a.expert_offset[e];
-  ffn_run(a, *a.max_rows, FfnReady{nullptr, 0});
+  ffn_run(a, maps, *a.max_rows, FfnReady{nullptr, 0});
 }
 
 }  // namespace mcb

@@ -59,7 +59,9 @@ typedef struct {
   uint64_t timeout_ns;
   const void* w1;              // packed interleaved gate/up matrix (E * 2I rows, hidden columns), see mcb_ffn.cuh
   const void* w2;              // packed down matrix (E * hidden rows, I columns)
-  const void* tmaps;           // device memory, MCB_FFN_TMAPS tensor maps of 128 bytes, 64-byte aligned (mcb_make_ffn_tmaps)
+  // MCB_FFN_TMAPS tensor maps of 128 bytes, 64-byte aligned (mcb_make_ffn_tmaps): in host memory, from where a launch copies
+  // them into its parameters; for ranks emulated inside one launch in device memory.
+  const void* tmaps;
   int32_t* sync;               // [2] zero between launches: CTAs that have copied their token rows, CTAs that have left
 } McbFfnArgs;
 
@@ -82,7 +84,7 @@ typedef struct {
   int32_t* tile_row0;
   int32_t* tile_rows;
   int32_t* num_m_tiles;        // device scalar
-  int32_t* sync;               // [4] scratch: blocks-done (2 phases), ready counter, spare
+  int32_t* sync;               // [4] zero between launches: blocks that have counted, blocks that have left; two words of the fused FFN
   int32_t max_pairs;           // capacity of the pair arrays
   int32_t max_tiles;           // capacity of the tile table
   uint32_t* status;

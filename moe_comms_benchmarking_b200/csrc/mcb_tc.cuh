@@ -153,6 +153,11 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar) {
 __device__ __forceinline__ void tma_prefetch_map(const void* map) {
   asm volatile("prefetch.tensormap [%0];" :: "l"(map) : "memory");
 }
+// Before the first use of a tensor map that the host has written to global memory (one in the kernel's parameters needs no
+// fence): a descriptor cached from what lay there before is not used.
+__device__ __forceinline__ void tma_acquire_map(const void* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" :: "l"(map) : "memory");
+}
 // Tile load / four-row gather into this CTA's shared memory, completing on a barrier of either CTA of the pair.
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* map, uint32_t bar, int c0, int c1) {
   asm volatile(

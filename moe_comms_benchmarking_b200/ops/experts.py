@@ -122,21 +122,18 @@ def make_weight_tmap(w2d: torch.Tensor):
     return (raw, addr)     # keep `raw` alive; `addr` is what launches take
 
 
-def make_ffn_tmaps(weights: "ExpertWeights", x: torch.Tensor, act: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
-    """The tensor maps of one FFN launch (token rows, activations, expert outputs, packed weights) as a device tensor."""
-    raw = torch.zeros(_ext.FFN_TMAPS * 128 + 64, dtype=torch.uint8)
-    addr = (raw.data_ptr() + 63) & ~63
+def make_ffn_tmaps(weights: "ExpertWeights", x: torch.Tensor, act: torch.Tensor, y: torch.Tensor):
+    """The tensor maps of one FFN launch (token rows, activations, expert outputs, packed weights) in host memory:
+    (keep-alive buffer, 64-byte aligned address)."""
+    raw = (C.c_uint8 * (_ext.FFN_TMAPS * 128 + 64))()
+    addr = (C.addressof(raw) + 63) & ~63
     lib = _ext.require()
     _ext.check(lib.mcb_make_ffn_tmaps(C.c_void_p(addr), C.c_void_p(x.data_ptr()), C.c_uint64(x.shape[0]),
                                       C.c_void_p(act.data_ptr()), C.c_void_p(y.data_ptr()),
                                       C.c_uint64(min(act.shape[0], y.shape[0])),
                                       C.c_void_p(weights.w1.data_ptr()), C.c_void_p(weights.w2.data_ptr()),
                                       weights.num_local_experts, weights.hidden, weights.intermediate), "make_ffn_tmaps")
-    off = addr - raw.data_ptr()
-    maps = raw[off:off + _ext.FFN_TMAPS * 128].to(act.device, non_blocking=True)    # pageable source: read before the call returns
-    if maps.data_ptr() % 64:
-        raise RuntimeError("device allocation is not 64-byte aligned")
-    return maps
+    return raw, addr
 
 
 class RouteBuffers:
@@ -157,7 +154,7 @@ class RouteBuffers:
         self.tile_row0 = torch.zeros(self.max_tiles, **i32)
         self.tile_rows = torch.zeros(self.max_tiles, **i32)
         self.num_m_tiles = torch.zeros(1, **i32)
-        self.sync = torch.zeros(4, **i32)
+        self.sync = torch.zeros(4, **i32)                # two words of the routing, two of the fused FFN
         self.max_rows = torch.zeros(1, **i32)            # largest pair count of one expert
         self.ffn_done = torch.zeros(num_local_experts, **i32)   # gate/up blocks finished per expert (fused FFN)
 
@@ -319,10 +316,9 @@ class ExpertFfnPlan:
             raise ValueError("down blocks wait for gate/up blocks of other CTAs: grid <= number of SMs")
         self.weights, self.grid = weights, grid
         tmaps = make_ffn_tmaps(weights, x, act, y)
-        sync = torch.zeros(2, dtype=torch.int32, device=y.device)
-        self._keep = (route, x, act, y, status, tmaps, sync)
+        self._keep = (route, x, act, y, status, tmaps)
         a = _ext.McbFfnArgs()
-        a.tmaps, a.sync = tmaps.data_ptr(), sync.data_ptr()
+        a.tmaps, a.sync = tmaps[1], route.sync[2:].data_ptr()
         a.x, a.x_row_bytes = x.data_ptr(), H * 2
         a.pair_token, a.pair_prob = route.pair_token.data_ptr(), route.pair_prob.data_ptr()
         a.expert_offset, a.max_rows = route.expert_offset.data_ptr(), route.max_rows.data_ptr()

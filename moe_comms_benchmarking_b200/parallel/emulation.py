@@ -225,8 +225,12 @@ class EmuWorld:
             ff.num_local_experts, ff.hidden, ff.intermediate = w.num_local_experts, w.hidden, w.intermediate
             ff.status, ff.timeout_ns = self.status[r].data_ptr(), int(timeout_s * 1e9)
             ff.w1, ff.w2 = w.w1.data_ptr(), w.w2.data_ptr()
-            keep += [make_ffn_tmaps(w, d["dst"][0].tensor, d["act"], d["y"]), torch.zeros(2, dtype=torch.int32, device=self.device)]
-            ff.tmaps, ff.sync = keep[-2].data_ptr(), keep[-1].data_ptr()
+            raw, addr = make_ffn_tmaps(w, d["dst"][0].tensor, d["act"], d["y"])
+            maps = torch.frombuffer(bytearray(C.string_at(addr, _ext.FFN_TMAPS * 128)), dtype=torch.uint8).to(self.device)
+            if maps.data_ptr() % 128:
+                raise RuntimeError("device allocation is not 128-byte aligned")
+            keep.append(maps)
+            ff.tmaps, ff.sync = maps.data_ptr(), route.sync[2:].data_ptr()
             cm = p.cmb
             cm.y, cm.pair_pos, cm.partial_off, cm.out = d["y"].data_ptr(), route.pair_pos.data_ptr(), d["partial"].offset, d["out"].data_ptr()
             cm.n_local, cm.step_meta = d["n_local"].data_ptr(), d["step_meta"].data_ptr()

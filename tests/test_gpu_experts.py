@@ -408,3 +408,40 @@ def test_layer_plan_follows_its_routing_plan(world1, form):
         heap.check_status()
         s = float(ref.abs().max())
         assert float((out[:T].float().cpu() - ref).abs().max()) < 0.03 * s + 1e-3, f"rep {rep}"
+
+
+@pytest.mark.parametrize("rows", [[40, 10], [100, 3]])       # token rows gathered, and copied into pair order
+def test_expert_ffn_plan_at_once_on_another_stream(world1, rows):
+    """A plan is ready when its constructor returns: plans over changing inputs, one after the other and each launched
+    on a stream of its own while the stream that it was built on is still busy.  The reference rounds the activations by
+    itself: one unit in the last place of bf16 (2^-8) apart for some, that and the rounding of y (2^-9) within 2^-6."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, T, H, I = len(rows), sum(rows), 256, 128
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(rows, device=DEV)).view(T, 1)
+    w = torch.ones(T, 1, device=DEV)
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    route = RouteBuffers(T, 1, E, DEV)
+    rp = RoutePlan(route, idx, w, torch.tensor([T], dtype=torch.int32, device=DEV), expert_begin=0, status=heap.status)
+    weights = ExpertWeights(E, H, I, DEV, seed=8, std=0.05)
+    wgu, wd = weights.w_gate_up.float(), weights.w_down.float()
+    bufs = [(torch.randn(T, H, device=DEV).to(torch.bfloat16), torch.zeros(T, I, dtype=torch.bfloat16, device=DEV),
+             torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)) for _ in range(3)]
+    side = torch.cuda.Stream()
+    for i in range(9):
+        x, act, y = bufs[i % 3]
+        act.zero_(); y.zero_()
+        rp.launch()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)            # about 10 ms
+        plan = ExpertFfnPlan(weights, route, x, act, y, heap.status)
+        plan.launch(stream=side)
+        side.synchronize()
+        got, tok = y.float(), route.pair_token[:T].long()
+        torch.cuda.synchronize()
+        heap.check_status()
+        for e, lo in ((0, 0), (1, rows[0])):
+            gu = x.float()[tok[lo:lo + rows[e]]] @ wgu[e].t()
+            want = (torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]).to(torch.bfloat16).float() @ wd[e].t()
+            assert float((got[lo:lo + rows[e]] - want).abs().max()) < 2 ** -6 * float(want.abs().max()), f"plan {i} expert {e}"
+        del plan
