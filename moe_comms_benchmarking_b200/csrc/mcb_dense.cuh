@@ -430,12 +430,12 @@ __device__ __forceinline__ GatheredRows agv_device(const McbCtx& c, const McbAgv
   }
   const long long start = (long long)bid * blockDim.x + threadIdx.x;
   const long long stride = (long long)nact * blockDim.x;
-  if (c.world == 1) {        // no peer to meet either
+  if (c.world == 1 && offset == 0) {        // no peer to meet; from row 0 on the packs are aligned whatever the rows hold
     __shared__ LocalRanges r;
     if (threadIdx.x == 0)
       for (int t = 0; t < LocalRanges::R; ++t) {
         const bool used = t < a.num_tensors;
-        r.set(t, used ? a.src[t] : nullptr, used ? c.heap_local + a.dst_off[t] + (uint64_t)offset * a.row_bytes[t] : nullptr, 0,
+        r.set(t, used ? a.src[t] : nullptr, used ? c.heap_local + a.dst_off[t] : nullptr, 0,
               used ? (long long)n * a.row_bytes[t] : 0);
       }
     __syncthreads();

@@ -173,3 +173,26 @@ def test_bench_contract_one_gpu():
     # the real-expert path and the all-to-all dispatcher are timed by child jobs and reported beside the headline
     assert set(line["fused_ms_by_global_batch"]) == {"64", "512", "4096"}, line.get("fused_detail")
     assert set(line["a2a_ms_by_global_batch"]) == {"1", "64", "512", "8192"}, line["a2a_ms_by_global_batch"]
+
+
+@pytest.mark.parametrize("K", [3, 22])           # rows of 12 and 24, 88 and 176 bytes: at most offsets not on a 16-byte boundary
+@pytest.mark.parametrize("offset", [0, 1, 2, 5])
+def test_all_gather_at_a_row_offset(world1, K, offset):
+    """Step metadata of the caller's own that puts this rank's rows behind `offset` others in the gathered tensors."""
+    from moe_comms_benchmarking_b200.ops.dense import AllGatherVPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    cap, n, H = 70, 61, 264
+    heap = SymmetricHeap(world1, 1 << 20, "cuda:0")
+    srcs = [torch.randn(cap, H, device="cuda:0").to(torch.bfloat16), torch.randint(0, 512, (cap, K), device="cuda:0"),
+            torch.rand(cap, K, device="cuda:0")]
+    dsts = [heap.alloc(f"d{i}", list(s.shape), s.dtype) for i, s in enumerate(srcs)]
+    meta = torch.tensor([offset + n, offset, n, 1], dtype=torch.int32, device="cuda:0")
+    plan = AllGatherVPlan(heap, dsts, srcs, torch.tensor([n], dtype=torch.int32, device="cuda:0"), meta, cap)
+    for d in dsts:
+        d.tensor.fill_(7)
+    plan.launch()
+    torch.cuda.synchronize()
+    heap.check_status()
+    for d, s in zip(dsts, srcs):
+        assert torch.equal(d.tensor[offset:offset + n], s[:n])
+        assert bool((d.tensor[:offset] == 7).all()) and bool((d.tensor[offset + n:] == 7).all())
