@@ -33,8 +33,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1) expe
   ffn_setup<false>(maps.map);
   pdl_wait();
   pdl_launch_dependents();
-  ffn_device(a, maps.map);
-  ffn_teardown();
+  const bool copied = ffn_device(a, maps.map);
+  ffn_teardown(a, copied);
 }
 
 template <bool EMU>
@@ -85,8 +85,8 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant_
   target += gridDim.x;
   stamp(3);
   stamp(4);
-  ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
-  ffn_teardown();
+  const bool copied = ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
+  ffn_teardown(p.ffn, copied);
   stamp(5);
   meet();                                                   // every y row is written before any is summed
   stamp(6);

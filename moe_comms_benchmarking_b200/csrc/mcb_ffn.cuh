@@ -237,11 +237,21 @@ __device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
   tc_fence_after();
 }
 
-// After it: TMEM back.  Nobody leaves before the other CTA of the pair is done with this one's shared memory.
-__device__ __forceinline__ void ffn_teardown() {
+// After it: TMEM back.  Nobody leaves before the other CTA of the pair is done with this one's shared memory.  `copied` is
+// what ffn_run returned: the last CTA out leaves the counters of the row copy at zero for the next launch.  A CTA counts
+// itself out behind the barrier: all its warps have added to the first counter and are done waiting for it.
+__device__ __forceinline__ void ffn_teardown(const McbFfnArgs& a, bool copied) {
   const FfnSmem sm;
   tc_fence_before();
   __syncthreads();
+  if (copied && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1) {
+      a.sync[0] = 0;
+      a.sync[1] = 0;
+      __threadfence();
+    }
+  }
   if (*sm.abort_flag) __nanosleep(50000);            // let any copy still in flight land before the CTA goes away
   cluster_sync();
   if (threadIdx.x >= 32 && threadIdx.x < 64) {
@@ -578,20 +588,13 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
   }
-  if (!gather && threadIdx.x == 0) {       // the last CTA out leaves the copy's counters at zero for the next launch
-    __threadfence();
-    if (atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1) {
-      a.sync[0] = 0;
-      a.sync[1] = 0;
-      __threadfence();
-    }
-  }
 }
 
 // Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
 // ffn_teardown, with the experts' offsets in the shared memory of FfnSmem::off (visible to all threads) and the largest
-// number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.
-__device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
+// number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.  Returns whether the token rows were copied
+// into pair order, for ffn_teardown.
+__device__ __forceinline__ bool ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
   const FfnSmem sm;
   const int E = a.num_local_experts;
   if (max_rows < 1) max_rows = 1;
@@ -610,13 +613,14 @@ __device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* 
   const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 31) & ~31);
   if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, maps, plan, n_slot, ready);
   else ffn_roles<1>(a, maps, plan, n_slot, ready);
+  return n_slot > kFfnGatherN;
 }
 
 // The same after a routing of its own launch, whose results are in global memory.
-__device__ __forceinline__ void ffn_device(const McbFfnArgs& a, const CUtensorMap* maps) {
+__device__ __forceinline__ bool ffn_device(const McbFfnArgs& a, const CUtensorMap* maps) {
   const FfnSmem sm;
   for (int e = threadIdx.x; e <= a.num_local_experts; e += blockDim.x) sm.off[e] = a.expert_offset[e];
-  ffn_run(a, maps, *a.max_rows, FfnReady{nullptr, 0});
+  return ffn_run(a, maps, *a.max_rows, FfnReady{nullptr, 0});
 }
 
 }  // namespace mcb

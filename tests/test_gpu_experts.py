@@ -445,3 +445,29 @@ def test_expert_ffn_plan_at_once_on_another_stream(world1, rows):
             want = (torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]).to(torch.bfloat16).float() @ wd[e].t()
             assert float((got[lo:lo + rows[e]] - want).abs().max()) < 2 ** -6 * float(want.abs().max()), f"plan {i} expert {e}"
         del plan
+
+
+@pytest.mark.parametrize("grid", [2, 6, 148])
+def test_expert_ffn_row_copy_counters_return(world1, grid):
+    """Launches back to back whose token rows are copied into pair order, with fewer and with more CTA pairs than units: the
+    counters of the copy are back at zero, and the last launch is as right as the first."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, H, I = 130, 256, 128
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    idx = (torch.arange(T, device=DEV) >= 70).long().view(T, 1)
+    route = RouteBuffers(T, 1, 2, DEV)
+    weights = ExpertWeights(2, H, I, DEV, seed=9, std=0.05)
+    act, y = torch.zeros(T, I, dtype=torch.bfloat16, device=DEV), torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)
+    rp = RoutePlan(route, idx, torch.ones(T, 1, device=DEV), torch.tensor([T], dtype=torch.int32, device=DEV), 0, heap.status)
+    plan = ExpertFfnPlan(weights, route, x, act, y, heap.status, grid=grid)
+    rows = []
+    for n in (1, 60):
+        for _ in range(n):
+            rp.launch(); plan.launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        assert route.sync.tolist() == [0] * 4
+        rows.append(y[route.pair_pos.flatten().long()].clone())
+    assert torch.equal(rows[0], rows[1])            # a token's row does not depend on its place among its expert's rows
