@@ -128,7 +128,7 @@ def make_ffn_tmaps(weights: "ExpertWeights", x: torch.Tensor, act: torch.Tensor,
     raw = (C.c_uint8 * (_ext.FFN_TMAPS * 128 + 64))()
     addr = (C.addressof(raw) + 63) & ~63
     lib = _ext.require()
-    _ext.check(lib.mcb_make_ffn_tmaps(C.c_void_p(addr), C.c_void_p(x.data_ptr()), C.c_uint64(x.shape[0]),
+    _ext.check(lib.mcb_make_ffn_tmaps(C.c_void_p(addr), C.c_void_p(x.data_ptr()), C.c_uint64(x.numel() // weights.hidden),
                                       C.c_void_p(act.data_ptr()), C.c_void_p(y.data_ptr()),
                                       C.c_uint64(min(act.shape[0], y.shape[0])),
                                       C.c_void_p(weights.w1.data_ptr()), C.c_void_p(weights.w2.data_ptr()),

@@ -471,3 +471,26 @@ def test_expert_ffn_row_copy_counters_return(world1, grid):
         assert route.sync.tolist() == [0] * 4
         rows.append(y[route.pair_pos.flatten().long()].clone())
     assert torch.equal(rows[0], rows[1])            # a token's row does not depend on its place among its expert's rows
+
+
+@pytest.mark.parametrize("shape", [(3, 20), (1, 1, 60)])
+def test_expert_ffn_token_rows_of_any_shape(world1, shape):
+    """Token rows as a tensor of more than two dimensions (a parity of gathered rows, say): the pair lists count its rows."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, K, E, H, I = 60, 2, 4, 256, 128
+    x, idx, w = _case(T, E, K, H, I, 23)
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    route = RouteBuffers(T, K, E, DEV)
+    weights = ExpertWeights(E, H, I, DEV, seed=9, std=0.05)
+    RoutePlan(route, idx, w, torch.tensor([T], dtype=torch.int32, device=DEV), 0, heap.status).launch()
+    act = torch.zeros(route.max_pairs, I, dtype=torch.bfloat16, device=DEV)
+    got = []
+    for rows in (x, x.view(*shape, H)):
+        y = torch.full((route.max_pairs, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+        route.ffn_done.zero_()
+        ExpertFfnPlan(weights, route, rows, act, y, heap.status).launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        got.append(y)
+    assert torch.equal(got[0], got[1]) and bool(got[0].count_nonzero() > got[0].numel() // 2)
