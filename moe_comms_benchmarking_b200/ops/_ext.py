@@ -264,6 +264,12 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def current_device() -> int:
+    """The calling thread's current GPU."""
+    import torch
+    return torch._C._cuda_getDevice() if hasattr(torch._C, "_cuda_getDevice") else torch.cuda.current_device()
+
+
 def _raw_stream_getter():
     """The current stream's handle without building a ``torch.cuda.Stream`` (3 us of a launch's 4 us of host time)."""
     import torch

@@ -15,6 +15,8 @@ import torch
 from ..config import Config
 from ..ops import _ext
 
+_Tensor = torch.Tensor
+
 
 class Dispatcher:
     name = "base"
@@ -66,7 +68,8 @@ class Dispatcher:
     def _load_rows(self, hidden, topk_idx, topk_weights, pinned: bool = False):
         """This rank's rows for the next step, stream-ordered: one kernel launch when the three tensors have the
         buffers' types, are contiguous and lie on this GPU (or, with ``pinned``, in pinned host memory); copies
-        otherwise (other types, strides or devices, which ``copy_`` converts)."""
+        otherwise (other types, strides, devices, negated views or subclasses, which ``copy_`` resolves; or another
+        GPU is current, to whose stream the launch would go)."""
         n = hidden.shape[0]
         if n > self.cap:
             raise ValueError(f"{n} local tokens exceed the per-rank capacity {self.cap}")
@@ -78,23 +81,28 @@ class Dispatcher:
             for t, b in enumerate(bufs):
                 a.dst[t] = b.data_ptr()
             a.n_local = self.n_local.data_ptr()
-            self._load_args, self._load_ref = a, C.byref(a)
-            self._load_row = [(b.dtype, b.device, b.shape[1], b.shape[1] * b.element_size()) for b in bufs]
-        a = self._load_args
-        for t, s in enumerate((hidden, topk_idx, topk_weights)):
-            dtype, device, cols, row_bytes = self._load_row[t]
-            ptr = s.data_ptr()
-            if (s.dtype is not dtype or s.shape != (n, cols) or ptr & 3 or not s.is_contiguous()
-                    or not (s.is_pinned() if pinned else s.device == device)):
-                break
-            a.src[t], a.bytes[t] = ptr, n * row_bytes
-        else:
-            a.n = n
-            err = _ext.require().mcb_launch_load_batch(self._load_ref, int(self.pdl), _ext.stream_handle())
-            _ext.check(err, "load_batch")
-            return
+            self._load_args, self._load_ref, self._load_src, self._load_bytes = a, C.byref(a), a.src, a.bytes
+            self._load_device = self.in_hidden.device.index
+            self._load_row = tuple(enumerate((b.dtype, b.device, b.shape[1], b.shape[1] * b.element_size()) for b in bufs))
+        a, src, nbytes = self._load_args, self._load_src, self._load_bytes
+        rows = (hidden, topk_idx, topk_weights)
+        if _ext.current_device() == self._load_device:
+            for t, (dtype, device, cols, row_bytes) in self._load_row:
+                s = rows[t]
+                if (s.dtype is not dtype or s.shape != (n, cols) or not s.is_contiguous() or s.is_neg() or type(s) is not _Tensor
+                        or not (s.is_pinned() if pinned else s.device == device)):
+                    break
+                ptr = s.data_ptr()
+                if ptr & 3:
+                    break
+                src[t], nbytes[t] = ptr, n * row_bytes
+            else:
+                a.n = n
+                err = _ext.require().mcb_launch_load_batch(self._load_ref, int(self.pdl), _ext.stream_handle())
+                _ext.check(err, "load_batch")
+                return
         if n:
-            for b, s in zip(bufs, (hidden, topk_idx, topk_weights)):
+            for b, s in zip(bufs, rows):
                 b[:n].copy_(s, non_blocking=True)
         self.n_local.fill_(n)
 
