@@ -109,13 +109,19 @@ __device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteS
   mx = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 31) { m.scan[warp] = r_inc; m.scan[32 + warp] = t_inc; m.scan[64 + warp] = mx; }
   __syncthreads();
-  int run = r_inc - rows, tile = t_inc - tiles, total = 0, total_tiles = 0;
-  for (int w = 0; w < nw; ++w) {
-    if (w < warp) { run += m.scan[w]; tile += m.scan[32 + w]; }
-    total += m.scan[w];
-    total_tiles += m.scan[32 + w];
-    mx = m.scan[64 + w] > mx ? m.scan[64 + w] : mx;
+  // Every warp scans the warps' sums for itself, lane w holding those of warp w.
+  int run = r_inc - rows, tile = t_inc - tiles;
+  r_inc = lane < nw ? m.scan[lane] : 0;
+  t_inc = lane < nw ? m.scan[32 + lane] : 0;
+  mx = __reduce_max_sync(0xffffffffu, lane < nw ? m.scan[64 + lane] : 0);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int r = __shfl_up_sync(0xffffffffu, r_inc, o), t = __shfl_up_sync(0xffffffffu, t_inc, o);
+    if (lane >= o) { r_inc += r; t_inc += t; }
   }
+  const int total = __shfl_sync(0xffffffffu, r_inc, 31), total_tiles = __shfl_sync(0xffffffffu, t_inc, 31);
+  const int r_before = __shfl_sync(0xffffffffu, r_inc, warp ? warp - 1 : 0), t_before = __shfl_sync(0xffffffffu, t_inc, warp ? warp - 1 : 0);
+  if (warp) { run += r_before; tile += t_before; }
   for (int e = e0; e < e1; ++e) {
     const int c = m.cnt[e];
     m.off[e] = run;
@@ -183,8 +189,8 @@ __device__ __forceinline__ void route_place(const McbRouteArgs& a, const int64_t
 }
 
 // The whole routing by the blocks of a launch that has nothing else to share a barrier with.  With few entries nobody waits
-// for another block: all count all entries and place their own (one block placing alone: 12.6 us a launch at 11264 entries,
-// now 8.6; 8.4 and 6.7 at 1408); with many the blocks wait for one another on a counter that only grows (the grid must be
+// for another block: all count all entries and place their own (one block alone: 21.9 us a launch at 11264 entries of 512
+// experts, now 5.8; 8.5 and 4.2 at 1408; 3.0 and 3.8 at 128 of 32, where the wider scan shows); with many the blocks wait for one another on a counter that only grows (the grid must be
 // co-resident).  Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.
 __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
   const RouteSmem m(smem);
