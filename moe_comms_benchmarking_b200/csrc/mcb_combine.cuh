@@ -7,9 +7,12 @@
 //   phase B  for the items of block b whose token this rank owns: out = sum over ranks of partial
 //            (multimem.ld_reduce in the switch, or peer loads).
 // A world of one writes phase A's sums straight to the output.  A warp serves an item with 1, 2 or 4 16-byte packs per
-// lane (32, 64 or 128 packs per item), as many as still give every warp of the grid an item, and keeps four to eight
-// pair rows in flight: with one token and two rows in flight the sum over 22 rows was a chain of eleven trips to L2
-// (7.9 us of a layer, now 2), with one warp per token 190 rows of 7168 values occupied an eighth of the chip (46 us, now 9).
+// lane (32, 64 or 128 packs per item), as many as still give every warp of the grid an item.  With one or two packs it keeps
+// eight or four pair rows in flight: with one token and two rows in flight the sum over 22 rows was a chain of eleven trips
+// to L2 (7.9 us of a layer, now 2), with one warp per token 190 rows of 7168 values occupied an eighth of the chip (46 us,
+// now 9).  With four packs every warp has an item and memory is the limit: one row at a time, with ordinary loads.  4096 rows
+// of 1024 values, 8 pairs each: 9.5 us (18.4 with four rows in flight and streaming loads, 11.4 with four rows, 12.4
+// with streaming loads); 22 pairs each, 184 MB of them: 39.6 (53, 61, 34).
 // Call from all threads of the block; works for any block size that is a multiple of 32.
 #pragma once
 #include "mcb_barrier.cuh"
@@ -52,7 +55,7 @@ struct CombineShape {
 // PL = packs per lane.
 template <int PL>
 __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineArgs& a, const CombineShape& s, uint32_t ep) {
-  constexpr int R = PL == 1 ? 8 : 4;               // pair rows in flight
+  constexpr int R = PL == 1 ? 8 : PL == 2 ? 4 : 1;               // pair rows in flight
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, bid = blockIdx.x;
   const uint8_t* y = reinterpret_cast<const uint8_t*>(a.y);
   const bool alone = c.world == 1;
@@ -83,7 +86,8 @@ __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineA
 #pragma unroll
           for (int u = 0; u < PL; ++u) {
             const int p = p0 + u * 32;
-            v[r][u] = live && p < s.packs ? ld_v4_stream(y + (uint64_t)pos * s.row_bytes + (uint64_t)p * 16) : make_uint4(0, 0, 0, 0);
+            const uint8_t* at = y + (uint64_t)pos * s.row_bytes + (uint64_t)p * 16;
+            v[r][u] = live && p < s.packs ? (PL == 4 ? ld_v4(at) : ld_v4_stream(at)) : make_uint4(0, 0, 0, 0);
           }
         }
 #pragma unroll
