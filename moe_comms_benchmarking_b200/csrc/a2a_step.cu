@@ -468,8 +468,7 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
   __shared__ int s_prefix[MCB_MAX_RANKS + 1];
   __shared__ int s_cnt[MCB_MAX_RANKS];
   __shared__ int s_max;
-  const int tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
+  const int tid = threadIdx.x, bid = blockIdx.x;
   const int W = c.world, L = a.num_layers;
   pdl_wait();
   pdl_launch_dependents();

@@ -4,12 +4,14 @@
 //   dispatch    every CTA pushes its share of the local tokens to all ranks (multimem.st + cross-GPU
 //               barrier, or flagged packets for small steps)                          mcb_dense.cuh
 //   routing     counts -> offsets -> pair lists for this rank's experts                  mcb_route.cuh
-//   experts     gate/up blocks, then down blocks, one persistent weight stream            mcb_ffn.cuh
+//   experts     gate/up and down units, one persistent weight stream                      mcb_ffn.cuh
 //   combine     per-token pre-sum of the local expert outputs into the symmetric buffer, block-matched
 //               cross-GPU barrier, multimem.ld_reduce of the rows this rank owns       mcb_combine.cuh
 //
-// separated by grid-wide barriers (the launch is cooperative: all CTAs are resident), except that every CTA works out
-// the experts' offsets itself and starts its weight stream before the others have placed their pairs.  The reference
+// The launch is cooperative: all CTAs are resident.  A grid-wide barrier follows the dispatch (not in a world of one that
+// routes by its own inputs) and the experts, and one falls inside the routing of many entries.  None stands between routing
+// and experts: every CTA works out the experts' offsets itself and starts its weight stream at once, and only the roles
+// that read pair lists or token rows wait for the other CTAs.  The reference
 // stops at the identity expert (bench_nvls.py:109-121); its dispatch and combine are the first and the
 // last phase here.  EMU = true runs several ranks inside one launch (gridDim.y = world, each y-slice
 // with its own argument block in device memory), which is how the cross-rank protocol of this kernel
@@ -84,7 +86,7 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant_
   }
   target += gridDim.x;
   stamp(3);
-  stamp(4);
+  stamp(4);                                                  // an empty phase, see McbLayerArgs::trace
   const bool copied = ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
   ffn_teardown(p.ffn, copied);
   stamp(5);

@@ -43,7 +43,6 @@ typedef struct {
 // persistent kernel over the pair lists written by the routing.
 typedef struct {
   const void* x;               // gathered tokens [T, hidden] bf16
-  uint64_t x_row_bytes;
   const int32_t* pair_token;   // [P] pair row -> gathered token
   const float* pair_prob;      // [P] routing weight of each pair row (NULL: 1)
   const int32_t* expert_offset;  // [E_loc + 1] first pair row of each local expert
@@ -75,7 +74,6 @@ typedef struct {
   int32_t num_local_experts;
   int32_t max_tokens;          // capacity of the gathered buffers (bounds check)
   int32_t* expert_count;       // [E_loc]        (scratch, zero between launches)
-  int32_t* expert_cursor;      // [E_loc]        (scratch, zero between launches)
   int32_t* expert_offset;      // [E_loc + 1]    first pair row of each expert
   int32_t* pair_token;         // [P] gathered-token index of each pair row
   float* pair_prob;            // [P] routing weight of each pair row
@@ -130,7 +128,8 @@ typedef struct alignas(64) {
   McbFfnArgs ffn;
   McbCombineArgs cmb;
   // Optional phase trace (null = off): block 0 stores the global timer (ns) at kernel entry and after
-  // dispatch, grid barrier, routing, grid barrier, experts, grid barrier, combine (8 words).
+  // dispatch, grid barrier, routing, grid barrier, experts, grid barrier, combine (8 words).  No barrier stands between
+  // routing and experts: that phase is empty, and the wait for the other blocks' pair lists is part of the experts.
   unsigned long long* trace;
   unsigned long long reserved0;
 } McbLayerArgs;

@@ -82,14 +82,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
       :: "r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
 }
 
-// Bulk copy of a contiguous, 16-byte aligned range of global memory into shared memory (no tensor
-// map, no multicast); completion is counted in bytes on the mbarrier.
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      :: "r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-
 // Asynchronous 16-byte global -> shared copy (L2 only), and "arrive on this mbarrier once all
 // my earlier cp.async copies have landed" (counts as one of the barrier's expected arrivals).
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {

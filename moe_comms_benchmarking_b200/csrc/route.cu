@@ -24,11 +24,9 @@ __global__ void __launch_bounds__(kRouteThreads, 1) route_kernel(const __grid_co
 }
 
 // ------------------------------------------------------------------------------------------------
-// Combine: block b owns the gathered tokens t with t % nact == b on EVERY rank.
-//   phase A  partial[t] = sum over the local (token, k) pairs of y[pair]       (this rank's heap)
-//   barrier  block b of every rank has written its tokens' partial sums
-//   phase B  for the tokens of block b that this rank owns: out = sum over ranks of partial[t]
-//            (multimem.ld_reduce in the switch, or peer loads).
+// Combine as a kernel of its own (mcb_combine.cuh): a block owns slices of the rows of gathered tokens, the same on EVERY
+// rank; it sums the local pairs of its slices, meets the matching block of every rank, and reduces across the ranks what
+// this rank owns.
 // ------------------------------------------------------------------------------------------------
 template <bool EMU>
 __global__ void __launch_bounds__(512) combine_kernel(const __grid_constant__ McbCtx ctx_p,

@@ -135,7 +135,7 @@ class McbRouteArgs(C.Structure):
     _fields_ = [
         ("topk_idx", _vp), ("topk_w", _vp), ("num_tokens", _vp),
         ("topk", _i32), ("expert_begin", _i32), ("num_local_experts", _i32), ("max_tokens", _i32),
-        ("expert_count", _vp), ("expert_cursor", _vp), ("expert_offset", _vp),
+        ("expert_count", _vp), ("expert_offset", _vp),
         ("pair_token", _vp), ("pair_prob", _vp), ("pair_pos", _vp),
         ("tile_expert", _vp), ("tile_row0", _vp), ("tile_rows", _vp), ("num_m_tiles", _vp), ("sync", _vp),
         ("max_pairs", _i32), ("max_tiles", _i32), ("status", _vp), ("timeout_ns", _u64),
@@ -145,7 +145,7 @@ class McbRouteArgs(C.Structure):
 
 class McbFfnArgs(C.Structure):
     _fields_ = [
-        ("x", _vp), ("x_row_bytes", _u64), ("pair_token", _vp), ("pair_prob", _vp), ("expert_offset", _vp),
+        ("x", _vp), ("pair_token", _vp), ("pair_prob", _vp), ("expert_offset", _vp),
         ("max_rows", _vp), ("act", _vp), ("y", _vp), ("ffn_done", _vp),
         ("num_local_experts", _i32), ("hidden", _i32), ("intermediate", _i32), ("reserved0", _i32),
         ("status", _vp), ("timeout_ns", _u64), ("w1", _vp), ("w2", _vp), ("tmaps", _vp), ("sync", _vp),

@@ -145,7 +145,6 @@ class RouteBuffers:
         self.max_tiles = num_local_experts + self.max_pairs // BLOCK_M + 1
         i32 = dict(dtype=torch.int32, device=device)
         self.expert_count = torch.zeros(num_local_experts, **i32)
-        self.expert_cursor = torch.zeros(num_local_experts, **i32)
         self.expert_offset = torch.zeros(num_local_experts + 1, **i32)
         self.pair_token = torch.zeros(max(self.max_pairs, 1), **i32)
         self.pair_prob = torch.zeros(max(self.max_pairs, 1), dtype=torch.float32, device=device)
@@ -175,7 +174,7 @@ class RoutePlan:
         a = _ext.McbRouteArgs()
         a.topk_idx, a.topk_w, a.num_tokens = topk_idx.data_ptr(), _ext.ptr(topk_w), num_tokens.data_ptr()
         a.topk, a.expert_begin, a.num_local_experts, a.max_tokens = bufs.topk, int(expert_begin), bufs.E, bufs.max_tokens
-        for f in ("expert_count", "expert_cursor", "expert_offset", "pair_token", "pair_prob", "pair_pos",
+        for f in ("expert_count", "expert_offset", "pair_token", "pair_prob", "pair_pos",
                   "tile_expert", "tile_row0", "tile_rows", "num_m_tiles", "sync", "max_rows", "ffn_done"):
             setattr(a, f, getattr(bufs, f).data_ptr())
         a.max_pairs, a.max_tiles = bufs.max_pairs, bufs.max_tiles
@@ -319,7 +318,7 @@ class ExpertFfnPlan:
         self._keep = (route, x, act, y, status, tmaps)
         a = _ext.McbFfnArgs()
         a.tmaps, a.sync = tmaps[1], route.sync[2:].data_ptr()
-        a.x, a.x_row_bytes = x.data_ptr(), H * 2
+        a.x = x.data_ptr()
         a.pair_token, a.pair_prob = route.pair_token.data_ptr(), route.pair_prob.data_ptr()
         a.expert_offset, a.max_rows = route.expert_offset.data_ptr(), route.max_rows.data_ptr()
         a.act, a.y, a.ffn_done = act.data_ptr(), y.data_ptr(), route.ffn_done.data_ptr()
@@ -379,6 +378,8 @@ class MoeLayerPlan:
         if self._ctx_version != id(self.heap.ctx()):      # the heap's context was rebuilt (e.g. a new timeout)
             self._fill()
 
+    # The barrier between routing and experts is gone: its phase is empty, and the wait for the other blocks' pair
+    # lists is part of the experts.
     PHASES = ("dispatch", "grid barrier", "routing", "grid barrier", "experts", "grid barrier", "combine")
 
     def phase_times(self):

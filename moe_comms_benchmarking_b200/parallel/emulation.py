@@ -212,13 +212,13 @@ class EmuWorld:
             ro.topk_idx, ro.topk_w = d["dst"][1].tensor.data_ptr(), d["dst"][2].tensor.data_ptr()
             ro.num_tokens = d["step_meta"].data_ptr()
             ro.topk, ro.expert_begin, ro.num_local_experts, ro.max_tokens = topk, d["expert_begin"], route.E, route.max_tokens
-            for f in ("expert_count", "expert_cursor", "expert_offset", "pair_token", "pair_prob", "pair_pos",
+            for f in ("expert_count", "expert_offset", "pair_token", "pair_prob", "pair_pos",
                       "tile_expert", "tile_row0", "tile_rows", "num_m_tiles", "sync", "max_rows", "ffn_done"):
                 setattr(ro, f, getattr(route, f).data_ptr())
             ro.max_pairs, ro.max_tiles = route.max_pairs, route.max_tiles
             ro.status, ro.timeout_ns = self.status[r].data_ptr(), int(timeout_s * 1e9)
             ff = p.ffn
-            ff.x, ff.x_row_bytes = d["dst"][0].tensor.data_ptr(), w.hidden * 2
+            ff.x = d["dst"][0].tensor.data_ptr()
             ff.pair_token, ff.pair_prob = route.pair_token.data_ptr(), route.pair_prob.data_ptr()
             ff.expert_offset, ff.max_rows = route.expert_offset.data_ptr(), route.max_rows.data_ptr()
             ff.act, ff.y, ff.ffn_done = d["act"].data_ptr(), d["y"].data_ptr(), route.ffn_done.data_ptr()

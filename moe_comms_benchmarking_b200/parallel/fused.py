@@ -12,9 +12,9 @@ expert computation the transport exists for.  Per layer and rank:
     combine    out[t] = sum_ranks sum_local-pairs y               csrc/route.cu   combine_kernel
 
 By default the whole layer is ONE cooperative kernel (``moe_layer_kernel`` in csrc/ffn.cu: dispatch,
-grid barrier, routing, grid barrier, the grouped FFN with the weights as the M operand and both
-projections in one persistent weight stream, grid barrier, combine), and a decode step is issued by
-one native call (count exchange + one launch per layer).  ``layer_kernel=False`` selects the older
+routing, the grouped FFN with the weights as the M operand and both projections in one persistent weight
+stream, combine; grid barriers behind the dispatch and the experts, none between routing and experts),
+and a decode step is issued by one native call (count exchange + one launch per layer).  ``layer_kernel=False`` selects the older
 form with the tokens as the M operand: two kernels per layer (``dispatch_route_fc1_kernel`` and
 ``fc2_combine_kernel`` in csrc/gemm.cu), or five with ``fuse_dispatch=False`` / ``fuse_combine=False``.
 

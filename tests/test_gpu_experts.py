@@ -86,10 +86,10 @@ def test_route_fc1_fc2_combine_against_oracle(world1, T, E, K, H, I):
                                             (3, 8, 2, 256, 128, 148), (4500, 8, 4, 256, 128, 148),
                                             (400, 8, 2, 256, 256, 3), (400, 8, 2, 256, 256, 5)])
 def test_expert_ffn_weights_as_m_against_oracle(world1, T, E, K, H, I, grid):
-    """The grouped FFN with the weights as the M = 128 operand (gate/up + SwiGLU + down in one
-    persistent launch): experts with no token, with a few, and with more than 256 (several passes
-    over the same weight block), more units than CTAs, interleaved gate/up rows; about 100 tokens per
-    expert (one block per pipeline stage, the next unit's gather indices fetched under the current one)."""
+    """The grouped FFN with the weights as the M operand of a CTA pair (gate/up + SwiGLU + down in one
+    persistent launch): experts with no token, with a few (rows gathered by TMA), with more than 64 (rows copied
+    into pair order) and more than 256 (several chunks), more units than CTA pairs, an odd grid, interleaved
+    gate/up rows."""
     from moe_comms_benchmarking_b200.ops import oracle
     from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
     from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
@@ -195,16 +195,16 @@ def test_moe_layer_kernel_emulated_ranks(lib, W, B, ll_rows):
 
 
 def test_fused_dispatcher_routes_more_than_one_block_of_entries(world1):
-    """More (token, expert) entries than one block routes alone, so the multi-block routing branch
-    (histogram per block, hand-over through the last block, cursors in global memory) runs INSIDE the
-    cooperative layer kernel; a sample of tokens is checked against the oracle."""
+    """More (token, expert) entries than every block counts by itself, so the routing that shares counts through global
+    counters and a grid-wide barrier runs INSIDE the cooperative layer kernel; a sample of tokens is checked against
+    the oracle."""
     from moe_comms_benchmarking_b200.config import Config
     from moe_comms_benchmarking_b200.parallel.fused import FusedExpertDispatcher
     from moe_comms_benchmarking_b200.utils.inputs import make_inputs
     cfg = Config(num_experts=16, topk=8, hidden=256, intermediate=128, ep_size=1, per_rank_cap=2304)
     d = FusedExpertDispatcher(cfg, world1, num_layers=1, weight_budget_gb=0.5)
     d.build()
-    h, i, w = make_inputs(cfg, 2304, DEV)          # 18432 entries > 16384
+    h, i, w = make_inputs(cfg, 2304, DEV)          # 18432 entries, 16 per thread are 6144
     d.setup_batch(h, i, w)
     for _ in range(2):
         d.decode_step(1)
