@@ -14,7 +14,7 @@
 //     image of their shared-memory tile, so a tile is contiguous in memory), activations as boxes of rows.
 //     Token rows come four at a time through the pair -> token list (tile::gather4, the routing permute fused
 //     into the load) while an expert has at most kFfnGatherN tokens.  One gather costs its issuing thread about
-//     100 cycles whatever it moves, which at more tokens is slower than the MMAs it feeds, so there the
+//     100 cycles whatever it moves, which at many tokens is slower than the MMAs it feeds, so there the
 //     rows are first copied into pair order (into the memory of the expert outputs, which an expert's down
 //     units overwrite only after all its gate/up units have read it) and come as boxes too;
 //   * work units are listed per CTA pair in shared memory before the roles start: experts without tokens are
@@ -31,15 +31,20 @@
 //     are neighbours in time), and without it 138 MB of them threw the kernel's own code, its inputs, the pair lists and the
 //     activations out of L2, so that every phase of the next layer began with trips to HBM.  88 layers of one token
 //     4595 -> 3757 us (dispatch 6.8 -> 3.8, experts 30.0 -> 27.2, combine 5.8 -> 3.1 us a layer), a layer of 37 tokens
-//     406 -> 384 us, of 190 wide tokens 454 -> 435 us, no difference at 4096;
+//     406 -> 384 us, of 190 wide tokens 454 -> 435 us, no difference at 4096.  Also with 8 sets of only 50 or 75 MB in use a
+//     layer is faster with it (30.5 -> 28.1, 36.6 -> 33.4 us), and an expert of several chunks (16 experts at 375 tokens
+//     47.6 -> 44.7); it costs only where ONE set of less than L2 is run again and again (75 MB 12.6 -> 17.3, 100 MB
+//     18.3 -> 21.2), which no launch can know;
 //   * weights and tokens have producer warps of their own, so the weight stream runs on while a down unit
 //     waits; eight epilogue warps read the accumulators with tcgen05.ld (a lane holds one output feature),
 //     turn them through a small shared-memory tile and store 16 bytes per lane, feature-contiguous;
 //   * every mbarrier wait is bounded and reports through the status words.
 // Measured on one B200 with 64 experts of 1024 x 1024 (402.7 MB of weights), against one CTA per unit of 128 weight rows
-// with token rows copied by cp.async and units numbered over all experts: 67 us (66 before) at 3 tokens per expert,
-// where the weight stream is the limit; 97 (113) at 173 and 150 (204) at 350 tokens per expert, where the SMs' reads from
-// L2 are; with skewed routing (8191 tokens, Zipf 1.2) 222 (536).  With 22 of 512 experts in use 36 (52).
+// with token rows copied by cp.async and units numbered over all experts: 64 us (66 before) at 3 tokens per expert,
+// where the weight stream is the limit; 89 (113) at 173 and 157 (204) at 350 tokens per expert; with skewed routing
+// (8191 tokens, Zipf 1.2) 222 (536).  With 22 of 512 experts in use 36 (52).  Launches of a few microseconds lose what a CTA
+// pair costs to set up and take down, and to gather: 8 experts of 512 x 256 at 1 / 32 / 128 tokens per expert 8.3 / 9.6 /
+// 12.9 us (7.2 / 7.7 / 10.4).
 #pragma once
 #include "mcb_tc.cuh"
 
@@ -51,7 +56,10 @@ constexpr int kFfnThreads = 32 * (2 + kFfnEpiWarps + kFfnTokWarps);      // weig
 constexpr int kFfnRowsM = 256;              // weight rows per unit (128 in each CTA of the pair)
 constexpr int kFfnBlockK = 64;              // 128 bytes of bf16
 constexpr int kFfnMaxN = 256;               // tokens per chunk
-constexpr int kFfnGatherN = 64;             // largest chunk whose token rows are gathered by TMA
+// Largest chunk whose token rows are gathered by TMA.  64 experts of 1024 x 1024, largest 90 / 110 / 128 tokens: 66 / 67 / 70 us
+// (70 / 71 / 75 with the copy into pair order from 65 on), 32 of 1024 x 512 at 64 tokens 24.3 (27.2), 8 of 7168 x 2048 at
+// 110: 111 (117); no difference with one popular expert, whose size decides for all.
+constexpr int kFfnGatherN = 128;
 constexpr int kFfnDoubleN = 128;            // up to this many tokens per chunk a stage holds two 64-column blocks
 constexpr int kFfnMaxStages = 10;
 constexpr int kFfnABytes = 128 * kFfnBlockK * 2;                 // 16 KiB of weights per CTA and 64-column block
@@ -172,8 +180,9 @@ __device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16
   return total;
 }
 
-// Down units follow their gate/up units at once-per-expert order only while the activations between them fit
-// comfortably in L2 (126 MB, shared with the weight stream, the tokens and the expert outputs).
+// Bytes of activations up to which all gate/up units come before all down units.  64 experts of 1024 x 1024 with 12 to 65 MB
+// of activations ran equally fast in either order (within the 6 % by which two runs differ); the line keeps the
+// activations well inside L2 (126 MB, shared with the weight stream, the tokens and the expert outputs).
 constexpr long long kFfnActL2Bytes = 24ll << 20;
 
 

@@ -22,7 +22,8 @@ constexpr int kRouteThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
 // Shared memory of a routing block: counts, own begins (later cursors), offsets, scan scratch.
 constexpr int kRouteSmemWords = 3 * kMaxLocalExperts + 1 + 3 * 32;
-// Entries per thread up to which every block counts all of them.
+// Entries per thread up to which every block counts all of them.  Layer kernel (384 threads), 64 experts: 4000 entries 37.4 us
+// (39.6 with the counts shared through global counters), 6080 42.1 (43.8), 8000 45.5 (45.4), 16000 62.8 (61.8), 24000 76.7 (72.7).
 constexpr int kRouteAllPerThread = 16;
 
 struct RouteSmem {
