@@ -94,7 +94,7 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant_
   stamp(6);
   if (blockIdx.x == gridDim.x - 1)                          // every block has read the counters of the routing
     for (int e = threadIdx.x; e < p.route.num_local_experts; e += blockDim.x) p.route.expert_count[e] = 0;
-  combine_body(c, p.cmb, ll_launch);      // partial sums alternate between two buffers, layer by layer
+  combine_body<false>(c, p.cmb, ll_launch);      // partial sums alternate between two buffers, layer by layer
   stamp(7);
   launch_end(c, MCB_SITE_FC1_FUSED, ll_launch, arrivals);
 }

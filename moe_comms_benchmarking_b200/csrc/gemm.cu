@@ -274,7 +274,7 @@ fc2_combine_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
   const uint32_t launch = launch_begin(c, MCB_SITE_FUSED_FC1);
   uint32_t* arrivals = epoch_ptr(c, MCB_SITE_LAYER, 0);
   grid_sync(c, arrivals, gridDim.x);
-  combine_body(c, cmb);
+  combine_body<false>(c, cmb);
   launch_end(c, MCB_SITE_FUSED_FC1, launch, arrivals);
 }
 

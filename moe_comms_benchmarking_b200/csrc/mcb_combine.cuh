@@ -10,9 +10,12 @@
 // lane (32, 64 or 128 packs per item), as many as still give every warp of the grid an item.  With one or two packs it keeps
 // eight or four pair rows in flight: with one token and two rows in flight the sum over 22 rows was a chain of eleven trips
 // to L2 (7.9 us of a layer, now 2), with one warp per token 190 rows of 7168 values occupied an eighth of the chip (46 us,
-// now 9).  With four packs every warp has an item and memory is the limit: one row at a time, with ordinary loads.  4096 rows
-// of 1024 values, 8 pairs each: 9.5 us (18.4 with four rows in flight and streaming loads, 11.4 with four rows, 12.4
-// with streaming loads); 22 pairs each, 184 MB of them: 39.6 (53, 61, 34).
+// now 9).  With four packs every warp has an item and memory is the limit; what is best there depends on the kernel around:
+//   combine_kernel (ALONE)  one row at a time, with ordinary loads.  4096 rows of 1024 values, 8 pairs each: 9.5 us (18.4 with
+//                           four rows in flight and streaming loads, 28 with two, 11.4 with four and ordinary loads); 22 pairs
+//                           each, 184 MB of them: 39.6 (53, 90, 61);
+//   behind the experts      two rows, with streaming loads.  The combine of the layer kernel at 4096 / 2048 tokens of 22 pairs:
+//                           41 / 24 us (44 / 26 with four rows, 59 / 37 with one and ordinary loads, 53 / 32 with one).
 // Call from all threads of the block; works for any block size that is a multiple of 32.
 #pragma once
 #include "mcb_barrier.cuh"
@@ -53,9 +56,9 @@ struct CombineShape {
 };
 
 // PL = packs per lane.
-template <int PL>
+template <int PL, bool ALONE>
 __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineArgs& a, const CombineShape& s, uint32_t ep) {
-  constexpr int R = PL == 1 ? 8 : PL == 2 ? 4 : 1;               // pair rows in flight
+  constexpr int R = PL == 1 ? 8 : PL == 2 ? 4 : (ALONE ? 1 : 2);       // pair rows in flight
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, bid = blockIdx.x;
   const uint8_t* y = reinterpret_cast<const uint8_t*>(a.y);
   const bool alone = c.world == 1;
@@ -87,7 +90,7 @@ __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineA
           for (int u = 0; u < PL; ++u) {
             const int p = p0 + u * 32;
             const uint8_t* at = y + (uint64_t)pos * s.row_bytes + (uint64_t)p * 16;
-            v[r][u] = live && p < s.packs ? (PL == 4 ? ld_v4(at) : ld_v4_stream(at)) : make_uint4(0, 0, 0, 0);
+            v[r][u] = live && p < s.packs ? (PL == 4 && ALONE ? ld_v4(at) : ld_v4_stream(at)) : make_uint4(0, 0, 0, 0);
           }
         }
 #pragma unroll
@@ -123,6 +126,7 @@ __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineA
   }
 }
 
+template <bool ALONE>
 __device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineArgs& a, uint32_t parity = 0u) {
   CombineShape s;
   s.T = a.step_meta[0];
@@ -143,9 +147,9 @@ __device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineAr
   s.nact = items < (long long)gridDim.x ? (int)items : (int)gridDim.x;
   if ((int)blockIdx.x >= s.nact) return;
   const uint32_t ep = *epoch_ptr(c, a.site, blockIdx.x);
-  if (pl == 4) combine_items<4>(c, a, s, ep);
-  else if (pl == 2) combine_items<2>(c, a, s, ep);
-  else combine_items<1>(c, a, s, ep);
+  if (pl == 4) combine_items<4, ALONE>(c, a, s, ep);
+  else if (pl == 2) combine_items<2, ALONE>(c, a, s, ep);
+  else combine_items<1, ALONE>(c, a, s, ep);
 }
 
 }  // namespace mcb

@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(512) combine_kernel(const __grid_constant__ Mc
   const McbCombineArgs& a = EMU ? eargs[blockIdx.y] : args_p;
   pdl_wait();
   pdl_launch_dependents();
-  combine_body(c, a);
+  combine_body<true>(c, a);
 }
 
 }  // namespace mcb
