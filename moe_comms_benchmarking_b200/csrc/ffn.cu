@@ -35,8 +35,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kFfnThreads, 1) expe
   ffn_setup<false>(maps.map);
   pdl_wait();
   pdl_launch_dependents();
-  const bool copied = ffn_device(a, maps.map);
-  ffn_teardown(a, copied);
+  ffn_device(a, maps.map);
+  ffn_teardown();
 }
 
 template <bool EMU>
@@ -87,8 +87,8 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant_
   target += gridDim.x;
   stamp(3);
   stamp(4);                                                  // an empty phase, see McbLayerArgs::trace
-  const bool copied = ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
-  ffn_teardown(p.ffn, copied);
+  ffn_run(p.ffn, maps, max_rows, FfnReady{arrivals, (int)target});
+  ffn_teardown();
   stamp(5);
   meet();                                                   // every y row is written before any is summed
   stamp(6);
@@ -122,7 +122,7 @@ static bool configure_ffn_kernels() {
 }
 
 static int check_ffn_args(const McbFfnArgs* a) {
-  if (!a || !a->x || !a->pair_token || !a->expert_offset || !a->max_rows || !a->act || !a->y || !a->ffn_done || !a->sync) return 1;
+  if (!a || !a->x || !a->pair_token || !a->expert_offset || !a->max_rows || !a->act || !a->y || !a->ffn_done) return 1;
   if (!a->w1 || !a->w2 || (reinterpret_cast<uintptr_t>(a->w1) & 15) || (reinterpret_cast<uintptr_t>(a->w2) & 15)) return 1;
   if (a->num_local_experts < 1 || a->num_local_experts > kFfnMaxExperts || a->hidden < 256 || a->hidden % 256 || a->intermediate < 128 || a->intermediate % 128) return 1;
   if (!a->tmaps || (reinterpret_cast<uintptr_t>(a->tmaps) & 63)) return 1;
@@ -132,17 +132,15 @@ static int check_ffn_args(const McbFfnArgs* a) {
 // The kernels run in CTA pairs: an odd grid is rounded down, one CTA is rounded up.
 static int pair_grid(int grid) { return grid < 2 ? 2 : grid & ~1; }
 
-// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory.  x: token rows; act, y: activations and expert outputs; w1, w2: the packed weights.
-int mcb_make_ffn_tmaps(void* out, const void* x, uint64_t x_rows, const void* act, const void* y, uint64_t pair_rows, const void* w1,
-                       const void* w2, int experts, int hidden, int intermediate) {
+// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory.  x: token rows; act: activations; w1, w2: the packed weights.
+int mcb_make_ffn_tmaps(void* out, const void* x, uint64_t x_rows, const void* act, uint64_t pair_rows, const void* w1, const void* w2,
+                       int experts, int hidden, int intermediate) {
   uint8_t* o = reinterpret_cast<uint8_t*>(out);
   const uint64_t E = experts, H = hidden, I = intermediate;
   if (!out || experts < 1 || hidden % 256 || intermediate % 128) return (int)cudaErrorInvalidValue;
   int err = make_tmap_bf16(o + MCB_FFN_MAP_X * 128, x, x_rows, H, 1);
-  for (int b = 0; b < 8 && !err; ++b) {
-    err = make_tmap_bf16(o + (MCB_FFN_MAP_ACT + b) * 128, act, pair_rows, I, 8 * (b + 1));
-    if (!err) err = make_tmap_bf16(o + (MCB_FFN_MAP_XP + b) * 128, y, pair_rows, H, 8 * (b + 1));
-  }
+  for (int b = 0; b < kFfnMaxGroups && !err; ++b)
+    err = make_tmap_bf16(o + (MCB_FFN_MAP_ACT + b) * 128, act, pair_rows, I, 4 * (b + 1));
   for (int d = 0; d < 2 && !err; ++d) {
     err = make_tmap_flat(o + (MCB_FFN_MAP_W1 + 2 * d) * 128, w1, E * 2 * I * H * 2, 8 * (d + 1));
     if (!err) err = make_tmap_flat(o + (MCB_FFN_MAP_W2 + 2 * d) * 128, w2, E * H * I * 2, 8 * (d + 1));

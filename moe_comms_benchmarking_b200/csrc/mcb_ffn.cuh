@@ -9,14 +9,16 @@
 //     and HALF of the token rows, so a token row enters the SMs once per 256 weight rows, and one thread of
 //     the pair issues the MMAs of both SMs.  A work unit is 256 weight rows x the whole reduction length x
 //     one chunk of up to 256 tokens of one expert; an expert's tokens are cut into equal chunks, rounded up
-//     to 32, and the accumulators are double buffered in TMEM;
+//     to 16, and the accumulators are double buffered in TMEM;
 //   * every operand arrives by TMA: weights as 16 or 32 KB tiles (pre-packed once into the swizzled K-major
 //     image of their shared-memory tile, so a tile is contiguous in memory), activations as boxes of rows.
-//     Token rows come four at a time through the pair -> token list (tile::gather4, the routing permute fused
-//     into the load) while an expert has at most kFfnGatherN tokens.  One gather costs its issuing thread about
-//     100 cycles whatever it moves, which at many tokens is slower than the MMAs it feeds, so there the
-//     rows are first copied into pair order (into the memory of the expert outputs, which an expert's down
-//     units overwrite only after all its gate/up units have read it) and come as boxes too;
+//     Token rows come four at a time through the pair -> token list (tile::gather4): the routing permute is
+//     fused into the load and no row is copied.  The TMA unit takes a gather every 12 cycles (128 rows in 390 cycles, a box
+//     of as many 330, an MMA step over 256 tokens 512), one thread issues one in 35 to 55: four warps share a
+//     chunk of up to 128 tokens, six a larger one.  With two warps that also fetched the token numbers, alone, the gathers
+//     were the limit, and above 128 tokens the rows were copied into pair order by all CTAs before the first unit
+//     (184 MB at 4096 tokens of top-22: 730 -> 672 us a layer without the copy; 64 experts at 173 tokens 91 -> 84, at 350 tokens
+//     154 -> 147, with Zipf routing 162 -> 152 us);
 //   * work units are listed per CTA pair in shared memory before the roles start: experts without tokens are
 //     left out of the numbering, so the pairs get equally many units whatever the routing, and a
 //     popular expert's chunks spread over the chip;
@@ -41,8 +43,8 @@
 //   * every mbarrier wait is bounded and reports through the status words.
 // Measured on one B200 with 64 experts of 1024 x 1024 (402.7 MB of weights), against one CTA per unit of 128 weight rows
 // with token rows copied by cp.async and units numbered over all experts: 64 us (66 before) at 3 tokens per expert,
-// where the weight stream is the limit; 89 (113) at 173 and 157 (204) at 350 tokens per expert; with skewed routing
-// (8191 tokens, Zipf 1.2) 222 (536).  With 22 of 512 experts in use 36 (52).  Launches of a few microseconds lose what a CTA
+// where the weight stream is the limit; 84 (113) at 173 and 147 (204) at 350 tokens per expert.  From about 170 tokens per
+// expert on the power cap decides: the clock falls to 1.2-1.4 GHz, and the same launches on rows of zeros take 76 and 122 us.  With 22 of 512 experts in use 36 (52).  Launches of a few microseconds lose what a CTA
 // pair costs to set up and take down, and to gather: 8 experts of 512 x 256 at 1 / 32 / 128 tokens per expert 8.3 / 9.6 /
 // 12.9 us (7.2 / 7.7 / 10.4).
 #pragma once
@@ -51,19 +53,21 @@
 namespace mcb {
 
 constexpr int kFfnEpiWarps = 8;
-constexpr int kFfnTokWarps = 2;
+constexpr int kFfnTokWarps = 6;             // four of them load chunks of up to kFfnDoubleN tokens: one token 41.2 us a layer, 43.6 with six
 constexpr int kFfnThreads = 32 * (2 + kFfnEpiWarps + kFfnTokWarps);      // weight TMA, MMA, epilogue, token TMA
 constexpr int kFfnRowsM = 256;              // weight rows per unit (128 in each CTA of the pair)
 constexpr int kFfnBlockK = 64;              // 128 bytes of bf16
 constexpr int kFfnMaxN = 256;               // tokens per chunk
-// Largest chunk whose token rows are gathered by TMA.  64 experts of 1024 x 1024, largest 90 / 110 / 128 tokens: 66 / 67 / 70 us
-// (70 / 71 / 75 with the copy into pair order from 65 on), 32 of 1024 x 512 at 64 tokens 24.3 (27.2), 8 of 7168 x 2048 at
-// 110: 111 (117); no difference with one popular expert, whose size decides for all.
-constexpr int kFfnGatherN = 128;
+constexpr int kFfnMaxGroups = (kFfnMaxN / 8 + kFfnTokWarps - 1) / kFfnTokWarps;      // groups of four rows per token warp and step
 constexpr int kFfnDoubleN = 128;            // up to this many tokens per chunk a stage holds two 64-column blocks
 constexpr int kFfnMaxStages = 10;
+// Stages of two blocks: four.  A fifth, where it fits, puts 24 MB of weights in flight on the chip instead of 19, and the CTAs then
+// share HBM less evenly: 512 experts of 1024 x 1024 at 16 / 37 / 64 / 128 / 512 tokens 235 / 379 / 428 / 462 / 496 us a layer (241 / 389 /
+// 443 / 477 / 513 with five); with three, 237 / 381 / 428 / 457 / 488, but 64 experts at 64 tokens 75.6 (73.4; 74.5 with five) and
+// 1024 / 4096 tokens 522 / 689 (519 / 680).  Only one token has a use for the fifth (42.0 against 41.6 us).
+constexpr int kFfnDoubleStages = 4;
 constexpr int kFfnABytes = 128 * kFfnBlockK * 2;                 // 16 KiB of weights per CTA and 64-column block
-constexpr int kFfnPipeBytes = 192 * 1024;   // 6 stages at 256 tokens, 5 of two blocks at 32
+constexpr int kFfnPipeBytes = 192 * 1024;   // 6 stages at 256 tokens, 4 of two blocks at 128
 constexpr int kFfnMaxExperts = 1024;        // local experts
 constexpr int kFfnListUnits = 256;          // units listed at a time
 // Shared memory behind the pipeline: barriers, unit list, epilogue tiles, expert offsets, chunk prefix, active experts.
@@ -74,8 +78,9 @@ constexpr int kFfnEpiBytes = kFfnEpiWarps * kFfnTileBytes;
 constexpr int kFfnOffBytes = (kFfnMaxExperts + 1) * 4 + 28;      // rounded to 32
 constexpr int kFfnCumBytes = kFfnOffBytes;
 constexpr int kFfnIdBytes = kFfnMaxExperts * 2;
-constexpr int kFfnSmemBytes = kFfnPipeBytes + 1024 /*align*/ + kFfnBarBytes + kFfnListBytes + kFfnEpiBytes + kFfnOffBytes +
-                              kFfnCumBytes + kFfnIdBytes;
+constexpr int kFfnTokIdxBytes = kFfnTokWarps * 128;              // token numbers of a unit's rows, at most 32 per token warp
+constexpr int kFfnSmemBytes = kFfnPipeBytes + 1024 /*align*/ + kFfnBarBytes + kFfnListBytes + kFfnEpiBytes + kFfnTokIdxBytes +
+                              kFfnOffBytes + kFfnCumBytes + kFfnIdBytes;
 
 __device__ __forceinline__ int ld_acquire_gpu_i32(const int* p) {
   int v;
@@ -92,9 +97,10 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
-// Equal chunks of an expert's `rows` tokens, at most kFfnMaxN each; all but the last are a multiple of 32.
+// Equal chunks of an expert's `rows` tokens, at most kFfnMaxN each; all but the last are a multiple of 16 (the step of N of a CTA
+// pair's MMA).
 __device__ __forceinline__ int ffn_chunks(int rows) { return (rows + kFfnMaxN - 1) / kFfnMaxN; }
-__device__ __forceinline__ int ffn_chunk_rows(int rows, int chunks) { return ((rows + chunks - 1) / chunks + 31) & ~31; }
+__device__ __forceinline__ int ffn_chunk_rows(int rows, int chunks) { return ((rows + chunks - 1) / chunks + 15) & ~15; }
 
 // One entry of the unit list.
 struct FfnUnit {
@@ -106,7 +112,14 @@ struct FfnUnit {
   __device__ __forceinline__ int e() const { return (int)(e_fc & 0x7fffffffu); }
   __device__ __forceinline__ int j() const { return (int)(j_ch & 0xfffu); }
   __device__ __forceinline__ int chunks() const { return (int)(j_ch >> 12); }
-  __device__ __forceinline__ int half() const { return ((n + 31) & ~31) >> 1; }      // token rows per CTA
+  __device__ __forceinline__ int half() const { return ((n + 15) & ~15) >> 1; }      // token rows per CTA
+  // Groups of four rows of that half that one of `warps` token warps fetches, and the first one of warp t.  Every warp has some at
+  // every size: where the groups do not divide by the warps, neighbours fetch the same rows to the same place.
+  __device__ __forceinline__ int groups(int warps) const { return ((half() >> 2) + warps - 1) / warps; }
+  __device__ __forceinline__ int first_group(int t, int warps) const {
+    const int g = groups(warps), last = (half() >> 2) - g;
+    return t * g < last ? t * g : last;
+  }
 };
 // What the unit numbering needs, the same in every CTA.  Slots are the experts that have tokens, in order;
 // slot s contributes its gate/up units and the down units of slot s - lag.
@@ -197,6 +210,7 @@ struct FfnSmem {
   volatile int* abort_flag;
   uint4* list;
   uint8_t* epi;
+  int* tok_idx;
   int* off;
   int* cum;
   uint16_t* ids;
@@ -212,7 +226,8 @@ struct FfnSmem {
     uint8_t* p = pipe + kFfnPipeBytes + kFfnBarBytes;
     list = reinterpret_cast<uint4*>(p);
     epi = p + kFfnListBytes;
-    off = reinterpret_cast<int*>(epi + kFfnEpiBytes);
+    tok_idx = reinterpret_cast<int*>(epi + kFfnEpiBytes);
+    off = tok_idx + kFfnTokIdxBytes / 4;
     cum = off + kFfnOffBytes / 4;
     ids = reinterpret_cast<uint16_t*>(cum + kFfnCumBytes / 4);
   }
@@ -246,21 +261,11 @@ __device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
   tc_fence_after();
 }
 
-// After it: TMEM back.  Nobody leaves before the other CTA of the pair is done with this one's shared memory.  `copied` is
-// what ffn_run returned: the last CTA out leaves the counters of the row copy at zero for the next launch.  A CTA counts
-// itself out behind the barrier: all its warps have added to the first counter and are done waiting for it.
-__device__ __forceinline__ void ffn_teardown(const McbFfnArgs& a, bool copied) {
+// After it: TMEM back.  Nobody leaves before the other CTA of the pair is done with this one's shared memory.
+__device__ __forceinline__ void ffn_teardown() {
   const FfnSmem sm;
   tc_fence_before();
   __syncthreads();
-  if (copied && threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&a.sync[1], 1) == (int)gridDim.x - 1) {
-      a.sync[0] = 0;
-      a.sync[1] = 0;
-      __threadfence();
-    }
-  }
   if (*sm.abort_flag) __nanosleep(50000);            // let any copy still in flight land before the CTA goes away
   cluster_sync();
   if (threadIdx.x >= 32 && threadIdx.x < 64) {
@@ -287,30 +292,6 @@ __device__ __forceinline__ void ffn_wait_count(const int* word, int want, const 
   }
 }
 
-// Token rows into pair order: row p of y = row pair_token[p] of x, for all `pairs` rows, over the warps that call it.
-// Eight 512-byte pieces per warp in flight; a.hidden is a multiple of 256, so a piece lies inside one row.
-__device__ __forceinline__ void ffn_permute_rows(const McbFfnArgs& a, int pairs, int wid, int nwarps) {
-  const int lane = threadIdx.x & 31, per_row = a.hidden / 256;
-  const long long pieces = (long long)pairs * per_row;
-  const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x) + lane * 16;
-  uint8_t* xp = reinterpret_cast<uint8_t*>(a.y) + lane * 16;
-  for (long long i0 = (long long)wid * 8; i0 < pieces; i0 += (long long)nwarps * 8) {
-    long long src[8];
-    uint4 v[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const long long i = i0 + k < pieces ? i0 + k : pieces - 1;
-      const int row = (int)(i / per_row);
-      src[k] = (long long)a.pair_token[row] * a.hidden * 2 + (i - (long long)row * per_row) * 512;
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = ld_v4(x + src[k]);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (i0 + k < pieces) st_v4(xp + (i0 + k) * 512, v[k]);
-  }
-}
-
 // a.w1 is the packed interleaved gate/up matrix (E * 2I rows, H columns), a.w2 the packed down matrix (E * H rows,
 // I columns): tile (128-row block v, column block kb) of a matrix with KB column blocks is the 16 KB at byte
 // (v * KB + kb) * 16384.
@@ -323,6 +304,7 @@ struct FfnReady {
 
 template <int NSUB>
 __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap* maps, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
+  constexpr int kTok = NSUB == 2 ? 4 : kFfnTokWarps;      // token warps of this launch
   const FfnSmem sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank();           // 0 = the CTA that issues the MMAs of the pair
@@ -331,12 +313,12 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
   const int total = plan.total();
   const uint32_t tmem_base = *sm.tmem_slot;
   const Abort ab{sm.abort_flag, a.status, a.timeout_ns};
-  const bool gather = n_slot <= kFfnGatherN;
 
   const int b_sub_bytes = (n_slot >> 1) * 128;                    // token half of one 64-column block
   const int stage_bytes = NSUB * (kFfnABytes + b_sub_bytes);
   int stages = kFfnPipeBytes / stage_bytes;
-  if (stages > kFfnMaxStages) stages = kFfnMaxStages;
+  constexpr int kStages = NSUB == 2 ? kFfnDoubleStages : kFfnMaxStages;
+  if (stages > kStages) stages = kStages;
 
   // Pipeline position of this warp's role, kept from one batch of the list to the next.
   int s = 0; uint32_t ph = 0;
@@ -362,15 +344,6 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
     if (lane == 0) ffn_wait_count(reinterpret_cast<const int*>(ready.word), ready.want, ab, 19, 0);
     __syncwarp();
   }
-  if (!gather && warp >= 2) {
-    // every warp but the weight producer and the MMA issuer takes a share of the copy into pair order
-    ffn_permute_rows(a, plan.off[a.num_local_experts], (int)blockIdx.x + (warp - 2) * (int)gridDim.x,
-                     (kFfnEpiWarps + kFfnTokWarps) * (int)gridDim.x);
-    fence_proxy_async_global();
-    __threadfence();
-    asm volatile("bar.sync 1, %0;" :: "n"(32 * (kFfnEpiWarps + kFfnTokWarps)) : "memory");
-    if (warp == 2 && lane == 0) atomicAdd(&a.sync[0], 1);
-  }
 
   for (int first = pair; first < total; first += kFfnListUnits * npairs) {
     int count = (total - first + npairs - 1) / npairs;
@@ -388,7 +361,7 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
           for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
             if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 11))) break;
             if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * NSUB * kFfnABytes);
-            tma_load_2d_pair_hint(sm.pipe + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row, stream);
+            tma_load_2d_pair_hint(smem_u32(sm.pipe) + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row, stream);
             if (++s == stages) { s = 0; ph ^= 1u; }
           }
         }
@@ -511,78 +484,77 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
         }
         if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
       }
-    } else {
+    } else if (warp < 2 + kFfnEpiWarps + kTok) {
       // ---------------- tokens: this CTA's half of the chunk into the swizzled K-major B tile ----------------
-      // Each of the two warps fetches half of the half, from one thread: four rows per gather, or one box.  Rows past
-      // the end of the chunk (they feed columns nobody reads) are fetched too, so that BOTH warps of both CTAs
+      // Each of the kTok warps fetches its groups of four rows, from one thread: a gather each, or one box.  Rows past
+      // the end of the chunk (they feed columns nobody reads) are fetched too, so that ALL warps of both CTAs
       // contribute bytes to every stage: one that the stage did not wait for could fall a whole ring behind and
-      // misread the parity of `empty`.  The gather indices of the next unit are requested while the current
-      // one is still being copied.
-      if (elect_one()) {
-        const int t = warp - 2 - kFfnEpiWarps;
-        constexpr int kOps = kFfnGatherN / 8 / kFfnTokWarps;
-        int nxt[kOps][4];
-        auto fetch_idx = [&](const FfnUnit& un) {
-          if (un.fc() || !gather) return;
-          const int rows = un.half() / kFfnTokWarps, base = rank * un.half() + t * rows;
-#pragma unroll
-          for (int k = 0; k < kOps; ++k) {
-            if (k * 4 >= rows) break;
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-              int r = base + k * 4 + m;
-              if (r >= un.n) r %= un.n;              // spread over the chunk's rows, not all on one
-              nxt[k][m] = a.pair_token[un.row0 + r];
-            }
-          }
-        };
-        fence_proxy_async_global();          // token rows written by ordinary stores before this point
-        fetch_idx(listed(0));
-        if (!gather && first == pair) {
-          ffn_wait_count(&a.sync[0], (int)gridDim.x, ab, 18, 0);
-          fence_proxy_async_global();
-        }
-        for (int i = 0; i < count && ok; ++i) {
-          const FfnUnit un = listed(i);
-          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
-          const int rows = un.half() / kFfnTokWarps;           // 8, 16, ... 64
-          const uint32_t bytes = (uint32_t)un.half() * 256u * NSUB;
-          const int row = un.row0 + rank * un.half() + t * rows;
-          const CUtensorMap* map = maps + (un.fc() ? MCB_FFN_MAP_ACT : MCB_FFN_MAP_XP) + (rows >> 3) - 1;
-          int cur[kOps][4];
-#pragma unroll
-          for (int k = 0; k < kOps; ++k)
-#pragma unroll
-            for (int m = 0; m < 4; ++m) cur[k][m] = nxt[k][m];
-          if (i + 1 < count) fetch_idx(listed(i + 1));
+      // misread the parity of `empty`.  The lanes fetch the token numbers of the next unit, one each, while the current one
+      // is still being copied, and hand them to the issuing thread through shared memory.
+      const int t = warp - 2 - kFfnEpiWarps;
+      constexpr int kOps = (kFfnMaxN / NSUB / 8 + kTok - 1) / kTok;
+      static_assert(kOps <= kFfnMaxGroups && kOps * 4 <= 32, "a map per box, a lane per row");
+      const uint32_t idx_slot = smem_u32(sm.tok_idx + t * 32);
+      const uint32_t pipe0 = smem_u32(sm.pipe) + NSUB * kFfnABytes, full0 = cluster_map(sm.full, 0);
+      auto fetch_idx = [&](const FfnUnit& un) {
+        const int rows = un.groups(kTok) * 4;
+        int r = rank * un.half() + un.first_group(t, kTok) * 4 + lane;
+        if (un.fc() || lane >= rows) return 0;
+        if (r >= un.n) r %= un.n;                  // spread over the chunk's rows, not all on one
+        return a.pair_token[un.row0 + r];
+      };
+      fence_proxy_async_global();          // token rows written by ordinary stores before this point
+      int nxt = fetch_idx(listed(0));
+      for (int i = 0; i < count && ok; ++i) {
+        const FfnUnit un = listed(i);
+        const int steps = (un.fc() ? I : H) / (kFfnBlockK * NSUB);
+        const int groups = un.groups(kTok), row_h = un.first_group(t, kTok) * 4;
+        if (!un.fc()) asm volatile("st.shared.b32 [%0], %1;" :: "r"(idx_slot + lane * 4), "r"(nxt) : "memory");
+        __syncwarp();
+        if (i + 1 < count) nxt = fetch_idx(listed(i + 1));
+        if (elect_one()) {
+          const uint32_t bytes = (uint32_t)(groups * kTok) * 1024u * NSUB;
+          int su = s; uint32_t pu = ph;
           if (un.fc()) {
+            const int row = un.row0 + rank * un.half() + row_h;
+            const CUtensorMap* map = maps + MCB_FFN_MAP_ACT + groups - 1;
             // the activations of this expert are complete once every epilogue warp of every gate/up unit has been counted
             ffn_wait_count(&a.ffn_done[un.e()], 2 * kFfnEpiWarps * plan.n1 * un.chunks(), ab, 15, (uint32_t)un.e());
             fence_proxy_async_global();
-          }
-          const bool box = un.fc() || !gather;
-          for (int kb = 0; kb < k_blocks; kb += NSUB) {
-            if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 16))) break;
-            uint8_t* dst = sm.pipe + s * stage_bytes + NSUB * kFfnABytes + t * rows * 128;
-            const uint32_t bar = cluster_map(&sm.full[s], 0);
-            if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[s], bytes);
-            if (box) {
+            for (int k = 0; k < steps; ++k) {
+              if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
+              if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
+              const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
 #pragma unroll
               for (int sub = 0; sub < NSUB; ++sub)
-                tma_load_2d_pair(dst + sub * b_sub_bytes, map, bar, (kb + sub) * kFfnBlockK, row);
-            } else {
+                tma_load_2d_pair(dst + sub * b_sub_bytes, map, full0 + su * 8, (k * NSUB + sub) * kFfnBlockK, row);
+              if (++su == stages) { su = 0; pu ^= 1u; }
+            }
+          } else {
+            uint4 idx[kOps];
 #pragma unroll
-              for (int k = 0; k < kOps; ++k) {
-                if (k * 4 >= rows) break;
+            for (int k = 0; k < kOps; ++k) idx[k] = lds_v4(idx_slot + k * 16);
+            for (int k = 0; k < steps; ++k) {
+              if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
+              if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
+              const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
+#pragma unroll
+              for (int g = 0; g < kOps; ++g) {
+                if (g >= groups) break;
 #pragma unroll
                 for (int sub = 0; sub < NSUB; ++sub)
-                  tma_gather4_pair(dst + sub * b_sub_bytes + k * 512, maps + MCB_FFN_MAP_X, bar,
-                                   (kb + sub) * kFfnBlockK, cur[k][0], cur[k][1], cur[k][2], cur[k][3]);
+                  tma_gather4_pair(dst + sub * b_sub_bytes + g * 512, maps + MCB_FFN_MAP_X, full0 + su * 8,
+                                   (k * NSUB + sub) * kFfnBlockK, idx[g].x, idx[g].y, idx[g].z, idx[g].w);
               }
+              if (++su == stages) { su = 0; pu ^= 1u; }
             }
-            if (++s == stages) { s = 0; ph ^= 1u; }
           }
         }
+        ok = __all_sync(0xffffffffu, ok);
+        s += steps % stages;
+        ph ^= (uint32_t)(steps / stages) & 1u;
+        if (s >= stages) { s -= stages; ph ^= 1u; }
+        __syncwarp();
       }
     }
     if (count == kFfnListUnits) {
@@ -601,9 +573,8 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
 
 // Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
 // ffn_teardown, with the experts' offsets in the shared memory of FfnSmem::off (visible to all threads) and the largest
-// number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.  Returns whether the token rows were copied
-// into pair order, for ffn_teardown.
-__device__ __forceinline__ bool ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
+// number of tokens of one expert; dynamic shared memory of at least kFfnSmemBytes.
+__device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
   const FfnSmem sm;
   const int E = a.num_local_experts;
   if (max_rows < 1) max_rows = 1;
@@ -618,18 +589,17 @@ __device__ __forceinline__ bool ffn_run(const McbFfnArgs& a, const CUtensorMap* 
     const int lag = (int)((long long)gridDim.x * 3 / 2 * plan.active / plan.total()) + 2;
     if (lag < plan.lag) plan.lag = lag;
   }
-  // Token tile of this launch: the largest expert, rounded up to 32, at most kFfnMaxN per chunk.
-  const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 31) & ~31);
+  // Token tile of this launch: the largest expert, rounded up to 16, at most kFfnMaxN per chunk.
+  const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 15) & ~15);
   if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, maps, plan, n_slot, ready);
   else ffn_roles<1>(a, maps, plan, n_slot, ready);
-  return n_slot > kFfnGatherN;
 }
 
 // The same after a routing of its own launch, whose results are in global memory.
-__device__ __forceinline__ bool ffn_device(const McbFfnArgs& a, const CUtensorMap* maps) {
+__device__ __forceinline__ void ffn_device(const McbFfnArgs& a, const CUtensorMap* maps) {
   const FfnSmem sm;
   for (int e = threadIdx.x; e <= a.num_local_experts; e += blockDim.x) sm.off[e] = a.expert_offset[e];
-  return ffn_run(a, maps, *a.max_rows, FfnReady{nullptr, 0});
+  ffn_run(a, maps, *a.max_rows, FfnReady{nullptr, 0});
 }
 
 }  // namespace mcb

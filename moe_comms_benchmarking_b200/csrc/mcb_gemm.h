@@ -8,13 +8,12 @@
 #define MCB_GEMM_FC1 0          // gate/up projection + SwiGLU epilogue
 #define MCB_GEMM_FC2 1          // down projection + per-row scale epilogue
 // Tensor maps of the fused FFN: token rows (gathered four at a time), gate/up and down tiles (16 KB, then 32 KB), and
-// activations and token rows in pair order in boxes of 8, 16, ... 64 rows.
+// activations in boxes of 4, 8, ... 24 rows.
 #define MCB_FFN_MAP_X 0
 #define MCB_FFN_MAP_W1 1
 #define MCB_FFN_MAP_W2 2
 #define MCB_FFN_MAP_ACT 5
-#define MCB_FFN_MAP_XP 13
-#define MCB_FFN_TMAPS 21
+#define MCB_FFN_TMAPS 11
 #define MCB_GEMM_ERR_TIMEOUT 5  // status code: a bounded mbarrier wait ran out
 
 #ifdef __cplusplus
@@ -48,7 +47,7 @@ typedef struct {
   const int32_t* expert_offset;  // [E_loc + 1] first pair row of each local expert
   const int32_t* max_rows;     // device scalar: largest pair count of one expert
   void* act;                   // [P, intermediate] bf16 (written by the gate/up blocks, read by the down blocks)
-  void* y;                     // [P, hidden] bf16 = prob * (act . Wd^T); holds the token rows in pair order before
+  void* y;                     // [P, hidden] bf16 = prob * (act . Wd^T)
   int32_t* ffn_done;           // [E_loc] warp shares of gate/up blocks finished (zeroed by the routing)
   int32_t num_local_experts;
   int32_t hidden;              // multiple of 256
@@ -61,7 +60,6 @@ typedef struct {
   // MCB_FFN_TMAPS tensor maps of 128 bytes, 64-byte aligned (mcb_make_ffn_tmaps): in host memory, from where a launch copies
   // them into its parameters; for ranks emulated inside one launch in device memory.
   const void* tmaps;
-  int32_t* sync;               // [2] zero between launches: CTAs that have copied their token rows, CTAs that have left
 } McbFfnArgs;
 
 // Routing of the gathered tokens to this rank's experts.
@@ -82,7 +80,7 @@ typedef struct {
   int32_t* tile_row0;
   int32_t* tile_rows;
   int32_t* num_m_tiles;        // device scalar
-  int32_t* sync;               // [4] zero between launches: blocks that have counted, blocks that have left; two words of the fused FFN
+  int32_t* sync;               // [4] zero between launches: blocks that have counted, blocks that have left, -, -
   int32_t max_pairs;           // capacity of the pair arrays
   int32_t max_tiles;           // capacity of the tile table
   uint32_t* status;

@@ -151,10 +151,10 @@ __device__ __forceinline__ void tma_acquire_map(const void* map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" :: "l"(map) : "memory");
 }
 // Tile load / four-row gather into this CTA's shared memory, completing on a barrier of either CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* map, uint32_t bar, int c0, int c1) {
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const void* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4}], [%2];"
-      :: "r"(smem_u32(smem_dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+      :: "r"(smem_dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
 // The same for data that nobody reads again: its lines are the first to leave L2.
 __device__ __forceinline__ uint64_t l2_evict_first() {
@@ -162,15 +162,15 @@ __device__ __forceinline__ uint64_t l2_evict_first() {
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
-__device__ __forceinline__ void tma_load_2d_pair_hint(void* smem_dst, const void* map, uint32_t bar, int c0, int c1, uint64_t policy) {
+__device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t smem_dst, const void* map, uint32_t bar, int c0, int c1, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-      :: "r"(smem_u32(smem_dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
+      :: "r"(smem_dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
 }
-__device__ __forceinline__ void tma_gather4_pair(void* smem_dst, const void* map, uint32_t bar, int c0, int r0, int r1, int r2, int r3) {
+__device__ __forceinline__ void tma_gather4_pair(uint32_t smem_dst, const void* map, uint32_t bar, int c0, int r0, int r1, int r2, int r3) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      :: "r"(smem_u32(smem_dst)), "l"(map), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+      :: "r"(smem_dst), "l"(map), "r"(bar), "r"(c0), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 // One warp of BOTH CTAs of the pair calls each of these.

@@ -148,7 +148,7 @@ class McbFfnArgs(C.Structure):
         ("x", _vp), ("pair_token", _vp), ("pair_prob", _vp), ("expert_offset", _vp),
         ("max_rows", _vp), ("act", _vp), ("y", _vp), ("ffn_done", _vp),
         ("num_local_experts", _i32), ("hidden", _i32), ("intermediate", _i32), ("reserved0", _i32),
-        ("status", _vp), ("timeout_ns", _u64), ("w1", _vp), ("w2", _vp), ("tmaps", _vp), ("sync", _vp),
+        ("status", _vp), ("timeout_ns", _u64), ("w1", _vp), ("w2", _vp), ("tmaps", _vp),
     ]
 
 
@@ -175,7 +175,7 @@ def layer_args_size() -> int:
 
 
 GEMM_FC1, GEMM_FC2 = 0, 1
-FFN_TMAPS = 21
+FFN_TMAPS = 11
 
 _STRUCTS = {
     "ctx": McbCtx, "load_args": McbLoadArgs, "meta_args": McbMetaArgs, "agv_args": McbAgvArgs, "rsv_args": McbRsvArgs,

@@ -123,14 +123,13 @@ def make_weight_tmap(w2d: torch.Tensor):
 
 
 def make_ffn_tmaps(weights: "ExpertWeights", x: torch.Tensor, act: torch.Tensor, y: torch.Tensor):
-    """The tensor maps of one FFN launch (token rows, activations, expert outputs, packed weights) in host memory:
+    """The tensor maps of one FFN launch (token rows, activations, packed weights) in host memory:
     (keep-alive buffer, 64-byte aligned address)."""
     raw = (C.c_uint8 * (_ext.FFN_TMAPS * 128 + 64))()
     addr = (C.addressof(raw) + 63) & ~63
     lib = _ext.require()
     _ext.check(lib.mcb_make_ffn_tmaps(C.c_void_p(addr), C.c_void_p(x.data_ptr()), C.c_uint64(x.numel() // weights.hidden),
-                                      C.c_void_p(act.data_ptr()), C.c_void_p(y.data_ptr()),
-                                      C.c_uint64(min(act.shape[0], y.shape[0])),
+                                      C.c_void_p(act.data_ptr()), C.c_uint64(min(act.shape[0], y.shape[0])),
                                       C.c_void_p(weights.w1.data_ptr()), C.c_void_p(weights.w2.data_ptr()),
                                       weights.num_local_experts, weights.hidden, weights.intermediate), "make_ffn_tmaps")
     return raw, addr
@@ -153,7 +152,7 @@ class RouteBuffers:
         self.tile_row0 = torch.zeros(self.max_tiles, **i32)
         self.tile_rows = torch.zeros(self.max_tiles, **i32)
         self.num_m_tiles = torch.zeros(1, **i32)
-        self.sync = torch.zeros(4, **i32)                # two words of the routing, two of the fused FFN
+        self.sync = torch.zeros(4, **i32)                # the routing uses two of them
         self.max_rows = torch.zeros(1, **i32)            # largest pair count of one expert
         self.ffn_done = torch.zeros(num_local_experts, **i32)   # gate/up blocks finished per expert (fused FFN)
 
@@ -317,7 +316,7 @@ class ExpertFfnPlan:
         tmaps = make_ffn_tmaps(weights, x, act, y)
         self._keep = (route, x, act, y, status, tmaps)
         a = _ext.McbFfnArgs()
-        a.tmaps, a.sync = tmaps[1], route.sync[2:].data_ptr()
+        a.tmaps = tmaps[1]
         a.x = x.data_ptr()
         a.pair_token, a.pair_prob = route.pair_token.data_ptr(), route.pair_prob.data_ptr()
         a.expert_offset, a.max_rows = route.expert_offset.data_ptr(), route.max_rows.data_ptr()

@@ -230,7 +230,7 @@ class EmuWorld:
             if maps.data_ptr() % 128:
                 raise RuntimeError("device allocation is not 128-byte aligned")
             keep.append(maps)
-            ff.tmaps, ff.sync = maps.data_ptr(), route.sync[2:].data_ptr()
+            ff.tmaps = maps.data_ptr()
             cm = p.cmb
             cm.y, cm.pair_pos, cm.partial_off, cm.out = d["y"].data_ptr(), route.pair_pos.data_ptr(), d["partial"].offset, d["out"].data_ptr()
             cm.n_local, cm.step_meta = d["n_local"].data_ptr(), d["step_meta"].data_ptr()

@@ -337,6 +337,17 @@ def test_expert_ffn_chunk_edges(world1, rows, H, I, grid):
             assert float((y[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} down"
 
 
+@pytest.mark.parametrize("rows", [
+    [1, 15, 16, 17, 48, 49, 80, 81, 112, 113, 128],                                     # four token warps, every number of row groups
+    [129, 144, 145, 160, 161, 176, 177, 192, 193, 208, 209, 224, 225, 240, 241, 256],   # six, dividing and not
+    [272, 273, 289, 350, 512, 513, 529, 16],                                            # equal chunks on either side of a multiple of 16
+])
+def test_expert_ffn_row_groups(world1, rows):
+    """Token rows in groups of four that the token warps share: where the groups do not divide by the warps, two of them fetch
+    the same rows.  Tolerance as in the test of the chunks."""
+    test_expert_ffn_chunk_edges(world1, rows, 512, 256, 148)
+
+
 @pytest.mark.parametrize("W,B", [(2, 900), (2, 2200), (1, 1), (1, 2100)])
 def test_moe_layer_kernel_routing_and_combine_branches(lib, W, B):
     """The whole-layer kernel where its routing and combine change form: four packs per lane in the combine (900 tokens),
