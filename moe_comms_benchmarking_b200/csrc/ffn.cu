@@ -67,16 +67,17 @@ moe_layer_kernel(const __grid_constant__ McbLayerArgs p_, const __grid_constant_
   RouteSmem m(reinterpret_cast<int*>(sm.pipe));              // the pipeline is not in use yet
   m.off = sm.off;
   const RouteShare share = route_share(p.route, (int)blockIdx.x, (int)gridDim.x);
-  if (route_counts_all(share)) {
-    route_count<true>(p.route, ids, m, 0, share.entries, share.lo);
+  const BlockGroup all;
+  if (route_counts_all(all, share)) {
+    route_count<true>(all, p.route, ids, m, 0, share.entries, share.lo);
   } else {
-    route_count<false>(p.route, ids, m, share.lo, share.hi, 0);
-    route_publish(p.route, m);
+    route_count<false>(all, p.route, ids, m, share.lo, share.hi, 0);
+    route_publish(all, p.route.num_local_experts, p.route.expert_count, m);
     meet();
-    route_collect(p.route, m);
+    route_collect(all, p.route.num_local_experts, p.route.expert_count, m);
   }
-  const int max_rows = route_offsets(p.route, m, blockIdx.x == 0);
-  route_place(p.route, ids, probs, m, share);
+  const int max_rows = route_offsets(all, p.route, m, blockIdx.x == 0);
+  route_place(all, p.route, ids, probs, m, share);
   // This block's pair rows (and gathered rows, when alone) are there.  Nobody waits here: the weight stream starts at
   // once, the roles that read rows or lists wait for all blocks.
   __syncthreads();
@@ -172,15 +173,25 @@ int mcb_launch_moe_layer(const McbLayerArgs* p, int grid, int pdl, cudaStream_t 
                        *reinterpret_cast<const FfnMaps*>(p->ffn.tmaps), (const McbLayerArgs*)nullptr);
 }
 
-// One decode step with real experts, issued natively: the count exchange, then num_layers layer
-// kernels; layer l uses the argument block (weight set) l % num_sets.
+// One decode step with real experts, issued natively: the count exchange, then num_layers layers; layer l uses the argument
+// block (weight set) l % num_sets.  With `step` (mcb_prepare_moe_step, over the same argument blocks) several layers share a
+// launch, without it each is a layer kernel.
 int mcb_launch_metadata(const McbCtx* ctx, const McbMetaArgs* args, int pdl, cudaStream_t stream);   // dense.cu
+int mcb_launch_moe_step(const McbMoeStepArgs* p, const McbLayerArgs* sets, int num_sets, int first, int num_layers, int grid, int pdl,
+                        cudaStream_t stream);                                                        // moe_step.cu
 
 int mcb_moe_decode_step(const McbCtx* ctx, const McbMetaArgs* meta, const McbLayerArgs* layers, int num_sets,
-                        int num_layers, int grid, int pdl, cudaStream_t stream) {
+                        int num_layers, int grid, int pdl, const McbMoeStepArgs* step, cudaStream_t stream) {
   if (!ctx || !meta || !layers || num_sets < 1 || num_layers < 0) return cudaErrorInvalidValue;
+  for (int s = 0; s < num_sets; ++s)
+    if (check_layer_args(&layers[s], grid)) return cudaErrorInvalidValue;
   int err = mcb_launch_metadata(ctx, meta, pdl, stream);
-  for (int l = 0; l < num_layers && err == 0; ++l) err = mcb_launch_moe_layer(&layers[l % num_sets], grid, pdl, stream);
+  const int together = !step || num_layers < 2 ? 1 : num_sets <= MCB_STEP_SETS ? num_layers : MCB_STEP_SETS;
+  for (int l = 0; l < num_layers && err == 0; l += together) {
+    const int n = num_layers - l < together ? num_layers - l : together;
+    err = n > 1 ? mcb_launch_moe_step(step, layers, num_sets, l, n, grid, pdl, stream)
+                : mcb_launch_moe_layer(&layers[l % num_sets], grid, pdl, stream);
+  }
   return err;
 }
 

@@ -16,7 +16,7 @@
 //                           each, 184 MB of them: 39.6 (53, 90, 61);
 //   behind the experts      two rows, with streaming loads.  The combine of the layer kernel at 4096 / 2048 tokens of 22 pairs:
 //                           41 / 24 us (44 / 26 with four rows, 59 / 37 with one and ordinary loads, 53 / 32 with one).
-// Call from all threads of the block; works for any block size that is a multiple of 32.
+// Call from all threads of the block (any size that is a multiple of 32), or in a world of one from `nwarps` of its warps.
 #pragma once
 #include "mcb_barrier.cuh"
 #include "mcb_gemm.h"
@@ -57,9 +57,10 @@ struct CombineShape {
 
 // PL = packs per lane.
 template <int PL, bool ALONE>
-__device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineArgs& a, const CombineShape& s, uint32_t ep) {
+__device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineArgs& a, const CombineShape& s, uint32_t ep, int warp,
+                                              int nwarps) {
   constexpr int R = PL == 1 ? 8 : PL == 2 ? 4 : (ALONE ? 1 : 2);       // pair rows in flight
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, bid = blockIdx.x;
+  const int lane = threadIdx.x & 31, bid = blockIdx.x;
   const uint8_t* y = reinterpret_cast<const uint8_t*>(a.y);
   const bool alone = c.world == 1;
   uint8_t* partial = c.heap_local + s.partial_off;
@@ -127,7 +128,8 @@ __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineA
 }
 
 template <bool ALONE>
-__device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineArgs& a, uint32_t parity = 0u) {
+__device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineArgs& a, uint32_t parity = 0u, int warp = threadIdx.x >> 5,
+                                             int nwarps = blockDim.x >> 5) {
   CombineShape s;
   s.T = a.step_meta[0];
   s.offset = a.step_meta[1];
@@ -139,7 +141,7 @@ __device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineAr
   s.row_bytes = (uint64_t)a.hidden * 2;
   s.partial_off = a.partial_off + (uint64_t)(parity & 1u) * a.partial_par_stride;
   // Packs per lane from sizes that are the same on every rank.
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  const long long warps = (long long)gridDim.x * nwarps;
   int pl = 4;
   while (pl > 1 && (long long)s.T * ((s.packs + 32 * pl - 1) / (32 * pl)) < warps) pl >>= 1;
   s.slices = (s.packs + 32 * pl - 1) / (32 * pl);
@@ -147,9 +149,9 @@ __device__ __forceinline__ void combine_body(const McbCtx& c, const McbCombineAr
   s.nact = items < (long long)gridDim.x ? (int)items : (int)gridDim.x;
   if ((int)blockIdx.x >= s.nact) return;
   const uint32_t ep = *epoch_ptr(c, a.site, blockIdx.x);
-  if (pl == 4) combine_items<4, ALONE>(c, a, s, ep);
-  else if (pl == 2) combine_items<2, ALONE>(c, a, s, ep);
-  else combine_items<1, ALONE>(c, a, s, ep);
+  if (pl == 4) combine_items<4, ALONE>(c, a, s, ep, warp, nwarps);
+  else if (pl == 2) combine_items<2, ALONE>(c, a, s, ep, warp, nwarps);
+  else combine_items<1, ALONE>(c, a, s, ep, warp, nwarps);
 }
 
 }  // namespace mcb

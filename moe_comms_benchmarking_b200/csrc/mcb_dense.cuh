@@ -98,28 +98,29 @@ struct LocalRanges {
     off = (i - (t ? end[t - 1] : 0)) * 16;
     return t;
   }
-  // The words behind the last whole pack of a range: one thread each, in block 0.
-  __device__ __forceinline__ bool word_of(int& t, long long& off) const {
-    t = threadIdx.x >> 2;
-    const int w = threadIdx.x & 3;
+  // The words behind the last whole pack of a range: one thread each (`tid` of those that copy), in block 0.
+  __device__ __forceinline__ bool word_of(int tid, int& t, long long& off) const {
+    t = tid >> 2;
+    const int w = tid & 3;
     if (blockIdx.x != 0 || t >= R || w >= words[t]) return false;
     off = (end[t] - (t ? end[t - 1] : 0)) * 16 + w * 4;
     return true;
   }
-  __device__ __forceinline__ uint32_t load_word() const {
+  __device__ __forceinline__ uint32_t load_word(int tid = threadIdx.x) const {
     int t; long long off;
-    return word_of(t, off) ? ld_b32(src[t] + off) : 0u;
+    return word_of(tid, t, off) ? ld_b32(src[t] + off) : 0u;
   }
-  __device__ __forceinline__ void store_word(uint32_t parity, uint32_t v) const {
+  __device__ __forceinline__ void store_word(uint32_t parity, uint32_t v, int tid = threadIdx.x) const {
     int t; long long off;
-    if (word_of(t, off)) st_b32(dst[t] + (parity ? par[t] : 0) + off, v);
+    if (word_of(tid, t, off)) st_b32(dst[t] + (parity ? par[t] : 0) + off, v);
   }
 };
 
-__device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parity, long long start, long long stride) {
+__device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parity, long long start, long long stride,
+                                            int tid = threadIdx.x) {
   constexpr int U = 8;
   const long long total = r.end[LocalRanges::R - 1];
-  const uint32_t word = r.load_word();
+  const uint32_t word = r.load_word(tid);
   for (long long i0 = start; i0 < total; i0 += stride * U) {
     uint4 v[U];
     uint8_t* dst[U];
@@ -138,7 +139,7 @@ __device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parit
     for (int u = 0; u < U; ++u)
       if (dst[u]) st_v4(dst[u], v[u]);
   }
-  r.store_word(parity, word);
+  r.store_word(parity, word, tid);
 }
 
 // The same range by range, each dealt from the first thread on: pack i of every range belongs to the same thread, so what

@@ -48,6 +48,7 @@
 // pair costs to set up and take down, and to gather: 8 experts of 512 x 256 at 1 / 32 / 128 tokens per expert 8.3 / 9.6 /
 // 12.9 us (7.2 / 7.7 / 10.4).
 #pragma once
+#include "mcb_group.cuh"
 #include "mcb_tc.cuh"
 
 namespace mcb {
@@ -58,7 +59,7 @@ constexpr int kFfnThreads = 32 * (2 + kFfnEpiWarps + kFfnTokWarps);      // weig
 constexpr int kFfnRowsM = 256;              // weight rows per unit (128 in each CTA of the pair)
 constexpr int kFfnBlockK = 64;              // 128 bytes of bf16
 constexpr int kFfnMaxN = 256;               // tokens per chunk
-constexpr int kFfnMaxGroups = (kFfnMaxN / 8 + kFfnTokWarps - 1) / kFfnTokWarps;      // groups of four rows per token warp and step
+constexpr int kFfnMaxGroups = kFfnMaxN / 8 / 4;      // groups of four rows per token warp and step, of at least four warps
 constexpr int kFfnDoubleN = 128;            // up to this many tokens per chunk a stage holds two 64-column blocks
 constexpr int kFfnMaxStages = 10;
 // Stages of two blocks: four.  A fifth, where it fits, puts 24 MB of weights in flight on the chip instead of 19, and the CTAs then
@@ -97,9 +98,9 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
-// Equal chunks of an expert's `rows` tokens, at most kFfnMaxN each; all but the last are a multiple of 16 (the step of N of a CTA
+// Equal chunks of an expert's `rows` tokens, at most `most` (a multiple of 16) each; all but the last are a multiple of 16 (the step of N of a CTA
 // pair's MMA).
-__device__ __forceinline__ int ffn_chunks(int rows) { return (rows + kFfnMaxN - 1) / kFfnMaxN; }
+__device__ __forceinline__ int ffn_chunks(int rows, int most) { return (rows + most - 1) / most; }
 __device__ __forceinline__ int ffn_chunk_rows(int rows, int chunks) { return ((rows + chunks - 1) / chunks + 15) & ~15; }
 
 // One entry of the unit list.
@@ -153,18 +154,29 @@ struct FfnPlanS {
     r.n = rows - c * cr < cr ? rows - c * cr : cr;
     return r;
   }
+  // Units first, first + step, ... into `out`, up to `most` of them; by `threads` threads, of which this is `tid`.
+  __device__ __forceinline__ void list(uint4* out, int most, int first, int step, int total, int tid, int threads) const {
+    for (int i = tid; i < most; i += threads) {
+      const long long u = first + (long long)i * step;
+      if (u < total) {
+        const FfnUnit un = unit((int)u);
+        out[i] = make_uint4(un.e_fc, un.j_ch, (uint32_t)un.row0, (uint32_t)un.n);
+      }
+    }
+  }
 };
 
-// Fills cum / ids from the expert offsets; returns the number of experts with tokens.  All threads of the CTA.
-__device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16_t* ids, int* scratch) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int per = (E + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int e0 = threadIdx.x * per, e1 = e0 + per < E ? e0 + per : E;
+// Fills cum / ids from the expert offsets; returns the number of experts with tokens.  All threads of the group.
+template <class Group>
+__device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, int most, int* cum, uint16_t* ids, int* scratch) {
+  const int tid = g.tid(), warp = tid >> 5, lane = tid & 31;
+  const int per = (E + g.size() - 1) / g.size();
+  const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
   int act = 0, chunks = 0;
   for (int e = e0; e < e1; ++e) {
     const int rows = off[e + 1] - off[e];
     act += rows > 0;
-    chunks += ffn_chunks(rows);
+    chunks += ffn_chunks(rows, most);
   }
   int a_inc = act, c_inc = chunks;
 #pragma unroll
@@ -173,9 +185,9 @@ __device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16
     if (lane >= o) { a_inc += a; c_inc += c; }
   }
   if (lane == 31) { scratch[warp] = a_inc; scratch[32 + warp] = c_inc; }
-  __syncthreads();
+  g.sync();
   int a_base = a_inc - act, c_base = c_inc - chunks, total = 0, total_c = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+  for (int w = 0; w < (g.size() >> 5); ++w) {
     if (w < warp) { a_base += scratch[w]; c_base += scratch[32 + w]; }
     total += scratch[w];
     total_c += scratch[32 + w];
@@ -186,10 +198,10 @@ __device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16
     ids[a_base] = (uint16_t)e;
     cum[a_base] = c_base;
     ++a_base;
-    c_base += ffn_chunks(rows);
+    c_base += ffn_chunks(rows, most);
   }
-  if (threadIdx.x == 0) cum[total] = total_c;
-  __syncthreads();
+  if (tid == 0) cum[total] = total_c;
+  g.sync();
   return total;
 }
 
@@ -198,6 +210,20 @@ __device__ __forceinline__ int ffn_slots(const int* off, int E, int* cum, uint16
 // activations well inside L2 (126 MB, shared with the weight stream, the tokens and the expert outputs).
 constexpr long long kFfnActL2Bytes = 24ll << 20;
 
+
+// Token tile of a launch: the largest expert, rounded up to 16, at most kFfnMaxN per chunk.
+__device__ __forceinline__ int ffn_token_tile(int max_rows) {
+  return max_rows < 1 ? 16 : max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 15) & ~15);
+}
+// The rest of the plan, once its offsets and slots are there.
+__device__ __forceinline__ void ffn_plan(FfnPlanS& plan, const McbFfnArgs& a, int active) {
+  plan.n1 = 2 * a.intermediate / kFfnRowsM; plan.n2 = a.hidden / kFfnRowsM;
+  plan.active = plan.lag = active;
+  if ((long long)plan.off[a.num_local_experts] * a.intermediate * 2 > kFfnActL2Bytes) {      // three rounds of the grid, in slots of average size
+    const int lag = (int)((long long)gridDim.x * 3 / 2 * active / plan.total()) + 2;
+    if (lag < plan.lag) plan.lag = lag;
+  }
+}
 
 // Shared memory of the FFN, carved out of the dynamic buffer.
 struct FfnSmem {
@@ -233,12 +259,43 @@ struct FfnSmem {
   }
 };
 
+// What a step of several layers in one launch (moe_step.cu) keeps behind the token numbers instead: offsets, chunk prefix and
+// active experts of the layer being listed, the counters of its routing, and the barriers of the two halves of the unit list.
+constexpr int kStepMaxExperts = 768;
+constexpr int kStepListUnits = kFfnListUnits / 2;
+struct StepSmem {
+  int* off;                  // [kStepMaxExperts + 1]
+  int* cum;                  // [kStepMaxExperts + 1]; the counts of the routing before the chunks are numbered
+  uint16_t* ids;             // [kStepMaxExperts]
+  int* begin;                // [kStepMaxExperts]
+  int* scan;                 // [96]
+  uint64_t* lfull;           // [2]
+  uint64_t* lempty;          // [2]
+  int* head;                 // [2][2] units of a half, whether it is the last one of its layer
+  int* word;                 // [2] hand-over among the epilogue warps, among the routing warps
+  static constexpr int kOff = kStepMaxExperts * 4 + 16;
+  static constexpr int kBytes = 2 * kOff + kStepMaxExperts * 2 + kStepMaxExperts * 4 + 96 * 4 + 64;
+  __device__ __forceinline__ explicit StepSmem(const FfnSmem& sm) {
+    off = sm.off;
+    cum = off + kOff / 4;
+    ids = reinterpret_cast<uint16_t*>(cum + kOff / 4);
+    begin = reinterpret_cast<int*>(ids + kStepMaxExperts);
+    scan = begin + kStepMaxExperts;
+    lfull = reinterpret_cast<uint64_t*>(scan + 96);
+    lempty = lfull + 2;
+    head = reinterpret_cast<int*>(lempty + 2);
+    word = head + 4;
+  }
+};
+constexpr int kStepSmemBytes = kFfnSmemBytes - kFfnOffBytes - kFfnCumBytes - kFfnIdBytes + StepSmem::kBytes;
+static_assert(kStepSmemBytes + 256 <= 227 * 1024, "fits beside the static shared memory");
+
 // The tensor maps of a launch, as a kernel parameter.
 struct FfnMaps {
   CUtensorMap map[MCB_FFN_TMAPS];
 };
 
-// Before the FFN, once per kernel: barriers, TMEM, tensor maps (GLOBAL: in global memory).  All threads of both CTAs of the pair; touches nothing
+// Before the FFN, once per kernel: barriers, TMEM, tensor maps (GLOBAL: in global memory; null: none).  All threads of both CTAs of the pair; touches nothing
 // that another kernel writes, so a kernel with other work to do first calls it at its very start.
 template <bool GLOBAL>
 __device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
@@ -251,7 +308,7 @@ __device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x >= 32 && threadIdx.x < 64) tmem_alloc_pair(sm.tmem_slot, 512);
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + MCB_FFN_TMAPS) {
+  if (maps && threadIdx.x >= 64 && threadIdx.x < 64 + MCB_FFN_TMAPS) {
     if (GLOBAL) tma_acquire_map(maps + (threadIdx.x - 64));
     tma_prefetch_map(maps + (threadIdx.x - 64));
   }
@@ -302,273 +359,302 @@ struct FfnReady {
   int want;
 };
 
-template <int NSUB>
-__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap* maps, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
-  constexpr int kTok = NSUB == 2 ? 4 : kFfnTokWarps;      // token warps of this launch
+// The warps' roles over lists of units.  A role keeps its position in the pipeline from one list to the next; every warp of
+// a role sees the same lists in the same order.  TOK: token warps.
+template <int NSUB, int TOK>
+struct FfnRoles {
+  const McbFfnArgs& a;
+  const CUtensorMap* xmap;           // token rows
+  // Activations by box, where the gate/up units write them, and expert outputs (of the layer at hand).
+  const CUtensorMap* actmap;
+  uint8_t* act_rows;
+  uint8_t* y_rows;
   const FfnSmem sm;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)cluster_ctarank();           // 0 = the CTA that issues the MMAs of the pair
-  const int H = a.hidden, I = a.intermediate;
-  const int npairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1;
-  const int total = plan.total();
-  const uint32_t tmem_base = *sm.tmem_slot;
-  const Abort ab{sm.abort_flag, a.status, a.timeout_ns};
-
-  const int b_sub_bytes = (n_slot >> 1) * 128;                    // token half of one 64-column block
-  const int stage_bytes = NSUB * (kFfnABytes + b_sub_bytes);
-  int stages = kFfnPipeBytes / stage_bytes;
-  constexpr int kStages = NSUB == 2 ? kFfnDoubleStages : kFfnMaxStages;
-  if (stages > kStages) stages = kStages;
-
-  // Pipeline position of this warp's role, kept from one batch of the list to the next.
+  const int warp, lane, rank;        // rank 0 = the CTA that issues the MMAs of the pair
+  const int H, I, n1, n2;
+  const uint32_t tmem_base;
+  const Abort ab;
+  const int b_sub_bytes, stage_bytes, stages;      // token half of one 64-column block, a stage, their number
+  // Position of this warp's role (each role uses its own of these).
   int s = 0; uint32_t ph = 0;
   int acc = 0; uint32_t acc_ph = 0;
   bool ok = true;
+  // A count that a down unit waits for before it writes its first row (null: nothing).
+  const int* y_free = nullptr;
+  int y_free_want = 0;
 
-  auto fill = [&](int first) {             // the units first, first + npairs, ... of this pair
-    for (int i = threadIdx.x; i < kFfnListUnits; i += blockDim.x) {
-      const long long u = first + (long long)i * npairs;
-      if (u < total) {
-        const FfnUnit un = plan.unit((int)u);
-        sm.list[i] = make_uint4(un.e_fc, un.j_ch, (uint32_t)un.row0, (uint32_t)un.n);
-      }
-    }
-    __syncthreads();
-  };
-  auto listed = [&](int i) {
-    const uint4 v = sm.list[i];
+  __device__ __forceinline__ FfnRoles(const McbFfnArgs& args, const CUtensorMap* x, const CUtensorMap* act, int n_slot)
+      : a(args), xmap(x), actmap(act), act_rows(reinterpret_cast<uint8_t*>(args.act)), y_rows(reinterpret_cast<uint8_t*>(args.y)), warp(threadIdx.x >> 5), lane(threadIdx.x & 31), rank((int)cluster_ctarank()),
+        H(args.hidden), I(args.intermediate), n1(2 * args.intermediate / kFfnRowsM), n2(args.hidden / kFfnRowsM),
+        tmem_base(*sm.tmem_slot), ab{sm.abort_flag, args.status, args.timeout_ns}, b_sub_bytes((n_slot >> 1) * 128),
+        stage_bytes(NSUB * (kFfnABytes + b_sub_bytes)), stages(stage_count(stage_bytes)) {}
+  static __device__ __forceinline__ int stage_count(int bytes) {
+    const int fit = kFfnPipeBytes / bytes, most = NSUB == 2 ? kFfnDoubleStages : kFfnMaxStages;
+    return fit < most ? fit : most;
+  }
+  static __device__ __forceinline__ FfnUnit listed(const uint4* list, int i) {
+    const uint4 v = list[i];
     return FfnUnit{v.x, v.y, (int)v.z, (int)v.w};
-  };
-  fill(pair);
-  if (ready.word && warp >= 2) {
-    if (lane == 0) ffn_wait_count(reinterpret_cast<const int*>(ready.word), ready.want, ab, 19, 0);
-    __syncwarp();
   }
 
-  for (int first = pair; first < total; first += kFfnListUnits * npairs) {
-    int count = (total - first + npairs - 1) / npairs;
-    if (count > kFfnListUnits) count = kFfnListUnits;
-    if (warp == 0) {
-      // ---------------- weights: 128 rows x 64 NSUB columns per CTA and stage ----------------
-      if (elect_one()) {
-        const uint64_t stream = l2_evict_first();
-        for (int i = 0; i < count && ok; ++i) {
-          const FfnUnit un = listed(i);
-          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
-          const CUtensorMap* map = maps + (un.fc() ? MCB_FFN_MAP_W2 : MCB_FFN_MAP_W1) + (NSUB - 1) * 2;
-          const int v = (un.e() * (un.fc() ? plan.n2 : plan.n1) + un.j()) * 2 + rank;     // 128-row block of the matrix
-          int row = v * k_blocks * (kFfnABytes / 2048);
-          for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
-            if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 11))) break;
-            if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * NSUB * kFfnABytes);
-            tma_load_2d_pair_hint(smem_u32(sm.pipe) + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row, stream);
-            if (++s == stages) { s = 0; ph ^= 1u; }
-          }
-        }
-      }
-    } else if (warp == 1) {
-      // ---------------- MMA: one thread of the leading CTA drives the tensor cores of both ----------------
-      if (rank == 0 && elect_one()) {
-        for (int i = 0; i < count && ok; ++i) {
-          const FfnUnit un = listed(i);
-          const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
-          const uint32_t idesc = umma_idesc_bf16(kFfnRowsM, (uint32_t)(un.half() * 2));
-          if (!(ok = mbar_wait(&sm.tempty[acc], acc_ph ^ 1u, ab, 12))) break;
-          tc_fence_after();
-          const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kFfnMaxN);
-          for (int kb = 0; kb < k_blocks; kb += NSUB) {
-            if (!(ok = mbar_wait(&sm.full[s], ph, ab, 13))) break;
-            tc_fence_after();
-            const uint32_t sa = smem_u32(sm.pipe + s * stage_bytes);
-#pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub) {
-              const uint64_t da = make_sw128_desc(sa + sub * kFfnABytes);
-              const uint64_t db = make_sw128_desc(sa + NSUB * kFfnABytes + sub * b_sub_bytes);
-#pragma unroll
-              for (int kk = 0; kk < kFfnBlockK / 16; ++kk)
-                umma_bf16_pair(d_tmem, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (kb | sub | kk) != 0);
-            }
-            umma_commit_pair(&sm.empty[s]);
-            if (++s == stages) { s = 0; ph ^= 1u; }
-          }
-          if (!ok) break;
-          umma_commit_pair(&sm.tfull[acc]);
-          if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
-        }
-      }
-    } else if (warp < 2 + kFfnEpiWarps) {
-      // ---------------- epilogue: TMEM (lane = weight row, column = token) -> global ----------------
-      const int q = warp & 3;                  // TMEM lane quarter this warp may read
-      const int hw = (warp - 2) >> 2;          // it takes the even or the odd 32-column groups
-      // A lane holds ONE feature of 32 tokens, memory wants the features of a token side by side: the values
-      // cross a small tile in shared memory ([column][feature], 64 or 32 bytes per row) and leave as 16-byte stores.
-      const uint32_t tile = smem_u32(sm.epi + (warp - 2) * kFfnTileBytes);
-      const uint32_t tempty_addr = cluster_map(sm.tempty, 0);
+  // One warp: 128 rows x 64 NSUB columns per CTA and stage.  wmaps: MCB_FFN_MAP_W1 ... of the weight set.
+  __device__ __forceinline__ void weights(const uint4* list, int count, const CUtensorMap* wmaps) {
+    if (elect_one()) {
+      const uint64_t stream = l2_evict_first();
       for (int i = 0; i < count && ok; ++i) {
-        const FfnUnit un = listed(i);
-        const int n = un.n;
-        if (!(ok = mbar_wait(&sm.tfull[acc], acc_ph, ab, 14))) break;
-        tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kFfnMaxN);
-        const int wrow = un.j() * kFfnRowsM + rank * 128 + q * 32;       // first weight row of the warp
-        auto release = [&] {                   // the accumulator has been read: hand it back before the stores
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster_relaxed(tempty_addr + acc * 8);
-        };
-        if (hw * 32 >= n) release();
-        if (!un.fc()) {
-          // rows alternate gate / up: lane pairs (2i, 2i + 1) hold the two halves of activation i; the even lane
-          // finishes the even columns, the odd lane the odd ones
-          const bool odd = lane & 1;
-          uint8_t* obase = reinterpret_cast<uint8_t*>(a.act) + (long long)un.row0 * I * 2 + wrow + (lane & 1) * 16;
-#pragma unroll 1
-          for (int cc = hw * 32; cc < n; cc += 64) {
-            uint32_t v[32];
-            tmem_ld32(t_row + cc, v);
-            tmem_ld_wait();
-            if (cc + 64 >= n) release();
-            // Each step over all columns before the next one: the stores keep their order with everything
-            // volatile, so a loop over columns would run one column's whole chain after the other.
-            uint32_t recv[16];
-            float r[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) recv[k] = __shfl_xor_sync(0xffffffffu, odd ? v[2 * k] : v[2 * k + 1], 1);
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const float g = __uint_as_float(odd ? recv[k] : v[2 * k]);
-              const float up = __uint_as_float(odd ? v[2 * k + 1] : recv[k]);
-              r[k] = silu(g) * up;
-            }
-#pragma unroll
-            for (int k = 0; k < 16; ++k) sts_bf16(tile + (2 * k + (lane & 1)) * 32 + (lane >> 1) * 2, r[k]);
-            __syncwarp();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {      // 32 columns x 16 features: lane l stores half (l & 1) of column 16h + (l >> 1)
-              const int cl = 16 * h + (lane >> 1);
-              const uint4 w = lds_v4(tile + cl * 32 + (lane & 1) * 16);
-              if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * I * 2, w);
-            }
-            __syncwarp();
-          }
-          // This warp's share of the gate/up unit is stored: make it visible to TMA loads of other CTAs and count
-          // it for the expert's down units (no barrier between the warps, so nothing can wait for a warp that
-          // has given up).
-          fence_proxy_async_global();
-          __threadfence();
-          __syncwarp();
-          if (lane == 0) atomicAdd(&a.ffn_done[un.e()], 1);
-        } else {
-          uint8_t* obase = reinterpret_cast<uint8_t*>(a.y) + ((long long)un.row0 * H + wrow) * 2 + (lane & 3) * 16;
-#pragma unroll 1
-          for (int cc = hw * 32; cc < n; cc += 64) {
-            const float mine = (a.pair_prob && cc + lane < n) ? a.pair_prob[un.row0 + cc + lane] : 1.0f;
-            uint32_t v[32];
-            tmem_ld32(t_row + cc, v);
-            tmem_ld_wait();
-            if (cc + 64 >= n) release();
-            float r[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) r[k] = __uint_as_float(v[k]) * __shfl_sync(0xffffffffu, mine, k);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) sts_bf16(tile + k * 64 + lane * 2, r[k]);
-            __syncwarp();
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {      // 32 columns x 32 features: lane l stores quarter (l & 3) of column 8h + (l >> 2)
-              const int cl = 8 * h + (lane >> 2);
-              const uint4 w = lds_v4(tile + cl * 64 + (lane & 3) * 16);
-              if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * H * 2, w);
-            }
-            __syncwarp();
-          }
+        const FfnUnit un = listed(list, i);
+        const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
+        const CUtensorMap* map = wmaps + un.fc() + (NSUB - 1) * 2;
+        const int v = (un.e() * (un.fc() ? n2 : n1) + un.j()) * 2 + rank;     // 128-row block of the matrix
+        int row = v * k_blocks * (kFfnABytes / 2048);
+        for (int kb = 0; kb < k_blocks; kb += NSUB, row += NSUB * kFfnABytes / 2048) {
+          if (!(ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 11))) break;
+          if (rank == 0) mbar_arrive_expect_tx(&sm.full[s], 2 * NSUB * kFfnABytes);
+          tma_load_2d_pair_hint(smem_u32(sm.pipe) + s * stage_bytes, map, cluster_map(&sm.full[s], 0), 0, row, stream);
+          if (++s == stages) { s = 0; ph ^= 1u; }
         }
+      }
+    }
+  }
+
+  // One warp of the leading CTA: one thread drives the tensor cores of both.
+  __device__ __forceinline__ void mma(const uint4* list, int count) {
+    if (elect_one()) {
+      for (int i = 0; i < count && ok; ++i) {
+        const FfnUnit un = listed(list, i);
+        const int k_blocks = (un.fc() ? I : H) / kFfnBlockK;
+        const uint32_t idesc = umma_idesc_bf16(kFfnRowsM, (uint32_t)(un.half() * 2));
+        if (!(ok = mbar_wait(&sm.tempty[acc], acc_ph ^ 1u, ab, 12))) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * kFfnMaxN);
+        for (int kb = 0; kb < k_blocks; kb += NSUB) {
+          if (!(ok = mbar_wait(&sm.full[s], ph, ab, 13))) break;
+          tc_fence_after();
+          const uint32_t sa = smem_u32(sm.pipe + s * stage_bytes);
+#pragma unroll
+          for (int sub = 0; sub < NSUB; ++sub) {
+            const uint64_t da = make_sw128_desc(sa + sub * kFfnABytes);
+            const uint64_t db = make_sw128_desc(sa + NSUB * kFfnABytes + sub * b_sub_bytes);
+#pragma unroll
+            for (int kk = 0; kk < kFfnBlockK / 16; ++kk)
+              umma_bf16_pair(d_tmem, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), idesc, (kb | sub | kk) != 0);
+          }
+          umma_commit_pair(&sm.empty[s]);
+          if (++s == stages) { s = 0; ph ^= 1u; }
+        }
+        if (!ok) break;
+        umma_commit_pair(&sm.tfull[acc]);
         if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
       }
-    } else if (warp < 2 + kFfnEpiWarps + kTok) {
-      // ---------------- tokens: this CTA's half of the chunk into the swizzled K-major B tile ----------------
-      // Each of the kTok warps fetches its groups of four rows, from one thread: a gather each, or one box.  Rows past
-      // the end of the chunk (they feed columns nobody reads) are fetched too, so that ALL warps of both CTAs
-      // contribute bytes to every stage: one that the stage did not wait for could fall a whole ring behind and
-      // misread the parity of `empty`.  The lanes fetch the token numbers of the next unit, one each, while the current one
-      // is still being copied, and hand them to the issuing thread through shared memory.
-      const int t = warp - 2 - kFfnEpiWarps;
-      constexpr int kOps = (kFfnMaxN / NSUB / 8 + kTok - 1) / kTok;
-      static_assert(kOps <= kFfnMaxGroups && kOps * 4 <= 32, "a map per box, a lane per row");
-      const uint32_t idx_slot = smem_u32(sm.tok_idx + t * 32);
-      const uint32_t pipe0 = smem_u32(sm.pipe) + NSUB * kFfnABytes, full0 = cluster_map(sm.full, 0);
-      auto fetch_idx = [&](const FfnUnit& un) {
-        const int rows = un.groups(kTok) * 4;
-        int r = rank * un.half() + un.first_group(t, kTok) * 4 + lane;
-        if (un.fc() || lane >= rows) return 0;
-        if (r >= un.n) r %= un.n;                  // spread over the chunk's rows, not all on one
-        return a.pair_token[un.row0 + r];
-      };
-      fence_proxy_async_global();          // token rows written by ordinary stores before this point
-      int nxt = fetch_idx(listed(0));
-      for (int i = 0; i < count && ok; ++i) {
-        const FfnUnit un = listed(i);
-        const int steps = (un.fc() ? I : H) / (kFfnBlockK * NSUB);
-        const int groups = un.groups(kTok), row_h = un.first_group(t, kTok) * 4;
-        if (!un.fc()) asm volatile("st.shared.b32 [%0], %1;" :: "r"(idx_slot + lane * 4), "r"(nxt) : "memory");
-        __syncwarp();
-        if (i + 1 < count) nxt = fetch_idx(listed(i + 1));
-        if (elect_one()) {
-          const uint32_t bytes = (uint32_t)(groups * kTok) * 1024u * NSUB;
-          int su = s; uint32_t pu = ph;
-          if (un.fc()) {
-            const int row = un.row0 + rank * un.half() + row_h;
-            const CUtensorMap* map = maps + MCB_FFN_MAP_ACT + groups - 1;
-            // the activations of this expert are complete once every epilogue warp of every gate/up unit has been counted
-            ffn_wait_count(&a.ffn_done[un.e()], 2 * kFfnEpiWarps * plan.n1 * un.chunks(), ab, 15, (uint32_t)un.e());
-            fence_proxy_async_global();
-            for (int k = 0; k < steps; ++k) {
-              if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
-              if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
-              const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
-#pragma unroll
-              for (int sub = 0; sub < NSUB; ++sub)
-                tma_load_2d_pair(dst + sub * b_sub_bytes, map, full0 + su * 8, (k * NSUB + sub) * kFfnBlockK, row);
-              if (++su == stages) { su = 0; pu ^= 1u; }
-            }
-          } else {
-            uint4 idx[kOps];
-#pragma unroll
-            for (int k = 0; k < kOps; ++k) idx[k] = lds_v4(idx_slot + k * 16);
-            for (int k = 0; k < steps; ++k) {
-              if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
-              if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
-              const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
-#pragma unroll
-              for (int g = 0; g < kOps; ++g) {
-                if (g >= groups) break;
-#pragma unroll
-                for (int sub = 0; sub < NSUB; ++sub)
-                  tma_gather4_pair(dst + sub * b_sub_bytes + g * 512, maps + MCB_FFN_MAP_X, full0 + su * 8,
-                                   (k * NSUB + sub) * kFfnBlockK, idx[g].x, idx[g].y, idx[g].z, idx[g].w);
-              }
-              if (++su == stages) { su = 0; pu ^= 1u; }
-            }
-          }
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        s += steps % stages;
-        ph ^= (uint32_t)(steps / stages) & 1u;
-        if (s >= stages) { s -= stages; ph ^= 1u; }
-        __syncwarp();
-      }
-    }
-    if (count == kFfnListUnits) {
-      __syncthreads();                     // the list is free for the next batch
-      fill(first + kFfnListUnits * npairs);
     }
   }
-  if (warp == 0 && elect_one()) {
-    // The last commits still arrive on both CTAs' `empty` barriers: nobody leaves before they have.
+
+  // kFfnEpiWarps warps, `ew` counts them from 0: TMEM (lane = weight row, column = token) -> global.
+  __device__ __forceinline__ void epilogue(const uint4* list, int begin, int count, int ew, const float* pair_prob, int* ffn_done) {
+    const int q = warp & 3;                  // TMEM lane quarter this warp may read
+    const int hw = ew >> 2;          // it takes the even or the odd 32-column groups
+    // A lane holds ONE feature of 32 tokens, memory wants the features of a token side by side: the values
+    // cross a small tile in shared memory ([column][feature], 64 or 32 bytes per row) and leave as 16-byte stores.
+    const uint32_t tile = smem_u32(sm.epi + ew * kFfnTileBytes);
+    const uint32_t tempty_addr = cluster_map(sm.tempty, 0);
+    for (int i = begin; i < count && ok; ++i) {
+      const FfnUnit un = listed(list, i);
+      const int n = un.n;
+      if (!(ok = mbar_wait(&sm.tfull[acc], acc_ph, ab, 14))) break;
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kFfnMaxN);
+      const int wrow = un.j() * kFfnRowsM + rank * 128 + q * 32;       // first weight row of the warp
+      auto release = [&] {                   // the accumulator has been read: hand it back before the stores
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(tempty_addr + acc * 8);
+      };
+      if (hw * 32 >= n) release();
+      if (!un.fc()) {
+        // rows alternate gate / up: lane pairs (2i, 2i + 1) hold the two halves of activation i; the even lane
+        // finishes the even columns, the odd lane the odd ones
+        const bool odd = lane & 1;
+        uint8_t* obase = act_rows + (long long)un.row0 * I * 2 + wrow + (lane & 1) * 16;
+#pragma unroll 1
+        for (int cc = hw * 32; cc < n; cc += 64) {
+          uint32_t v[32];
+          tmem_ld32(t_row + cc, v);
+          tmem_ld_wait();
+          if (cc + 64 >= n) release();
+          // Each step over all columns before the next one: the stores keep their order with everything
+          // volatile, so a loop over columns would run one column's whole chain after the other.
+          uint32_t recv[16];
+          float r[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) recv[k] = __shfl_xor_sync(0xffffffffu, odd ? v[2 * k] : v[2 * k + 1], 1);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const float g = __uint_as_float(odd ? recv[k] : v[2 * k]);
+            const float up = __uint_as_float(odd ? v[2 * k + 1] : recv[k]);
+            r[k] = silu(g) * up;
+          }
+#pragma unroll
+          for (int k = 0; k < 16; ++k) sts_bf16(tile + (2 * k + (lane & 1)) * 32 + (lane >> 1) * 2, r[k]);
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {      // 32 columns x 16 features: lane l stores half (l & 1) of column 16h + (l >> 1)
+            const int cl = 16 * h + (lane >> 1);
+            const uint4 w = lds_v4(tile + cl * 32 + (lane & 1) * 16);
+            if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * I * 2, w);
+          }
+          __syncwarp();
+        }
+        // This warp's share of the gate/up unit is stored: make it visible to TMA loads of other CTAs and count
+        // it for the expert's down units (no barrier between the warps, so nothing can wait for a warp that
+        // has given up).
+        fence_proxy_async_global();
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) atomicAdd(&ffn_done[un.e()], 1);
+      } else {
+        if (y_free) {
+          if (lane == 0) ffn_wait_count(y_free, y_free_want, ab, 20, (uint32_t)un.e());
+          __syncwarp();
+          y_free = nullptr;
+        }
+        uint8_t* obase = y_rows + ((long long)un.row0 * H + wrow) * 2 + (lane & 3) * 16;
+#pragma unroll 1
+        for (int cc = hw * 32; cc < n; cc += 64) {
+          const float mine = (pair_prob && cc + lane < n) ? pair_prob[un.row0 + cc + lane] : 1.0f;
+          uint32_t v[32];
+          tmem_ld32(t_row + cc, v);
+          tmem_ld_wait();
+          if (cc + 64 >= n) release();
+          float r[32];
+#pragma unroll
+          for (int k = 0; k < 32; ++k) r[k] = __uint_as_float(v[k]) * __shfl_sync(0xffffffffu, mine, k);
+#pragma unroll
+          for (int k = 0; k < 32; ++k) sts_bf16(tile + k * 64 + lane * 2, r[k]);
+          __syncwarp();
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {      // 32 columns x 32 features: lane l stores quarter (l & 3) of column 8h + (l >> 2)
+            const int cl = 8 * h + (lane >> 2);
+            const uint4 w = lds_v4(tile + cl * 64 + (lane & 3) * 16);
+            if (cc + cl < n) st_v4(obase + (long long)(cc + cl) * H * 2, w);
+          }
+          __syncwarp();
+        }
+      }
+      if (++acc == 2) { acc = 0; acc_ph ^= 1u; }
+    }
+  }
+
+  // TOK warps, `t` counts them from 0: this CTA's half of the chunk into the swizzled K-major B tile.
+  __device__ __forceinline__ void tokens(const uint4* list, int count, int t, const int* pair_token, const int* ffn_done) {
+    // Each of the TOK warps fetches its groups of four rows, from one thread: a gather each, or one box.  Rows past
+    // the end of the chunk (they feed columns nobody reads) are fetched too, so that ALL warps of both CTAs
+    // contribute bytes to every stage: one that the stage did not wait for could fall a whole ring behind and
+    // misread the parity of `empty`.  The lanes fetch the token numbers of the next unit, one each, while the current one
+    // is still being copied, and hand them to the issuing thread through shared memory.
+    constexpr int kOps = (kFfnMaxN / NSUB / 8 + TOK - 1) / TOK;
+    static_assert(kOps <= kFfnMaxGroups && kOps * 4 <= 32, "a map per box, a lane per row");
+    const uint32_t idx_slot = smem_u32(sm.tok_idx + t * 32);
+    const uint32_t pipe0 = smem_u32(sm.pipe) + NSUB * kFfnABytes, full0 = cluster_map(sm.full, 0);
+    auto fetch_idx = [&](const FfnUnit& un) {
+      const int rows = un.groups(TOK) * 4;
+      int r = rank * un.half() + un.first_group(t, TOK) * 4 + lane;
+      if (un.fc() || lane >= rows) return 0;
+      if (r >= un.n) r %= un.n;                  // spread over the chunk's rows, not all on one
+      return pair_token[un.row0 + r];
+    };
+    fence_proxy_async_global();          // token rows written by ordinary stores before this point
+    int nxt = fetch_idx(listed(list, 0));
+    for (int i = 0; i < count && ok; ++i) {
+      const FfnUnit un = listed(list, i);
+      const int steps = (un.fc() ? I : H) / (kFfnBlockK * NSUB);
+      const int groups = un.groups(TOK), row_h = un.first_group(t, TOK) * 4;
+      if (!un.fc()) asm volatile("st.shared.b32 [%0], %1;" :: "r"(idx_slot + lane * 4), "r"(nxt) : "memory");
+      __syncwarp();
+      if (i + 1 < count) nxt = fetch_idx(listed(list, i + 1));
+      if (elect_one()) {
+        const uint32_t bytes = (uint32_t)(groups * TOK) * 1024u * NSUB;
+        int su = s; uint32_t pu = ph;
+        if (un.fc()) {
+          const int row = un.row0 + rank * un.half() + row_h;
+          const CUtensorMap* map = actmap + groups - 1;
+          // the activations of this expert are complete once every epilogue warp of every gate/up unit has been counted
+          ffn_wait_count(&ffn_done[un.e()], 2 * kFfnEpiWarps * n1 * un.chunks(), ab, 15, (uint32_t)un.e());
+          fence_proxy_async_global();
+          for (int k = 0; k < steps; ++k) {
+            if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
+            if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
+            const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
+#pragma unroll
+            for (int sub = 0; sub < NSUB; ++sub)
+              tma_load_2d_pair(dst + sub * b_sub_bytes, map, full0 + su * 8, (k * NSUB + sub) * kFfnBlockK, row);
+            if (++su == stages) { su = 0; pu ^= 1u; }
+          }
+        } else {
+          uint4 idx[kOps];
+#pragma unroll
+          for (int k = 0; k < kOps; ++k) idx[k] = lds_v4(idx_slot + k * 16);
+          for (int k = 0; k < steps; ++k) {
+            if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
+            if (rank == 0 && t == 0) mbar_arrive_expect_tx(&sm.full[su], bytes);
+            const uint32_t dst = pipe0 + su * stage_bytes + row_h * 128;
+#pragma unroll
+            for (int g = 0; g < kOps; ++g) {
+              if (g >= groups) break;
+#pragma unroll
+              for (int sub = 0; sub < NSUB; ++sub)
+                tma_gather4_pair(dst + sub * b_sub_bytes + g * 512, xmap, full0 + su * 8,
+                                 (k * NSUB + sub) * kFfnBlockK, idx[g].x, idx[g].y, idx[g].z, idx[g].w);
+            }
+            if (++su == stages) { su = 0; pu ^= 1u; }
+          }
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      s += steps % stages;
+      ph ^= (uint32_t)(steps / stages) & 1u;
+      if (s >= stages) { s -= stages; ph ^= 1u; }
+      __syncwarp();
+    }
+  }
+
+  // The weight warp, after its last unit: the last commits still arrive on both CTAs' `empty` barriers, and nobody leaves
+  // before they have.
+  __device__ __forceinline__ void drain() {
+    if (!elect_one()) return;
     for (int i = 0; i < stages && ok; ++i) {
       ok = mbar_wait(&sm.empty[s], ph ^ 1u, ab, 17);
       if (++s == stages) { s = 0; ph ^= 1u; }
     }
   }
+};
+
+template <int NSUB>
+__device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap* maps, const FfnPlanS& plan, const int n_slot, const FfnReady ready) {
+  constexpr int kTok = NSUB == 2 ? 4 : kFfnTokWarps;      // token warps of this launch
+  FfnRoles<NSUB, kTok> r(a, maps + MCB_FFN_MAP_X, maps + MCB_FFN_MAP_ACT, n_slot);
+  const int npairs = (int)gridDim.x >> 1, pair = (int)blockIdx.x >> 1, total = plan.total();
+  auto fill = [&](int first) {             // the units first, first + npairs, ... of this pair
+    plan.list(r.sm.list, kFfnListUnits, first, npairs, total, (int)threadIdx.x, (int)blockDim.x);
+    __syncthreads();
+  };
+  fill(pair);
+  if (ready.word && r.warp >= 2) {
+    if (r.lane == 0) ffn_wait_count(reinterpret_cast<const int*>(ready.word), ready.want, r.ab, 19, 0);
+    __syncwarp();
+  }
+  for (int first = pair; first < total; first += kFfnListUnits * npairs) {
+    int count = (total - first + npairs - 1) / npairs;
+    if (count > kFfnListUnits) count = kFfnListUnits;
+    if (r.warp == 0) r.weights(r.sm.list, count, maps + MCB_FFN_MAP_W1);
+    else if (r.warp == 1) { if (r.rank == 0) r.mma(r.sm.list, count); }
+    else if (r.warp < 2 + kFfnEpiWarps) r.epilogue(r.sm.list, 0, count, r.warp - 2, a.pair_prob, a.ffn_done);
+    else if (r.warp < 2 + kFfnEpiWarps + kTok) r.tokens(r.sm.list, count, r.warp - 2 - kFfnEpiWarps, a.pair_token, a.ffn_done);
+    if (count == kFfnListUnits) {
+      __syncthreads();                     // the list is free for the next batch
+      fill(first + kFfnListUnits * npairs);
+    }
+  }
+  if (r.warp == 0) r.drain();
 }
 
 // Call from all kFfnThreads threads of every CTA of the grid (clusters of two CTAs along x), between ffn_setup and
@@ -577,20 +663,12 @@ __device__ __forceinline__ void ffn_roles(const McbFfnArgs& a, const CUtensorMap
 __device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* maps, int max_rows, const FfnReady ready) {
   const FfnSmem sm;
   const int E = a.num_local_experts;
-  if (max_rows < 1) max_rows = 1;
   fence_proxy_async_smem();                // the pipeline's memory may have been in ordinary use until here
   __syncthreads();
+  const int n_slot = ffn_token_tile(max_rows);
   FfnPlanS plan;
   plan.off = sm.off; plan.cum = sm.cum; plan.ids = sm.ids;
-  plan.n1 = 2 * a.intermediate / kFfnRowsM; plan.n2 = a.hidden / kFfnRowsM;
-  plan.active = ffn_slots(sm.off, E, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi));
-  plan.lag = plan.active;
-  if ((long long)sm.off[E] * a.intermediate * 2 > kFfnActL2Bytes) {      // three rounds of the grid, in slots of average size
-    const int lag = (int)((long long)gridDim.x * 3 / 2 * plan.active / plan.total()) + 2;
-    if (lag < plan.lag) plan.lag = lag;
-  }
-  // Token tile of this launch: the largest expert, rounded up to 16, at most kFfnMaxN per chunk.
-  const int n_slot = max_rows > kFfnMaxN ? kFfnMaxN : ((max_rows + 15) & ~15);
+  ffn_plan(plan, a, ffn_slots(BlockGroup{}, sm.off, E, n_slot, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi)));
   if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, maps, plan, n_slot, ready);
   else ffn_roles<1>(a, maps, plan, n_slot, ready);
 }

@@ -8,12 +8,12 @@
 #define MCB_GEMM_FC1 0          // gate/up projection + SwiGLU epilogue
 #define MCB_GEMM_FC2 1          // down projection + per-row scale epilogue
 // Tensor maps of the fused FFN: token rows (gathered four at a time), gate/up and down tiles (16 KB, then 32 KB), and
-// activations in boxes of 4, 8, ... 24 rows.
+// activations in boxes of 4, 8, ... 32 rows.
 #define MCB_FFN_MAP_X 0
 #define MCB_FFN_MAP_W1 1
 #define MCB_FFN_MAP_W2 2
 #define MCB_FFN_MAP_ACT 5
-#define MCB_FFN_TMAPS 11
+#define MCB_FFN_TMAPS 13
 #define MCB_GEMM_ERR_TIMEOUT 5  // status code: a bounded mbarrier wait ran out
 
 #ifdef __cplusplus
@@ -131,4 +131,28 @@ typedef struct alignas(64) {
   unsigned long long* trace;
   unsigned long long reserved0;
 } McbLayerArgs;
+
+#define MCB_STEP_SETS 16        // weight sets of one launch (four tensor maps each, in its parameters)
+#define MCB_STEP_SYNC_WORDS 160 // counters of a step, 128 bytes apart
+
+// Several layers of a world of one as ONE launch (moe_step.cu).  `layer` is what a layer kernel takes, of any weight set; the
+// buffers that layers in flight do not share come three times (pair lists and counters) or twice: [0] those of the last layer,
+// which are layer.route's and layer.ffn's own.
+typedef struct alignas(64) {
+  McbLayerArgs layer;
+  const int64_t* ids;            // expert ids, weights (null: 1) and rows of this rank's tokens where the all-gather reads them
+  const float* probs;
+  const void* x;
+  int32_t* pair_token[3];
+  float* pair_prob[3];
+  int32_t* pair_pos[3];
+  int32_t* ffn_done[3];
+  void* act[2];                  // the second ones hold two_rows pair rows; larger steps use one buffer for all layers
+  void* y[2];
+  int64_t two_rows;
+  int32_t* expert_count;         // [3][E_loc], zero between launches
+  int32_t* sync;                 // [MCB_STEP_SYNC_WORDS], zero between launches
+  alignas(64) unsigned long long map_x[16];    // token rows
+  unsigned long long map_act[2][8][16];        // activations, by box
+} McbMoeStepArgs;
 #endif

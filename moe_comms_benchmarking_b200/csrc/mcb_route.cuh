@@ -15,6 +15,7 @@
 #pragma once
 #include "mcb_barrier.cuh"
 #include "mcb_gemm.h"
+#include "mcb_group.cuh"
 
 namespace mcb {
 
@@ -30,6 +31,7 @@ struct RouteSmem {
   int *cnt, *begin, *off, *scan;
   __device__ __forceinline__ explicit RouteSmem(int* base)
       : cnt(base), begin(base + kMaxLocalExperts), off(base + 2 * kMaxLocalExperts), scan(base + 3 * kMaxLocalExperts + 1) {}
+  __device__ __forceinline__ RouteSmem(int* cnt_, int* begin_, int* off_, int* scan_) : cnt(cnt_), begin(begin_), off(off_), scan(scan_) {}
 };
 
 // This block's share of the entries.
@@ -47,53 +49,57 @@ __device__ __forceinline__ RouteShare route_share(const McbRouteArgs& a, int blo
   s.hi = s.lo + per < s.entries ? s.lo + per : s.entries;
   return s;
 }
-__device__ __forceinline__ bool route_counts_all(const RouteShare& s) {
-  return s.entries <= (long long)kRouteAllPerThread * blockDim.x;
+template <class Group>
+__device__ __forceinline__ bool route_counts_all(const Group& g, const RouteShare& s) {
+  return s.entries <= (long long)kRouteAllPerThread * g.size();
 }
 
-// Counts the entries [lo, hi) into m.cnt and, with SPLIT, those before `split` into m.begin too.  All threads of the block.
-template <bool SPLIT>
-__device__ __forceinline__ void route_count(const McbRouteArgs& a, const int64_t* topk_idx, const RouteSmem& m, long long lo,
+// Counts the entries [lo, hi) into m.cnt and, with SPLIT, those before `split` into m.begin too.  All threads of the group.
+template <bool SPLIT, class Group>
+__device__ __forceinline__ void route_count(const Group& g, const McbRouteArgs& a, const int64_t* topk_idx, const RouteSmem& m, long long lo,
                                             long long hi, long long split) {
-  const int tid = threadIdx.x, E = a.num_local_experts;
-  for (int e = tid; e < E; e += blockDim.x) { m.cnt[e] = 0; m.begin[e] = 0; }
-  __syncthreads();
-  for (long long i0 = lo + tid; i0 < hi; i0 += blockDim.x * 4) {
+  const int tid = g.tid(), threads = g.size(), E = a.num_local_experts;
+  for (int e = tid; e < E; e += threads) { m.cnt[e] = 0; m.begin[e] = 0; }
+  g.sync();
+  for (long long i0 = lo + tid; i0 < hi; i0 += threads * 4) {
     long long e[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + u * blockDim.x;
+      const long long i = i0 + u * threads;
       e[u] = i < hi ? topk_idx[i] - a.expert_begin : -1;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (e[u] >= 0 && e[u] < E) {
         atomicAdd(&m.cnt[(int)e[u]], 1);
-        if (SPLIT && i0 + u * blockDim.x < split) atomicAdd(&m.begin[(int)e[u]], 1);
+        if (SPLIT && i0 + u * threads < split) atomicAdd(&m.begin[(int)e[u]], 1);
       }
   }
-  __syncthreads();
+  g.sync();
 }
 
 // Many entries, before the barrier: this block's counts into the counters; m.begin = where its entries begin.
-__device__ __forceinline__ void route_publish(const McbRouteArgs& a, const RouteSmem& m) {
-  for (int e = threadIdx.x; e < a.num_local_experts; e += blockDim.x)
-    m.begin[e] = m.cnt[e] ? atomicAdd(&a.expert_count[e], m.cnt[e]) : 0;
+template <class Group>
+__device__ __forceinline__ void route_publish(const Group& g, int E, int* expert_count, const RouteSmem& m) {
+  for (int e = g.tid(); e < E; e += g.size())
+    m.begin[e] = m.cnt[e] ? atomicAdd(&expert_count[e], m.cnt[e]) : 0;
 }
 // ... and after it: the counts of all blocks.
-__device__ __forceinline__ void route_collect(const McbRouteArgs& a, const RouteSmem& m) {
-  for (int e = threadIdx.x; e < a.num_local_experts; e += blockDim.x)
-    m.cnt[e] = *reinterpret_cast<volatile int*>(&a.expert_count[e]);
-  __syncthreads();
+template <class Group>
+__device__ __forceinline__ void route_collect(const Group& g, int E, const int* expert_count, const RouteSmem& m) {
+  for (int e = g.tid(); e < E; e += g.size())
+    m.cnt[e] = *reinterpret_cast<const volatile int*>(&expert_count[e]);
+  g.sync();
 }
 
 // Offsets of the experts (exclusive prefix of m.cnt) into m.off[0 .. E] by a block-wide scan; the block that `writes` puts
 // them, the 128-row tile table of the tokens-as-rows GEMMs, the largest count and the zeroed "gate/up done" counters of
-// the fused FFN into global memory.  Returns the largest count in every thread.  All threads of the block.
-__device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteSmem& m, bool writes) {
-  const int E = a.num_local_experts, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
-  const int per = (E + (int)blockDim.x - 1) / (int)blockDim.x;
-  const int e0 = threadIdx.x * per, e1 = e0 + per < E ? e0 + per : E;
+// the fused FFN into global memory.  Returns the largest count in every thread.  All threads of the group.
+template <class Group>
+__device__ __forceinline__ int route_offsets(const Group& g, const McbRouteArgs& a, const RouteSmem& m, bool writes) {
+  const int tid = g.tid(), E = a.num_local_experts, warp = tid >> 5, lane = tid & 31, nw = g.size() >> 5;
+  const int per = (E + g.size() - 1) / g.size();
+  const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
   int rows = 0, tiles = 0, mx = 0;
   for (int e = e0; e < e1; ++e) {
     const int c = m.cnt[e];
@@ -109,7 +115,7 @@ __device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteS
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 31) { m.scan[warp] = r_inc; m.scan[32 + warp] = t_inc; m.scan[64 + warp] = mx; }
-  __syncthreads();
+  g.sync();
   // Every warp scans the warps' sums for itself, lane w holding those of warp w.
   int run = r_inc - rows, tile = t_inc - tiles;
   r_inc = lane < nw ? m.scan[lane] : 0;
@@ -139,7 +145,7 @@ __device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteS
     }
     run += c;
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     m.off[E] = total;
     if (writes) {
       a.expert_offset[E] = total;
@@ -152,27 +158,28 @@ __device__ __forceinline__ int route_offsets(const McbRouteArgs& a, const RouteS
       *a.num_m_tiles = total_tiles < a.max_tiles ? total_tiles : a.max_tiles;
     }
   }
-  __syncthreads();
+  g.sync();
   return mx;
 }
 
 // Places this block's entries: pair row = offset of the expert + where the block's entries of it begin + a cursor (m.begin
-// is used up).  All threads of the block.
-__device__ __forceinline__ void route_place(const McbRouteArgs& a, const int64_t* topk_idx, const float* topk_w,
+// is used up).  All threads of the group.
+template <class Group>
+__device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& a, const int64_t* topk_idx, const float* topk_w,
                                             const RouteSmem& m, const RouteShare& s) {
-  const int E = a.num_local_experts;
-  for (long long i0 = s.lo + threadIdx.x; i0 < s.hi; i0 += blockDim.x * 4) {
+  const int E = a.num_local_experts, threads = g.size();
+  for (long long i0 = s.lo + g.tid(); i0 < s.hi; i0 += threads * 4) {
     long long e[4];
     float w[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + u * blockDim.x;
+      const long long i = i0 + u * threads;
       e[u] = i < s.hi ? topk_idx[i] - a.expert_begin : -1;
       w[u] = i < s.hi && topk_w ? topk_w[i] : 1.0f;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long i = i0 + u * blockDim.x;
+      const long long i = i0 + u * threads;
       if (i >= s.hi) break;
       int pos = -1;
       if (e[u] >= 0 && e[u] < E) {
@@ -197,16 +204,17 @@ __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
   const RouteSmem m(smem);
   const int tid = threadIdx.x;
   const RouteShare s = route_share(a, (int)blockIdx.x, (int)gridDim.x);
-  if (route_counts_all(s)) {
+  const BlockGroup g;
+  if (route_counts_all(g, s)) {
     if (s.lo >= s.hi && blockIdx.x != 0) return;
-    route_count<true>(a, a.topk_idx, m, 0, s.entries, s.lo);
-    route_offsets(a, m, blockIdx.x == 0);
-    route_place(a, a.topk_idx, a.topk_w, m, s);
+    route_count<true>(g, a, a.topk_idx, m, 0, s.entries, s.lo);
+    route_offsets(g, a, m, blockIdx.x == 0);
+    route_place(g, a, a.topk_idx, a.topk_w, m, s);
     return;
   }
   volatile int* arrived = a.sync;                            // back at zero when the last block has left
-  route_count<false>(a, a.topk_idx, m, s.lo, s.hi, 0);
-  route_publish(a, m);
+  route_count<false>(g, a, a.topk_idx, m, s.lo, s.hi, 0);
+  route_publish(g, a.num_local_experts, a.expert_count, m);
   __syncthreads();
   if (tid == 0) {
     __threadfence();
@@ -223,9 +231,9 @@ __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
     __threadfence();
   }
   __syncthreads();
-  route_collect(a, m);
-  route_offsets(a, m, blockIdx.x == 0);
-  route_place(a, a.topk_idx, a.topk_w, m, s);
+  route_collect(g, a.num_local_experts, a.expert_count, m);
+  route_offsets(g, a, m, blockIdx.x == 0);
+  route_place(g, a, a.topk_idx, a.topk_w, m, s);
   __shared__ int s_last;
   __syncthreads();
   if (tid == 0) {

@@ -175,7 +175,8 @@ def layer_args_size() -> int:
 
 
 GEMM_FC1, GEMM_FC2 = 0, 1
-FFN_TMAPS = 11
+FFN_TMAPS = 13
+STEP_SETS, STEP_SYNC_WORDS = 16, 160
 
 _STRUCTS = {
     "ctx": McbCtx, "load_args": McbLoadArgs, "meta_args": McbMetaArgs, "agv_args": McbAgvArgs, "rsv_args": McbRsvArgs,
@@ -190,7 +191,8 @@ _LAUNCHERS = {
     "mcb_launch_load_batch": "pip", "mcb_launch_metadata": "ppip", "mcb_launch_agv": "ppiiip", "mcb_launch_rsv": "ppiiip",
     "mcb_launch_dense_step": "ppiiip", "mcb_launch_a2a_dispatch": "ppiiip", "mcb_launch_a2a_combine": "ppiiip",
     "mcb_launch_a2a_step": "ppiiip", "mcb_launch_route": "piip", "mcb_launch_expert_ffn": "piip",
-    "mcb_launch_combine": "ppiiip", "mcb_launch_moe_layer": "piip",
+    "mcb_launch_combine": "ppiiip", "mcb_launch_moe_layer": "piip", "mcb_moe_decode_step": "pppiiiipp",
+    "mcb_prepare_moe_step": "ppip" + "p" * 8 + "i",
 }
 
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libmcb.so"

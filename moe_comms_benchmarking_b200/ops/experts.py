@@ -21,6 +21,11 @@ from ..parallel.symm_heap import HeapTensor, SymmetricHeap
 
 NUM_SMS = 148
 BLOCK_M = 128
+# Activations (or expert outputs) of a layer up to which the layers of a step alternate between two buffers of them: nobody then waits
+# for the slowest CTA of the layer before, but twice the memory is written, which leaves L2 from some size on.  512 experts of
+# 1024 x 1024, one / 64 / 128 / 256 tokens (11.5 MB) 23.8 / 409 / 448 / 459 us a layer (26.1 / 411 / 452 / 459 with one buffer); 300 tokens
+# of 16 experts of 2048 x 1408 (4.9 MB) 41.4 (43.3); 60 tokens of 32 of 7168 x 2048 (6.9 MB) 392 (386).
+STEP_TWO_BUFFERS_BYTES = 6 << 20
 
 
 def _swizzle(t: torch.Tensor) -> torch.Tensor:
@@ -347,7 +352,9 @@ def local_routing(heap: SymmetricHeap, agv: "_ext.McbAgvArgs", route: "_ext.McbR
 class MoeLayerPlan:
     """One whole MoE layer per launch (``moe_layer_kernel``: dispatch, routing, experts, combine), for
     one or several weight sets; ``launch(s)`` runs the layer with set ``s``, ``decode_step(n)`` issues the
-    count exchange and ``n`` layers natively (layer l uses set l % sets)."""
+    count exchange and ``n`` layers natively (layer l uses set l % sets).  In a world of one the layers of a step share a
+    launch (csrc/moe_step.cu; up to 16 of them where there are more sets than that) unless a layer writes what the next one
+    reads or a phase trace is taken."""
 
     def __init__(self, heap: SymmetricHeap, agv, route: RoutePlan, ffns: list[ExpertFfnPlan], combine: ExpertCombinePlan,
                  meta, grid: int = NUM_SMS, trace: bool = False):
@@ -358,6 +365,7 @@ class MoeLayerPlan:
         self.trace = torch.zeros(8, dtype=torch.int64, device=heap.device) if trace else None
         self._raw, self._addr, self._stride = _aligned_layer_args(len(ffns))
         self._ctx_version = None
+        self._step = self._step_bufs = None
         self._fill()
 
     def _fill(self):
@@ -371,7 +379,40 @@ class MoeLayerPlan:
             C.memmove(C.addressof(p.cmb), C.addressof(self.combine.args), C.sizeof(_ext.McbCombineArgs))
             p.trace = self.trace.data_ptr() if self.trace is not None else None
             p.local_ids, p.local_probs = local_routing(self.heap, self.agv.args, self.route.args)
+        self._prepare_step()
         self._ctx_version = id(ctx)
+
+    def _prepare_step(self):
+        """Several layers of a step in one launch, where the layers allow it (``mcb_prepare_moe_step`` in csrc/moe_step.cu)."""
+        self._step = None
+        if self.heap.world != 1 or self.trace is not None:
+            return
+        b, f = self.route.bufs, self.ffns[0].args
+        if self._step_bufs is None:         # pair lists and counters of two more layers in flight
+            sizes = [2 * b.max_pairs, 2 * b.max_pairs, 2 * b.max_tokens * b.topk, 2 * b.E, 3 * b.E, _ext.STEP_SYNC_WORDS]
+            starts = [0]
+            for n in sizes:
+                starts.append(starts[-1] + (n + 31) // 32 * 32)
+            mem = torch.zeros(starts[-1], dtype=torch.int32, device=self.heap.device)
+            mem[starts[2]:starts[3]] = -1
+            keep, ptrs = [mem], [mem.data_ptr() + 4 * s for s in starts[:-1]]
+            # ... and their activations and expert outputs
+            rows = max(1, min(b.max_pairs, STEP_TWO_BUFFERS_BYTES // (2 * max(f.hidden, f.intermediate))))
+            keep += [torch.empty(rows, cols, dtype=torch.bfloat16, device=mem.device) for cols in (f.intermediate, f.hidden)]
+            ptrs += [t.data_ptr() for t in keep[1:]] + [rows]
+            if mem.is_cuda:
+                torch.cuda.current_stream(mem.device).synchronize()        # a step may run on another stream
+            self._step_bufs = (keep, ptrs)
+        lib = _ext.require()
+        raw = (C.c_uint8 * (lib.mcb_sizeof_step_args() + 64))()
+        addr = (C.addressof(raw) + 63) & ~63
+        if lib.mcb_prepare_moe_step(addr, self._addr, len(self.ffns), C.byref(self.meta.args), *self._step_bufs[1]) == 0:
+            self._step = (raw, addr)
+
+    def launches(self, num_layers: int) -> int:
+        """Kernel launches of ``decode_step(num_layers)``: the count exchange and those of the layers."""
+        together = 1 if self._step is None or num_layers < 2 else num_layers if len(self.ffns) <= _ext.STEP_SETS else _ext.STEP_SETS
+        return 1 + -(-num_layers // together)
 
     def _sync_ctx(self):
         if self._ctx_version != id(self.heap.ctx()):      # the heap's context was rebuilt (e.g. a new timeout)
@@ -401,6 +442,6 @@ class MoeLayerPlan:
     def decode_step(self, num_layers: int, pdl: bool = False, stream=None):
         lib = _ext.require()
         self._sync_ctx()
-        _ext.check(lib.mcb_moe_decode_step(self.heap.ctx_ref(), C.byref(self.meta.args), C.c_void_p(self._addr),
-                                           len(self.ffns), int(num_layers), self.grid, int(pdl),
+        _ext.check(lib.mcb_moe_decode_step(self.heap.ctx_ref(), C.byref(self.meta.args), self._addr, len(self.ffns),
+                                           int(num_layers), self.grid, int(pdl), self._step[1] if self._step else None,
                                            _ext.stream_handle(stream)), "moe_decode_step")

@@ -14,7 +14,8 @@ expert computation the transport exists for.  Per layer and rank:
 By default the whole layer is ONE cooperative kernel (``moe_layer_kernel`` in csrc/ffn.cu: dispatch,
 routing, the grouped FFN with the weights as the M operand and both projections in one persistent weight
 stream, combine; grid barriers behind the dispatch and the experts, none between routing and experts),
-and a decode step is issued by one native call (count exchange + one launch per layer).  ``layer_kernel=False`` selects the older
+and a decode step is issued by one native call: the count exchange and one launch per layer, or in a world of
+one a launch for all layers (``moe_step_kernel`` in csrc/moe_step.cu), whose weight stream runs through.  ``layer_kernel=False`` selects the older
 form with the tokens as the M operand: two kernels per layer (``dispatch_route_fc1_kernel`` and
 ``fc2_combine_kernel`` in csrc/gemm.cu), or five with ``fuse_dispatch=False`` / ``fuse_combine=False``.
 
@@ -55,7 +56,8 @@ class FusedExpertDispatcher(Dispatcher):
         self.fuse_dispatch = bool(fuse_dispatch)
         self.layer_kernel = bool(layer_kernel)
         self.phase_trace = bool(phase_trace) and self.layer_kernel
-        self.kernel_launches_per_step = lambda nl: 1 + (
+        self.layer_plan = None
+        self.kernel_launches_per_step = lambda nl: self.layer_plan.launches(nl) if self.layer_plan else 1 + (
             1 if self.layer_kernel else 5 - int(self.fuse_combine) - 2 * int(self.fuse_dispatch)) * nl
 
     @staticmethod

@@ -506,3 +506,77 @@ def test_expert_ffn_token_rows_of_any_shape(world1, shape):
         heap.check_status()
         got.append(y)
     assert torch.equal(got[0], got[1]) and bool(got[0].count_nonzero() > got[0].numel() // 2)
+
+
+@pytest.mark.parametrize("E,K,H,I,T,layers,sets,grid", [
+    (8, 2, 256, 128, 3, 2, 1, 148),          # two layers; fewer units than CTA pairs
+    (8, 2, 256, 128, 90, 40, 20, 148),       # more weight sets than one launch takes, buffers used many times over
+    (64, 6, 768, 512, 700, 5, 2, 148),       # counts of the later layers through the shared counters
+    (6, 3, 512, 384, 1500, 4, 3, 148),       # several chunks per expert, one block per stage
+    (40, 4, 256, 128, 200, 7, 2, 2),         # one pair of CTAs: more units than half a list holds
+    (768, 22, 256, 128, 65, 3, 1, 30),       # as many experts as fit
+    (769, 5, 256, 128, 40, 3, 1, 148),       # one more: layer by layer
+    (4, 2, 2048, 256, 1600, 3, 2, 148),      # one buffer of expert outputs for all layers
+])
+def test_step_of_several_layers(world1, E, K, H, I, T, layers, sets, grid):
+    """decode_step with its layers in one launch against the same layers launched one by one, bit for bit (both add the same
+    products in the same order), and the rows that it gathers; smaller batches and none through the same plan; twice, so counters
+    come back clean."""
+    from moe_comms_benchmarking_b200.config import Config
+    from moe_comms_benchmarking_b200.ops.experts import MoeLayerPlan
+    from moe_comms_benchmarking_b200.parallel.fused import FusedExpertDispatcher
+    cfg = Config(num_experts=E, topk=K, hidden=H, intermediate=I, ep_size=1, per_rank_cap=T + 3, probs="softmax")
+    d = FusedExpertDispatcher(cfg, world1, num_layers=layers, weight_budget_gb=(sets * 6 * E * H * I + 1) / 2**30)
+    d.build()
+    plan = MoeLayerPlan(d.heap, d.agv_plan, d.route_plan, d.ffn, d.combine_plan, d.meta_plan, grid=grid)
+    assert len(d.ffn) == sets and (plan._step is None) == (E > 768)
+    for n in (T, T // 3 + 1, 0, T):
+        x, idx, w = _case(max(n, 1), E, K, H, I, n + 31)
+        d.setup_batch(x[:n], idx[:n], w[:n])
+        d.metadata()
+        for l in range(layers):
+            plan.launch(l % sets)
+        torch.cuda.synchronize()
+        want = d.out.clone()
+        for rep in range(2):
+            for t in (d.out_buf, d.y, d.act, d.agv_h.tensor):
+                t.fill_(float("nan"))
+            plan.decode_step(layers)
+            torch.cuda.synchronize()
+            d.check_health()
+            assert torch.equal(d.out, want), f"{n} tokens, rep {rep}"
+            assert torch.equal(d.agv_h.tensor[:n], x[:n]) and torch.equal(d.agv_r.tensor[:n], idx[:n]) and torch.equal(d.agv_p.tensor[:n], w[:n])
+    d.destroy()
+
+
+def test_step_on_its_own_output_goes_layer_by_layer(world1):
+    """Layers that read what the layer before has written keep their order: rows gathered from the combined output."""
+    from moe_comms_benchmarking_b200.ops.dense import AllGatherVPlan, MetadataPlan
+    from moe_comms_benchmarking_b200.ops.experts import (ExpertCombinePlan, ExpertFfnPlan, ExpertWeights, MoeLayerPlan,
+                                                         RouteBuffers, RoutePlan)
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, E, K, H, I = 40, 6, 3, 256, 128
+    x, idx, w = _case(T, E, K, H, I, 27)
+    heap = SymmetricHeap(world1, 2 << 20, DEV)
+    gx, gi, gw = heap.alloc("gx", [T, H], torch.bfloat16), heap.alloc("gi", [T, K], torch.int64), heap.alloc("gw", [T, K], torch.float32)
+    n, meta = torch.tensor([T], dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    route = RouteBuffers(T, K, E, DEV)
+    act = torch.zeros(route.max_pairs, I, dtype=torch.bfloat16, device=DEV)
+    y = torch.zeros(route.max_pairs, H, dtype=torch.bfloat16, device=DEV)
+    rows = x.clone()
+    partial = heap.alloc("partial", [2, T, H], torch.bfloat16)
+    ffn = [ExpertFfnPlan(ExpertWeights(E, H, I, DEV, seed=s, std=0.05), route, gx.tensor, act, y, heap.status) for s in (3, 4)]
+    plan = MoeLayerPlan(heap, AllGatherVPlan(heap, [gx, gi, gw], [rows, idx, w], n, meta, T),
+                        RoutePlan(route, gi.tensor, gw.tensor, meta[0:1], expert_begin=0, status=heap.status), ffn,
+                        ExpertCombinePlan(heap, y, route, partial, rows, n, meta, T), MetadataPlan(heap, n, meta, T))
+    assert plan._step is None and plan.launches(3) == 4
+    plan.meta.launch()
+    for l in range(3):
+        plan.launch(l % 2)
+    torch.cuda.synchronize()
+    want = rows.clone()
+    rows.copy_(x)
+    plan.decode_step(3)
+    torch.cuda.synchronize()
+    heap.check_status()
+    assert torch.equal(rows, want) and not torch.equal(rows, x)
