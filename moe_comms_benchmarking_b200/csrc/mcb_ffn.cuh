@@ -234,6 +234,7 @@ struct FfnSmem {
   uint64_t* tempty;          // [2], used in the leading CTA
   uint32_t* tmem_slot;
   volatile int* abort_flag;
+  int* acts_there;           // down units whose activations are complete, counted by the first token warp
   uint4* list;
   uint8_t* epi;
   int* tok_idx;
@@ -249,6 +250,7 @@ struct FfnSmem {
     tempty = tfull + 2;
     tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    acts_there = reinterpret_cast<int*>(tmem_slot + 2);
     uint8_t* p = pipe + kFfnPipeBytes + kFfnBarBytes;
     list = reinterpret_cast<uint4*>(p);
     epi = p + kFfnListBytes;
@@ -305,6 +307,7 @@ __device__ __forceinline__ void ffn_setup(const CUtensorMap* maps) {
     for (int s = 0; s < kFfnMaxStages; ++s) { mbar_init(&sm.full[s], 2); mbar_init(&sm.empty[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sm.tfull[i], 1); mbar_init(&sm.tempty[i], 2 * kFfnEpiWarps); }
     *sm.abort_flag = 0;
+    *sm.acts_there = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x >= 32 && threadIdx.x < 64) tmem_alloc_pair(sm.tmem_slot, 512);
@@ -349,6 +352,25 @@ __device__ __forceinline__ void ffn_wait_count(const int* word, int want, const 
   }
 }
 
+// The same for a count in this CTA's shared memory.
+__device__ __forceinline__ void ffn_wait_told(const int* word, int want, const Abort& ab, uint32_t what) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 0;; ++i) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(smem_u32(word)) : "memory");
+    if (v >= want || *ab.flag) return;
+    if ((i & 1023u) != 1023u) continue;
+    if (t0 == 0) t0 = now_ns();
+    if (now_ns() - t0 > ab.timeout_ns) {
+      *ab.flag = 1;
+      if (ab.status && atomicCAS(ab.status, 0u, (uint32_t)MCB_GEMM_ERR_TIMEOUT) == 0u) {
+        ab.status[1] = 26; ab.status[2] = blockIdx.x; ab.status[3] = what;
+      }
+      return;
+    }
+  }
+}
+
 // a.w1 is the packed interleaved gate/up matrix (E * 2I rows, H columns), a.w2 the packed down matrix (E * H rows,
 // I columns): tile (128-row block v, column block kb) of a matrix with KB column blocks is the 16 KB at byte
 // (v * KB + kb) * 16384.
@@ -378,6 +400,7 @@ struct FfnRoles {
   // Position of this warp's role (each role uses its own of these).
   int s = 0; uint32_t ph = 0;
   int acc = 0; uint32_t acc_ph = 0;
+  int downs = 0;                     // down units so far
   bool ok = true;
   // A count that a down unit waits for before it writes its first row (null: nothing).
   const int* y_free = nullptr;
@@ -577,8 +600,15 @@ struct FfnRoles {
         if (un.fc()) {
           const int row = un.row0 + rank * un.half() + row_h;
           const CUtensorMap* map = actmap + groups - 1;
-          // the activations of this expert are complete once every epilogue warp of every gate/up unit has been counted
-          ffn_wait_count(&ffn_done[un.e()], 2 * kFfnEpiWarps * n1 * un.chunks(), ab, 15, (uint32_t)un.e());
+          // The activations of this expert are complete once every epilogue warp of every gate/up unit has been counted.  One
+          // warp asks for the count and tells the others: the answers come from one or two lines that the counting goes through too.
+          ++downs;
+          if (t == 0) {
+            ffn_wait_count(&ffn_done[un.e()], 2 * kFfnEpiWarps * n1 * un.chunks(), ab, 15, (uint32_t)un.e());
+            asm volatile("st.release.cta.shared.b32 [%0], %1;" :: "r"(smem_u32(sm.acts_there)), "r"(downs) : "memory");
+          } else {
+            ffn_wait_told(sm.acts_there, downs, ab, (uint32_t)un.e());
+          }
           fence_proxy_async_global();
           for (int k = 0; k < steps; ++k) {
             if (!(ok = mbar_wait(&sm.empty[su], pu ^ 1u, ab, 16))) break;
