@@ -380,8 +380,7 @@ __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArg
   };
 
   if (W == 1) {
-    // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.
-    // The identity expert on bf16 rows returns the row just delivered, which is still in registers.
+    // Emulated alone (else a2a_alone_kernel): a slice is delivered and combined in one go.
     const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
     for (int l = 0; l < L; ++l) {
       const uint32_t par = (layer_base + (uint32_t)l) & 1u;
@@ -459,6 +458,44 @@ __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArg
   if (tid == 0) *epoch_ptr(c, MCB_SITE_A2A_STEP, bid) = ep;
 }
 
+// Opening and end of a step, for all threads of every block.
+struct A2AStep {
+  int n, ep_max;
+  uint32_t step_seq, layer_base;
+};
+__device__ __forceinline__ A2AStep a2a_step_open(const McbCtx& c, const McbA2AStepArgs& a, int* s_cnt, int* s_prefix, int* s_max) {
+  volatile uint32_t* state = a.state;
+  A2AStep st;
+  st.step_seq = state[MCB_STATE_STEP_SEQ];
+  st.layer_base = state[MCB_STATE_LAYER_BASE];
+  const int L = a.num_layers;
+  st.n = step_count_exchange(c, MCB_SITE_A2A_STEP_META, a.counts_off, st.step_seq, *a.n_local, a.cap, s_cnt, s_prefix, s_max);
+  st.ep_max = *s_max;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.step_meta[0] = s_prefix[c.world];
+    a.step_meta[1] = s_prefix[c.rank];
+    a.step_meta[2] = st.ep_max;
+    a.step_meta[4] = (int)(st.step_seq + 1u);
+    a.step_meta[5] = L > 0 ? (int)((st.layer_base + (uint32_t)L - 1u) & 1u) : 0;
+    a.step_meta[7] = (int)(st.layer_base + (uint32_t)L);     // stamp of the last layer's rows
+  }
+  return st;
+}
+// The last block out advances the sequence words.
+__device__ __forceinline__ void a2a_step_close(const McbA2AStepArgs& a, const A2AStep& st) {
+  volatile uint32_t* state = a.state;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(a.state + MCB_STATE_FINISHED, 1u) == gridDim.x - 1u) {
+      state[MCB_STATE_STEP_SEQ] = st.step_seq + 1u;
+      state[MCB_STATE_LAYER_BASE] = st.layer_base + (uint32_t)a.num_layers;
+      state[MCB_STATE_FINISHED] = 0u;
+      __threadfence();
+    }
+  }
+}
+
 template <bool EMU>
 __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ McbCtx ctx_p,
                                                        const __grid_constant__ McbA2AStepArgs args_p,
@@ -468,23 +505,10 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
   __shared__ int s_prefix[MCB_MAX_RANKS + 1];
   __shared__ int s_cnt[MCB_MAX_RANKS];
   __shared__ int s_max;
-  const int tid = threadIdx.x, bid = blockIdx.x;
-  const int W = c.world, L = a.num_layers;
+  const int W = c.world;
   pdl_wait();
   pdl_launch_dependents();
-  volatile uint32_t* state = a.state;
-  const uint32_t step_seq = state[MCB_STATE_STEP_SEQ], layer_base = state[MCB_STATE_LAYER_BASE];
-  const int n = step_count_exchange(c, MCB_SITE_A2A_STEP_META, a.counts_off, step_seq, *a.n_local, a.cap, s_cnt,
-                                    s_prefix, &s_max);
-  const int ep_max = s_max;
-  if (bid == 0 && tid == 0) {
-    a.step_meta[0] = s_prefix[W];
-    a.step_meta[1] = s_prefix[c.rank];
-    a.step_meta[2] = ep_max;
-    a.step_meta[4] = (int)(step_seq + 1u);
-    a.step_meta[5] = L > 0 ? (int)((layer_base + (uint32_t)L - 1u) & 1u) : 0;
-    a.step_meta[7] = (int)(layer_base + (uint32_t)L);     // stamp of the last layer's rows
-  }
+  const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
   const int valid = s_prefix[W];
   LLShape shp;
   shp.xdata = a.fp8 ? a.hidden / 8 : a.hidden / 4;
@@ -493,23 +517,223 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
   shp.xw = 1 + shp.xdata + shp.scales + shp.meta;
   shp.yw = a.hidden / 4;
   const bool ll = W > 1 && a.ll_rows > 0 && valid > 0 && valid <= a.ll_rows && (!a.fp8 || a.hidden % 256 == 0);
-  if (bid == 0 && tid == 0) a.step_meta[6] = ll ? 1 : 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = ll ? 1 : 0;
   if (ll) {
-    packet_layers(c, a, shp, s_prefix, n, valid, layer_base);
+    packet_layers(c, a, shp, s_prefix, st.n, valid, st.layer_base);
   } else {
-    barrier_layers(c, a, n, ep_max, layer_base);
+    barrier_layers(c, a, st.n, st.ep_max, st.layer_base);
   }
-  // ---- the last block out advances the sequence words ----
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(a.state + MCB_STATE_FINISHED, 1u) == gridDim.x - 1u) {
-      state[MCB_STATE_STEP_SEQ] = step_seq + 1u;
-      state[MCB_STATE_LAYER_BASE] = layer_base + (uint32_t)L;
-      state[MCB_STATE_FINISHED] = 0u;
-      __threadfence();
+  a2a_step_close(a, st);
+}
+
+__device__ __forceinline__ BarrierShape barrier_shape(const McbCtx& c, const McbA2AStepArgs& a) {
+  BarrierShape s;
+  s.row_packs = a.hidden / 8;
+  s.slices = (s.row_packs + kSlicePacks - 1) / kSlicePacks;
+  s.nblk = a.hidden / 128;
+  s.meta_chunks = (int)(a.meta_row_bytes >> 4);
+  s.epr = a.num_experts / c.world;
+  s.row_bytes = (uint64_t)a.hidden * 2;
+  s.xrow_bytes = a.fp8 ? (uint64_t)a.hidden : s.row_bytes;     // bytes of a dispatched row
+  return s;
+}
+
+// ---- a world of one -----------------------------------------------------------------------------------
+// Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.  The identity expert on
+// bf16 rows returns the row just delivered, which is still in registers.  PL = packs per lane; a lane holds one expert id (topk at most 32, others take
+// barrier_alone).
+template <bool FP8, int PL>
+struct AloneSlice {
+  const McbA2AStepArgs& a;
+  const int lane, row_packs;
+  const bool echo, has_id;
+  int t, p0;
+  bool head;                 // the row's first slice: its warp writes the metadata row
+  const uint8_t *x, *y;
+  uint8_t *out, *recv, *scales, *meta;
+  const int64_t* ids;
+  const float* ws;
+
+  __device__ __forceinline__ AloneSlice(const McbA2AStepArgs& args)
+      : a(args), lane(threadIdx.x & 31), row_packs(args.hidden / 8), echo(!FP8 && args.y_off == args.recv_x_off), has_id(lane < args.topk) {}
+  __device__ __forceinline__ int slices() const { return (row_packs + 32 * PL - 1) / (32 * PL); }
+  __device__ __forceinline__ void at(const McbCtx& c, long long item) {
+    const int per_row = slices();
+    t = (int)(item / per_row);
+    p0 = (int)(item - (long long)t * per_row) * 32 * PL + lane;
+    head = p0 == lane;
+    const uint64_t row = (uint64_t)c.rank * a.cap + t, row_bytes = (uint64_t)a.hidden * 2;
+    x = reinterpret_cast<const uint8_t*>(a.x) + t * row_bytes + p0 * 16;
+    y = c.heap_local + a.y_off + row * row_bytes + p0 * 16;
+    out = reinterpret_cast<uint8_t*>(a.out) + t * row_bytes + p0 * 16;
+    recv = c.heap_local + a.recv_x_off + (FP8 ? row * a.hidden + p0 * 8 : row * row_bytes + p0 * 16);
+    scales = c.heap_local + a.recv_scale_off + row * (uint64_t)(a.hidden / 128) * 4 + (p0 >> 4) * 4;
+    meta = c.heap_local + a.recv_meta_off + row * a.meta_row_bytes + lane * 16;
+    ids = a.topk_idx + (int64_t)t * a.topk + lane;
+    ws = a.topk_w ? a.topk_w + (int64_t)t * a.topk + lane : nullptr;
+  }
+  __device__ __forceinline__ void load(bool on, uint64_t par, uint4 (&v)[PL], uint4 (&w)[PL], long long& id, float& wt) const {
+#pragma unroll
+    for (int u = 0; u < PL; ++u) {
+      const bool live = on && p0 + u * 32 < row_packs;
+      v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
+      if (!echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
+    }
+    id = on && has_id ? *reinterpret_cast<const volatile int64_t*>(ids) : 0;
+    wt = on && head && has_id ? (ws ? *reinterpret_cast<const volatile float*>(ws) : 1.0f) : 0.0f;
+  }
+  __device__ __forceinline__ void deliver(const McbCtx& c, uint64_t par, uint32_t stamp, const uint4 (&v)[PL], const uint4 (&w)[PL], long long id,
+                                          float wt) const {
+    const bool good = has_id && id >= 0 && id < a.num_experts;
+    if (has_id && !good) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)t, (uint32_t)id);
+    const bool sent = __any_sync(0xffffffffu, good);
+    if (sent) {
+      uint8_t* dst = recv + par * a.x_par_stride;
+      if (FP8) {
+        float scale[PL + 1];
+#pragma unroll
+        for (int u = 0; u < PL; u += 2) block_absmax_pair(v[u], v[u + 1 < PL ? u + 1 : u], scale[u], scale[u + 1]);
+#pragma unroll
+        for (int u = 0; u < PL; ++u) {
+          scale[u] = e4m3_scale(scale[u]);
+          const uint2 q = quant_pack_e4m3(v[u], scale[u]);
+          if (p0 + u * 32 >= row_packs) continue;
+          st_v2(dst + u * 256, q);
+          if ((lane & 15) == 0) st_b32(scales + par * a.scale_par_stride + u * 8, __float_as_uint(scale[u]));
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < PL; ++u)
+          if (p0 + u * 32 < row_packs) st_v4(dst + u * 512, v[u]);
+      }
+      if (head) {            // chunk j of the metadata row, as in meta_chunk, from the lanes that hold its ids and weights
+        const int k0 = lane == 0 ? 0 : 2 * lane - 1, k1 = 2 * lane;
+        const uint32_t my_id = has_id ? (uint32_t)id : 0xffffffffu, my_w = __float_as_uint(wt);
+        const uint32_t id0 = __shfl_sync(0xffffffffu, my_id, k0), w0 = __shfl_sync(0xffffffffu, my_w, k0);
+        const uint32_t id1 = __shfl_sync(0xffffffffu, my_id, k1), w1 = __shfl_sync(0xffffffffu, my_w, k1);
+        const bool have0 = k0 < a.topk, have1 = k1 < a.topk;
+        uint4 m = make_uint4(have0 ? id0 : 0xffffffffu, have0 ? w0 : 0u, have1 ? id1 : 0xffffffffu, have1 ? w1 : 0u);
+        if (lane == 0) m = make_uint4(stamp, (uint32_t)t, id0, w0);
+        if (lane < (int)(a.meta_row_bytes >> 4)) st_v4(meta + par * a.meta_par_stride, m);
+      }
+    }
+    // the sum over one destination's row
+#pragma unroll
+    for (int u = 0; u < PL; ++u) {
+      if (p0 + u * 32 >= row_packs) continue;
+      float acc[8] = {};
+      if (sent) acc_bf16x8(acc, echo ? v[u] : w[u]);
+      st_v4(out + u * 512, make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
+                                      pack_bf16x2(acc[6], acc[7])));
     }
   }
+};
+
+// At most one slice per warp: where it comes from and goes to is worked out once for all layers.  Nothing that a layer reads is
+// written in the step (a.apart), so the loads of D layers go out together and are delivered layer by layer.
+template <bool FP8, int PL, int D>
+__device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  AloneSlice<FP8, PL> s(a);
+  const int item = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;      // the smallest steps spread over the chip
+  if (item >= n * s.slices()) return;
+  s.at(c, item);
+  for (int l0 = 0; l0 < a.num_layers; l0 += D) {
+    uint4 v[D][PL], w[D][PL];
+    long long id[D];
+    float wt[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) s.load(l0 + d < a.num_layers, (layer_base + (uint32_t)(l0 + d)) & 1u, v[d], w[d], id[d], wt[d]);
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (l0 + d >= a.num_layers) break;
+      s.deliver(c, (layer_base + (uint32_t)(l0 + d)) & 1u, layer_base + (uint32_t)(l0 + d) + 1u, v[d], w[d], id[d], wt[d]);
+    }
+  }
+}
+
+// Layer after layer.
+template <bool FP8>
+__device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  AloneSlice<FP8, 4> s(a);
+  const long long mine = (long long)n * s.slices(), step = (long long)gridDim.x * (blockDim.x >> 5);
+  for (int l = 0; l < a.num_layers; ++l)
+    for (long long i = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x; i < mine; i += step) {
+      uint4 v[4], w[4];
+      long long id;
+      float wt;
+      s.at(c, i);
+      s.load(true, (layer_base + (uint32_t)l) & 1u, v, w, id, wt);
+      s.deliver(c, (layer_base + (uint32_t)l) & 1u, layer_base + (uint32_t)l + 1u, v, w, id, wt);
+    }
+}
+
+// As few packs per lane as still give every slice a warp of its own; false: the layers are left to barrier_alone.  One B200, against
+// layers one by one through pointers to the arguments: 88 layers of 9 / 333 rows of 1024 values: e4m3 228 -> 50 / 244 -> 63 us, bf16
+// 166 -> 46 / 168 -> 48; 58 layers of 333 rows of 7168: e4m3 209 -> 122, bf16 149 -> 106; more slices than warps: 48 layers of 3000 rows of 2048
+// e4m3 492 -> 347, bf16 331 -> 219, 58 of 2048 rows of 7168 e4m3 1313 -> 974.  Beyond 15 MB of bf16 rows the four copies of a row
+// (input, both parities, output) reach the size of one die's L2, and what counts is what stays there: 5000 / 8192 rows of 2048
+// took 613 / 1275 us this way and 575 / 1021 (now 509 / 907) in barrier_alone, with streaming stores 667 / 1171, with the warps of a
+// block in step 673 / 1322.
+constexpr long long kAloneBf16Bytes = 15ll << 20;
+template <bool FP8>
+__device__ __forceinline__ bool alone_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
+  auto fits = [&](int pl) { return a.apart && (long long)n * ((packs + 32 * pl - 1) / (32 * pl)) <= warps; };
+  if (fits(1)) alone_few<FP8, 1, 8>(c, a, n, layer_base);
+  else if (fits(2)) alone_few<FP8, 2, 4>(c, a, n, layer_base);
+  else if (fits(4)) alone_few<FP8, 4, 2>(c, a, n, layer_base);
+  else if (FP8 || n * packs * 16 <= kAloneBf16Bytes) alone_many<FP8>(c, a, n, layer_base);
+  else return false;
+  return true;
+}
+
+// Layer after layer in a world of one, any number of ids: a slice is delivered and combined in one go, with every load of it in flight
+// at once.
+__device__ __forceinline__ void barrier_alone(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const BarrierShape s = barrier_shape(c, a);
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
+  const long long mine = (long long)n * s.slices;
+  // one warp per block first, so that the smallest steps spread over the chip
+  const long long nact = mine < (long long)gridDim.x ? mine : (long long)gridDim.x;
+  if ((long long)blockIdx.x >= nact) return;
+  const long long first = blockIdx.x + (long long)warp * nact, step = nact * (blockDim.x >> 5);
+  const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
+  for (int l = 0; l < a.num_layers; ++l) {
+    const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+    const uint32_t stamp = layer_base + (uint32_t)l + 1u;
+    for (long long i = first; i < mine; i += step) {
+      RowSlice r;
+      r.t = (int)(i / s.slices);
+      r.p0 = (int)(i - (long long)r.t * s.slices) * kSlicePacks;
+      r.row = (uint64_t)c.rank * a.cap + r.t;
+      uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
+      load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
+      if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
+      if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
+      const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
+      push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
+      float acc[4][8] = {};
+      if (m.w[0]) {
+        if (echo) add_packs(acc, v);
+        else add_packs(acc, y);
+      }
+      store_out(a, s, r, acc, lane);
+    }
+  }
+}
+
+// The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
+// through pointers after every store.
+template <bool FP8>
+__global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbA2AStepArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
+  __shared__ int s_prefix[2], s_cnt[1], s_max;
+  const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
+  if (a.topk > 32 || !alone_layers<FP8>(c, a, st.n, st.layer_base)) barrier_alone(c, a, st.n, st.layer_base);
+  a2a_step_close(a, st);
 }
 
 }  // namespace mcb
@@ -530,10 +754,38 @@ static int check_a2a_step(const McbCtx* ctx, const McbA2AStepArgs* a, int grid, 
   return 0;
 }
 
+// Whether a step in a world of one writes nothing that it reads (an output on its input, expert outputs among received rows),
+// and no row by two ways: its layers may then run into each other.
+int mcb_a2a_step_apart(const McbCtx* ctx, const McbA2AStepArgs* a) {
+  if (ctx->world != 1) return 0;
+  struct Range { uint64_t at, bytes; };
+  auto meet = [](Range x, Range y) { return x.at && y.at && x.bytes && y.bytes && x.at < y.at + y.bytes && y.at < x.at + x.bytes; };
+  auto at = [](const void* p) { return reinterpret_cast<uint64_t>(p); };
+  const uint64_t heap = at(ctx->heap_local), cap = (uint64_t)a->cap, row = (uint64_t)a->hidden * 2;
+  const bool echo = !a->fp8 && a->y_off == a->recv_x_off;
+  const Range reads[] = {{at(a->x), cap * row}, {at(a->topk_idx), cap * a->topk * 8}, {at(a->topk_w), cap * a->topk * 4},
+                         {heap + a->y_off, echo ? 0 : a->y_par_stride + cap * row}};
+  const Range writes[] = {{at(a->out), cap * row}, {heap + a->recv_x_off, a->x_par_stride + cap * (a->fp8 ? row / 2 : row)},
+                          {heap + a->recv_scale_off, a->fp8 ? a->scale_par_stride + cap * (a->hidden / 128) * 4 : 0},
+                          {heap + a->recv_meta_off, a->meta_par_stride + cap * a->meta_row_bytes}};
+  for (int w = 0; w < 4; ++w) {
+    for (const Range& r : reads)
+      if (meet(r, writes[w])) return 0;
+    for (int v = 0; v < w; ++v)
+      if (meet(writes[v], writes[w])) return 0;
+  }
+  return 1;
+}
+
 int mcb_launch_a2a_step(const McbCtx* ctx, const McbA2AStepArgs* args, int grid, int threads, int pdl,
                         cudaStream_t stream) {
   if (check_a2a_step(ctx, args, grid, threads)) return cudaErrorInvalidValue;
-  return launch_kernel(a2a_step_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, *args,
+  McbA2AStepArgs a = *args;
+  a.apart = mcb_a2a_step_apart(ctx, args);
+  if (ctx->world == 1)
+    return a.fp8 ? launch_kernel(a2a_alone_kernel<true>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a)
+                 : launch_kernel(a2a_alone_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
+  return launch_kernel(a2a_step_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a,
                        (const McbCtx*)nullptr, (const McbA2AStepArgs*)nullptr);
 }
 

@@ -248,7 +248,7 @@ typedef struct {
   uint64_t ll_y_off;
   uint64_t credit_off;         // heap: uint32 credit[grid][MCB_MAX_RANKS] (zero at start)
   int32_t ll_src_rows;         // min(cap, ll_rows)
-  int32_t reserved1;
+  int32_t apart;               // world of one: the step writes nothing that it reads (mcb_launch_a2a_step sets it)
 } McbA2AStepArgs;
 
 // All-to-all-V combine: out[t,:] = sum over destination ranks d of y_d[rank][slot_map[t][d],:].

@@ -108,7 +108,7 @@ class McbA2AStepArgs(C.Structure):
         ("meta_row_bytes", _u32), ("hidden", _i32), ("topk", _i32), ("num_experts", _i32), ("cap", _i32),
         ("fp8", _i32), ("num_layers", _i32), ("ll_rows", _i32),
         ("step_meta", _vp), ("counts_off", _u64), ("state", _vp),
-        ("ll_x_off", _u64), ("ll_y_off", _u64), ("credit_off", _u64), ("ll_src_rows", _i32), ("reserved1", _i32),
+        ("ll_x_off", _u64), ("ll_y_off", _u64), ("credit_off", _u64), ("ll_src_rows", _i32), ("apart", _i32),
     ]
 
 

@@ -317,6 +317,73 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
     w.check_status()
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,K,n,layers,grid,threads", [
+    (128, 1, 1, 1, 148, 512),            # half a slice of one pack per lane, one id
+    (1024, 32, 5, 17, 148, 512),         # 17 metadata chunks; a remainder of layers
+    (1152, 5, 8, 9, 2, 320),             # 20 warps: two packs per lane, 16 packs in the last slice
+    (1152, 5, 9, 3, 2, 320),             # four packs per lane
+    (2048, 8, 5, 2, 10, 64),             # as many slices as warps
+    (2048, 8, 6, 4, 5, 64),              # more slices than warps
+    (7168, 33, 3, 4, 148, 512),          # more ids than lanes
+])
+def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads):
+    """A step in a world of one whose layers run into each other, against the kernel of the emulated ranks, which takes
+    layer after layer: every received byte of both parities and the combined rows.  An id outside the experts is reported by
+    both and the rest delivered."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, cap = 40, n + 2
+    w, heap = EmuWorld(1, 8 << 20, DEV), SymmetricHeap(world1, 8 << 20, DEV)
+    b, bufs = w.a2a_step_buffers(cap, H, K, fp8), A2AStepBuffers(heap, cap, H, K, fp8)
+    g = torch.Generator(device=DEV).manual_seed(37)
+    x, y = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((cap, H), (2, 1, cap, H)))
+    x[0, :9] = torch.tensor([0.0, -0.0, float("inf"), -float("inf"), float("nan"), 1e-40, -1e-40, 3e38, 448.0])
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(cap)])
+    wt = torch.rand(cap, K, device=DEV, generator=g)
+    count = torch.tensor([n], dtype=torch.int32, device=DEV)
+    metas = [torch.zeros(8, dtype=torch.int32, device=DEV) for _ in range(2)]
+    outs = [torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    for buf in [b[k][0].tensor for k in ("recv_x", "recv_meta")] + [bufs.recv_x.tensor, bufs.recv_meta.tensor]:
+        buf.zero_()
+    if fp8:
+        b["recv_scale"][0].tensor.zero_(); bufs.recv_scale.tensor.zero_()
+        b["y"][0].tensor.copy_(y); bufs.y.tensor.copy_(y)
+    plan = A2AStepPlan(heap, bufs, x, idx, wt, outs[1], count, metas[1], E, layers, grid=grid, threads=threads)
+    assert lib.mcb_a2a_step_apart(heap.ctx_ref(), plan._ref) == 1
+    same = lambda s, t: torch.equal(s.contiguous().view(torch.uint8), t.contiguous().view(torch.uint8))
+    for step in range(3):
+        if step == 2:
+            idx[n - 1, 0] = -1
+            idx[0] = E
+        w.a2a_step(b, [x], [idx], [wt], [outs[0]], [count], [metas[0]], E, layers, grid=grid, threads=threads)
+        plan.launch()
+        torch.cuda.synchronize()
+        assert same(outs[0], outs[1]) and same(metas[0], metas[1]), f"step {step}"
+        for name in ("recv_x", "recv_meta") + (("recv_scale",) if fp8 else ()):
+            assert same(b[name][0].tensor, getattr(bufs, name).tensor), f"{name} in step {step}"
+        assert int(w.status[0][0]) == int(heap.status.view(torch.int32)[0]) == (4 if step == 2 else 0)        # MCB_ERR_ROUTING
+
+
+@pytest.mark.parametrize("form", ["out_on_x", "out_on_ids", "echo"])
+def test_a2a_step_that_reads_what_it_writes(lib, world1, form):
+    """The host tells steps whose layers may run into each other from those that write what they read."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    heap = SymmetricHeap(world1, 4 << 20, DEV)
+    bufs = A2AStepBuffers(heap, 8, 256, 8, False)
+    mem = torch.zeros(8 * 256 * 4, dtype=torch.bfloat16, device=DEV)
+    x, out = mem[:2048].view(8, 256), mem[4096:6144].view(8, 256)
+    idx = torch.zeros(8, 8, dtype=torch.int64, device=DEV)
+    if form == "out_on_x":
+        out = mem[1024:3072].view(8, 256)
+    if form == "out_on_ids":
+        idx = mem[6016:6272].view(torch.int64).view(8, 8)
+    count, meta = torch.tensor([8], dtype=torch.int32, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    plan = A2AStepPlan(heap, bufs, x, idx, None, out, count, meta, 4, 3)
+    assert lib.mcb_a2a_step_apart(heap.ctx_ref(), plan._ref) == int(form == "echo")
+
+
 def _all_quotients(exponent):
     """Blocks of 128 values whose largest has each of the 128 bf16 significands, the others every significand at
     distances of 0 .. 23 binades with alternating signs, and both zeros: every quotient the quantisation can meet."""
