@@ -667,24 +667,19 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
     }
 }
 
-// As few packs per lane as still give every slice a warp of its own; false: the layers are left to barrier_alone.  One B200, against
-// layers one by one through pointers to the arguments: 88 layers of 9 / 333 rows of 1024 values: e4m3 228 -> 50 / 244 -> 63 us, bf16
-// 166 -> 46 / 168 -> 48; 58 layers of 333 rows of 7168: e4m3 209 -> 122, bf16 149 -> 106; more slices than warps: 48 layers of 3000 rows of 2048
-// e4m3 492 -> 347, bf16 331 -> 219, 58 of 2048 rows of 7168 e4m3 1313 -> 974.  Beyond 15 MB of bf16 rows the four copies of a row
-// (input, both parities, output) reach the size of one die's L2, and what counts is what stays there: 5000 / 8192 rows of 2048
-// took 613 / 1275 us this way and 575 / 1021 (now 509 / 907) in barrier_alone, with streaming stores 667 / 1171, with the warps of a
-// block in step 673 / 1322.
-constexpr long long kAloneBf16Bytes = 15ll << 20;
+// As few packs per lane as still give every slice a warp of its own.  One B200, against layers one by one through pointers to the
+// arguments: 88 layers of 9 / 333 rows of 1024 values: e4m3 228 -> 50 / 244 -> 63 us, bf16 166 -> 46 / 168 -> 48; 58 layers of 333 rows
+// of 7168: e4m3 209 -> 122, bf16 149 -> 106; more slices than warps: 48 layers of 3000 rows of 2048 e4m3 492 -> 347, bf16 331 -> 219, of 8192
+// rows 1252 -> 906 and 1010 -> 796, 58 of 2048 rows of 7168 1313 -> 974 and 1007 -> 788.  Neither streaming stores nor keeping the warps
+// of a block in step helped the largest ones.
 template <bool FP8>
-__device__ __forceinline__ bool alone_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+__device__ __forceinline__ void alone_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
   auto fits = [&](int pl) { return a.apart && (long long)n * ((packs + 32 * pl - 1) / (32 * pl)) <= warps; };
   if (fits(1)) alone_few<FP8, 1, 8>(c, a, n, layer_base);
   else if (fits(2)) alone_few<FP8, 2, 4>(c, a, n, layer_base);
   else if (fits(4)) alone_few<FP8, 4, 2>(c, a, n, layer_base);
-  else if (FP8 || n * packs * 16 <= kAloneBf16Bytes) alone_many<FP8>(c, a, n, layer_base);
-  else return false;
-  return true;
+  else alone_many<FP8>(c, a, n, layer_base);
 }
 
 // Layer after layer in a world of one, any number of ids: a slice is delivered and combined in one go, with every load of it in flight
@@ -732,7 +727,8 @@ __global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ 
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
-  if (a.topk > 32 || !alone_layers<FP8>(c, a, st.n, st.layer_base)) barrier_alone(c, a, st.n, st.layer_base);
+  if (a.topk <= 32) alone_layers<FP8>(c, a, st.n, st.layer_base);
+  else barrier_alone(c, a, st.n, st.layer_base);
   a2a_step_close(a, st);
 }
 
