@@ -508,6 +508,36 @@ def test_expert_ffn_token_rows_of_any_shape(world1, shape):
     assert torch.equal(got[0], got[1]) and bool(got[0].count_nonzero() > got[0].numel() // 2)
 
 
+@pytest.mark.parametrize("T,grid", [(4097, 1), (4097, 3), (3277, 1), (5000, 128), (12300, 3)])
+def test_route_many_entries(world1, T, grid):
+    """Routing whose entries are shared out over waiting blocks: all of a thread's kept until they are placed, more than that,
+    and blocks without any; every entry of a local expert in its expert's rows once, the others marked, twice."""
+    from moe_comms_benchmarking_b200.ops.experts import RouteBuffers, RoutePlan
+    E, K, first = 24, 5, 7
+    _, idx, w = _case(T, 40, K, 8, 8, 41)
+    route = RouteBuffers(T + 3, K, E, DEV)
+    pad = lambda t: torch.cat([t, t[:3]]).contiguous()
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    ids, ws = pad(idx), pad(w)
+    plan = RoutePlan(route, ids, ws, torch.tensor([T], dtype=torch.int32, device=DEV), expert_begin=first, status=status, grid=grid)
+    local = (idx >= first) & (idx < first + E)
+    counts = torch.bincount((idx[local] - first).flatten(), minlength=E)
+    for rep in range(2):
+        for t in (route.pair_token, route.pair_pos, route.pair_prob):
+            t.fill_(-7)
+        plan.launch()
+        torch.cuda.synchronize()
+        assert not status.any() and not route.sync.any() and not route.expert_count.any()
+        assert torch.equal(route.expert_offset.long(), torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+        pos = route.pair_pos[:T]
+        assert bool((pos[~local] == -1).all()) and torch.equal(pos[local].sort().values.long(), torch.arange(int(counts.sum()), device=DEV))
+        t, k = local.nonzero(as_tuple=True)
+        at = pos[t, k].long()
+        assert torch.equal(route.pair_token[at].long(), t) and torch.equal(route.pair_prob[at], w[t, k])
+        assert torch.equal(torch.bucketize(at, route.expert_offset.long(), right=True) - 1, idx[t, k] - first)
+        assert bool((route.pair_pos[T:] == -7).all()) and int(route.max_rows) == int(counts.max())
+
+
 @pytest.mark.parametrize("E,K,H,I,T,layers,sets,grid", [
     (8, 2, 256, 128, 3, 2, 1, 148),          # two layers; fewer units than CTA pairs
     (8, 2, 256, 128, 90, 40, 20, 148),       # more weight sets than one launch takes, buffers used many times over
