@@ -289,10 +289,25 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
 // layer reads is written in the step (else: a.in_order), so the loads of D layers go out together and are stored layer
 // by layer; the layers of such a step run into each other.  With one layer at a time each layer was a trip to L2: 88 layers
 // of hidden 1024 and top-22, one B200: 57 -> 37 us with one
-// token, 47 -> 34 with 200, 62 -> 55 with 333, where the second pack per thread begins.
+// token, 47 -> 34 with 200, 62 -> 55 with 333, where the second pack per thread begins; with e4m3 rows, whose packs go along, 100 -> 52, 109 ->
+// 47 (100 tokens) and 115 -> 59.
 template <bool FP8, int S, int D>
 __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, long long start,
                                           long long stride, uint32_t layer_base) {
+  // e4m3: packs of bf16 rows, and where their values and their block's scale go
+  const int H = (int)a.fp8_hidden, ppr = FP8 ? H / 8 : 1, nblk = H / 128;
+  const uint8_t* rows = reinterpret_cast<const uint8_t*>(a.src[0]);
+  uint8_t *q_dst[S], *s_dst[S];
+  bool quant[S];
+#pragma unroll
+  for (int u = 0; u < S; ++u) {
+    const long long i = start + u * stride;
+    quant[u] = FP8 && i < (long long)n * ppr;
+    const int row = (int)(i / ppr), pk = (int)(i - (long long)row * ppr);
+    q_dst[u] = c.heap_local + a.dst_off[0] + (uint64_t)row * H + (uint64_t)pk * 8;
+    s_dst[u] = c.heap_local + a.dst_off[3] + ((uint64_t)row * nblk + (pk >> 4)) * 4;
+  }
+
   const long long total = r.end[LocalRanges::R - 1];
   const uint8_t* src[S];
   uint8_t* dst[S];
@@ -309,21 +324,39 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
     par_off[u] = r.par[t];
   }
   for (int l0 = 0; l0 < a.num_layers; l0 += D) {
-    uint4 v[D][S];
+    uint4 v[D][S], h[D * S];
     uint32_t w[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      if (l0 + d >= a.num_layers) break;
+      if (FP8) {
+#pragma unroll
+        for (int u = 0; u < S; ++u)
+          h[d * S + u] = quant[u] && l0 + d < a.num_layers ? ld_v4_stream(rows + (start + u * stride) * 16) : make_uint4(0, 0, 0, 0);
+      }
+      if (l0 + d >= a.num_layers) continue;
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) v[d][u] = ld_v4_stream(src[u]);
       w[d] = r.load_word();
     }
+    float scale[D * S];
+    if (FP8) {
+#pragma unroll
+      for (int k = 0; k < D * S; k += 2) block_absmax_pair(h[k], h[k + 1], scale[k], scale[k + 1]);
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       if (l0 + d >= a.num_layers) break;
       const uint32_t par = (layer_base + (uint32_t)(l0 + d)) & 1u;
-      if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
+      if (FP8) {
+#pragma unroll
+        for (int u = 0; u < S; ++u) {
+          if (!quant[u]) continue;
+          const float sc = e4m3_scale(scale[d * S + u]);
+          st_v2(q_dst[u] + (par ? a.dst_par_stride[0] : 0), quant_pack_e4m3(h[d * S + u], sc));
+          if ((threadIdx.x & 15) == 0) st_b32(s_dst[u] + (par ? a.dst_par_stride[3] : 0), __float_as_uint(sc));
+        }
+      }
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) st_v4(dst[u] + (par ? par_off[u] : 0), v[d][u]);
@@ -356,14 +389,12 @@ __device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStep
     return;
   }
 
-  // Few packs: eight of them in flight per thread, those of several layers where a layer has fewer.
-  if (FP8) {
-    if (total <= stride * 4) { local_few<FP8, 4, 1>(c, a, r, n, start, stride, layer_base); return; }
-  } else {
-    if (total <= stride) { local_few<FP8, 1, 8>(c, a, r, n, start, stride, layer_base); return; }
-    if (total <= stride * 2) { local_few<FP8, 2, 4>(c, a, r, n, start, stride, layer_base); return; }
-    if (total <= stride * 4) { local_few<FP8, 4, 2>(c, a, r, n, start, stride, layer_base); return; }
-  }
+  // Few packs: eight of them in flight per thread, and as many of rows to quantise, those of several layers where a layer has
+  // fewer.
+  const long long rows = FP8 ? (long long)n * (a.fp8_hidden / 8) : 0, most = total > rows ? total : rows;
+  if (most <= stride) { local_few<FP8, 1, 8>(c, a, r, n, start, stride, layer_base); return; }
+  if (most <= stride * 2) { local_few<FP8, 2, 4>(c, a, r, n, start, stride, layer_base); return; }
+  if (most <= stride * 4) { local_few<FP8, 4, 2>(c, a, r, n, start, stride, layer_base); return; }
   for (int l = 0; l < a.num_layers; ++l) {
     const uint32_t par = (layer_base + (uint32_t)l) & 1u;
     if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
@@ -544,8 +575,9 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
 
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.  One B200, 88 layers of hidden 1024 and top-22, against the same code called by the step
-// kernel: e4m3 1 / 333 / 8192 rows 134 -> 100 / 152 -> 115 / 1215 -> 1014 us, 58 layers of 333 rows of 7168 200 -> 148; bf16 1 / 100 rows
-// 40 -> 34 / 34 -> 30, 48 layers of 9 rows of 2048 25 -> 20; the largest bf16 steps are bound by L2 either way (702 -> 700).
+// kernel: e4m3 1 / 333 / 8192 rows 134 -> 100 / 152 -> 115 / 1215 -> 1014 us, 58 layers of 333 rows of 7168 200 -> 148 (52, 59 and 111 with
+// several layers in flight); bf16 1 / 100 rows 40 -> 34 / 34 -> 30, 48 layers of 9 rows of 2048 25 -> 20; the largest bf16 steps are
+// bound by L2 either way (702 -> 700).
 template <bool FP8>
 __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
   __shared__ int s_prefix[2], s_cnt[1], s_max;

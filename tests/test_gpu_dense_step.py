@@ -296,3 +296,37 @@ def test_world_of_one_step_on_its_own_rows(lib, form, n, layers):
             else:
                 assert torch.equal(gh.tensor[p, :n], rows[p])
             assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 17])          # 32 packs to quantise a row on 96 threads: up to 1, 2, 4 per thread and more
+@pytest.mark.parametrize("layers", [1, 3, 8, 9])
+@pytest.mark.parametrize("out_cols", [256, 64])             # as many packs of expert outputs, and fewer than are quantised
+def test_world_of_one_quantised_layers_in_flight(lib, n, layers, out_cols):
+    """e4m3 dispatch of a world of one: the bytes, scales and copies of the last two layers, whatever number of layers is in flight."""
+    from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    cap, H, K = 20, 256, 3
+    g = torch.Generator(device=DEV).manual_seed(n)
+    heap = SymmetricHeap(None, 1 << 20, DEV)
+    x = torch.randn(cap, H, device=DEV, generator=g).to(torch.bfloat16)
+    ids, w = torch.randint(0, 64, (cap, K), device=DEV, generator=g), torch.rand(cap, K, device=DEV, generator=g)
+    gh, gs = heap.alloc("gh", [2, cap, H], torch.uint8), heap.alloc("gs", [2, cap, H // 128], torch.float32)
+    gi, gw = heap.alloc("gi", [2, cap, K], torch.int64), heap.alloc("gw", [2, cap, K], torch.float32)
+    rsv = heap.alloc("rsv", [cap, out_cols], torch.bfloat16)
+    rsv.tensor.normal_()
+    out, meta = torch.zeros(cap, out_cols, dtype=torch.bfloat16, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    plan = DenseStepPlan(heap, [gh, gi, gw, gs], [x, ids, w, None], out, rsv, torch.tensor([n], dtype=torch.int32, device=DEV), meta, cap,
+                         layers, grid=1, threads=96, fp8_hidden=H)
+    q, scale = oracle.quant_e4m3_1x128(x[:n].float().cpu())
+    for step in range(2):
+        for t in (gh, gs, gi, gw):
+            t.tensor.zero_()
+        plan.launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        par = int(meta[5])
+        assert torch.equal(out[:n], rsv.tensor[:n])
+        for p in {par, (par + layers - 1) % 2}:
+            assert torch.equal(gh.tensor[p, :n].cpu(), q.view(torch.uint8)) and torch.equal(gs.tensor[p, :n].cpu(), scale)
+            assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
+        assert not gh.tensor[:, n:].any() and not gs.tensor[:, n:].any()
