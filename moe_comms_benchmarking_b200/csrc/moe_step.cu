@@ -360,6 +360,8 @@ int mcb_prepare_moe_step(McbMoeStepArgs* out, const McbLayerArgs* sets, int num_
   const uint64_t rows = (uint64_t)g.cap, pairs = (uint64_t)r.max_pairs;
   const Range written[] = {range(f.act, pairs * f.intermediate * 2), range(f.y, pairs * f.hidden * 2), range(cmb.out, (uint64_t)cmb.cap * f.hidden * 2)};
   for (int t = 0; t < g.num_tensors; ++t) {
+    for (const Range& w : written)      // a row written by two ways has the order of its layers
+      if (overlap(w, range(p.ctx.heap_local + g.dst_off[t], rows * g.row_bytes[t]))) return 1;
     const Range src = range(g.src[t], rows * g.row_bytes[t]);
     for (const Range& w : written)
       if (overlap(src, w)) return 1;

@@ -600,6 +600,11 @@ def test_step_on_its_own_output_goes_layer_by_layer(world1):
                         RoutePlan(route, gi.tensor, gw.tensor, meta[0:1], expert_begin=0, status=heap.status), ffn,
                         ExpertCombinePlan(heap, y, route, partial, rows, n, meta, T), MetadataPlan(heap, n, meta, T))
     assert plan._step is None and plan.launches(3) == 4
+    for out in (gx.tensor, torch.zeros_like(rows)):         # an output on the gathered rows, and one of its own
+        p = MoeLayerPlan(heap, AllGatherVPlan(heap, [gx, gi, gw], [rows, idx, w], n, meta, T),
+                         RoutePlan(route, gi.tensor, gw.tensor, meta[0:1], expert_begin=0, status=heap.status), ffn,
+                         ExpertCombinePlan(heap, y, route, partial, out, n, meta, T), MetadataPlan(heap, n, meta, T))
+        assert (p._step is None) == (out is gx.tensor)
     plan.meta.launch()
     for l in range(3):
         plan.launch(l % 2)
