@@ -227,7 +227,7 @@ __device__ __forceinline__ void gemm_device(const CUtensorMap& w_map, const McbG
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) __nanosleep(50000);        // let any copy still in flight land before the CTA goes away
+  if (*abort_flag) settle();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

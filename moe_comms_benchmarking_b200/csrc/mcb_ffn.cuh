@@ -326,7 +326,7 @@ __device__ __forceinline__ void ffn_teardown() {
   const FfnSmem sm;
   tc_fence_before();
   __syncthreads();
-  if (*sm.abort_flag) __nanosleep(50000);            // let any copy still in flight land before the CTA goes away
+  if (*sm.abort_flag) settle();
   cluster_sync();
   if (threadIdx.x >= 32 && threadIdx.x < 64) {
     tc_fence_after();

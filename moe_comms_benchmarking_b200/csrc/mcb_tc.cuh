@@ -45,6 +45,13 @@ __device__ __forceinline__ uint64_t now_ns() {
   return t;
 }
 
+// Before a CTA that has given up frees its TMEM and goes away: time for copies and MMAs in flight to land.  (A single nanosleep may
+// return at once: any time from zero to twice the one asked for.)
+__device__ __forceinline__ void settle() {
+  const uint64_t t0 = now_ns();
+  while (now_ns() - t0 < 50000u) __nanosleep(1000);
+}
+
 // Bounded wait.  Returns false once this CTA has given up (now or earlier).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const Abort& ab, uint32_t where) {
   uint64_t t0 = 0;

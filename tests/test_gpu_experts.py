@@ -615,3 +615,34 @@ def test_step_on_its_own_output_goes_layer_by_layer(world1):
     torch.cuda.synchronize()
     heap.check_status()
     assert torch.equal(rows, want) and not torch.equal(rows, x)
+
+
+@pytest.mark.parametrize("rows,grid", [([40, 10], 148), ([140, 3], 148), ([300] * 12, 6)])
+def test_expert_ffn_whose_wait_runs_out(world1, rows, grid):
+    """Down units whose activations are never complete (the counters held back): the launch ends by itself and says so in the
+    status words, with copies and MMAs landed; the next one is right."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import DeviceStatusError, SymmetricHeap
+    E, T, H, I = len(rows), sum(rows), 512, 256
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    x = torch.randn(T, H, device=DEV).to(torch.bfloat16)
+    idx = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(rows, device=DEV)).view(T, 1)
+    route = RouteBuffers(T, 1, E, DEV)
+    act, y = torch.zeros(T, I, dtype=torch.bfloat16, device=DEV), torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)
+    rp = RoutePlan(route, idx, torch.ones(T, 1, device=DEV), torch.tensor([T], dtype=torch.int32, device=DEV), 0, heap.status)
+    ffn = ExpertFfnPlan(ExpertWeights(E, H, I, DEV, seed=9, std=0.05), route, x, act, y, heap.status, grid=grid, timeout_s=0.05)
+    out = []
+    for held in (False, True, False):
+        rp.launch()
+        if held:
+            route.ffn_done.fill_(-(1 << 20))
+        ffn.launch()
+        torch.cuda.synchronize()
+        if held:
+            with pytest.raises(DeviceStatusError) as e:
+                heap.check_status()
+            assert e.value.code == 5 and 11 <= e.value.words[1] <= 26
+        else:
+            heap.check_status()
+            out.append(y[route.pair_pos.flatten().long()].clone())
+    assert torch.equal(*out)
