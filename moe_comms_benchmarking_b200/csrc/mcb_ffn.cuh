@@ -274,7 +274,7 @@ struct StepSmem {
   uint64_t* lfull;           // [2]
   uint64_t* lempty;          // [2]
   int* head;                 // [2][2] units of a half, whether it is the last one of its layer
-  int* word;                 // [2] hand-over among the epilogue warps, among the routing warps
+  int* word;                 // [4] hand-over among the epilogue warps (0, 2) and among the routing warps (1, 3)
   static constexpr int kOff = kStepMaxExperts * 4 + 16;
   static constexpr int kBytes = 2 * kOff + kStepMaxExperts * 2 + kStepMaxExperts * 4 + 96 * 4 + 64;
   __device__ __forceinline__ explicit StepSmem(const FfnSmem& sm) {

@@ -61,9 +61,14 @@ struct StepRoute {
   int counted = 0;             // layers whose counts went through the counters
 
   __device__ __forceinline__ StepRoute(const McbMoeStepArgs& args, const LocalRanges& ranges, const StepSmem& smem, const Abort& abort, int tokens)
-      : p(args), rows(ranges), st(smem), ab(abort), r(args.layer.route), T(tokens) {}
+      : p(args), rows(ranges), st(smem), ab(abort), r(args.layer.route), T(tokens) {
+    if (two() && p.two_rows < r.max_pairs) r.max_pairs = (int)p.two_rows;
+  }
+  // Whether the layers alternate between two buffers of activations and expert outputs.
+  __device__ __forceinline__ bool two() const { return (long long)T * p.layer.route.topk <= p.two_rows; }
 
-  // Returns the largest number of rows of an expert.
+  // Returns the largest number of rows of an expert, -1 once this CTA has given up: counts that are not complete would place rows
+  // beyond the buffers.
   template <class Group>
   __device__ __forceinline__ int layer(const Group& g, int set) {
     const int grid = (int)gridDim.x, bid = (int)blockIdx.x, E = r.num_local_experts;
@@ -91,8 +96,10 @@ struct StepRoute {
         __threadfence();
         atomicAdd(&p.sync[kStepCounted], 1);
         ffn_wait_count(&p.sync[kStepCounted], counted * grid, ab, 21, (uint32_t)counted);
+        st.word[3] = *ab.flag;
       }
       g.sync();
+      if (st.word[3]) return -1;
       route_collect(g, E, count, m);
     }
     const int mx = route_offsets(g, r, m, bid == 0);
@@ -120,14 +127,17 @@ __device__ __forceinline__ void step_roles(const McbMoeStepArgs& p, const StepWe
     const RouteGroup g;
     int base = 0;              // pair of the layer's first unit
     int half = 0; uint32_t half_ph = 0;
-    bool go = true;
-    for (int l = 0; l < layers && go; ++l) {
+    for (int l = 0; l < layers; ++l) {
       if (l > 0) {
         // the buffers are those of layer l - 3
-        if (l > 2 && g.tid() == 0) ffn_wait_count(&p.sync[kStepCombined], (l - 2) * grid, r.ab, 22, (uint32_t)l);
+        if (g.tid() == 0) {
+          if (l > 2) ffn_wait_count(&p.sync[kStepCombined], (l - 2) * grid, r.ab, 22, (uint32_t)l);
+          st.word[1] = *r.ab.flag;
+        }
         g.sync();
+        if (st.word[1]) return;
         if (g.tid() < 4) tma_prefetch_map(&w.map[(first_set + l) % sets][g.tid()]);
-        route.layer(g, (layers - 1 - l) % 3);
+        if (route.layer(g, (layers - 1 - l) % 3) < 0) return;
       }
       FfnPlanS plan;
       plan.off = st.off; plan.cum = st.cum; plan.ids = st.ids;
@@ -136,13 +146,13 @@ __device__ __forceinline__ void step_roles(const McbMoeStepArgs& p, const StepWe
       int first = pair - base;
       if (first < 0) first += npairs;
       base = (base + total) % npairs;
-      for (bool last = false; !last && go; first += kStepListUnits * npairs) {
+      for (bool last = false; !last; first += kStepListUnits * npairs) {
         int count = first < total ? (total - first + npairs - 1) / npairs : 0;
         last = count <= kStepListUnits;
         if (!last) count = kStepListUnits;
         if (g.tid() == 0) st.word[1] = mbar_wait(&st.lempty[half], half_ph ^ 1u, r.ab, 23);
         g.sync();
-        go = st.word[1] != 0;
+        if (!st.word[1]) return;             // the half may still be read
         plan.list(r.sm.list + half * kStepListUnits, count, first, npairs, total, g.tid(), g.size());
         if (g.tid() == 0) { st.head[half * 2] = count; st.head[half * 2 + 1] = last; }
         g.sync();
@@ -156,7 +166,7 @@ __device__ __forceinline__ void step_roles(const McbMoeStepArgs& p, const StepWe
 
   int half = 0; uint32_t half_ph = 0;
   const bool epilogue = r.warp >= 2 && r.warp < 2 + kFfnEpiWarps, tokens = r.warp >= 2 + kFfnEpiWarps;
-  const bool two = (long long)route.T * p.layer.route.topk <= p.two_rows;
+  const bool two = route.two();
   const EpilogueGroup g;
   bool go = true;
   // One round more than there are layers: the sums of a layer are taken in the next one.
@@ -211,10 +221,17 @@ __device__ __forceinline__ void step_roles(const McbMoeStepArgs& p, const StepWe
           if (pending && (begin < count || last)) {
             // This CTA's share of the sums, behind the experts of all CTAs.
             pending = false;
-            if (g.tid() == 0) ffn_wait_count(&p.sync[kStepExperts], l * grid, r.ab, 25, (uint32_t)l);
+            if (g.tid() == 0) {
+              ffn_wait_count(&p.sync[kStepExperts], l * grid, r.ab, 25, (uint32_t)l);
+              // No rows to sum (the sums are zero) where nothing was routed or this CTA has given up: the list may still hold
+              // positions of an earlier, larger step.
+              st.word[2] = *r.sm.abort_flag || route.T == 0 ? 0 : p.layer.cmb.topk;
+            }
             g.sync();
             McbCombineArgs cmb = p.layer.cmb;
             cmb.pair_pos = p.pair_pos[(layers - l) % 3];
+
+            cmb.topk = st.word[2];
             cmb.y = p.y[two ? (layers - l) & 1 : 0];
             combine_body<false>(p.layer.ctx, cmb, 0u, r.warp - 2, kFfnEpiWarps);
             g.sync();
@@ -283,8 +300,10 @@ moe_step_kernel(const __grid_constant__ McbMoeStepArgs p, const __grid_constant_
   const int mx = route.layer(BlockGroup{}, (layers - 1) % 3);      // the first layer's by all warps
   const int n_slot = ffn_token_tile(mx);
   __syncthreads();
-  if (n_slot <= kFfnDoubleN) step_roles<2>(p, w, route, layers, first_set, sets, n_slot);
-  else step_roles<1>(p, w, route, layers, first_set, sets, n_slot);
+  if (mx >= 0) {
+    if (n_slot <= kFfnDoubleN) step_roles<2>(p, w, route, layers, first_set, sets, n_slot);
+    else step_roles<1>(p, w, route, layers, first_set, sets, n_slot);
+  }
   ffn_teardown();
   if (threadIdx.x == 0) {
     __threadfence();

@@ -646,3 +646,72 @@ def test_expert_ffn_whose_wait_runs_out(world1, rows, grid):
             heap.check_status()
             out.append(y[route.pair_pos.flatten().long()].clone())
     assert torch.equal(*out)
+
+
+def _step_behind_a_larger_one(world1, small, layers=4, K=6):
+    """A plan whose three sets of pair lists hold the positions of a step that fills one buffer of expert outputs, with a batch
+    of `small` tokens loaded that alternates between two; its waits end after 50 ms.  (dispatcher, plan, output of the batch)"""
+    from moe_comms_benchmarking_b200.config import Config
+    from moe_comms_benchmarking_b200.ops.experts import STEP_TWO_BUFFERS_BYTES, MoeLayerPlan
+    from moe_comms_benchmarking_b200.parallel.fused import FusedExpertDispatcher
+    E, H, I, T = 8, 256, 128, 2100
+    assert small * K * 2 * H <= STEP_TWO_BUFFERS_BYTES < T * K * 2 * H
+    cfg = Config(num_experts=E, topk=K, hidden=H, intermediate=I, ep_size=1, per_rank_cap=T, probs="softmax")
+    d = FusedExpertDispatcher(cfg, world1, num_layers=2, weight_budget_gb=1.0)
+    d.build()
+    for f in d.ffn:
+        f.args.timeout_ns = 50_000_000
+    plan = MoeLayerPlan(d.heap, d.agv_plan, d.route_plan, d.ffn, d.combine_plan, d.meta_plan)
+    assert plan._step is not None
+    for n in (T, small):
+        d.setup_batch(*_case(n, E, K, H, I, n + 43))
+        plan.decode_step(layers)
+    torch.cuda.synchronize()
+    d.check_health()
+    return d, plan, d.out.clone()
+
+
+def test_step_with_a_refused_count(world1):
+    """More tokens than the capacity: reported, nothing is routed, and no position of an earlier, larger step is summed (the
+    second buffer of expert outputs does not hold its rows).  The next step is right."""
+    from moe_comms_benchmarking_b200.parallel.symm_heap import DeviceStatusError
+    d, plan, want = _step_behind_a_larger_one(world1, 300)
+    n = int(d.n_local)
+    for bad in (d.cap + 1, 1 << 30):
+        d.n_local.fill_(bad)
+        for y in (d.y, plan._step_bufs[0][2]):
+            y.fill_(float("nan"))
+        plan.decode_step(4)
+        torch.cuda.synchronize()
+        with pytest.raises(DeviceStatusError) as e:
+            d.check_health()
+        assert e.value.code == 2 and not d.out_buf.isnan().any()
+        d.n_local.fill_(n)
+        plan.decode_step(4)
+        torch.cuda.synchronize()
+        d.check_health()
+        assert torch.equal(d.out, want)
+    d.destroy()
+
+
+@pytest.mark.parametrize("word,small", [("routed", 300), ("counted", 300), ("counted", 2000), ("experts", 300), ("combined", 300)])
+def test_step_whose_waits_run_out(world1, word, small):
+    """Each counter that CTAs of a step wait for, held back so that it is never reached: the launch ends by itself, says so in
+    the status words, and leaves its counters clean for the next one.  With 2000 tokens the first layer's counts are shared too."""
+    from moe_comms_benchmarking_b200.parallel.symm_heap import DeviceStatusError
+    d, plan, want = _step_behind_a_larger_one(world1, small)
+    mem, b = plan._step_bufs[0][0], d.route
+    sync = mem[mem.numel() - 160:]
+    assert not sync.any()
+    sync[{"routed": 0, "counted": 32, "experts": 64, "combined": 96}[word]] = -(1 << 20)
+    plan.decode_step(4)
+    torch.cuda.synchronize()
+    with pytest.raises(DeviceStatusError) as e:
+        d.check_health()
+    assert e.value.code == 5 and 11 <= e.value.words[1] <= 26
+    assert not sync.any()
+    plan.decode_step(4)
+    torch.cuda.synchronize()
+    d.check_health()
+    assert torch.equal(d.out, want)
+    d.destroy()
