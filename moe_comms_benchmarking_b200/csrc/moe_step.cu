@@ -340,6 +340,47 @@ bool same_but_weights(const McbLayerArgs& a, const McbLayerArgs& b) {
          a.local_probs == b.local_probs;
 }
 
+// The rows of this rank's tokens where its all-gather reads them, if the layers can go into one launch.  Null where they cannot: more
+// ranks than one, rows or routing that are not read there, plans that do not fit together or differ in more than their weights, too
+// many experts, a phase trace, or a layer that writes what the next one reads (rows taken from the output of the layer before, say)
+// or writes memory by two ways (an output in the activations, which a layer of its own is done with by then).
+const void* joined_rows(const McbLayerArgs* sets, int num_sets, const McbMetaArgs* meta) {
+  if (!sets || num_sets < 1 || !meta) return nullptr;
+  const McbLayerArgs& p = sets[0];
+  const McbRouteArgs& r = p.route;
+  const McbFfnArgs& f = p.ffn;
+  const McbAgvArgs& g = p.agv;
+  const McbCombineArgs& cmb = p.cmb;
+  if (p.ctx.world != 1 || p.trace || !p.local_ids || r.num_local_experts > kStepMaxExperts) return nullptr;
+  for (int s = 1; s < num_sets; ++s)
+    if (!same_but_weights(p, sets[s]) || sets[s].trace) return nullptr;
+  if (f.pair_token != r.pair_token || (f.pair_prob && f.pair_prob != r.pair_prob) || f.expert_offset != r.expert_offset ||
+      f.ffn_done != r.ffn_done || f.num_local_experts != r.num_local_experts)
+    return nullptr;
+  if (cmb.y != f.y || cmb.pair_pos != r.pair_pos || cmb.topk != r.topk || cmb.hidden != f.hidden || cmb.n_local != g.n_local ||
+      cmb.step_meta != g.step_meta || r.num_tokens != g.step_meta || meta->n_local != g.n_local || meta->step_meta != g.step_meta ||
+      meta->cap > g.cap || meta->cap > r.max_tokens || meta->cap > cmb.cap)
+    return nullptr;
+  const void* x = nullptr;
+  for (int t = 0; t < g.num_tensors; ++t)
+    if (p.ctx.heap_local + g.dst_off[t] == f.x && g.row_bytes[t] == 2u * (uint32_t)f.hidden) x = g.src[t];
+  const uint64_t rows = (uint64_t)g.cap, pairs = (uint64_t)r.max_pairs;
+  const Range written[] = {range(f.act, pairs * f.intermediate * 2), range(f.y, pairs * f.hidden * 2), range(cmb.out, (uint64_t)cmb.cap * f.hidden * 2)};
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < i; ++j)
+      if (overlap(written[i], written[j])) return nullptr;
+  for (int t = 0; t < g.num_tensors; ++t) {
+    for (const Range& w : written)      // a row written by two ways has the order of its layers
+      if (overlap(w, range(p.ctx.heap_local + g.dst_off[t], rows * g.row_bytes[t]))) return nullptr;
+    const Range src = range(g.src[t], rows * g.row_bytes[t]);
+    for (const Range& w : written)
+      if (overlap(src, w)) return nullptr;
+    for (int u = 0; u < g.num_tensors; ++u)
+      if (overlap(src, range(p.ctx.heap_local + g.dst_off[u], rows * g.row_bytes[u]))) return nullptr;
+  }
+  return x;
+}
+
 bool configure_step_kernel() {
   static const bool ok = cudaFuncSetAttribute(moe_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmemBytes) == cudaSuccess;
   return ok;
@@ -347,46 +388,22 @@ bool configure_step_kernel() {
 
 }  // namespace
 
+// Whether several layers of a step can go into one launch.
+int mcb_moe_step_joins(const McbLayerArgs* sets, int num_sets, const McbMetaArgs* meta) { return joined_rows(sets, num_sets, meta) != nullptr; }
+
 // Fills `out` (64-byte aligned host memory) for steps of several layers in one launch and returns 0, or 1 where the layers cannot
-// go into one: more ranks than one, rows or routing that are not read where this rank's all-gather reads them, plans that do not
-// fit together or differ in more than their weights, too many experts, a phase trace, or a layer that writes what the next one
-// reads (rows taken from the output of the layer before, say).  The further buffers come from the caller: two times pair_token and
+// go into one (mcb_moe_step_joins).  The further buffers come from the caller: two times pair_token and
 // pair_prob (route.max_pairs each), pair_pos (max_tokens x topk, -1) and ffn_done (num_local_experts), expert_count (3 x
 // num_local_experts) and sync (MCB_STEP_SYNC_WORDS), all zero but for pair_pos; act and y of two_rows rows, or null.
 int mcb_prepare_moe_step(McbMoeStepArgs* out, const McbLayerArgs* sets, int num_sets, const McbMetaArgs* meta, int32_t* pair_token,
                          float* pair_prob, int32_t* pair_pos, int32_t* ffn_done, int32_t* expert_count, int32_t* sync, void* act,
                          void* y, int two_rows) {
-  if (!out || !sets || num_sets < 1 || !meta || !pair_token || !pair_prob || !pair_pos || !ffn_done || !expert_count || !sync) return 1;
+  const void* x = joined_rows(sets, num_sets, meta);
+  if (!x || !out || !pair_token || !pair_prob || !pair_pos || !ffn_done || !expert_count || !sync) return 1;
   const McbLayerArgs& p = sets[0];
   const McbRouteArgs& r = p.route;
   const McbFfnArgs& f = p.ffn;
-  const McbAgvArgs& g = p.agv;
-  const McbCombineArgs& cmb = p.cmb;
-  if (p.ctx.world != 1 || p.trace || !p.local_ids || r.num_local_experts > kStepMaxExperts) return 1;
-  for (int s = 1; s < num_sets; ++s)
-    if (!same_but_weights(p, sets[s]) || sets[s].trace) return 1;
-  if (f.pair_token != r.pair_token || (f.pair_prob && f.pair_prob != r.pair_prob) || f.expert_offset != r.expert_offset ||
-      f.ffn_done != r.ffn_done || f.num_local_experts != r.num_local_experts)
-    return 1;
-  if (cmb.y != f.y || cmb.pair_pos != r.pair_pos || cmb.topk != r.topk || cmb.hidden != f.hidden || cmb.n_local != g.n_local ||
-      cmb.step_meta != g.step_meta || r.num_tokens != g.step_meta || meta->n_local != g.n_local || meta->step_meta != g.step_meta ||
-      meta->cap > g.cap || meta->cap > r.max_tokens || meta->cap > cmb.cap)
-    return 1;
-  const void* x = nullptr;
-  for (int t = 0; t < g.num_tensors; ++t)
-    if (p.ctx.heap_local + g.dst_off[t] == f.x && g.row_bytes[t] == 2u * (uint32_t)f.hidden) x = g.src[t];
-  if (!x) return 1;
-  const uint64_t rows = (uint64_t)g.cap, pairs = (uint64_t)r.max_pairs;
-  const Range written[] = {range(f.act, pairs * f.intermediate * 2), range(f.y, pairs * f.hidden * 2), range(cmb.out, (uint64_t)cmb.cap * f.hidden * 2)};
-  for (int t = 0; t < g.num_tensors; ++t) {
-    for (const Range& w : written)      // a row written by two ways has the order of its layers
-      if (overlap(w, range(p.ctx.heap_local + g.dst_off[t], rows * g.row_bytes[t]))) return 1;
-    const Range src = range(g.src[t], rows * g.row_bytes[t]);
-    for (const Range& w : written)
-      if (overlap(src, w)) return 1;
-    for (int u = 0; u < g.num_tensors; ++u)
-      if (overlap(src, range(p.ctx.heap_local + g.dst_off[u], rows * g.row_bytes[u]))) return 1;
-  }
+  const uint64_t rows = (uint64_t)p.agv.cap, pairs = (uint64_t)r.max_pairs;
   memset(out, 0, sizeof *out);
   out->layer = p;
   out->ids = p.local_ids;

@@ -192,7 +192,7 @@ _LAUNCHERS = {
     "mcb_launch_dense_step": "ppiiip", "mcb_launch_a2a_dispatch": "ppiiip", "mcb_launch_a2a_combine": "ppiiip",
     "mcb_launch_a2a_step": "ppiiip", "mcb_launch_route": "piip", "mcb_launch_expert_ffn": "piip",
     "mcb_launch_combine": "ppiiip", "mcb_launch_moe_layer": "piip", "mcb_moe_decode_step": "pppiiiipp",
-    "mcb_prepare_moe_step": "ppip" + "p" * 8 + "i",
+    "mcb_moe_step_joins": "pip", "mcb_prepare_moe_step": "ppip" + "p" * 8 + "i",
 }
 
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libmcb.so"

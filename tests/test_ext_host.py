@@ -314,3 +314,43 @@ def test_weight_tile_packing_round_trip():
     assert torch.equal(il[:, 0::2], split[:, :4]) and torch.equal(il[:, 1::2], split[:, 4:])
     with pytest.raises(ValueError):
         pack_weight_tiles(torch.zeros(1, 100, 64, dtype=torch.bfloat16))
+
+
+def _step_args(act=1 << 32, y=2 << 32, out=3 << 32):
+    """Argument blocks of two layers over buffers at made-up addresses: 16 rows of 256 values, 2 experts per token, 128 activations."""
+    from moe_comms_benchmarking_b200.ops.experts import _aligned_layer_args
+    cap, K, H = 16, 2, 256
+    raw, addr, stride = _aligned_layer_args(2)
+    meta = _ext.McbMetaArgs()
+    meta.n_local, meta.step_meta, meta.cap = 0x1000, 0x1100, cap
+    for s in range(2):
+        p = _ext.McbLayerArgs.from_address(addr + s * stride)
+        p.ctx.world, p.ctx.heap_local = 1, 4 << 32
+        g, r, f, c = p.agv, p.route, p.ffn, p.cmb
+        g.num_tensors, g.cap, g.n_local, g.step_meta = 3, cap, 0x1000, 0x1100
+        for t, nbytes in enumerate((2 * H, 8 * K, 4 * K)):
+            g.src[t], g.dst_off[t], g.row_bytes[t] = (5 + t) << 32, t << 20, nbytes
+        r.num_local_experts, r.topk, r.max_tokens, r.max_pairs, r.num_tokens = 4, K, cap, cap * K, 0x1100
+        r.pair_token, r.pair_prob, r.pair_pos, r.expert_offset, r.ffn_done = 0x2000, 0x3000, 0x4000, 0x5000, 0x6000
+        f.x, f.pair_token, f.pair_prob, f.expert_offset, f.ffn_done = 4 << 32, 0x2000, 0x3000, 0x5000, 0x6000
+        f.act, f.y, f.num_local_experts, f.hidden, f.intermediate, f.w1 = act, y, 4, H, 128, 0x7000 + s
+        c.y, c.pair_pos, c.topk, c.hidden, c.cap, c.out, c.n_local, c.step_meta = y, 0x4000, K, H, cap, out, 0x1000, 0x1100
+        p.local_ids, p.local_probs = g.src[1], g.src[2]
+    return raw, addr, meta
+
+
+def test_step_joins_only_layers_that_keep_apart(lib):
+    """Layers share a launch where none writes what another one reads or writes: activations (8 KB), expert outputs (16 KB) and combined
+    rows (8 KB) apart from one another, from the gathered rows and from their sources."""
+    def joins(**at):
+        raw, addr, meta = _step_args(**at)
+        return lib.mcb_moe_step_joins(addr, 2, C.addressof(meta))
+    act, y, rows, src = 1 << 32, 2 << 32, 4 << 32, 5 << 32
+    assert joins() == 1 and joins(out=act + 8192) == 1 and joins(y=act + 8192, out=act + 8192 + 16384) == 1
+    for out in (act, act + 8176, act - 8176, y, y + 16368, rows, rows + 8176, rows + (1 << 20), src, src + 8176, 6 << 32):
+        assert joins(out=out) == 0, hex(out)
+    for at in (act, act + 8176, act - 16368, rows, src):
+        assert joins(y=at) == 0, hex(at)
+    raw, addr, meta = _step_args()
+    meta.cap = 17
+    assert lib.mcb_moe_step_joins(addr, 2, C.addressof(meta)) == 0

@@ -715,3 +715,32 @@ def test_step_whose_waits_run_out(world1, word, small):
     d.check_health()
     assert torch.equal(d.out, want)
     d.destroy()
+
+
+def test_step_with_its_output_in_the_activations_goes_layer_by_layer(world1):
+    """A combined output in the memory of the activations: a layer of its own is done with them before it writes the first row."""
+    from moe_comms_benchmarking_b200.ops.dense import AllGatherVPlan, MetadataPlan
+    from moe_comms_benchmarking_b200.ops.experts import (ExpertCombinePlan, ExpertFfnPlan, ExpertWeights, MoeLayerPlan,
+                                                         RouteBuffers, RoutePlan)
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, E, K, H, I = 600, 6, 3, 256, 128
+    x, idx, w = _case(T, E, K, H, I, 29)
+    heap = SymmetricHeap(world1, 8 << 20, DEV)
+    gx, gi, gw = heap.alloc("gx", [T, H], torch.bfloat16), heap.alloc("gi", [T, K], torch.int64), heap.alloc("gw", [T, K], torch.float32)
+    n, meta = torch.tensor([T], dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    route = RouteBuffers(T, K, E, DEV)
+    act = torch.zeros(route.max_pairs, I, dtype=torch.bfloat16, device=DEV)
+    y = torch.zeros(route.max_pairs, H, dtype=torch.bfloat16, device=DEV)
+    partial = heap.alloc("partial", [2, T, H], torch.bfloat16)
+    ffn = [ExpertFfnPlan(ExpertWeights(E, H, I, DEV, seed=s, std=0.05), route, gx.tensor, act, y, heap.status) for s in (3, 4)]
+    got = []
+    for out in (act.view(-1)[:T * H].view(T, H), torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)):
+        plan = MoeLayerPlan(heap, AllGatherVPlan(heap, [gx, gi, gw], [x, idx, w], n, meta, T),
+                            RoutePlan(route, gi.tensor, gw.tensor, meta[0:1], expert_begin=0, status=heap.status), ffn,
+                            ExpertCombinePlan(heap, y, route, partial, out, n, meta, T), MetadataPlan(heap, n, meta, T))
+        assert (plan._step is None) == (not got)
+        plan.decode_step(5)
+        torch.cuda.synchronize()
+        heap.check_status()
+        got.append(out.clone())
+    assert torch.equal(*got) and bool(got[0].any())
