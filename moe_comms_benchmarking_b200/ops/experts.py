@@ -383,10 +383,13 @@ class MoeLayerPlan:
         self._ctx_version = id(ctx)
 
     def _prepare_step(self):
-        """Several layers of a step in one launch, where the layers allow it (``mcb_prepare_moe_step`` in csrc/moe_step.cu)."""
+        """Several layers of a step in one launch, where the layers allow it (``mcb_moe_step_joins`` in csrc/moe_step.cu)."""
         self._step = None
         if self.heap.world != 1 or self.trace is not None:
             return
+        lib = _ext.require()
+        if not lib.mcb_moe_step_joins(self._addr, len(self.ffns), C.addressof(self.meta.args)):
+            return                          # before anything is allocated
         b, f = self.route.bufs, self.ffns[0].args
         if self._step_bufs is None:         # pair lists and counters of two more layers in flight
             sizes = [2 * b.max_pairs, 2 * b.max_pairs, 2 * b.max_tokens * b.topk, 2 * b.E, 3 * b.E, _ext.STEP_SYNC_WORDS]
@@ -403,7 +406,6 @@ class MoeLayerPlan:
             if mem.is_cuda:
                 torch.cuda.current_stream(mem.device).synchronize()        # a step may run on another stream
             self._step_bufs = (keep, ptrs)
-        lib = _ext.require()
         raw = (C.c_uint8 * (lib.mcb_sizeof_step_args() + 64))()
         addr = (C.addressof(raw) + 63) & ~63
         if lib.mcb_prepare_moe_step(addr, self._addr, len(self.ffns), C.byref(self.meta.args), *self._step_bufs[1]) == 0:

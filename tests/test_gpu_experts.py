@@ -744,3 +744,17 @@ def test_step_with_its_output_in_the_activations_goes_layer_by_layer(world1):
         heap.check_status()
         got.append(out.clone())
     assert torch.equal(*got) and bool(got[0].any())
+
+
+@pytest.mark.parametrize("E,trace", [(768, False), (769, False), (8, True)])
+def test_plan_that_goes_layer_by_layer_keeps_no_step_buffers(world1, E, trace):
+    """Pair lists and buffers of further layers in flight are there only where layers share a launch."""
+    from moe_comms_benchmarking_b200.config import Config
+    from moe_comms_benchmarking_b200.parallel.fused import FusedExpertDispatcher
+    cfg = Config(num_experts=E, topk=4, hidden=256, intermediate=128, ep_size=1, per_rank_cap=8)
+    d = FusedExpertDispatcher(cfg, world1, num_layers=1, weight_budget_gb=1.0, phase_trace=trace)
+    d.build()
+    joins = E <= 768 and not trace
+    assert (d.layer_plan._step is not None) == joins and (d.layer_plan._step_bufs is not None) == joins
+    assert d.layer_plan.launches(4) == (2 if joins else 5)
+    d.destroy()
