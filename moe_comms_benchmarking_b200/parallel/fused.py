@@ -201,9 +201,10 @@ class FusedExpertDispatcher(Dispatcher):
         return oracle.moe_layer(hidden.cpu(), topk_idx.cpu(), topk_w.cpu(), torch.cat(wgu), torch.cat(wd))
 
     def validate(self):
-        """One full layer against the CPU oracle at B = 2*ep, at B = 1 (idle ranks) and, when the
-        capacity allows, at a realistic batch (up to 4096 tokens over all ranks, multi-block routing,
-        every expert busy) where a sample of this rank's tokens is compared."""
+        """One full layer, and a decode step through all weight sets whose last layer uses the same one, against the
+        CPU oracle at B = 2*ep, at B = 1 (idle ranks) and, when the capacity allows, at a realistic batch (up to
+        4096 tokens over all ranks, multi-block routing, every expert busy) where a sample of this rank's tokens
+        is compared."""
         from ..utils.inputs import make_inputs
         cfg, rank = self.cfg, self.cfg.rank
         results = []
@@ -220,23 +221,31 @@ class FusedExpertDispatcher(Dispatcher):
             # ones: meet on the host first, or the idle ranks' bounded device waits run out.
             self._sync_all()
             self.setup_batch(h, i, w)
-            for rep in range(2 if B == big else 1):     # twice at the large batch: counters must come back clean
-                self.metadata()
-                self.layer(0)
+            n, layers = counts[rank], len(self.weights) + 1
+            sample = torch.arange(n) if n <= 16 else torch.arange(0, n, max(1, n // 8))[:8]
+            ref = self.reference_output(h[sample], i[sample], w[sample]) if n else None
+            self._sync_all()
+
+            def one_layer():
+                for rep in range(2 if B == big else 1):     # twice at the large batch: counters must come back clean
+                    self.metadata()
+                    self.layer(0)
+
+            # A step of several layers may be other kernels than its layers one by one: it is what decoding runs.
+            for what, call in (("MoE layer", one_layer), (f"step of {layers}", lambda: self.decode_step(layers))):
+                self.out_buf.fill_(float("nan"))
+                call()
                 self._sync_all()
-            if counts[rank]:
-                n = counts[rank]
-                sample = torch.arange(n) if n <= 16 else torch.arange(0, n, max(1, n // 8))[:8]
-                ref = self.reference_output(h[sample], i[sample], w[sample])
-                got = self.out[sample].float().cpu()
-                scale = float(ref.abs().max()) + 1e-6
-                err = float((got - ref).abs().max())
-                ok = err / scale < 0.05
-                detail = (f"n={n} ({sample.numel()} token(s) compared) max|got-ref|={err:.5f} "
-                          f"({100 * err / scale:.2f}% of {scale:.4f})")
-            else:
-                ok, detail = True, "n=0 (idle rank still runs its experts on other ranks' tokens)"
-            results.append((f"fused MoE layer vs oracle B={B:<4d}", bool(ok), detail))
+                if n:
+                    got = self.out[sample].float().cpu()
+                    scale = float(ref.abs().max()) + 1e-6
+                    err = float((got - ref).abs().max())
+                    ok = err / scale < 0.05
+                    detail = (f"n={n} ({sample.numel()} token(s) compared) max|got-ref|={err:.5f} "
+                              f"({100 * err / scale:.2f}% of {scale:.4f})")
+                else:
+                    ok, detail = True, "n=0 (idle rank still runs its experts on other ranks' tokens)"
+                results.append((f"fused {what} vs oracle B={B:<4d}", bool(ok), detail))
         try:
             self.check_health()
         except Exception as e:

@@ -758,3 +758,21 @@ def test_plan_that_goes_layer_by_layer_keeps_no_step_buffers(world1, E, trace):
     assert (d.layer_plan._step is not None) == joins and (d.layer_plan._step_bufs is not None) == joins
     assert d.layer_plan.launches(4) == (2 if joins else 5)
     d.destroy()
+
+
+def test_validate_sees_the_kernels_of_a_step(world1, monkeypatch):
+    """The self-check runs decode steps through every weight set, and finds a step that delivers nothing."""
+    from moe_comms_benchmarking_b200.config import Config
+    from moe_comms_benchmarking_b200.parallel.fused import FusedExpertDispatcher
+    cfg = Config(num_experts=16, topk=4, hidden=256, intermediate=128, ep_size=1, per_rank_cap=48)
+    d = FusedExpertDispatcher(cfg, world1, num_layers=3, weight_budget_gb=1.0)
+    d.build()
+    results = d.validate()
+    assert all(ok for _, ok, _ in results), results
+    steps = []
+    with monkeypatch.context() as m:
+        m.setattr(d.layer_plan, "decode_step", lambda layers, *a, **kw: steps.append(layers))
+        broken = d.validate()
+    assert steps and set(steps) == {len(d.weights) + 1}
+    assert {name for name, ok, _ in broken if not ok} == {name for name, _, _ in results if "step" in name} != set()
+    d.destroy()
