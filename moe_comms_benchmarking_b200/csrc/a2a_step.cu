@@ -347,29 +347,68 @@ __device__ __forceinline__ void store_out(const McbA2AStepArgs& a, const Barrier
   }
 }
 
-// Barrier-mode layers of a step: push -> one block-matched barrier -> pull + fp32 sum.  Out of line, as above.
-__device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, int ep_max, uint32_t layer_base) {
-  const int tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int W = c.world, L = a.num_layers;
+__device__ __forceinline__ BarrierShape barrier_shape(const McbCtx& c, const McbA2AStepArgs& a) {
   BarrierShape s;
   s.row_packs = a.hidden / 8;
   s.slices = (s.row_packs + kSlicePacks - 1) / kSlicePacks;
   s.nblk = a.hidden / 128;
   s.meta_chunks = (int)(a.meta_row_bytes >> 4);
-  s.epr = a.num_experts / W;
+  s.epr = a.num_experts / c.world;
   s.row_bytes = (uint64_t)a.hidden * 2;
   s.xrow_bytes = a.fp8 ? (uint64_t)a.hidden : s.row_bytes;     // bytes of a dispatched row
+  return s;
+}
+
+// Layer after layer in a world of one, any number of ids: a slice is delivered and combined in one go, with every load of it in flight
+// at once.
+__device__ __forceinline__ void barrier_alone(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const BarrierShape s = barrier_shape(c, a);
+  const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
+  const long long mine = (long long)n * s.slices;
+  // one warp per block first, so that the smallest steps spread over the chip
+  const long long nact = mine < (long long)gridDim.x ? mine : (long long)gridDim.x;
+  if ((long long)blockIdx.x >= nact) return;
+  const long long first = blockIdx.x + (long long)warp * nact, step = nact * (blockDim.x >> 5);
+  const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
+  for (int l = 0; l < a.num_layers; ++l) {
+    const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+    const uint32_t stamp = layer_base + (uint32_t)l + 1u;
+    for (long long i = first; i < mine; i += step) {
+      RowSlice r;
+      r.t = (int)(i / s.slices);
+      r.p0 = (int)(i - (long long)r.t * s.slices) * kSlicePacks;
+      r.row = (uint64_t)c.rank * a.cap + r.t;
+      uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
+      load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
+      if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
+      if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
+      const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
+      push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
+      float acc[4][8] = {};
+      if (m.w[0]) {
+        if (echo) add_packs(acc, v);
+        else add_packs(acc, y);
+      }
+      store_out(a, s, r, acc, lane);
+    }
+  }
+}
+
+// Barrier-mode layers of a step: push -> one block-matched barrier -> pull + fp32 sum.  Out of line, as above.
+__device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, int ep_max, uint32_t layer_base) {
+  const int tid = threadIdx.x, bid = blockIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nwarps = blockDim.x >> 5;
+  const int W = c.world, L = a.num_layers;
+  const BarrierShape s = barrier_shape(c, a);
   const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
   const uint64_t slot0 = (uint64_t)c.rank * a.cap;             // first row of this source on a destination
-  // As many blocks as the largest rank needs, the same on every rank: with peers full blocks (each costs a flag per
-  // rank and layer), alone one warp per block first, so that the smallest steps spread over the chip.
-  const long long items = (long long)ep_max * s.slices;
-  const long long want = W == 1 ? items : (items + nwarps - 1) / nwarps;
+  // As many full blocks as the largest rank needs (each costs a flag per rank and layer), the same on every rank.
+  const long long want = ((long long)ep_max * s.slices + nwarps - 1) / nwarps;
   const int nact = (int)(want > (long long)gridDim.x ? (long long)gridDim.x : want);
   if (bid >= nact) return;
   const long long mine = (long long)n * s.slices;
-  const long long first = W == 1 ? bid + (long long)warp * nact : (long long)bid * nwarps + warp;
+  const long long first = (long long)bid * nwarps + warp;
   const long long step = (long long)nact * nwarps;
   auto slice_of = [&](long long i) {
     RowSlice r;
@@ -378,31 +417,6 @@ __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArg
     r.row = slot0 + r.t;
     return r;
   };
-
-  if (W == 1) {
-    // Emulated alone (else a2a_alone_kernel): a slice is delivered and combined in one go.
-    const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
-    for (int l = 0; l < L; ++l) {
-      const uint32_t par = (layer_base + (uint32_t)l) & 1u;
-      const uint32_t stamp = layer_base + (uint32_t)l + 1u;
-      for (long long i = first; i < mine; i += step) {
-        const RowSlice r = slice_of(i);
-        uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
-        load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
-        if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
-        if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
-        const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
-        push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
-        float acc[4][8] = {};
-        if (m.w[0]) {
-          if (echo) add_packs(acc, v);
-          else add_packs(acc, y);
-        }
-        store_out(a, s, r, acc, lane);
-      }
-    }
-    return;
-  }
 
   uint32_t ep = *epoch_ptr(c, MCB_SITE_A2A_STEP, bid);
   for (int l = 0; l < L; ++l) {
@@ -458,7 +472,7 @@ __device__ __noinline__ void barrier_layers(const McbCtx& c, const McbA2AStepArg
   if (tid == 0) *epoch_ptr(c, MCB_SITE_A2A_STEP, bid) = ep;
 }
 
-// Opening and end of a step, for all threads of every block.
+// Opening of a step, for all threads of every block.
 struct A2AStep {
   int n, ep_max;
   uint32_t step_seq, layer_base;
@@ -480,20 +494,6 @@ __device__ __forceinline__ A2AStep a2a_step_open(const McbCtx& c, const McbA2ASt
     a.step_meta[7] = (int)(st.layer_base + (uint32_t)L);     // stamp of the last layer's rows
   }
   return st;
-}
-// The last block out advances the sequence words.
-__device__ __forceinline__ void a2a_step_close(const McbA2AStepArgs& a, const A2AStep& st) {
-  volatile uint32_t* state = a.state;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(a.state + MCB_STATE_FINISHED, 1u) == gridDim.x - 1u) {
-      state[MCB_STATE_STEP_SEQ] = st.step_seq + 1u;
-      state[MCB_STATE_LAYER_BASE] = st.layer_base + (uint32_t)a.num_layers;
-      state[MCB_STATE_FINISHED] = 0u;
-      __threadfence();
-    }
-  }
 }
 
 template <bool EMU>
@@ -520,22 +520,12 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = ll ? 1 : 0;
   if (ll) {
     packet_layers(c, a, shp, s_prefix, st.n, valid, st.layer_base);
+  } else if (EMU && W == 1) {      // else a2a_alone_kernel
+    barrier_alone(c, a, st.n, st.layer_base);
   } else {
     barrier_layers(c, a, st.n, st.ep_max, st.layer_base);
   }
-  a2a_step_close(a, st);
-}
-
-__device__ __forceinline__ BarrierShape barrier_shape(const McbCtx& c, const McbA2AStepArgs& a) {
-  BarrierShape s;
-  s.row_packs = a.hidden / 8;
-  s.slices = (s.row_packs + kSlicePacks - 1) / kSlicePacks;
-  s.nblk = a.hidden / 128;
-  s.meta_chunks = (int)(a.meta_row_bytes >> 4);
-  s.epr = a.num_experts / c.world;
-  s.row_bytes = (uint64_t)a.hidden * 2;
-  s.xrow_bytes = a.fp8 ? (uint64_t)a.hidden : s.row_bytes;     // bytes of a dispatched row
-  return s;
+  step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
 }
 
 // ---- a world of one -----------------------------------------------------------------------------------
@@ -682,42 +672,6 @@ __device__ __forceinline__ void alone_layers(const McbCtx& c, const McbA2AStepAr
   else alone_many<FP8>(c, a, n, layer_base);
 }
 
-// Layer after layer in a world of one, any number of ids: a slice is delivered and combined in one go, with every load of it in flight
-// at once.
-__device__ __forceinline__ void barrier_alone(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const BarrierShape s = barrier_shape(c, a);
-  const uint8_t* x = reinterpret_cast<const uint8_t*>(a.x);
-  const long long mine = (long long)n * s.slices;
-  // one warp per block first, so that the smallest steps spread over the chip
-  const long long nact = mine < (long long)gridDim.x ? mine : (long long)gridDim.x;
-  if ((long long)blockIdx.x >= nact) return;
-  const long long first = blockIdx.x + (long long)warp * nact, step = nact * (blockDim.x >> 5);
-  const bool echo = !a.fp8 && a.y_off == a.recv_x_off;
-  for (int l = 0; l < a.num_layers; ++l) {
-    const uint32_t par = (layer_base + (uint32_t)l) & 1u;
-    const uint32_t stamp = layer_base + (uint32_t)l + 1u;
-    for (long long i = first; i < mine; i += step) {
-      RowSlice r;
-      r.t = (int)(i / s.slices);
-      r.p0 = (int)(i - (long long)r.t * s.slices) * kSlicePacks;
-      r.row = (uint64_t)c.rank * a.cap + r.t;
-      uint4 v[4], y[4], meta = make_uint4(0, 0, 0, 0);
-      load_packs(v, x + (uint64_t)r.t * s.row_bytes, r.p0, s.row_packs, lane);
-      if (!echo) load_packs(y, c.heap_local + a.y_off + (uint64_t)par * a.y_par_stride + r.row * s.row_bytes, r.p0, s.row_packs, lane);
-      if (r.p0 == 0 && lane < s.meta_chunks) meta = meta_chunk(a, r.t, lane, stamp);
-      const DestMask m = dest_mask(c, a, r.t, s.epr, lane);
-      push_slice(c, a, s, r, m, v, meta, par, stamp, lane);
-      float acc[4][8] = {};
-      if (m.w[0]) {
-        if (echo) add_packs(acc, v);
-        else add_packs(acc, y);
-      }
-      store_out(a, s, r, acc, lane);
-    }
-  }
-}
-
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.
 template <bool FP8>
@@ -729,7 +683,7 @@ __global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ 
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
   if (a.topk <= 32) alone_layers<FP8>(c, a, st.n, st.layer_base);
   else barrier_alone(c, a, st.n, st.layer_base);
-  a2a_step_close(a, st);
+  step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
 }
 
 }  // namespace mcb

@@ -602,16 +602,7 @@ __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant_
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
   const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
   if ((int)blockIdx.x < nact) local_layers<FP8>(c, a, n, nact, layer_base);
-  __syncthreads();
-  if (threadIdx.x == 0) {     // the last block out advances the sequence words
-    __threadfence();
-    if (atomicAdd(a.state + MCB_STATE_FINISHED, 1u) == gridDim.x - 1u) {
-      state[MCB_STATE_STEP_SEQ] = step_seq + 1u;
-      state[MCB_STATE_LAYER_BASE] = layer_base + (uint32_t)L;
-      state[MCB_STATE_FINISHED] = 0u;
-      __threadfence();
-    }
-  }
+  step_close(a.state, step_seq, layer_base + (uint32_t)L);
 }
 
 }  // namespace mcb

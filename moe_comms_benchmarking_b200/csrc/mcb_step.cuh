@@ -1,4 +1,4 @@
-// The count exchange that opens a persistent decode step (dense and all-to-all alike).
+// The count exchange that opens a persistent decode step and what ends one (dense and all-to-all alike).
 #pragma once
 #include "mcb_barrier.cuh"
 
@@ -54,6 +54,21 @@ __device__ __forceinline__ int step_count_exchange(const McbCtx& c, int site, ui
   }
   __syncthreads();
   return n;
+}
+
+// The last block out advances the sequence words of a step without packets.  Call from all threads of every block.
+__device__ __forceinline__ void step_close(uint32_t* words, uint32_t step_seq, uint32_t next_layer_base) {
+  volatile uint32_t* state = words;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(words + MCB_STATE_FINISHED, 1u) == gridDim.x - 1u) {
+      state[MCB_STATE_STEP_SEQ] = step_seq + 1u;
+      state[MCB_STATE_LAYER_BASE] = next_layer_base;
+      state[MCB_STATE_FINISHED] = 0u;
+      __threadfence();
+    }
+  }
 }
 
 // Credits of the packet modes: credit[block][source rank] = number of packet layers whose packets the
