@@ -482,3 +482,72 @@ def test_barrier_rounds_and_bounded_wait(lib):
     assert float((x * 2).sum()) == 16.0          # the context is still usable
     w.barrier_test(grid=8, rounds=1)
     w.check_status()
+
+
+@pytest.mark.parametrize("H,n,layers,grid,threads", [(1024, 5, 9, 148, 512), (7168, 3, 6, 148, 512), (1152, 40, 4, 2, 320)])
+def test_a2a_step_in_place(world1, H, n, layers, grid, threads):
+    """A step whose output is its input, e4m3 rows: each layer sends what the layer before has put out, so the received rows of
+    either parity are the expert outputs of the other one.  Fewer slices than warps and more."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, K, cap = 16, 4, n + 1
+    heap = SymmetricHeap(world1, 16 << 20, DEV)
+    bufs = A2AStepBuffers(heap, cap, H, K, True)
+    g = torch.Generator(device=DEV).manual_seed(53)
+    x, y = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((cap, H), (2, 1, cap, H)))
+    bufs.y.tensor.copy_(y)
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(cap)])
+    idx[n - 1] = -1 if n > 4 else idx[n - 1]            # a row for no expert: zero from the first layer on
+    wt = torch.rand(cap, K, device=DEV, generator=g)
+    meta = torch.zeros(8, dtype=torch.int32, device=DEV)
+    before = x.clone()
+    A2AStepPlan(heap, bufs, x, idx, wt, x, torch.tensor([n], dtype=torch.int32, device=DEV), meta, E, layers, grid=grid, threads=threads).launch()
+    torch.cuda.synchronize()
+    if n > 4:
+        with pytest.raises(DeviceStatusError):
+            heap.check_status()
+    last = int(meta[5])                                 # parity of the last layer
+    sent = n - 1 if n > 4 else n
+    assert torch.equal(x[:sent], y[last, 0, :sent]) and torch.equal(x[n:], before[n:]) and not x[sent:n].any()
+    for par in (0, 1):                                  # sent in a layer of parity `par`: what the layer before has put out
+        q, scale = oracle.quant_e4m3_1x128(y[1 - par, 0, :sent].float().cpu())
+        assert torch.equal(bufs.recv_x.tensor[par, 0, :sent].cpu(), q.view(torch.uint8))
+        assert torch.equal(bufs.recv_scale.tensor[par, 0, :sent].cpu(), scale)
+        words = bufs.recv_meta.tensor[par, 0, :sent].view(torch.int32).view(sent, -1)
+        assert bool((words[:, 0] == int(meta[7]) - (par != last)).all())
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("K", [1, 2, 31, 32, 33, 64, 65])
+def test_a2a_step_alone_metadata(world1, fp8, K):
+    """Received rows and metadata of a step in a world of one against values made in torch, up to and beyond one id per lane."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, H, n, layers = 80, 1152, 6, 5
+    heap = SymmetricHeap(world1, 16 << 20, DEV)
+    bufs = A2AStepBuffers(heap, n, H, K, fp8)
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, y = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((n, H), (2, 1, n, H)))
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(n)])
+    wt = torch.rand(n, K, device=DEV, generator=g)
+    out, meta = torch.zeros(n, H, dtype=torch.bfloat16, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    if fp8:
+        bufs.y.tensor.copy_(y)
+    bufs.recv_meta.tensor.zero_()
+    A2AStepPlan(heap, bufs, x, idx, wt, out, torch.tensor([n], dtype=torch.int32, device=DEV), meta, E, layers).launch()
+    torch.cuda.synchronize()
+    heap.check_status()
+    last = int(meta[5])
+    assert torch.equal(out, y[last, 0] if fp8 else x)
+    for par in (0, 1):
+        words = bufs.recv_meta.tensor[par, 0].contiguous().view(torch.int32).view(n, -1)
+        want = torch.zeros_like(words)
+        want[:, 2::2] = -1                              # no id
+        want[:, 0], want[:, 1] = int(meta[7]) - (par != last), torch.arange(n, device=DEV)
+        want[:, 2:2 + 2 * K:2], want[:, 3:3 + 2 * K:2] = idx.int(), wt.view(torch.int32)
+        assert torch.equal(words, want)
+        if fp8:
+            q, scale = oracle.quant_e4m3_1x128(x.float().cpu())
+            assert torch.equal(bufs.recv_x.tensor[par, 0].cpu(), q.view(torch.uint8)) and torch.equal(bufs.recv_scale.tensor[par, 0].cpu(), scale)
+        else:
+            assert torch.equal(bufs.recv_x.tensor[par, 0], x)
