@@ -98,9 +98,9 @@ __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
   return v;
 }
 
-// Equal chunks of an expert's `rows` tokens, at most `most` (a multiple of 16) each; all but the last are a multiple of 16 (the step of N of a CTA
+// Equal chunks of an expert's `rows` tokens, at most kFfnMaxN each; all but the last are a multiple of 16 (the step of N of a CTA
 // pair's MMA).
-__device__ __forceinline__ int ffn_chunks(int rows, int most) { return (rows + most - 1) / most; }
+__device__ __forceinline__ int ffn_chunks(int rows) { return (rows + kFfnMaxN - 1) / kFfnMaxN; }
 __device__ __forceinline__ int ffn_chunk_rows(int rows, int chunks) { return ((rows + chunks - 1) / chunks + 15) & ~15; }
 
 // One entry of the unit list.
@@ -168,7 +168,7 @@ struct FfnPlanS {
 
 // Fills cum / ids from the expert offsets; returns the number of experts with tokens.  All threads of the group.
 template <class Group>
-__device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, int most, int* cum, uint16_t* ids, int* scratch) {
+__device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, int* cum, uint16_t* ids, int* scratch) {
   const int tid = g.tid(), warp = tid >> 5, lane = tid & 31;
   const int per = (E + g.size() - 1) / g.size();
   const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
@@ -176,7 +176,7 @@ __device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, 
   for (int e = e0; e < e1; ++e) {
     const int rows = off[e + 1] - off[e];
     act += rows > 0;
-    chunks += ffn_chunks(rows, most);
+    chunks += ffn_chunks(rows);
   }
   int a_inc = act, c_inc = chunks;
 #pragma unroll
@@ -198,7 +198,7 @@ __device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, 
     ids[a_base] = (uint16_t)e;
     cum[a_base] = c_base;
     ++a_base;
-    c_base += ffn_chunks(rows, most);
+    c_base += ffn_chunks(rows);
   }
   if (tid == 0) cum[total] = total_c;
   g.sync();
@@ -698,7 +698,7 @@ __device__ __forceinline__ void ffn_run(const McbFfnArgs& a, const CUtensorMap* 
   const int n_slot = ffn_token_tile(max_rows);
   FfnPlanS plan;
   plan.off = sm.off; plan.cum = sm.cum; plan.ids = sm.ids;
-  ffn_plan(plan, a, ffn_slots(BlockGroup{}, sm.off, E, n_slot, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi)));
+  ffn_plan(plan, a, ffn_slots(BlockGroup{}, sm.off, E, sm.cum, sm.ids, reinterpret_cast<int*>(sm.epi)));
   if (n_slot <= kFfnDoubleN) ffn_roles<2>(a, maps, plan, n_slot, ready);
   else ffn_roles<1>(a, maps, plan, n_slot, ready);
 }

@@ -141,7 +141,7 @@ __device__ __forceinline__ void step_roles(const McbMoeStepArgs& p, const StepWe
       }
       FfnPlanS plan;
       plan.off = st.off; plan.cum = st.cum; plan.ids = st.ids;
-      ffn_plan(plan, a, ffn_slots(g, st.off, a.num_local_experts, n_slot, st.cum, st.ids, st.scan));
+      ffn_plan(plan, a, ffn_slots(g, st.off, a.num_local_experts, st.cum, st.ids, st.scan));
       const int total = plan.total();
       int first = pair - base;
       if (first < 0) first += npairs;
