@@ -170,7 +170,7 @@ struct FfnPlanS {
 template <class Group>
 __device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, int* cum, uint16_t* ids, int* scratch) {
   const int tid = g.tid(), warp = tid >> 5, lane = tid & 31;
-  const int per = (E + g.size() - 1) / g.size();
+  const int per = (E + (int)g.size() - 1) / (int)g.size();
   const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
   int act = 0, chunks = 0;
   for (int e = e0; e < e1; ++e) {
@@ -187,7 +187,7 @@ __device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, 
   if (lane == 31) { scratch[warp] = a_inc; scratch[32 + warp] = c_inc; }
   g.sync();
   int a_base = a_inc - act, c_base = c_inc - chunks, total = 0, total_c = 0;
-  for (int w = 0; w < (g.size() >> 5); ++w) {
+  for (int w = 0; w < (int)(g.size() >> 5); ++w) {
     if (w < warp) { a_base += scratch[w]; c_base += scratch[32 + w]; }
     total += scratch[w];
     total_c += scratch[32 + w];

@@ -58,7 +58,8 @@ __device__ __forceinline__ bool route_counts_all(const Group& g, const RouteShar
 template <bool SPLIT, class Group>
 __device__ __forceinline__ void route_count(const Group& g, const McbRouteArgs& a, const int64_t* topk_idx, const RouteSmem& m, long long lo,
                                             long long hi, long long split) {
-  const int tid = g.tid(), threads = g.size(), E = a.num_local_experts;
+  const int tid = g.tid(), E = a.num_local_experts;
+  const unsigned threads = g.size();
   for (int e = tid; e < E; e += threads) { m.cnt[e] = 0; m.begin[e] = 0; }
   g.sync();
   for (long long i0 = lo + tid; i0 < hi; i0 += threads * 4) {
@@ -97,8 +98,8 @@ __device__ __forceinline__ void route_collect(const Group& g, int E, const int* 
 // the fused FFN into global memory.  Returns the largest count in every thread.  All threads of the group.
 template <class Group>
 __device__ __forceinline__ int route_offsets(const Group& g, const McbRouteArgs& a, const RouteSmem& m, bool writes) {
-  const int tid = g.tid(), E = a.num_local_experts, warp = tid >> 5, lane = tid & 31, nw = g.size() >> 5;
-  const int per = (E + g.size() - 1) / g.size();
+  const int tid = g.tid(), E = a.num_local_experts, warp = tid >> 5, lane = tid & 31, nw = (int)(g.size() >> 5);
+  const int per = (E + (int)g.size() - 1) / (int)g.size();
   const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
   int rows = 0, tiles = 0, mx = 0;
   for (int e = e0; e < e1; ++e) {
@@ -167,7 +168,8 @@ __device__ __forceinline__ int route_offsets(const Group& g, const McbRouteArgs&
 template <class Group>
 __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& a, const int64_t* topk_idx, const float* topk_w,
                                             const RouteSmem& m, const RouteShare& s) {
-  const int E = a.num_local_experts, threads = g.size();
+  const int E = a.num_local_experts;
+  const unsigned threads = g.size();
   for (long long i0 = s.lo + g.tid(); i0 < s.hi; i0 += threads * 4) {
     long long e[4];
     float w[4];
