@@ -118,11 +118,11 @@ def run_child(world, impl, batches, extra):
 def run_fused_child(world, batches, args):
     """Times the real-expert path (config: 512 experts, SwiGLU FFN 1024 -> 1024 -> 1024 per expert, bf16 weights
     N(0, 0.02^2), 88 layers) with ``run.py --impl fused``; returns ({global batch: ms per step}, details)."""
+    from moe_comms_benchmarking_b200.ops.experts import step_launches
     ms = run_child(world, "fused", batches, ["--reps", "5", "--warmup", "3", "--weight-budget-gb", str(args.fused_weight_gb)])
     experts_per_rank = 512 // world
     sets = max(1, min(NUM_LAYERS, int(args.fused_weight_gb * 2**30 // (experts_per_rank * 3 * 1024 * 1024 * 2))))
-    together = 1 if world > 1 else NUM_LAYERS if sets <= 16 else 16         # layers of one launch
-    detail = {"kernels_per_step": 1 + -(-NUM_LAYERS // together), "protocol": "run.py --impl fused: graph replays back to back, max over ranks",
+    detail = {"kernels_per_step": step_launches(NUM_LAYERS, sets, joined=world == 1), "protocol": "run.py --impl fused: graph replays back to back, max over ranks",
               "weights_mb_per_layer_and_rank": round(experts_per_rank * 3 * 1024 * 1024 * 2 / 1e6, 1),
               "expert": "SwiGLU FFN, hidden 1024 -> intermediate 1024 -> 1024, bf16, N(0, 0.02^2)"}
     return ms, detail

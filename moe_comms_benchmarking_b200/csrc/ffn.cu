@@ -125,7 +125,8 @@ static bool configure_ffn_kernels() {
 static int check_ffn_args(const McbFfnArgs* a) {
   if (!a || !a->x || !a->pair_token || !a->expert_offset || !a->max_rows || !a->act || !a->y || !a->ffn_done) return 1;
   if (!a->w1 || !a->w2 || (reinterpret_cast<uintptr_t>(a->w1) & 15) || (reinterpret_cast<uintptr_t>(a->w2) & 15)) return 1;
-  if (a->num_local_experts < 1 || a->num_local_experts > kFfnMaxExperts || a->hidden < 256 || a->hidden % 256 || a->intermediate < 128 || a->intermediate % 128) return 1;
+  if (a->num_local_experts < 1 || a->num_local_experts > kFfnMaxExperts) return 1;
+  if (a->hidden < 256 || a->hidden % 256 || a->intermediate < 128 || a->intermediate % 128) return 1;
   if (!a->tmaps || (reinterpret_cast<uintptr_t>(a->tmaps) & 63)) return 1;
   return 0;
 }
@@ -133,7 +134,8 @@ static int check_ffn_args(const McbFfnArgs* a) {
 // The kernels run in CTA pairs: an odd grid is rounded down, one CTA is rounded up.
 static int pair_grid(int grid) { return grid < 2 ? 2 : grid & ~1; }
 
-// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory.  x: token rows; act: activations; w1, w2: the packed weights.
+// The tensor maps of one FFN launch (MCB_FFN_TMAPS x 128 bytes) into 64-byte aligned host memory.  x: token rows; act: activations;
+// w1, w2: the packed weights.
 int mcb_make_ffn_tmaps(void* out, const void* x, uint64_t x_rows, const void* act, uint64_t pair_rows, const void* w1, const void* w2,
                        int experts, int hidden, int intermediate) {
   uint8_t* o = reinterpret_cast<uint8_t*>(out);

@@ -17,8 +17,8 @@
 //     of as many 330, an MMA step over 256 tokens 512), one thread issues one in 35 to 55: four warps share a
 //     chunk of up to 128 tokens, six a larger one.  With two warps that also fetched the token numbers, alone, the gathers
 //     were the limit, and above 128 tokens the rows were copied into pair order by all CTAs before the first unit
-//     (184 MB at 4096 tokens of top-22: 730 -> 672 us a layer without the copy; 64 experts at 173 tokens 91 -> 84, at 350 tokens
-//     154 -> 147, with Zipf routing 162 -> 152 us);
+//     (184 MB at 4096 tokens of top-22: 730 -> 672 us a layer without the copy from a cool chip, 896 -> 830 in runs long enough
+//     for the power cap; 64 experts at 173 tokens 91 -> 84, at 350 tokens 154 -> 147, with Zipf routing 162 -> 152 us);
 //   * work units are listed per CTA pair in shared memory before the roles start: experts without tokens are
 //     left out of the numbering, so the pairs get equally many units whatever the routing, and a
 //     popular expert's chunks spread over the chip;
@@ -44,9 +44,9 @@
 // Measured on one B200 with 64 experts of 1024 x 1024 (402.7 MB of weights), against one CTA per unit of 128 weight rows
 // with token rows copied by cp.async and units numbered over all experts: 64 us (66 before) at 3 tokens per expert,
 // where the weight stream is the limit; 84 (113) at 173 and 147 (204) at 350 tokens per expert.  From about 170 tokens per
-// expert on the power cap decides: the clock falls to 1.2-1.4 GHz, and the same launches on rows of zeros take 76 and 122 us.  With 22 of 512 experts in use 36 (52).  Launches of a few microseconds lose what a CTA
-// pair costs to set up and take down, and to gather: 8 experts of 512 x 256 at 1 / 32 / 128 tokens per expert 8.3 / 9.6 /
-// 12.9 us (7.2 / 7.7 / 10.4).
+// expert on the power cap decides: the clock falls to 1.2-1.4 GHz, and the same launches on rows of zeros take 76 and 122 us.  With
+// 22 of 512 experts in use 36 (52).  Launches of a few microseconds lose what a CTA pair costs to set up and take down, and to
+// gather: 8 experts of 512 x 256 at 1 / 32 / 128 tokens per expert 8.3 / 9.6 / 12.9 us (7.2 / 7.7 / 10.4).
 #pragma once
 #include "mcb_group.cuh"
 #include "mcb_tc.cuh"
@@ -407,10 +407,10 @@ struct FfnRoles {
   int y_free_want = 0;
 
   __device__ __forceinline__ FfnRoles(const McbFfnArgs& args, const CUtensorMap* x, const CUtensorMap* act, int n_slot)
-      : a(args), xmap(x), actmap(act), act_rows(reinterpret_cast<uint8_t*>(args.act)), y_rows(reinterpret_cast<uint8_t*>(args.y)), warp(threadIdx.x >> 5), lane(threadIdx.x & 31), rank((int)cluster_ctarank()),
-        H(args.hidden), I(args.intermediate), n1(2 * args.intermediate / kFfnRowsM), n2(args.hidden / kFfnRowsM),
-        tmem_base(*sm.tmem_slot), ab{sm.abort_flag, args.status, args.timeout_ns}, b_sub_bytes((n_slot >> 1) * 128),
-        stage_bytes(NSUB * (kFfnABytes + b_sub_bytes)), stages(stage_count(stage_bytes)) {}
+      : a(args), xmap(x), actmap(act), act_rows(reinterpret_cast<uint8_t*>(args.act)), y_rows(reinterpret_cast<uint8_t*>(args.y)),
+        warp(threadIdx.x >> 5), lane(threadIdx.x & 31), rank((int)cluster_ctarank()), H(args.hidden), I(args.intermediate),
+        n1(2 * args.intermediate / kFfnRowsM), n2(args.hidden / kFfnRowsM), tmem_base(*sm.tmem_slot), ab{sm.abort_flag, args.status, args.timeout_ns},
+        b_sub_bytes((n_slot >> 1) * 128), stage_bytes(NSUB * (kFfnABytes + b_sub_bytes)), stages(stage_count(stage_bytes)) {}
   static __device__ __forceinline__ int stage_count(int bytes) {
     const int fit = kFfnPipeBytes / bytes, most = NSUB == 2 ? kFfnDoubleStages : kFfnMaxStages;
     return fit < most ? fit : most;

@@ -23,8 +23,11 @@ constexpr int kRouteThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
 // Shared memory of a routing block: counts, own begins (later cursors), offsets, scan scratch.
 constexpr int kRouteSmemWords = 3 * kMaxLocalExperts + 1 + 3 * 32;
-// Entries per thread up to which every block counts all of them.  Layer kernel (384 threads), 64 experts: 4000 entries 37.4 us
-// (39.6 with the counts shared through global counters), 6080 42.1 (43.8), 8000 45.5 (45.4), 16000 62.8 (61.8), 24000 76.7 (72.7).
+// Entries per thread up to which every block counts all of them.  Either way forced, one B200, us a layer with 64 experts of
+// 512 x 256 and top-8, all counted by every block (counts shared through global counters):
+//   layer kernel, 512 threads      4096 entries 30.8 (34.6), 8192 35.9 (38.2), 12288 41.7 (42.3), 16384 47.4 (47.3), 24576 58.6 (56.4)
+//   step, 64 threads of a block    1024 entries 14.5 (15.0), 2048 14.8 (15.3), 3072 15.9 (15.4), 4096 18.1 (16.2), 8192 25.8 (20.0)
+// The line lies on the safe side of both crossings (about 32 and 40 entries per thread): beyond them counting all costs ever more.
 constexpr int kRouteAllPerThread = 16;
 
 struct RouteSmem {
@@ -200,9 +203,10 @@ __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& 
 
 // The whole routing by the blocks of a launch that has nothing else to share a barrier with.  With few entries nobody waits
 // for another block: all count all entries and place their own (one block alone: 21.9 us a launch at 11264 entries of 512
-// experts, now 5.8; 8.5 and 4.2 at 1408; 3.0 and 3.8 at 128 of 32, where the wider scan shows); with many the blocks wait for one another on a counter that only grows (the grid must be
-// co-resident).  There a thread keeps its first kRouteKept entries from the counting to the placing, and the last block to have read the
-// counters is found while the others place: 22528 / 45056 / 90112 entries, 64 of 512 experts local, 10.4 -> 8.5 / 10.5 -> 8.5 / 10.6 -> 9.3 us.
+// experts, now 5.8; 8.5 and 4.2 at 1408; 3.0 and 3.8 at 128 of 32, where the wider scan shows); with many the blocks wait for one
+// another on a counter that only grows (the grid must be co-resident).  There a thread keeps its first kRouteKept entries from the
+// counting to the placing, and the last block to have read the counters is found while the others place: 22528 / 45056 / 90112
+// entries, 64 of 512 experts local, 10.4 -> 8.5 / 10.5 -> 8.5 / 10.6 -> 9.3 us.
 // Shares are runs of entries: with entries dealt to the blocks in turn, an expert's rows come in another order, and FFN and
 // combine of 8191 tokens with Zipf routing were 2 % slower; asked for before the number of tokens is known, few entries took
 // 8.4 us (7.2).  Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.

@@ -14,13 +14,17 @@
 //
 // The pair lists and counters of a layer alternate between three sets of buffers, so that routing layer l + 1 waits for the
 // sums of layer l - 2 only.  With two sets (and the sums right behind a layer's last unit) the stream stood still for 5 of
-// 26 us a layer at one token, waiting for the routing that waited for the sums.  Measured on one B200 against a launch per layer,
-// 8 layers of 512 experts of 1024 x 1024, top-22: 1 / 4 / 16 / 37 / 128 / 512 / 1024 tokens 23.5 / 72.7 / 219 / 361 / 448 / 475 / 494 us a
-// layer (41.5 / 89 / 235 / 379 / 462 / 496 / 519); 88 layers of one token 1942 us (3565), whose weights alone are 1860 at the speed
-// of a copy; 64 experts of 768 x 512, one token, 12.3 us (23.5); 4 wide layers of 190 tokens 402 (420).  At 4096 tokens the power cap
-// decides and both are equal (670-780 us, as warm as the chip is).  Four accumulators instead of two changed nothing.  The units are numbered through all layers (the first unit of a layer goes to the pair behind the one
-// that has the last unit of the layer before), so a layer whose units do not fill its last round costs no round.
-// All layers read the same rows, ids and weights, which nothing in the step writes (the host checks that, mcb_prepare_moe_step), so
+// 26 us a layer at one token, waiting for the routing that waited for the sums.  Measured on one B200 against a launch per layer, both
+// kept running for a second (nvidia-smi beside them), 8 layers of 512 experts of 1024 x 1024, top-22, us a layer:
+//   tokens              1       4      16      37     128     512    1024    4096
+//   one launch       23.6    72.6     226     339     455     492     520     800     1.9 GHz at one token, 1.6-1.5 up to 512, 1.4, 1.05
+//   a launch each    41.7    89.5     244     353     474     503     541     792     1.97, 1.96, 1.67-1.6, 1.43, 1.1 GHz
+// From 4 tokens on the power cap is active in both (1000 W); runs of a few milliseconds on a cool chip are up to 15 % shorter at 4096.
+// 88 layers of one token 1980 us (3630), whose weights alone are 1860 at the speed of a copy; 64 experts of 768 x 512, one token of
+// top-6, 9.3 us a layer (22.5); 4 wide layers (7168 x 2048, 32 experts) of 190 tokens 422 (441).  Four accumulators instead of two
+// changed nothing.  The units are numbered through all layers (the first unit of a layer goes to the pair behind the one that has the
+// last unit of the layer before), so a layer whose units do not fill its last round costs no round.
+// All layers read the same rows, ids and weights, which nothing in the step writes (the host checks that, mcb_moe_step_joins), so
 // the experts gather the rows at their source and nobody waits for the copy.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -365,7 +369,8 @@ const void* joined_rows(const McbLayerArgs* sets, int num_sets, const McbMetaArg
   for (int t = 0; t < g.num_tensors; ++t)
     if (p.ctx.heap_local + g.dst_off[t] == f.x && g.row_bytes[t] == 2u * (uint32_t)f.hidden) x = g.src[t];
   const uint64_t rows = (uint64_t)g.cap, pairs = (uint64_t)r.max_pairs;
-  const Range written[] = {range(f.act, pairs * f.intermediate * 2), range(f.y, pairs * f.hidden * 2), range(cmb.out, (uint64_t)cmb.cap * f.hidden * 2)};
+  const Range written[] = {range(f.act, pairs * f.intermediate * 2), range(f.y, pairs * f.hidden * 2),
+                           range(cmb.out, (uint64_t)cmb.cap * f.hidden * 2)};
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < i; ++j)
       if (overlap(written[i], written[j])) return nullptr;
@@ -424,7 +429,9 @@ int mcb_prepare_moe_step(McbMoeStepArgs* out, const McbLayerArgs* sets, int num_
   static_assert(sizeof out->map_act[0] == kFfnMaxGroups * sizeof(CUtensorMap), "a map per box");
   for (int i = 0; i < 2; ++i)
     for (int b = 0; b < kFfnMaxGroups; ++b)
-      if (make_tmap_bf16(out->map_act[i][b], out->act[i], i && out->two_rows ? (uint64_t)out->two_rows : pairs, (uint64_t)f.intermediate, 4 * (b + 1))) return 1;
+      if (make_tmap_bf16(out->map_act[i][b], out->act[i], i && out->two_rows ? (uint64_t)out->two_rows : pairs, (uint64_t)f.intermediate,
+                         4 * (b + 1)))
+        return 1;
   return 0;
 }
 

@@ -349,12 +349,20 @@ def local_routing(heap: SymmetricHeap, agv: "_ext.McbAgvArgs", route: "_ext.McbR
     return (ids, probs) if ids and (probs or not route.topk_w) else (None, None)
 
 
+def step_launches(num_layers: int, sets: int, joined: bool) -> int:
+    """Kernel launches of a decode step with ``sets`` weight sets whose layers share launches or do not."""
+    together = 1 if not joined or num_layers < 2 else num_layers if sets <= _ext.STEP_SETS else _ext.STEP_SETS
+    return 1 + -(-num_layers // together)
+
+
 class MoeLayerPlan:
     """One whole MoE layer per launch (``moe_layer_kernel``: dispatch, routing, experts, combine), for
     one or several weight sets; ``launch(s)`` runs the layer with set ``s``, ``decode_step(n)`` issues the
     count exchange and ``n`` layers natively (layer l uses set l % sets).  In a world of one the layers of a step share a
-    launch (csrc/moe_step.cu; up to 16 of them where there are more sets than that) unless a layer writes what the next one
-    reads or a phase trace is taken."""
+    launch (csrc/moe_step.cu; up to 16 of them where there are more sets than that).  They go one by one where a phase trace
+    is taken, there are more than 768 experts, the all-gather does not bring the rows, ids and weights that experts and routing
+    read, the plans do not belong together (other buffers, counts or capacities), or a layer writes what the next one reads or
+    memory that it writes in another way too."""
 
     def __init__(self, heap: SymmetricHeap, agv, route: RoutePlan, ffns: list[ExpertFfnPlan], combine: ExpertCombinePlan,
                  meta, grid: int = NUM_SMS, trace: bool = False):
@@ -413,8 +421,7 @@ class MoeLayerPlan:
 
     def launches(self, num_layers: int) -> int:
         """Kernel launches of ``decode_step(num_layers)``: the count exchange and those of the layers."""
-        together = 1 if self._step is None or num_layers < 2 else num_layers if len(self.ffns) <= _ext.STEP_SETS else _ext.STEP_SETS
-        return 1 + -(-num_layers // together)
+        return step_launches(num_layers, len(self.ffns), self._step is not None)
 
     def _sync_ctx(self):
         if self._ctx_version != id(self.heap.ctx()):      # the heap's context was rebuilt (e.g. a new timeout)

@@ -168,7 +168,7 @@ class FusedExpertDispatcher(Dispatcher):
         self.layer(0)
 
     def decode_step(self, num_layers: int):
-        if self.layer_kernel:       # one native call: count exchange + one launch per layer
+        if self.layer_kernel:       # one native call: count exchange + one launch per layer, or one for several (MoeLayerPlan)
             self.layer_plan.decode_step(num_layers, self.pdl and self.coop_pdl)
             return
         self.metadata()

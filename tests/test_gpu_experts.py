@@ -87,8 +87,8 @@ def test_route_fc1_fc2_combine_against_oracle(world1, T, E, K, H, I):
                                             (400, 8, 2, 256, 256, 3), (400, 8, 2, 256, 256, 5)])
 def test_expert_ffn_weights_as_m_against_oracle(world1, T, E, K, H, I, grid):
     """The grouped FFN with the weights as the M operand of a CTA pair (gate/up + SwiGLU + down in one
-    persistent launch): experts with no token, with a few (rows gathered by TMA), with more than 128 (rows copied
-    into pair order) and more than 256 (several chunks), more units than CTA pairs, an odd grid, interleaved
+    persistent launch): experts with no token, with a few, with more than 128 (one column block per pipeline
+    stage) and more than 256 (several chunks), more units than CTA pairs, an odd grid, interleaved
     gate/up rows."""
     from moe_comms_benchmarking_b200.ops import oracle
     from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
@@ -294,7 +294,7 @@ def test_layer_kernel_phase_trace_world1(world1):
     ([1, 31, 32, 33, 0, 64], 256, 128, 148),             # gathered token rows: below, at and above a multiple of 32, an idle expert
     ([65, 0, 3], 512, 256, 6),                           # rows gathered past 64, fewer CTA pairs than units
     ([128, 97, 96, 127, 33, 0], 256, 128, 148),          # up to 32 gathered rows per producer, two column blocks per stage
-    ([129, 1], 256, 128, 148),                           # rows copied into pair order, one column block per stage; more CTAs than units
+    ([129, 1], 256, 128, 148),                           # one column block per stage; more CTAs than units
     ([256, 257, 0, 513, 5], 256, 384, 148),              # one, two and three chunks of an expert
     ([40] * 200, 512, 256, 2),                           # more units than one list holds
     ([2600, 300, 1, 900, 2400, 700], 256, 2048, 148),    # activations beyond the L2 bound: down units follow at a distance
@@ -422,7 +422,7 @@ def test_layer_plan_follows_its_routing_plan(world1, form):
         assert float((out[:T].float().cpu() - ref).abs().max()) < 0.03 * s + 1e-3, f"rep {rep}"
 
 
-@pytest.mark.parametrize("rows", [[40, 10], [140, 3]])       # token rows gathered, and copied into pair order
+@pytest.mark.parametrize("rows", [[40, 10], [140, 3]])       # two column blocks per pipeline stage, and one
 def test_expert_ffn_plan_at_once_on_another_stream(world1, rows):
     """A plan is ready when its constructor returns: plans over changing inputs, one after the other and each launched
     on a stream of its own while the stream that it was built on is still busy.  The reference rounds the activations by
@@ -461,8 +461,8 @@ def test_expert_ffn_plan_at_once_on_another_stream(world1, rows):
 
 @pytest.mark.parametrize("grid", [2, 6, 148])
 def test_expert_ffn_row_copy_counters_return(world1, grid):
-    """Launches back to back whose token rows are copied into pair order, with fewer and with more CTA pairs than units: the
-    counters of the copy are back at zero, and the last launch is as right as the first."""
+    """Launches back to back with fewer and with more CTA pairs than units: the counters of the routing are back at zero, and the
+    last launch is as right as the first."""
     from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
     from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
     T, H, I = 290, 256, 128
