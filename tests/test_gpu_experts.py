@@ -776,3 +776,45 @@ def test_validate_sees_the_kernels_of_a_step(world1, monkeypatch):
     assert steps and set(steps) == {len(d.weights) + 1}
     assert {name for name, ok, _ in broken if not ok} == {name for name, _, _ in results if "step" in name} != set()
     d.destroy()
+
+
+@pytest.mark.parametrize("form", ["plain", "no_weights", "two_tensors", "order", "odd_ids", "own_weights"])
+def test_step_forms_like_single_layers(world1, form):
+    """What a joined step accepts against the same layers launched one by one, bit for bit: no routing weights, fewer tensors or another
+    order of them in the all-gather, ids of no expert and an expert twice in a row.  Weights that the all-gather does not bring are
+    the caller's own, and the layers go one by one."""
+    from moe_comms_benchmarking_b200.ops.dense import AllGatherVPlan, MetadataPlan
+    from moe_comms_benchmarking_b200.ops.experts import (ExpertCombinePlan, ExpertFfnPlan, ExpertWeights, MoeLayerPlan,
+                                                         RouteBuffers, RoutePlan)
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, cap, E, K, H, I = 310, 333, 6, 5, 256, 128
+    pad = lambda t: torch.cat([t, t[:cap - T]]).contiguous()
+    x, idx, w = (pad(t) for t in _case(T, E, K, H, I, 61))
+    if form == "odd_ids":
+        idx[::3, 0], idx[1::3, 1], idx[2::3, 2], idx[::2, 3], idx[7] = -1, E, 1 << 40, idx[::2, 4], -5
+    heap = SymmetricHeap(world1, 8 << 20, DEV)
+    gx, gi, gw = heap.alloc("gx", [cap, H], torch.bfloat16), heap.alloc("gi", [cap, K], torch.int64), heap.alloc("gw", [cap, K], torch.float32)
+    pairs = {"two_tensors": [(gx, x), (gi, idx)], "order": [(gw, w), (gi, idx), (gx, x)]}.get(form, [(gx, x), (gi, idx), (gw, w)])
+    r_w = {"no_weights": None, "two_tensors": None, "own_weights": w.clone()}.get(form, gw.tensor)
+    n, meta = torch.tensor([T], dtype=torch.int32, device=DEV), torch.zeros(4, dtype=torch.int32, device=DEV)
+    route = RouteBuffers(cap, K, E, DEV)
+    act = torch.zeros(route.max_pairs, I, dtype=torch.bfloat16, device=DEV)
+    y = torch.zeros(route.max_pairs, H, dtype=torch.bfloat16, device=DEV)
+    out, partial = torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV), heap.alloc("partial", [2, cap, H], torch.bfloat16)
+    ffn = [ExpertFfnPlan(ExpertWeights(E, H, I, DEV, seed=s, std=0.05), route, gx.tensor, act, y, heap.status) for s in (3, 4, 5)]
+    plan = MoeLayerPlan(heap, AllGatherVPlan(heap, [d for d, _ in pairs], [s for _, s in pairs], n, meta, cap),
+                        RoutePlan(route, gi.tensor, r_w, meta[0:1], expert_begin=0, status=heap.status), ffn,
+                        ExpertCombinePlan(heap, y, route, partial, out, n, meta, cap), MetadataPlan(heap, n, meta, cap))
+    assert (plan._step is None) == (form == "own_weights")
+    plan.meta.launch()
+    for l in range(5):
+        plan.launch(l % 3)
+    torch.cuda.synchronize()
+    want, rows = out.clone(), [d.tensor[:T].clone() for d, _ in pairs]
+    for rep in range(2):
+        for t in [out, y, act] + [d.tensor for d, _ in pairs]:
+            t.zero_()
+        plan.decode_step(5)
+        torch.cuda.synchronize()
+        heap.check_status()
+        assert torch.equal(out, want) and bool(out[:T].any()) and all(torch.equal(d.tensor[:T], r) for (d, _), r in zip(pairs, rows))
