@@ -285,15 +285,21 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
 }
 
 // ---- a world of one: the layers of a step are local copies ------------------------------------------------------
+// The part of a step that a block has a share in: layers [first, last), as block `block` of those that a layer fills.
+struct LocalPart {
+  int block, first, last;
+};
+
 // Up to S packs per thread and layer: where they come from and go to is worked out once for all layers.  Nothing that a
 // layer reads is written in the step (else: a.in_order), so the loads of D layers go out together and are stored layer
 // by layer; the layers of such a step run into each other.  With one layer at a time each layer was a trip to L2: 88 layers
 // of hidden 1024 and top-22, one B200: 57 -> 37 us with one
 // token, 47 -> 34 with 200, 62 -> 55 with 333, where the second pack per thread begins; with e4m3 rows, whose packs go along, 100 -> 52, 109 ->
 // 47 (100 tokens) and 115 -> 59.
-template <bool FP8, int S, int D>
-__device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, long long start,
-                                          long long stride, uint32_t layer_base) {
+template <bool FP8, int S, int D, bool PARTS = false>
+__device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, const LocalPart& part,
+                                          long long start, long long stride, uint32_t layer_base) {
+  const int last = PARTS ? part.last : a.num_layers, block = PARTS ? part.block : (int)blockIdx.x;
   // e4m3: packs of bf16 rows, and where their values and their block's scale go
   const int H = (int)a.fp8_hidden, ppr = FP8 ? H / 8 : 1, nblk = H / 128;
   const uint8_t* rows = reinterpret_cast<const uint8_t*>(a.src[0]);
@@ -323,7 +329,7 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
     dst[u] = r.dst[t] + off;
     par_off[u] = r.par[t];
   }
-  for (int l0 = 0; l0 < a.num_layers; l0 += D) {
+  for (int l0 = PARTS ? part.first : 0; l0 < last; l0 += D) {
     uint4 v[D][S], h[D * S];
     uint32_t w[D];
 #pragma unroll
@@ -331,13 +337,13 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
       if (FP8) {
 #pragma unroll
         for (int u = 0; u < S; ++u)
-          h[d * S + u] = quant[u] && l0 + d < a.num_layers ? ld_v4_stream(rows + (start + u * stride) * 16) : make_uint4(0, 0, 0, 0);
+          h[d * S + u] = quant[u] && l0 + d < last ? ld_v4_stream(rows + (start + u * stride) * 16) : make_uint4(0, 0, 0, 0);
       }
-      if (l0 + d >= a.num_layers) continue;
+      if (l0 + d >= last) continue;
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) v[d][u] = ld_v4_stream(src[u]);
-      w[d] = r.load_word();
+      w[d] = r.load_word(threadIdx.x, block);
     }
     float scale[D * S];
     if (FP8) {
@@ -346,7 +352,7 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
     }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      if (l0 + d >= a.num_layers) break;
+      if (l0 + d >= last) break;
       const uint32_t par = (layer_base + (uint32_t)(l0 + d)) & 1u;
       if (FP8) {
 #pragma unroll
@@ -360,26 +366,32 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
 #pragma unroll
       for (int u = 0; u < S; ++u)
         if (live[u]) st_v4(dst[u] + (par ? par_off[u] : 0), v[d][u]);
-      r.store_word(par, w[d]);
+      r.store_word(par, w[d], threadIdx.x, block);
     }
   }
 }
 
+// What a layer copies; quantised values and scales are pushed on their own.  All threads of the block.
 template <bool FP8>
-__device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
-  __shared__ LocalRanges r;
+__device__ __forceinline__ void local_ranges(LocalRanges& r, const McbCtx& c, const McbDenseStepArgs& a, int n) {
   constexpr int R = LocalRanges::R;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    for (int t = 0; t < R - 1; ++t) {       // quantised values and scales are pushed on their own
+  if (threadIdx.x == 0) {
+    for (int t = 0; t < R - 1; ++t) {
       const bool used = t < a.num_tensors && !(FP8 && (t == 0 || t == 3));
       r.set(t, a.src[t], c.heap_local + a.dst_off[t], a.dst_par_stride[t], used ? (long long)n * a.row_bytes[t] : 0);
     }
     r.set(R - 1, c.heap_local + a.rsv_off, reinterpret_cast<uint8_t*>(a.out), 0, (long long)n * a.rsv_row_bytes);
   }
   __syncthreads();
-  const long long start = (long long)blockIdx.x * blockDim.x + tid, stride = (long long)nact * blockDim.x;
-  const long long total = r.end[R - 1];
+}
+
+// Layers that fill `nact` blocks, all of these.
+template <bool FP8>
+__device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
+  __shared__ LocalRanges r;
+  local_ranges<FP8>(r, c, a, n);
+  const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)nact * blockDim.x;
+  const long long total = r.end[LocalRanges::R - 1];
   if (a.in_order) {
     for (int l = 0; l < a.num_layers; ++l) {
       const uint32_t par = (layer_base + (uint32_t)l) & 1u;
@@ -392,14 +404,36 @@ __device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStep
   // Few packs: eight of them in flight per thread, and as many of rows to quantise, those of several layers where a layer has
   // fewer.
   const long long rows = FP8 ? (long long)n * (a.fp8_hidden / 8) : 0, most = total > rows ? total : rows;
-  if (most <= stride) { local_few<FP8, 1, 8>(c, a, r, n, start, stride, layer_base); return; }
-  if (most <= stride * 2) { local_few<FP8, 2, 4>(c, a, r, n, start, stride, layer_base); return; }
-  if (most <= stride * 4) { local_few<FP8, 4, 2>(c, a, r, n, start, stride, layer_base); return; }
+  const LocalPart whole{};
+  if (most <= stride) { local_few<FP8, 1, 8>(c, a, r, n, whole, start, stride, layer_base); return; }
+  if (most <= stride * 2) { local_few<FP8, 2, 4>(c, a, r, n, whole, start, stride, layer_base); return; }
+  if (most <= stride * 4) { local_few<FP8, 4, 2>(c, a, r, n, whole, start, stride, layer_base); return; }
   for (int l = 0; l < a.num_layers; ++l) {
     const uint32_t par = (layer_base + (uint32_t)l) & 1u;
     if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
     copy_ranges(r, par, start, stride);
   }
+}
+
+// Layers of which the grid holds several: `parts` runs of layers side by side, `nact` blocks each (a pack per thread).  Nothing that a
+// layer reads is written in the step, and all layers of a parity deliver the same rows, so the runs need no order.  In one block after
+// the other a step was a chain of trips to L2, eight layers each.  One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 rows:
+// 29 -> 6.4 / 35 -> 10.5 / 25 -> 14.6 us, with e4m3 rows 45 -> 8.4 / 53 -> 12.5 / 41 -> 20; 58 layers of one row of 7168 18.7 -> 6.5.  From two
+// layers on that the grid holds no size was faster one after the other.
+template <bool FP8>
+__device__ __forceinline__ int local_parts(const McbDenseStepArgs& a, int n, int nact) {
+  if (a.in_order || nact < 1 || (FP8 && (long long)n * (a.fp8_hidden / 8) > (long long)nact * blockDim.x)) return 1;
+  const int fit = (int)(gridDim.x / (unsigned)nact);
+  return fit < a.num_layers ? fit : a.num_layers;
+}
+template <bool FP8>
+__device__ __forceinline__ void local_layers_apart(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, int parts, uint32_t layer_base) {
+  __shared__ LocalRanges r;
+  const unsigned p = blockIdx.x / (unsigned)nact, L = (unsigned)a.num_layers;
+  if (p >= (unsigned)parts) return;
+  local_ranges<FP8>(r, c, a, n);
+  const LocalPart part{(int)(blockIdx.x - p * nact), (int)(L * p / parts), (int)(L * (p + 1) / parts)};
+  local_few<FP8, 1, 8, true>(c, a, r, n, part, (long long)part.block * blockDim.x + threadIdx.x, (long long)nact * blockDim.x, layer_base);
 }
 
 template <bool EMU, bool CHECK, bool FP8>
@@ -601,7 +635,9 @@ __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant_
   for (int t = 0; t < MCB_MAX_TENSORS; ++t)
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
   const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
-  if ((int)blockIdx.x < nact) local_layers<FP8>(c, a, n, nact, layer_base);
+  const int parts = local_parts<FP8>(a, n, nact);
+  if ((int)blockIdx.x < nact && parts < 2) local_layers<FP8>(c, a, n, nact, layer_base);
+  if (parts > 1) local_layers_apart<FP8>(c, a, n, nact, parts, layer_base);      // this order of the two spills less
   step_close(a.state, step_seq, layer_base + (uint32_t)L);
 }
 

@@ -98,21 +98,21 @@ struct LocalRanges {
     off = (i - (t ? end[t - 1] : 0)) * 16;
     return t;
   }
-  // The words behind the last whole pack of a range: one thread each (`tid` of those that copy), in block 0.
-  __device__ __forceinline__ bool word_of(int tid, int& t, long long& off) const {
+  // The words behind the last whole pack of a range: one thread each (`tid` of those that copy), in the first block of those that copy.
+  __device__ __forceinline__ bool word_of(int tid, int block, int& t, long long& off) const {
     t = tid >> 2;
     const int w = tid & 3;
-    if (blockIdx.x != 0 || t >= R || w >= words[t]) return false;
+    if (block != 0 || t >= R || w >= words[t]) return false;
     off = (end[t] - (t ? end[t - 1] : 0)) * 16 + w * 4;
     return true;
   }
-  __device__ __forceinline__ uint32_t load_word(int tid = threadIdx.x) const {
+  __device__ __forceinline__ uint32_t load_word(int tid = threadIdx.x, int block = blockIdx.x) const {
     int t; long long off;
-    return word_of(tid, t, off) ? ld_b32(src[t] + off) : 0u;
+    return word_of(tid, block, t, off) ? ld_b32(src[t] + off) : 0u;
   }
-  __device__ __forceinline__ void store_word(uint32_t parity, uint32_t v, int tid = threadIdx.x) const {
+  __device__ __forceinline__ void store_word(uint32_t parity, uint32_t v, int tid = threadIdx.x, int block = blockIdx.x) const {
     int t; long long off;
-    if (word_of(tid, t, off)) st_b32(dst[t] + (parity ? par[t] : 0) + off, v);
+    if (word_of(tid, block, t, off)) st_b32(dst[t] + (parity ? par[t] : 0) + off, v);
   }
 };
 

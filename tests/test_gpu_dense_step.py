@@ -330,3 +330,44 @@ def test_world_of_one_quantised_layers_in_flight(lib, n, layers, out_cols):
             assert torch.equal(gh.tensor[p, :n].cpu(), q.view(torch.uint8)) and torch.equal(gs.tensor[p, :n].cpu(), scale)
             assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
         assert not gh.tensor[:, n:].any() and not gs.tensor[:, n:].any()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("n,layers,grid,threads", [
+    (1, 88, 148, 512),           # a layer per block
+    (1, 3, 148, 512),            # more blocks than layers
+    (5, 17, 7, 96),              # two or more runs of unequal length, one of them longer than the layers in flight
+    (5, 9, 2, 160),              # the grid holds one layer and a rest
+    (4, 0, 148, 512),
+])
+def test_world_of_one_layers_side_by_side(lib, fp8, n, layers, grid, threads):
+    """Steps whose layers leave blocks over: runs of them go side by side.  What the last two layers deliver, and nothing besides."""
+    from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    cap, H, K = 8, 256, 3
+    g = torch.Generator(device=DEV).manual_seed(n + layers)
+    heap = SymmetricHeap(None, 1 << 20, DEV)
+    x = torch.randn(cap, H, device=DEV, generator=g).to(torch.bfloat16)
+    ids, w = torch.randint(0, 64, (cap, K), device=DEV, generator=g), torch.rand(cap, K, device=DEV, generator=g)
+    gh, gs = heap.alloc("gh", [2, cap, H], torch.uint8 if fp8 else torch.bfloat16), heap.alloc("gs", [2, cap, H // 128], torch.float32)
+    gi, gw = heap.alloc("gi", [2, cap, K], torch.int64), heap.alloc("gw", [2, cap, K], torch.float32)
+    rsv = heap.alloc("rsv", [cap, H], torch.bfloat16)
+    rsv.tensor.normal_()
+    out, meta = torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+    plan = DenseStepPlan(heap, [gh, gi, gw] + [gs] * fp8, [x, ids, w] + [None] * fp8, out, rsv, torch.tensor([n], dtype=torch.int32, device=DEV),
+                         meta, cap, layers, grid=grid, threads=threads, fp8_hidden=H if fp8 else 0)
+    q, scale = oracle.quant_e4m3_1x128(x[:n].float().cpu())
+    for step in range(3):
+        for t in (gh, gs, gi, gw):
+            t.tensor.zero_()
+        plan.launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        par = int(meta[5])
+        assert not layers or par == (step * layers + layers - 1) % 2
+        assert torch.equal(out[:n], rsv.tensor[:n] if layers else torch.zeros_like(out[:n])) and not out[n:].any()
+        for p in (0, 1):
+            there = p in [(par + l) % 2 for l in range(min(layers, 2))]
+            want = [(q.view(torch.uint8) if fp8 else x[:n]).to(DEV), ids[:n], w[:n]] + [scale.to(DEV)] * fp8
+            for t, v in zip((gh, gi, gw, gs), want):
+                assert torch.equal(t.tensor[p, :n], v if there else torch.zeros_like(v)) and not t.tensor[p, n:].any()
