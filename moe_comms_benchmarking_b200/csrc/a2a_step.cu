@@ -532,8 +532,10 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
 // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.  The identity expert on
 // bf16 rows returns the row just delivered, which is still in registers.  PL = packs per lane; a lane holds one expert id (topk at most 32, others take
 // barrier_alone).
-template <bool FP8, int PL>
+enum AloneWork { kAloneBoth, kAloneDispatch, kAloneCombine };
+template <bool FP8, int PL, AloneWork WORK = kAloneBoth>
 struct AloneSlice {
+  static constexpr bool kSends = WORK != kAloneCombine, kSums = WORK != kAloneDispatch;
   const McbA2AStepArgs& a;
   const int lane, row_packs;
   const bool echo, has_id;
@@ -562,22 +564,40 @@ struct AloneSlice {
     ids = a.topk_idx + (int64_t)t * a.topk + lane;
     ws = a.topk_w ? a.topk_w + (int64_t)t * a.topk + lane : nullptr;
   }
+  __device__ __forceinline__ void load_meta(bool on, long long& id, float& wt) const {
+    id = on && has_id ? *reinterpret_cast<const volatile int64_t*>(ids) : 0;
+    wt = on && head && has_id ? (ws ? *reinterpret_cast<const volatile float*>(ws) : 1.0f) : 0.0f;
+  }
+  // Whether the row goes anywhere.
+  __device__ __forceinline__ bool sends(const McbCtx& c, long long id) const {
+    const bool good = has_id && id >= 0 && id < a.num_experts;
+    if (has_id && !good) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)t, (uint32_t)id);
+    return __any_sync(0xffffffffu, good);
+  }
+  // Chunk j of the metadata row, as in meta_chunk, from the lanes that hold its ids and weights.
+  __device__ __forceinline__ void deliver_meta(uint64_t par, uint32_t stamp, long long id, float wt) const {
+    const int k0 = lane == 0 ? 0 : 2 * lane - 1, k1 = 2 * lane;
+    const uint32_t my_id = has_id ? (uint32_t)id : 0xffffffffu, my_w = __float_as_uint(wt);
+    const uint32_t id0 = __shfl_sync(0xffffffffu, my_id, k0), w0 = __shfl_sync(0xffffffffu, my_w, k0);
+    const uint32_t id1 = __shfl_sync(0xffffffffu, my_id, k1), w1 = __shfl_sync(0xffffffffu, my_w, k1);
+    const bool have0 = k0 < a.topk, have1 = k1 < a.topk;
+    uint4 m = make_uint4(have0 ? id0 : 0xffffffffu, have0 ? w0 : 0u, have1 ? id1 : 0xffffffffu, have1 ? w1 : 0u);
+    if (lane == 0) m = make_uint4(stamp, (uint32_t)t, id0, w0);
+    if (lane < (int)(a.meta_row_bytes >> 4)) st_v4(meta + par * a.meta_par_stride, m);
+  }
   __device__ __forceinline__ void load(bool on, uint64_t par, uint4 (&v)[PL], uint4 (&w)[PL], long long& id, float& wt) const {
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
       const bool live = on && p0 + u * 32 < row_packs;
-      v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
-      if (!echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
+      if (kSends || echo) v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
+      if (kSums && !echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
     }
-    id = on && has_id ? *reinterpret_cast<const volatile int64_t*>(ids) : 0;
-    wt = on && head && has_id ? (ws ? *reinterpret_cast<const volatile float*>(ws) : 1.0f) : 0.0f;
+    load_meta(on, id, wt);
   }
   __device__ __forceinline__ void deliver(const McbCtx& c, uint64_t par, uint32_t stamp, const uint4 (&v)[PL], const uint4 (&w)[PL], long long id,
                                           float wt) const {
-    const bool good = has_id && id >= 0 && id < a.num_experts;
-    if (has_id && !good) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)t, (uint32_t)id);
-    const bool sent = __any_sync(0xffffffffu, good);
-    if (sent) {
+    const bool sent = sends(c, id);
+    if (kSends && sent) {
       uint8_t* dst = recv + par * a.x_par_stride;
       if (FP8) {
         float scale[PL + 1];
@@ -596,18 +616,10 @@ struct AloneSlice {
         for (int u = 0; u < PL; ++u)
           if (p0 + u * 32 < row_packs) st_v4(dst + u * 512, v[u]);
       }
-      if (head) {            // chunk j of the metadata row, as in meta_chunk, from the lanes that hold its ids and weights
-        const int k0 = lane == 0 ? 0 : 2 * lane - 1, k1 = 2 * lane;
-        const uint32_t my_id = has_id ? (uint32_t)id : 0xffffffffu, my_w = __float_as_uint(wt);
-        const uint32_t id0 = __shfl_sync(0xffffffffu, my_id, k0), w0 = __shfl_sync(0xffffffffu, my_w, k0);
-        const uint32_t id1 = __shfl_sync(0xffffffffu, my_id, k1), w1 = __shfl_sync(0xffffffffu, my_w, k1);
-        const bool have0 = k0 < a.topk, have1 = k1 < a.topk;
-        uint4 m = make_uint4(have0 ? id0 : 0xffffffffu, have0 ? w0 : 0u, have1 ? id1 : 0xffffffffu, have1 ? w1 : 0u);
-        if (lane == 0) m = make_uint4(stamp, (uint32_t)t, id0, w0);
-        if (lane < (int)(a.meta_row_bytes >> 4)) st_v4(meta + par * a.meta_par_stride, m);
-      }
+      if (head) deliver_meta(par, stamp, id, wt);
     }
     // the sum over one destination's row
+    if (!kSums) return;
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
       if (p0 + u * 32 >= row_packs) continue;
@@ -615,6 +627,22 @@ struct AloneSlice {
       if (sent) acc_bf16x8(acc, echo ? v[u] : w[u]);
       st_v4(out + u * 512, make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
                                       pack_bf16x2(acc[6], acc[7])));
+    }
+  }
+  // Layers [first, last) of the slice, the loads of D of them in flight together.
+  template <int D>
+  __device__ __forceinline__ void layers(const McbCtx& c, int first, int last, uint32_t layer_base) const {
+    for (int l0 = first; l0 < last; l0 += D) {
+      uint4 v[D][PL], w[D][PL];
+      long long id[D];
+      float wt[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) load(l0 + d < last, (layer_base + (uint32_t)(l0 + d)) & 1u, v[d], w[d], id[d], wt[d]);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        if (l0 + d >= last) break;
+        deliver(c, (layer_base + (uint32_t)(l0 + d)) & 1u, layer_base + (uint32_t)(l0 + d) + 1u, v[d], w[d], id[d], wt[d]);
+      }
     }
   }
 };
@@ -627,16 +655,59 @@ __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs&
   const int item = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;      // the smallest steps spread over the chip
   if (item >= n * s.slices()) return;
   s.at(c, item);
+  s.template layers<D>(c, 0, a.num_layers, layer_base);
+}
+
+// The same for so few slices that the warps of the chip hold those of several layers: `parts` runs of layers side by side, which leave
+// the same rows behind in any order.  What a layer does leave behind of its own goes layer after layer: the metadata rows, which
+// carry the number of their layer, by a further warp each, and the sums over expert outputs, which alternate between two buffers, by
+// a further warp per slice.  One B200, against one warp per slice for all layers, 88 layers of 1 / 37 / 200 rows of 1024 values:
+// bf16 33 -> 16 / 35 -> 19 / 37 -> 27 us, e4m3 with 1 / 37 / 100 rows 43 -> 17 / 45 -> 20 / 45 -> 25; 58 layers of one row of 7168
+// 25 -> 12.5 and 31 -> 12.5.  What is left is the chain of the metadata rows (four trips to L2 for 88 layers) or of the sums (eight).
+template <bool FP8>
+__device__ __forceinline__ void alone_apart(const McbCtx& c, const McbA2AStepArgs& a, int n, bool echo, int parts, uint32_t layer_base) {
+  AloneSlice<FP8, 1> s(a);
+  const unsigned L = (unsigned)a.num_layers, items = (unsigned)(n * s.slices());
+  unsigned at = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;
+  const unsigned p = at / items;
+  if (p < (unsigned)parts) {
+    const int first = (int)(L * p / parts), last = (int)(L * (p + 1) / parts);
+    if (echo) {
+      s.at(c, at - p * items);
+      s.head = false;
+      s.template layers<8>(c, first, last, layer_base);
+    } else {
+      AloneSlice<FP8, 1, kAloneDispatch> d(a);
+      d.at(c, at - p * items);
+      d.head = false;
+      d.template layers<8>(c, first, last, layer_base);
+    }
+    return;
+  }
+  at -= parts * items;
+  if (!echo) {
+    if (at < items) {
+      AloneSlice<FP8, 1, kAloneCombine> d(a);
+      d.at(c, at);
+      d.head = false;
+      d.template layers<12>(c, 0, a.num_layers, layer_base);
+      return;
+    }
+    at -= items;
+  }
+  if (at >= (unsigned)n) return;
+  constexpr int D = 22;
+  s.at(c, (long long)at * s.slices());
   for (int l0 = 0; l0 < a.num_layers; l0 += D) {
-    uint4 v[D][PL], w[D][PL];
     long long id[D];
     float wt[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) s.load(l0 + d < a.num_layers, (layer_base + (uint32_t)(l0 + d)) & 1u, v[d], w[d], id[d], wt[d]);
+    for (int d = 0; d < D; ++d) s.load_meta(l0 + d < a.num_layers, id[d], wt[d]);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
       if (l0 + d >= a.num_layers) break;
-      s.deliver(c, (layer_base + (uint32_t)(l0 + d)) & 1u, layer_base + (uint32_t)(l0 + d) + 1u, v[d], w[d], id[d], wt[d]);
+      const uint32_t l = layer_base + (uint32_t)(l0 + d);
+      if (s.sends(c, id[d])) s.deliver_meta(l & 1u, l + 1u, id[d], wt[d]);
     }
   }
 }
@@ -665,6 +736,12 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
 template <bool FP8>
 __device__ __forceinline__ void alone_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
+  if (a.apart && n > 0) {
+    const bool echo = !FP8 && a.y_off == a.recv_x_off;
+    const long long items = n * ((packs + 31) / 32), fit = (warps - n) / items - !echo;
+    const int parts = (int)(fit < a.num_layers ? fit : a.num_layers);
+    if (parts > 1) { alone_apart<FP8>(c, a, n, echo, parts, layer_base); return; }
+  }
   auto fits = [&](int pl) { return a.apart && (long long)n * ((packs + 32 * pl - 1) / (32 * pl)) <= warps; };
   if (fits(1)) alone_few<FP8, 1, 8>(c, a, n, layer_base);
   else if (fits(2)) alone_few<FP8, 2, 4>(c, a, n, layer_base);

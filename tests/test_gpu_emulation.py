@@ -326,6 +326,8 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
     (2048, 8, 5, 2, 10, 64),             # as many slices as warps
     (2048, 8, 6, 4, 5, 64),              # more slices than warps
     (7168, 33, 3, 4, 148, 512),          # more ids than lanes
+    (1152, 5, 3, 9, 6, 256),             # 48 warps, 15 slices: two or three runs of the layers side by side
+    (256, 2, 2, 33, 8, 64),              # six or seven runs, and more layers than one warp has in flight
 ])
 def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads):
     """A step in a world of one whose layers run into each other, against the kernel of the emulated ranks, which takes
