@@ -24,7 +24,7 @@
 //     popular expert's chunks spread over the chip;
 //   * both projections run in one persistent stream.  While the activations of all experts fit in L2 the gate/up
 //     units of every expert come first, then the down units; above that a down unit follows its gate/up
-//     units at a distance of three rounds of the grid, while its activations are still in L2.  A down
+//     units at a distance of several rounds of the grid (ffn_plan), while its activations are still in L2.  A down
 //     unit waits for a counter of its expert's finished gate/up units; units are taken in list order, so the
 //     wait cannot deadlock;
 //   * the gate/up matrix is stored interleaved (row 2i = gate row i, row 2i + 1 = up row i): the two values
@@ -219,8 +219,12 @@ __device__ __forceinline__ int ffn_token_tile(int max_rows) {
 __device__ __forceinline__ void ffn_plan(FfnPlanS& plan, const McbFfnArgs& a, int active) {
   plan.n1 = 2 * a.intermediate / kFfnRowsM; plan.n2 = a.hidden / kFfnRowsM;
   plan.active = plan.lag = active;
-  if ((long long)plan.off[a.num_local_experts] * a.intermediate * 2 > kFfnActL2Bytes) {      // three rounds of the grid, in slots of average size
-    const int lag = (int)((long long)gridDim.x * 3 / 2 * active / plan.total()) + 2;
+  if ((long long)plan.off[a.num_local_experts] * a.intermediate * 2 > kFfnActL2Bytes) {
+    // So many slots, of average size, that their down units alone make two rounds of the grid: that is how far the last slot's are from
+    // its gate/up units.  With three rounds of all units (one of down units) they waited there: 8191 tokens with Zipf routing, an
+    // eighth of 512 experts, 129.6 -> 127.2 us (three rounds of down units 126.5, all gate/up units first 126.9); 4096 tokens of all
+    // experts the same (three rounds of down units 0.3 % slower).
+    const int lag = (int)((long long)gridDim.x * active / (plan.n2 * plan.cum[active])) + 2;
     if (lag < plan.lag) plan.lag = lag;
   }
 }
