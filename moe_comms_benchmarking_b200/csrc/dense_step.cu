@@ -285,92 +285,6 @@ __device__ __forceinline__ void fp8_push(const McbCtx& c, const McbDenseStepArgs
 }
 
 // ---- a world of one: the layers of a step are local copies ------------------------------------------------------
-// The part of a step that a block has a share in: layers [first, last), as block `block` of those that a layer fills.
-struct LocalPart {
-  int block, first, last;
-};
-
-// Up to S packs per thread and layer: where they come from and go to is worked out once for all layers.  Nothing that a
-// layer reads is written in the step (else: a.in_order), so the loads of D layers go out together and are stored layer
-// by layer; the layers of such a step run into each other.  With one layer at a time each layer was a trip to L2: 88 layers
-// of hidden 1024 and top-22, one B200: 57 -> 37 us with one
-// token, 47 -> 34 with 200, 62 -> 55 with 333, where the second pack per thread begins; with e4m3 rows, whose packs go along, 100 -> 52, 109 ->
-// 47 (100 tokens) and 115 -> 59.
-template <bool FP8, int S, int D, bool PARTS = false>
-__device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, const LocalPart& part,
-                                          long long start, long long stride, uint32_t layer_base) {
-  const int last = PARTS ? part.last : a.num_layers, block = PARTS ? part.block : (int)blockIdx.x;
-  // e4m3: packs of bf16 rows, and where their values and their block's scale go
-  const int H = (int)a.fp8_hidden, ppr = FP8 ? H / 8 : 1, nblk = H / 128;
-  const uint8_t* rows = reinterpret_cast<const uint8_t*>(a.src[0]);
-  uint8_t *q_dst[S], *s_dst[S];
-  bool quant[S];
-#pragma unroll
-  for (int u = 0; u < S; ++u) {
-    const long long i = start + u * stride;
-    quant[u] = FP8 && i < (long long)n * ppr;
-    const int row = (int)(i / ppr), pk = (int)(i - (long long)row * ppr);
-    q_dst[u] = c.heap_local + a.dst_off[0] + (uint64_t)row * H + (uint64_t)pk * 8;
-    s_dst[u] = c.heap_local + a.dst_off[3] + ((uint64_t)row * nblk + (pk >> 4)) * 4;
-  }
-
-  const long long total = r.end[LocalRanges::R - 1];
-  const uint8_t* src[S];
-  uint8_t* dst[S];
-  uint64_t par_off[S];
-  bool live[S];
-#pragma unroll
-  for (int u = 0; u < S; ++u) {
-    const long long i = start + u * stride;
-    live[u] = i < total;
-    long long off = 0;
-    const int t = live[u] ? r.find(i, off) : 0;
-    src[u] = r.src[t] + off;
-    dst[u] = r.dst[t] + off;
-    par_off[u] = r.par[t];
-  }
-  for (int l0 = PARTS ? part.first : 0; l0 < last; l0 += D) {
-    uint4 v[D][S], h[D * S];
-    uint32_t w[D];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (FP8) {
-#pragma unroll
-        for (int u = 0; u < S; ++u)
-          h[d * S + u] = quant[u] && l0 + d < last ? ld_v4_stream(rows + (start + u * stride) * 16) : make_uint4(0, 0, 0, 0);
-      }
-      if (l0 + d >= last) continue;
-#pragma unroll
-      for (int u = 0; u < S; ++u)
-        if (live[u]) v[d][u] = ld_v4_stream(src[u]);
-      w[d] = r.load_word(threadIdx.x, block);
-    }
-    float scale[D * S];
-    if (FP8) {
-#pragma unroll
-      for (int k = 0; k < D * S; k += 2) block_absmax_pair(h[k], h[k + 1], scale[k], scale[k + 1]);
-    }
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (l0 + d >= last) break;
-      const uint32_t par = (layer_base + (uint32_t)(l0 + d)) & 1u;
-      if (FP8) {
-#pragma unroll
-        for (int u = 0; u < S; ++u) {
-          if (!quant[u]) continue;
-          const float sc = e4m3_scale(scale[d * S + u]);
-          st_v2(q_dst[u] + (par ? a.dst_par_stride[0] : 0), quant_pack_e4m3(h[d * S + u], sc));
-          if ((threadIdx.x & 15) == 0) st_b32(s_dst[u] + (par ? a.dst_par_stride[3] : 0), __float_as_uint(sc));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < S; ++u)
-        if (live[u]) st_v4(dst[u] + (par ? par_off[u] : 0), v[d][u]);
-      r.store_word(par, w[d], threadIdx.x, block);
-    }
-  }
-}
-
 // What a layer copies; quantised values and scales are pushed on their own.  All threads of the block.
 template <bool FP8>
 __device__ __forceinline__ void local_ranges(LocalRanges& r, const McbCtx& c, const McbDenseStepArgs& a, int n) {
@@ -385,55 +299,124 @@ __device__ __forceinline__ void local_ranges(LocalRanges& r, const McbCtx& c, co
   __syncthreads();
 }
 
-// Layers that fill `nact` blocks, all of these.
+// Layers [first, last) of one pack per lane, the loads of eight of them in flight together.
+template <class Load, class Store>
+__device__ __forceinline__ void local_layers_of(int first, int last, Load load, Store store) {
+  constexpr int D = 8;
+  for (int l0 = first; l0 < last; l0 += D) {
+    uint4 v[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) v[d] = l0 + d < last ? load() : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int d = 0; d < D; d += 2) store(v[d], v[d + 1], l0 + d < last, l0 + d + 1 < last, l0 + d);
+  }
+}
+
+// Nothing that a layer reads is written in the step (else: a.in_order), and all layers of a parity deliver the same rows, so the layers
+// need no order.  Bound by L2: a warp takes all layers of a few packs, so that the chip works on a few MB at a time, and every warp gets
+// the same number of packs whatever the batch.  Layer after layer over all rows, large steps went through up to 90 MB of L2 in every
+// layer, small ones left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
+// One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against layers one after the other:
+//   bf16   29 -> 6.4 / 35 -> 8.5 / 25 -> 12.6 / 49 -> 33 / 41 -> 34 / 169 -> 112 / 655 -> 411 us (15 TB/s read and written)
+//   e4m3   45 -> 8.5 / 53 -> 10.5 / 41 -> 14.5 / 52 -> 33 / 41 -> 37 / 154 -> 121 / 923 -> 451 us
+// and 58 layers of hidden 7168 and top-8, 1 / 64 / 512 / 2048 rows, bf16 19 -> 6.5 / 29 -> 21 / 178 -> 116 / 961 -> 425, e4m3 with 512 / 2048
+// rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.
+template <bool FP8>
+__device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, uint32_t layer_base) {
+  const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
+  const int warp = (int)(blockIdx.x + (threadIdx.x >> 5) * gridDim.x);         // the smallest steps spread over the chip
+  const long long packs = r.end[LocalRanges::R - 1], groups = (packs + 31) >> 5;
+  auto quantise = [&] {
+    // Two packs (16 values) per lane, so eight lanes hold a block of 128 values and a lane stores 16 bytes: 13 to 18 % faster than one.
+    const int H = (int)a.fp8_hidden, ppr = H / 16, nblk = H / 128;
+    const long long total = (long long)n * ppr;                // a multiple of 8
+    local_share((total + 31) >> 5, a.num_layers, warp, warps, [&](long long g, int first, int last) {
+      const long long i = g * 32 + lane;
+      const bool live = i < total;
+      const int row = (int)(i / ppr), pk = (int)(i - (long long)row * ppr);
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src[0]) + i * 32;
+      uint8_t* q_dst = c.heap_local + a.dst_off[0] + (uint64_t)row * H + (uint64_t)pk * 16;
+      uint8_t* s_dst = c.heap_local + a.dst_off[3] + ((uint64_t)row * nblk + (pk >> 3)) * 4;
+      constexpr int D = 4;
+      for (int l0 = first; l0 < last; l0 += D) {
+        uint4 v[D][2];
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int d = 0; d < D; d += 2) {
+          const uint32_t m0 = max_bf16x2(pack_absmax2(v[d][0]), pack_absmax2(v[d][1])), m1 = max_bf16x2(pack_absmax2(v[d + 1][0]), pack_absmax2(v[d + 1][1]));
+          uint32_t m = max_bf16x2(__byte_perm(m0, m1, 0x5410), __byte_perm(m0, m1, 0x7632));
+#pragma unroll
+          for (int sh = 4; sh >= 1; sh >>= 1) m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, sh));
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            if (!live || l0 + d + k >= last) continue;
+            const uint32_t par = (layer_base + (uint32_t)(l0 + d + k)) & 1u;
+            const float sc = e4m3_scale(k ? bf16_hi(m) : bf16_lo(m));
+            const uint2 q0 = quant_pack_e4m3(v[d + k][0], sc), q1 = quant_pack_e4m3(v[d + k][1], sc);
+            st_v4(q_dst + (par ? a.dst_par_stride[0] : 0), make_uint4(q0.x, q0.y, q1.x, q1.y));
+            if ((lane & 7) == 0) st_b32(s_dst + (par ? a.dst_par_stride[3] : 0), __float_as_uint(sc));
+          }
+        }
+      }
+    });
+  };
+  auto copy = [&] {
+    const int from = FP8 ? (warp + warps / 2) % warps : warp;       // small steps: not the warps that quantise
+    // The group behind the last one: the words behind the last whole pack of each range.
+    local_share(groups + 1, a.num_layers, from, warps, [&](long long g, int first, int last) {
+      if (g == groups) {
+        for (int l0 = first; l0 < last; l0 += 8) {
+          uint32_t w[8];
+#pragma unroll
+          for (int d = 0; d < 8; ++d) w[d] = l0 + d < last ? r.load_word(lane, 0) : 0u;
+#pragma unroll
+          for (int d = 0; d < 8; ++d)
+            if (l0 + d < last) r.store_word((layer_base + (uint32_t)(l0 + d)) & 1u, w[d], lane, 0);
+        }
+        return;
+      }
+      const long long i = g * 32 + lane;
+      const bool live = i < packs;
+      long long off = 0;
+      const int t = live ? r.find(i, off) : 0;
+      const uint8_t* src = r.src[t] + off;
+      uint8_t* dst = r.dst[t] + off;
+      const uint64_t par_off = r.par[t];
+      local_layers_of(first, last, [&] { return live ? ld_v4_stream(src) : make_uint4(0, 0, 0, 0); },
+                      [&](uint4 v0, uint4 v1, bool on0, bool on1, int l) {
+        const uint32_t par = (layer_base + (uint32_t)l) & 1u;
+        if (live && on0) st_v4(dst + (par ? par_off : 0), v0);
+        if (live && on1) st_v4(dst + (par ? 0 : par_off), v1);
+      });
+    });
+  };
+  if (!FP8) { copy(); return; }
+  // Half of the warps of an SM quantise while the others copy: 5 to 10 % faster than all of them in step.
+  const int odd = (int)(threadIdx.x >> 5) & 1;
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    if (k == odd) quantise();
+    else copy();
+  }
+}
+
+// `nact`: blocks that a layer fills, if the layers keep their order.
 template <bool FP8>
 __device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
+  if (n <= 0) return;
   __shared__ LocalRanges r;
   local_ranges<FP8>(r, c, a, n);
+  if (!a.in_order) { local_dealt<FP8>(c, a, r, n, layer_base); return; }
+  if ((int)blockIdx.x >= nact) return;
   const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)nact * blockDim.x;
-  const long long total = r.end[LocalRanges::R - 1];
-  if (a.in_order) {
-    for (int l = 0; l < a.num_layers; ++l) {
-      const uint32_t par = (layer_base + (uint32_t)l) & 1u;
-      if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
-      copy_ranges_in_order(r, par, start, stride);
-    }
-    return;
-  }
-
-  // Few packs: eight of them in flight per thread, and as many of rows to quantise, those of several layers where a layer has
-  // fewer.
-  const long long rows = FP8 ? (long long)n * (a.fp8_hidden / 8) : 0, most = total > rows ? total : rows;
-  const LocalPart whole{};
-  if (most <= stride) { local_few<FP8, 1, 8>(c, a, r, n, whole, start, stride, layer_base); return; }
-  if (most <= stride * 2) { local_few<FP8, 2, 4>(c, a, r, n, whole, start, stride, layer_base); return; }
-  if (most <= stride * 4) { local_few<FP8, 4, 2>(c, a, r, n, whole, start, stride, layer_base); return; }
   for (int l = 0; l < a.num_layers; ++l) {
     const uint32_t par = (layer_base + (uint32_t)l) & 1u;
     if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
-    copy_ranges(r, par, start, stride);
+    copy_ranges_in_order(r, par, start, stride);
   }
-}
-
-// Layers of which the grid holds several: `parts` runs of layers side by side, `nact` blocks each (a pack per thread).  Nothing that a
-// layer reads is written in the step, and all layers of a parity deliver the same rows, so the runs need no order.  In one block after
-// the other a step was a chain of trips to L2, eight layers each.  One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 rows:
-// 29 -> 6.4 / 35 -> 10.5 / 25 -> 14.6 us, with e4m3 rows 45 -> 8.4 / 53 -> 12.5 / 41 -> 20; 58 layers of one row of 7168 18.7 -> 6.5.  From two
-// layers on that the grid holds no size was faster one after the other.
-template <bool FP8>
-__device__ __forceinline__ int local_parts(const McbDenseStepArgs& a, int n, int nact) {
-  if (a.in_order || nact < 1 || (FP8 && (long long)n * (a.fp8_hidden / 8) > (long long)nact * blockDim.x)) return 1;
-  const int fit = (int)(gridDim.x / (unsigned)nact);
-  return fit < a.num_layers ? fit : a.num_layers;
-}
-template <bool FP8>
-__device__ __forceinline__ void local_layers_apart(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, int parts, uint32_t layer_base) {
-  __shared__ LocalRanges r;
-  const unsigned p = blockIdx.x / (unsigned)nact, L = (unsigned)a.num_layers;
-  if (p >= (unsigned)parts) return;
-  local_ranges<FP8>(r, c, a, n);
-  const LocalPart part{(int)(blockIdx.x - p * nact), (int)(L * p / parts), (int)(L * (p + 1) / parts)};
-  local_few<FP8, 1, 8, true>(c, a, r, n, part, (long long)part.block * blockDim.x + threadIdx.x, (long long)nact * blockDim.x, layer_base);
 }
 
 template <bool EMU, bool CHECK, bool FP8>
@@ -520,7 +503,7 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
     }
   } else if (EMU && W == 1 && !CHECK) {      // else dense_alone_kernel
     const int nloc = active_blocks((int)gridDim.x, n, bytes_per_row + a.rsv_row_bytes, (int)blockDim.x);
-    if (bid < nloc) local_layers<FP8>(c, a, n, nloc, layer_base);
+    local_layers<FP8>(c, a, n, nloc, layer_base);
   } else if (grp >= 0 && lb < nact) {
     // ---- barrier mode ----------------------------------------------------------------------------
     uint32_t ep = *epoch_ptr(c, MCB_SITE_STEP, bid);
@@ -608,10 +591,7 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
 }
 
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
-// through pointers after every store.  One B200, 88 layers of hidden 1024 and top-22, against the same code called by the step
-// kernel: e4m3 1 / 333 / 8192 rows 134 -> 100 / 152 -> 115 / 1215 -> 1014 us, 58 layers of 333 rows of 7168 200 -> 148 (52, 59 and 111 with
-// several layers in flight); bf16 1 / 100 rows 40 -> 34 / 34 -> 30, 48 layers of 9 rows of 2048 25 -> 20; the largest bf16 steps are
-// bound by L2 either way (702 -> 700).
+// through pointers after every store.
 template <bool FP8>
 __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
   __shared__ int s_prefix[2], s_cnt[1], s_max;
@@ -635,9 +615,7 @@ __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant_
   for (int t = 0; t < MCB_MAX_TENSORS; ++t)
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
   const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
-  const int parts = local_parts<FP8>(a, n, nact);
-  if ((int)blockIdx.x < nact && parts < 2) local_layers<FP8>(c, a, n, nact, layer_base);
-  if (parts > 1) local_layers_apart<FP8>(c, a, n, nact, parts, layer_base);      // this order of the two spills less
+  local_layers<FP8>(c, a, n, nact, layer_base);
   step_close(a.state, step_seq, layer_base + (uint32_t)L);
 }
 

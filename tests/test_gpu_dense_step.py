@@ -334,14 +334,16 @@ def test_world_of_one_quantised_layers_in_flight(lib, n, layers, out_cols):
 
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("n,layers,grid,threads", [
-    (1, 88, 148, 512),           # a layer per block
-    (1, 3, 148, 512),            # more blocks than layers
-    (5, 17, 7, 96),              # two or more runs of unequal length, one of them longer than the layers in flight
-    (5, 9, 2, 160),              # the grid holds one layer and a rest
+    (1, 88, 148, 512),           # more warps than groups of packs times layers
+    (1, 3, 148, 512),
+    (5, 17, 7, 96),              # runs that begin and end inside a group's layers
+    (5, 9, 2, 160),
+    (7, 19, 1, 32),              # all by one warp
     (4, 0, 148, 512),
 ])
-def test_world_of_one_layers_side_by_side(lib, fp8, n, layers, grid, threads):
-    """Steps whose layers leave blocks over: runs of them go side by side.  What the last two layers deliver, and nothing besides."""
+def test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads):
+    """The layers of a step, dealt to the warps in runs of a group of packs after the other.  What the last two layers deliver, and
+    nothing besides."""
     from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
     from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
     cap, H, K = 8, 256, 3
