@@ -532,10 +532,8 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
 // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.  The identity expert on
 // bf16 rows returns the row just delivered, which is still in registers.  PL = packs per lane; a lane holds one expert id (topk at most 32, others take
 // barrier_alone).
-enum AloneWork { kAloneBoth, kAloneDispatch, kAloneCombine };
-template <bool FP8, int PL, AloneWork WORK = kAloneBoth>
+template <bool FP8, int PL>
 struct AloneSlice {
-  static constexpr bool kSends = WORK != kAloneCombine, kSums = WORK != kAloneDispatch;
   const McbA2AStepArgs& a;
   const int lane, row_packs;
   const bool echo, has_id;
@@ -564,9 +562,9 @@ struct AloneSlice {
     ids = a.topk_idx + (int64_t)t * a.topk + lane;
     ws = a.topk_w ? a.topk_w + (int64_t)t * a.topk + lane : nullptr;
   }
-  __device__ __forceinline__ void load_meta(bool on, long long& id, float& wt) const {
-    id = on && has_id ? *reinterpret_cast<const volatile int64_t*>(ids) : 0;
-    wt = on && head && has_id ? (ws ? *reinterpret_cast<const volatile float*>(ws) : 1.0f) : 0.0f;
+  __device__ __forceinline__ long long load_id(bool on) const { return on && has_id ? *reinterpret_cast<const volatile int64_t*>(ids) : 0; }
+  __device__ __forceinline__ float load_weight(bool on) const {
+    return on && has_id ? (ws ? *reinterpret_cast<const volatile float*>(ws) : 1.0f) : 0.0f;
   }
   // Whether the row goes anywhere.
   __device__ __forceinline__ bool sends(const McbCtx& c, long long id) const {
@@ -589,15 +587,16 @@ struct AloneSlice {
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
       const bool live = on && p0 + u * 32 < row_packs;
-      if (kSends || echo) v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
-      if (kSums && !echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
+      v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
+      if (!echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
     }
-    load_meta(on, id, wt);
+    id = load_id(on);
+    wt = load_weight(on && head);
   }
   __device__ __forceinline__ void deliver(const McbCtx& c, uint64_t par, uint32_t stamp, const uint4 (&v)[PL], const uint4 (&w)[PL], long long id,
                                           float wt) const {
     const bool sent = sends(c, id);
-    if (kSends && sent) {
+    if (sent) {
       uint8_t* dst = recv + par * a.x_par_stride;
       if (FP8) {
         float scale[PL + 1];
@@ -619,7 +618,6 @@ struct AloneSlice {
       if (head) deliver_meta(par, stamp, id, wt);
     }
     // the sum over one destination's row
-    if (!kSums) return;
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
       if (p0 + u * 32 >= row_packs) continue;
@@ -629,90 +627,137 @@ struct AloneSlice {
                                       pack_bf16x2(acc[6], acc[7])));
     }
   }
-  // Layers [first, last) of the slice, the loads of D of them in flight together.
-  template <int D>
-  __device__ __forceinline__ void layers(const McbCtx& c, int first, int last, uint32_t layer_base) const {
-    for (int l0 = first; l0 < last; l0 += D) {
-      uint4 v[D][PL], w[D][PL];
-      long long id[D];
-      float wt[D];
-#pragma unroll
-      for (int d = 0; d < D; ++d) load(l0 + d < last, (layer_base + (uint32_t)(l0 + d)) & 1u, v[d], w[d], id[d], wt[d]);
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        if (l0 + d >= last) break;
-        deliver(c, (layer_base + (uint32_t)(l0 + d)) & 1u, layer_base + (uint32_t)(l0 + d) + 1u, v[d], w[d], id[d], wt[d]);
-      }
-    }
-  }
 };
 
-// At most one slice per warp: where it comes from and goes to is worked out once for all layers.  Nothing that a layer reads is
-// written in the step (a.apart), so the loads of D layers go out together and are delivered layer by layer.
-template <bool FP8, int PL, int D>
-__device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
-  AloneSlice<FP8, PL> s(a);
-  const int item = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;      // the smallest steps spread over the chip
-  if (item >= n * s.slices()) return;
-  s.at(c, item);
-  s.template layers<D>(c, 0, a.num_layers, layer_base);
+// The sum over one destination's row, as the fp32 accumulation from zero rounds it: 0 + v, which drops the sign of a zero.  bf16 adds two
+// values exactly where one of them is zero, so it takes one instruction for two values.
+__device__ __forceinline__ uint32_t plus_zero_bf16x2(uint32_t v) {
+  uint32_t r;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+  return r;
+}
+__device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
+  return sent ? make_uint4(plus_zero_bf16x2(v.x), plus_zero_bf16x2(v.y), plus_zero_bf16x2(v.z), plus_zero_bf16x2(v.w)) : make_uint4(0, 0, 0, 0);
 }
 
-// The same for so few slices that the warps of the chip hold those of several layers: `parts` runs of layers side by side, which leave
-// the same rows behind in any order.  What a layer does leave behind of its own goes layer after layer: the metadata rows, which
-// carry the number of their layer, by a further warp each, and the sums over expert outputs, which alternate between two buffers, by
-// a further warp per slice.  One B200, against one warp per slice for all layers, 88 layers of 1 / 37 / 200 rows of 1024 values:
-// bf16 33 -> 16 / 35 -> 19 / 37 -> 27 us, e4m3 with 1 / 37 / 100 rows 43 -> 17 / 45 -> 20 / 45 -> 25; 58 layers of one row of 7168
-// 25 -> 12.5 and 31 -> 12.5.  What is left is the chain of the metadata rows (four trips to L2 for 88 layers) or of the sums (eight).
+// The layers of a step that writes nothing that it reads (a.apart), dealt to the warps; topk at most 32.
+//   pieces   32 packs of a row (64 to quantise, two per lane) and their layers.  All layers of a parity deliver the same rows, so these
+//            need no order: every warp takes a run of (piece, layer), a piece's layers one after the other.
+//   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token, which carries the
+//            number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
+//            expert on bf16 rows returns the row: its sums are the pieces' own.)
+// A warp with one chain more than others takes fewer pieces.  Bound by L2; the chip works on a few MB at a time.  One B200, against
+// layers one after the other, in slices of up to 128 packs a warp:
+//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows
+//     bf16   35 -> 16.7 / 35 -> 18.7 / 41 -> 35 / 77 -> 72 / 271 -> 265 us
+//     e4m3   43 -> 16.6 / 45 -> 16.7 / 56 -> 38 / 91 -> 75 / 404 -> 272 us
+//   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 4096 rows
+//     bf16   25 -> 14.6 / 27 -> 21 / 99 -> 97 / 265 -> 283 / 1690 -> 1088 us
+//     e4m3   31 -> 14.6 / 35 -> 21 / 113 -> 100 / 401 -> 278 / 2211 -> 1120 us
+// The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.
 template <bool FP8>
-__device__ __forceinline__ void alone_apart(const McbCtx& c, const McbA2AStepArgs& a, int n, bool echo, int parts, uint32_t layer_base) {
+__device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  constexpr int K = FP8 ? 2 : 1;             // packs per lane of a piece
+  constexpr int kCost = K + (FP8 ? 0 : 1);   // of a piece, against a layer of a chain
   AloneSlice<FP8, 1> s(a);
-  const unsigned L = (unsigned)a.num_layers, items = (unsigned)(n * s.slices());
-  unsigned at = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;
-  const unsigned p = at / items;
-  if (p < (unsigned)parts) {
-    const int first = (int)(L * p / parts), last = (int)(L * (p + 1) / parts);
-    if (echo) {
-      s.at(c, at - p * items);
-      s.head = false;
-      s.template layers<8>(c, first, last, layer_base);
-    } else {
-      AloneSlice<FP8, 1, kAloneDispatch> d(a);
-      d.at(c, at - p * items);
-      d.head = false;
-      d.template layers<8>(c, first, last, layer_base);
-    }
-    return;
-  }
-  at -= parts * items;
-  if (!echo) {
-    if (at < items) {
-      AloneSlice<FP8, 1, kAloneCombine> d(a);
-      d.at(c, at);
-      d.head = false;
-      d.template layers<12>(c, 0, a.num_layers, layer_base);
-      return;
-    }
-    at -= items;
-  }
-  if (at >= (unsigned)n) return;
-  constexpr int D = 22;
-  s.at(c, (long long)at * s.slices());
-  for (int l0 = 0; l0 < a.num_layers; l0 += D) {
-    long long id[D];
-    float wt[D];
+  const int lane = s.lane, L = a.num_layers, per_row = (s.row_packs + 32 * K - 1) / (32 * K);
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5), warp = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x;
+  const long long sums = s.echo ? 0 : (long long)n * s.slices(), chains = sums + n, items = (long long)n * per_row * L;
+  const uint64_t row_bytes = (uint64_t)a.hidden * 2;
+
+  auto chain = [&] {
+    for (long long k = warp; k < chains; k += warps) {
+      const bool sum = k < sums;
+      s.at(c, sum ? k : (k - sums) * s.slices());
+      if (sum) {
+        constexpr int D = 8;
+        const bool live = s.p0 < s.row_packs, sent = s.sends(c, s.load_id(true));
+        for (int l0 = 0; l0 < L; l0 += D) {
+          uint4 v[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) s.load_meta(l0 + d < a.num_layers, id[d], wt[d]);
+          for (int d = 0; d < D; ++d)
+            v[d] = live && l0 + d < L ? ld_v4_stream(s.y + ((layer_base + (uint32_t)(l0 + d)) & 1u ? a.y_par_stride : 0)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      if (l0 + d >= a.num_layers) break;
-      const uint32_t l = layer_base + (uint32_t)(l0 + d);
-      if (s.sends(c, id[d])) s.deliver_meta(l & 1u, l + 1u, id[d], wt[d]);
+          for (int d = 0; d < D; ++d)
+            if (live && l0 + d < L) st_v4(s.out, alone_sum(sent, v[d]));
+        }
+      } else {
+        constexpr int D = 22;
+        for (int l0 = 0; l0 < L; l0 += D) {
+          long long id[D];
+          float wt[D];
+#pragma unroll
+          for (int d = 0; d < D; ++d) { id[d] = s.load_id(l0 + d < L); wt[d] = s.load_weight(l0 + d < L); }
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            if (l0 + d >= L) break;
+            const uint32_t l = layer_base + (uint32_t)(l0 + d);
+            if (s.sends(c, id[d])) s.deliver_meta(l & 1u, l + 1u, id[d], wt[d]);
+          }
+        }
+      }
     }
+  };
+
+  auto pieces = [&] {
+    const long long extra = chains % warps, level = (kCost * items + chains * L) / warps, most = chains / warps * L + L;
+    long long less = extra && level > most ? (level - most) / kCost : 0;             // items of a warp with a chain more
+    if (extra && less * extra > items) less = 0;
+    const long long rest = items - less * extra, others = warps - extra;
+    auto begin = [&](long long w) { return w < extra ? w * less : less * extra + rest * (w - extra) / others; };
+    local_runs(begin(warp), begin(warp + 1), L, [&](long long piece, int first, int last) {
+      constexpr int D = FP8 ? 2 : 8;
+      s.at(c, (piece / per_row) * s.slices());                                       // its row
+      const int p = (int)(piece % per_row) * 32 * K + lane * K;
+      const bool live = p < s.row_packs;
+      const uint64_t row = (uint64_t)c.rank * a.cap + s.t;
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + s.t * row_bytes + p * 16;
+      uint8_t* out = reinterpret_cast<uint8_t*>(a.out) + s.t * row_bytes + p * 16;
+      uint8_t* recv = c.heap_local + a.recv_x_off + (FP8 ? row * a.hidden + p * 8 : row * row_bytes + p * 16);
+      uint8_t* scales = c.heap_local + a.recv_scale_off + (row * (a.hidden / 128) + (p >> 4)) * 4;
+      const bool sent = s.sends(c, s.load_id(true));                                  // its layers have the same ids
+      for (int l0 = first; l0 < last; l0 += D) {
+        uint4 v[D][K];
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+          for (int k = 0; k < K; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int d = 0; d < D; d += 2) {
+          float m[2];
+          if constexpr (FP8) block_absmax_wide(v[d], v[d + 1], m[0], m[1]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (l0 + d + e >= last) break;
+            const uint32_t par = (layer_base + (uint32_t)(l0 + d + e)) & 1u;
+            const uint4* r = v[d + e];
+            uint8_t* dst = recv + (par ? a.x_par_stride : 0);
+            if constexpr (FP8) {
+              const float scale = e4m3_scale(m[e]);
+              if (sent && live) {
+                const uint2 q0 = quant_pack_e4m3(r[0], scale), q1 = quant_pack_e4m3(r[1], scale);
+                st_v4(dst, make_uint4(q0.x, q0.y, q1.x, q1.y));
+                if ((lane & 7) == 0) st_b32(scales + (par ? a.scale_par_stride : 0), __float_as_uint(scale));
+              }
+            } else {
+              if (sent && live) st_v4(dst, r[0]);
+              if (s.echo && live) st_v4(out, alone_sum(sent, r[0]));
+            }
+          }
+        }
+      }
+    });
+  };
+  // Half of the warps of an SM begin with their chains.
+  const int odd = (int)(threadIdx.x >> 5) & 1;
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    if (k == odd) chain();
+    else pieces();
   }
 }
 
-// Layer after layer.
+// Layer after layer: steps that read what they write.
 template <bool FP8>
 __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   AloneSlice<FP8, 4> s(a);
@@ -728,27 +773,6 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
     }
 }
 
-// As few packs per lane as still give every slice a warp of its own.  One B200, against layers one by one through pointers to the
-// arguments: 88 layers of 9 / 333 rows of 1024 values: e4m3 228 -> 50 / 244 -> 63 us, bf16 166 -> 46 / 168 -> 48; 58 layers of 333 rows
-// of 7168: e4m3 209 -> 122, bf16 149 -> 106; more slices than warps: 48 layers of 3000 rows of 2048 e4m3 492 -> 347, bf16 331 -> 219, of 8192
-// rows 1252 -> 906 and 1010 -> 796, 58 of 2048 rows of 7168 1313 -> 974 and 1007 -> 788.  Neither streaming stores nor keeping the warps
-// of a block in step helped the largest ones.
-template <bool FP8>
-__device__ __forceinline__ void alone_layers(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
-  if (a.apart && n > 0) {
-    const bool echo = !FP8 && a.y_off == a.recv_x_off;
-    const long long items = n * ((packs + 31) / 32), fit = (warps - n) / items - !echo;
-    const int parts = (int)(fit < a.num_layers ? fit : a.num_layers);
-    if (parts > 1) { alone_apart<FP8>(c, a, n, echo, parts, layer_base); return; }
-  }
-  auto fits = [&](int pl) { return a.apart && (long long)n * ((packs + 32 * pl - 1) / (32 * pl)) <= warps; };
-  if (fits(1)) alone_few<FP8, 1, 8>(c, a, n, layer_base);
-  else if (fits(2)) alone_few<FP8, 2, 4>(c, a, n, layer_base);
-  else if (fits(4)) alone_few<FP8, 4, 2>(c, a, n, layer_base);
-  else alone_many<FP8>(c, a, n, layer_base);
-}
-
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.
 template <bool FP8>
@@ -758,8 +782,9 @@ __global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ 
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
-  if (a.topk <= 32) alone_layers<FP8>(c, a, st.n, st.layer_base);
-  else barrier_alone(c, a, st.n, st.layer_base);
+  if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
+  else if (a.apart) alone_dealt<FP8>(c, a, st.n, st.layer_base);
+  else alone_many<FP8>(c, a, st.n, st.layer_base);
   step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
 }
 

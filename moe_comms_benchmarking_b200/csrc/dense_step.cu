@@ -346,15 +346,13 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
           for (int k = 0; k < 2; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int d = 0; d < D; d += 2) {
-          const uint32_t m0 = max_bf16x2(pack_absmax2(v[d][0]), pack_absmax2(v[d][1])), m1 = max_bf16x2(pack_absmax2(v[d + 1][0]), pack_absmax2(v[d + 1][1]));
-          uint32_t m = max_bf16x2(__byte_perm(m0, m1, 0x5410), __byte_perm(m0, m1, 0x7632));
-#pragma unroll
-          for (int sh = 4; sh >= 1; sh >>= 1) m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, sh));
+          float m[2];
+          block_absmax_wide(v[d], v[d + 1], m[0], m[1]);
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             if (!live || l0 + d + k >= last) continue;
             const uint32_t par = (layer_base + (uint32_t)(l0 + d + k)) & 1u;
-            const float sc = e4m3_scale(k ? bf16_hi(m) : bf16_lo(m));
+            const float sc = e4m3_scale(m[k]);
             const uint2 q0 = quant_pack_e4m3(v[d + k][0], sc), q1 = quant_pack_e4m3(v[d + k][1], sc);
             st_v4(q_dst + (par ? a.dst_par_stride[0] : 0), make_uint4(q0.x, q0.y, q1.x, q1.y));
             if ((lane & 7) == 0) st_b32(s_dst + (par ? a.dst_par_stride[3] : 0), __float_as_uint(sc));

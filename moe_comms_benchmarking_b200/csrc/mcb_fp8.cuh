@@ -69,6 +69,16 @@ __device__ __forceinline__ void block_absmax_pair(uint4 v0, uint4 v1, float& m0,
   m1 = bf16_hi(m);
 }
 
+// The same where a lane holds two neighbouring packs and eight lanes a block: of the lane's packs p0 and of its packs p1.
+__device__ __forceinline__ void block_absmax_wide(const uint4* p0, const uint4* p1, float& m0, float& m1) {
+  const uint32_t a = max_bf16x2(pack_absmax2(p0[0]), pack_absmax2(p0[1])), b = max_bf16x2(pack_absmax2(p1[0]), pack_absmax2(p1[1]));
+  uint32_t m = max_bf16x2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
+#pragma unroll
+  for (int sh = 4; sh >= 1; sh >>= 1) m = max_bf16x2(m, __shfl_xor_sync(0xffffffffu, m, sh));
+  m0 = bf16_lo(m);
+  m1 = bf16_hi(m);
+}
+
 // Scale of a 128-value block from its largest magnitude (1 if that is zero or the block has only NaNs).
 __device__ __forceinline__ float e4m3_scale(float amax) {
   if (e4m3_ordinary(amax)) return div_corrected(amax, 448.0f, 1.0f / 448.0f);

@@ -56,18 +56,22 @@ __device__ __forceinline__ int step_count_exchange(const McbCtx& c, int site, ui
   return n;
 }
 
-// A world of one: the share of warp `warp` of `warps` in `groups` pieces of `layers` layers each, a run of (piece, layer), a piece's layers one
-// after the other.
+// A world of one: items [i, end) of pieces of `layers` layers each, as runs of layers of a piece.
 template <class Body>
-__device__ __forceinline__ void local_share(long long groups, int layers, int warp, int warps, Body body) {
-  const long long items = groups * layers, end = items * (warp + 1) / warps;
-  for (long long i = items * warp / warps; i < end;) {
+__device__ __forceinline__ void local_runs(long long i, long long end, int layers, Body body) {
+  while (i < end) {
     const long long g = i / layers;
     const int first = (int)(i - g * layers);
     const int last = end - i < layers - first ? first + (int)(end - i) : layers;
     body(g, first, last);
     i += last - first;
   }
+}
+// The share of warp `warp` of `warps` in all items of `groups` pieces.
+template <class Body>
+__device__ __forceinline__ void local_share(long long groups, int layers, int warp, int warps, Body body) {
+  const long long items = groups * layers;
+  local_runs(items * warp / warps, items * (warp + 1) / warps, layers, body);
 }
 
 // The last block out advances the sequence words of a step without packets.  Call from all threads of every block.

@@ -326,8 +326,9 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
     (2048, 8, 5, 2, 10, 64),             # as many slices as warps
     (2048, 8, 6, 4, 5, 64),              # more slices than warps
     (7168, 33, 3, 4, 148, 512),          # more ids than lanes
-    (1152, 5, 3, 9, 6, 256),             # 48 warps, 15 slices: two or three runs of the layers side by side
-    (256, 2, 2, 33, 8, 64),              # six or seven runs, and more layers than one warp has in flight
+    (1152, 5, 3, 9, 6, 256),             # 48 warps: a chain each for some, runs that begin and end inside a piece's layers
+    (256, 2, 2, 33, 8, 64),              # more layers than a chain has in flight
+    (1152, 5, 7, 5, 1, 64),              # two warps: many chains each, one of them one more
 ])
 def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads):
     """A step in a world of one whose layers run into each other, against the kernel of the emulated ranks, which takes
@@ -341,6 +342,7 @@ def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, 
     g = torch.Generator(device=DEV).manual_seed(37)
     x, y = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((cap, H), (2, 1, cap, H)))
     x[0, :9] = torch.tensor([0.0, -0.0, float("inf"), -float("inf"), float("nan"), 1e-40, -1e-40, 3e38, 448.0])
+    y[:, 0, 0, :9] = x[0, :9]
     idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(cap)])
     wt = torch.rand(cap, K, device=DEV, generator=g)
     count = torch.tensor([n], dtype=torch.int32, device=DEV)
