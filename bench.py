@@ -221,8 +221,8 @@ def run_native(args):
             "e2e": {"value": round(e2e_ms, 4), "unit": "ms", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": launches,
             "sweep_ms_by_global_batch": {k: round(v, 4) for k, v in sweep_ms.items()},
-            "sweep_note": "world of one: a step of either dispatcher is local copies, at small batches with the loads of up to 8 layers in flight "
-                          "together" if world == 1 and args.native_impl == "dense" and not args.no_persistent else "",
+            "sweep_note": "world of one: a step of either dispatcher is local copies whose layers need no order; a warp takes all layers of a few "
+                          "rows' parts" if world == 1 and args.native_impl == "dense" and not args.no_persistent else "",
             "fused_ms_by_global_batch": fused_ms, "fused_detail": fused_detail,
             "a2a_ms_by_global_batch": a2a_ms,
             "clocks": clocks,

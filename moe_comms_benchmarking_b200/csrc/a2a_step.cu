@@ -646,13 +646,13 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 //   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token, which carries the
 //            number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
-// A warp with one chain more than others takes fewer pieces.  Bound by L2; the chip works on a few MB at a time.  One B200, against
-// layers one after the other, in slices of up to 128 packs a warp:
+// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 (6 TB/s with bf16 rows); the
+// loads of a piece's layers hit L1.  One B200, against layers one after the other, in slices of up to 128 packs a warp:
 //   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows
 //     bf16   35 -> 16.7 / 35 -> 18.7 / 41 -> 35 / 77 -> 72 / 271 -> 265 us
 //     e4m3   43 -> 16.6 / 45 -> 16.7 / 56 -> 38 / 91 -> 75 / 404 -> 272 us
 //   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 4096 rows
-//     bf16   25 -> 14.6 / 27 -> 21 / 99 -> 97 / 265 -> 283 / 1690 -> 1088 us
+//     bf16   25 -> 14.6 / 27 -> 21 / 99 -> 97 / 265 -> 283 (263 -> 267 on another) / 1690 -> 1088 us
 //     e4m3   31 -> 14.6 / 35 -> 21 / 113 -> 100 / 401 -> 278 / 2211 -> 1120 us
 // The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.
 template <bool FP8>

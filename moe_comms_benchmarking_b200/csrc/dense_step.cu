@@ -313,11 +313,12 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 }
 
 // Nothing that a layer reads is written in the step (else: a.in_order), and all layers of a parity deliver the same rows, so the layers
-// need no order.  Bound by L2: a warp takes all layers of a few packs, so that the chip works on a few MB at a time, and every warp gets
-// the same number of packs whatever the batch.  Layer after layer over all rows, large steps went through up to 90 MB of L2 in every
-// layer, small ones left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
+// need no order: a warp takes all layers of a few packs, and every warp gets the same number of (pack, layer) whatever the batch.  Large
+// steps are bound by the stores into L2 (7.6 TB/s at 8192 rows): the chip works on a few MB at a time, and what a warp loads in one layer
+// after the other it finds in L1.  Layer after layer over all rows, large steps went through up to 90 MB of L2 in every layer, small ones
+// left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
 // One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against layers one after the other:
-//   bf16   29 -> 6.4 / 35 -> 8.5 / 25 -> 12.6 / 49 -> 33 / 41 -> 34 / 169 -> 112 / 655 -> 411 us (15 TB/s read and written)
+//   bf16   29 -> 6.4 / 35 -> 8.5 / 25 -> 12.6 / 49 -> 33 / 41 -> 34 / 169 -> 112 / 655 -> 411 us
 //   e4m3   45 -> 8.5 / 53 -> 10.5 / 41 -> 14.5 / 52 -> 33 / 41 -> 37 / 154 -> 121 / 923 -> 451 us
 // and 58 layers of hidden 7168 and top-8, 1 / 64 / 512 / 2048 rows, bf16 19 -> 6.5 / 29 -> 21 / 178 -> 116 / 961 -> 425, e4m3 with 512 / 2048
 // rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.
