@@ -2,9 +2,36 @@
 // small device-memory utilities.
 #include <cuda_runtime.h>
 
-#include "mcb_ctx.h"
+#include "mcb_gemm.h"
 
 extern "C" {
+
+int mcb_launch_metadata(const McbCtx*, const McbMetaArgs*, int, cudaStream_t);
+int mcb_launch_agv(const McbCtx*, const McbAgvArgs*, int, int, int, cudaStream_t);
+int mcb_launch_rsv(const McbCtx*, const McbRsvArgs*, int, int, int, cudaStream_t);
+int mcb_launch_dense_step(const McbCtx*, const McbDenseStepArgs*, int, int, int, cudaStream_t);
+int mcb_launch_a2a_dispatch(const McbCtx*, const McbA2ADispatchArgs*, int, int, int, cudaStream_t);
+int mcb_launch_a2a_combine(const McbCtx*, const McbA2ACombineArgs*, int, int, int, cudaStream_t);
+int mcb_launch_a2a_step(const McbCtx*, const McbA2AStepArgs*, int, int, int, cudaStream_t);
+int mcb_launch_combine(const McbCtx*, const McbCombineArgs*, int, int, int, cudaStream_t);
+
+int mcb_sizeof_launch() { return (int)sizeof(McbLaunch); }
+
+int mcb_launch(const McbLaunch* l, cudaStream_t stream) {
+  if (!l) return (int)cudaErrorInvalidValue;
+  const int g = l->grid, t = l->threads, pdl = l->pdl;
+  switch (l->op) {
+    case MCB_OP_METADATA:     return mcb_launch_metadata(l->ctx, static_cast<const McbMetaArgs*>(l->args), pdl, stream);
+    case MCB_OP_AGV:          return mcb_launch_agv(l->ctx, static_cast<const McbAgvArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_RSV:          return mcb_launch_rsv(l->ctx, static_cast<const McbRsvArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_DENSE_STEP:   return mcb_launch_dense_step(l->ctx, static_cast<const McbDenseStepArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_A2A_DISPATCH: return mcb_launch_a2a_dispatch(l->ctx, static_cast<const McbA2ADispatchArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_A2A_COMBINE:  return mcb_launch_a2a_combine(l->ctx, static_cast<const McbA2ACombineArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_A2A_STEP:     return mcb_launch_a2a_step(l->ctx, static_cast<const McbA2AStepArgs*>(l->args), g, t, pdl, stream);
+    case MCB_OP_COMBINE:      return mcb_launch_combine(l->ctx, static_cast<const McbCombineArgs*>(l->args), g, t, pdl, stream);
+  }
+  return (int)cudaErrorInvalidValue;
+}
 
 int mcb_sizeof_ctx() { return (int)sizeof(McbCtx); }
 int mcb_sizeof_meta_args() { return (int)sizeof(McbMetaArgs); }

@@ -272,6 +272,14 @@ typedef struct {
   int32_t reserved0;
 } McbNormArgs;
 
+// A launch with all its arguments but the stream, which a caller keeps: the call from Python then converts two values instead of six.
+enum { MCB_OP_METADATA = 0, MCB_OP_AGV, MCB_OP_RSV, MCB_OP_DENSE_STEP, MCB_OP_A2A_DISPATCH, MCB_OP_A2A_COMBINE, MCB_OP_A2A_STEP, MCB_OP_COMBINE };
+typedef struct {
+  const McbCtx* ctx;
+  const void* args;              // argument block of the operation
+  int32_t op, grid, threads, pdl;
+} McbLaunch;
+
 #ifdef __cplusplus
 }
 #endif

@@ -81,12 +81,10 @@ class A2ADispatchPlan:
         a.hidden, a.topk, a.num_experts, a.cap = bufs.hidden, bufs.topk, int(num_experts), bufs.cap
         a.fp8 = 1 if bufs.fp8 else 0
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_A2A_DISPATCH, a, "a2a_dispatch")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
-        _ext.check(lib.mcb_launch_a2a_dispatch(self.heap.ctx_ref(), self._ref, self.grid,
-                                               self.threads, int(pdl), _ext.stream_handle(stream)),
-                   "a2a_dispatch")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 class A2ACombinePlan:
@@ -103,13 +101,11 @@ class A2ACombinePlan:
         a.slot_map, a.n_local = bufs.slot_map.data_ptr(), n_local.data_ptr()
         a.hidden, a.cap = bufs.hidden, bufs.cap
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_A2A_COMBINE, a, "a2a_combine")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_A2A_COMBINE, self.grid)
-        _ext.check(lib.mcb_launch_a2a_combine(self.heap.ctx_ref(), self._ref, self.grid,
-                                              self.threads, int(pdl), _ext.stream_handle(stream)),
-                   "a2a_combine")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 def a2a_meta_row_bytes(topk: int) -> int:
@@ -230,11 +226,10 @@ class A2AStepPlan:
             a.ll_rows, a.ll_src_rows = bufs.ll_rows, min(bufs.cap, bufs.ll_rows)
             a.ll_x_off, a.ll_y_off, a.credit_off = bufs.ll_x.offset, bufs.ll_y.offset, bufs.credits.offset
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_A2A_STEP, a, "a2a_step")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
-        _ext.check(lib.mcb_launch_a2a_step(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
-                                           int(pdl), _ext.stream_handle(stream)), "a2a_step")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 def a2a_decode_step(heap, d: A2ADispatchPlan, c: A2ACombinePlan, num_layers: int, pdl: bool = False, stream=None):

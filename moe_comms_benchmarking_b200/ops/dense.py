@@ -75,11 +75,10 @@ class MetadataPlan:
         a.step_meta = step_meta.data_ptr()
         a.cap = int(cap)
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_METADATA, a, "metadata")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
-        _ext.check(lib.mcb_launch_metadata(self.heap.ctx_ref(), self._ref, int(pdl),
-                                           _ext.stream_handle(stream)), "metadata")
+        self._launch(self.heap, pdl=pdl, stream=stream)
 
 
 class AllGatherVPlan:
@@ -123,12 +122,11 @@ class AllGatherVPlan:
             a.ll_off, a.ll_rows = ll_stage.offset, int(ll_rows)
             self._keep += (ll_stage,)
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_AGV, a, "all_gather_v")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_AGV_LL, self.grid)
-        _ext.check(lib.mcb_launch_agv(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
-                                      int(pdl), _ext.stream_handle(stream)), "all_gather_v")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 class ReduceScatterVPlan:
@@ -165,12 +163,11 @@ class ReduceScatterVPlan:
             a.ll_src_rows = min(int(cap), int(ll_rows))
             self._keep += (ll_stage,)
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_RSV, a, "reduce_scatter_v")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
         self.heap.level_launch_counters(_ext.SITE_RSV_LL, self.grid)
-        _ext.check(lib.mcb_launch_rsv(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
-                                      int(pdl), _ext.stream_handle(stream)), "reduce_scatter_v")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 def dense_decode_step(heap, meta: MetadataPlan, agv: AllGatherVPlan, rsv: ReduceScatterVPlan,
@@ -292,11 +289,10 @@ class DenseStepPlan:
             a.delay_ns, a.delay_every = int(delay_ns), max(1, int(delay_every))
             self._keep += (check_errors,)
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_DENSE_STEP, a, "dense_step")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
-        _ext.check(lib.mcb_launch_dense_step(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
-                                             int(pdl), _ext.stream_handle(stream)), "dense_step")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 # ---- uniform-count collectives (tensor-parallel style) ------------------------------------------

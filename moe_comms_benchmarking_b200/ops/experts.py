@@ -245,11 +245,10 @@ class ExpertCombinePlan:
         a.hidden, a.topk, a.cap, a.site = hidden, route.topk, int(cap), int(site)
         a.partial_par_stride = partial.nbytes // 2 if two else 0
         self.args, self._ref = a, C.byref(a)
+        self._launch = _ext.Launcher(_ext.OP_COMBINE, a, "expert_combine")
 
     def launch(self, pdl: bool = False, stream=None):
-        lib = _ext.require()
-        _ext.check(lib.mcb_launch_combine(self.heap.ctx_ref(), self._ref, self.grid, self.threads,
-                                          int(pdl), _ext.stream_handle(stream)), "expert_combine")
+        self._launch(self.heap, self.grid, self.threads, pdl, stream)
 
 
 class Fc2CombinePlan:

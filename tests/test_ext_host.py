@@ -354,3 +354,32 @@ def test_step_joins_only_layers_that_keep_apart(lib):
     raw, addr, meta = _step_args()
     meta.cap = 17
     assert lib.mcb_moe_step_joins(addr, 2, C.addressof(meta)) == 0
+
+
+def test_launcher_follows_context_grid_and_stream(monkeypatch):
+    """The kept block of a plan's launches names the heap's present context, grid, threads and PDL, and errors are raised."""
+    import types
+    from moe_comms_benchmarking_b200.ops import _ext
+    seen, err = [], 0
+
+    def launch(addr, stream):
+        b = _ext.McbLaunch.from_address(addr)
+        seen.append((b.ctx, b.args, b.op, b.grid, b.threads, b.pdl, stream))
+        return err
+
+    monkeypatch.setattr(_ext, "_lib", types.SimpleNamespace(mcb_launch=launch, mcb_error_string=lambda e: b"refused"))
+    monkeypatch.setattr(_ext, "_current_raw_stream", lambda: 7)
+    one, two, args = _ext.McbCtx(), _ext.McbCtx(), _ext.McbAgvArgs()
+    heap = types.SimpleNamespace(ctx=lambda: one)
+    go = _ext.Launcher(_ext.OP_AGV, args, "all_gather_v")
+    at = lambda c: C.addressof(c)
+    go(heap, 148, 512, False)
+    go(heap, 148, 512, True, types.SimpleNamespace(cuda_stream=9))
+    go(heap, 16, 512, True)
+    heap.ctx = lambda: two
+    go(heap, 16, 64, True)
+    assert seen == [(at(one), at(args), _ext.OP_AGV, 148, 512, 0, 7), (at(one), at(args), _ext.OP_AGV, 148, 512, 1, 9),
+                    (at(one), at(args), _ext.OP_AGV, 16, 512, 1, 7), (at(two), at(args), _ext.OP_AGV, 16, 64, 1, 7)]
+    err = 1
+    with pytest.raises(_ext.CudaLaunchError, match="all_gather_v"):
+        go(heap, 16, 64, True)
