@@ -643,17 +643,18 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 // The layers of a step that writes nothing that it reads (a.apart), dealt to the warps; topk at most 32.
 //   pieces   32 packs of a row (64 to quantise, two per lane) and their layers.  All layers of a parity deliver the same rows, so these
 //            need no order: every warp takes a run of (piece, layer), a piece's layers one after the other.
-//   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token, which carries the
-//            number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
+//   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token and parity, which
+//            carries the number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
 // A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 (6 TB/s with bf16 rows); the
 // loads of a piece's layers hit L1.  One B200, against layers one after the other, in slices of up to 128 packs a warp:
 //   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows
-//     bf16   35 -> 16.7 / 35 -> 18.7 / 41 -> 35 / 77 -> 72 / 271 -> 265 us
-//     e4m3   43 -> 16.6 / 45 -> 16.7 / 56 -> 38 / 91 -> 75 / 404 -> 272 us
+//     bf16   35 -> 10.6 / 37 -> 12.6 / 41 -> 33 / 77 -> 72 / 271 -> 265 us
+//     e4m3   45 -> 10.8 / 45 -> 12.6 / 56 -> 37 / 91 -> 76 / 404 -> 272 us
 //   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 4096 rows
-//     bf16   25 -> 14.6 / 27 -> 21 / 99 -> 97 / 265 -> 283 (263 -> 267 on another) / 1690 -> 1088 us
-//     e4m3   31 -> 14.6 / 35 -> 21 / 113 -> 100 / 401 -> 278 / 2211 -> 1120 us
+//     bf16   25 -> 8.5 / 27 -> 18 / 99 -> 93 / 263 -> 268 (265 -> 283 on another) / 1690 -> 1088 us
+//     e4m3   31 -> 10.5 / 35 -> 19 / 112 -> 100 / 407 -> 283 / 2211 -> 1120 us
+// With one chain for both parities of a metadata row, its chunks put together by shuffles, the smallest steps took 16.7 and 14.6 us.
 // The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.
 template <bool FP8>
 __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
@@ -662,13 +663,13 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
   AloneSlice<FP8, 1> s(a);
   const int lane = s.lane, L = a.num_layers, per_row = (s.row_packs + 32 * K - 1) / (32 * K);
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5), warp = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x;
-  const long long sums = s.echo ? 0 : (long long)n * s.slices(), chains = sums + n, items = (long long)n * per_row * L;
+  const long long sums = s.echo ? 0 : (long long)n * s.slices(), chains = sums + 2ll * n, items = (long long)n * per_row * L;
   const uint64_t row_bytes = (uint64_t)a.hidden * 2;
 
   auto chain = [&] {
     for (long long k = warp; k < chains; k += warps) {
       const bool sum = k < sums;
-      s.at(c, sum ? k : (k - sums) * s.slices());
+      s.at(c, sum ? k : (k - sums >> 1) * s.slices());
       if (sum) {
         constexpr int D = 8;
         const bool live = s.p0 < s.row_packs, sent = s.sends(c, s.load_id(true));
@@ -682,17 +683,34 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
             if (live && l0 + d < L) st_v4(s.out, alone_sum(sent, v[d]));
         }
       } else {
-        constexpr int D = 22;
-        for (int l0 = 0; l0 < L; l0 += D) {
-          long long id[D];
-          float wt[D];
-#pragma unroll
-          for (int d = 0; d < D; ++d) { id[d] = s.load_id(l0 + d < L); wt[d] = s.load_weight(l0 + d < L); }
+        // Chunk j of the row (meta_chunk) by lane j, which reads the two ids and weights in it itself.
+        const uint32_t par = (uint32_t)(k - sums) & 1u;
+        const int k0 = lane ? 2 * lane - 1 : 0, k1 = 2 * lane;
+        const bool have0 = k0 < a.topk, have1 = k1 < a.topk, mine = lane < (int)(a.meta_row_bytes >> 4);
+        const int64_t* ids = a.topk_idx + (int64_t)s.t * a.topk;
+        const float* ws = a.topk_w ? a.topk_w + (int64_t)s.t * a.topk : nullptr;
+        uint8_t* meta = s.meta + (par ? a.meta_par_stride : 0);
+        constexpr int D = 8;
+        for (int l0 = (int)((layer_base ^ par) & 1u); l0 < L; l0 += 2 * D) {
+          uint2 id[D][2];
+          uint32_t wt[D][2];
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            if (l0 + d >= L) break;
-            const uint32_t l = layer_base + (uint32_t)(l0 + d);
-            if (s.sends(c, id[d])) s.deliver_meta(l & 1u, l + 1u, id[d], wt[d]);
+            const bool on = l0 + 2 * d < L;
+            id[d][0] = on && have0 ? ld_v2(ids + k0) : make_uint2(~0u, ~0u);
+            id[d][1] = on && have1 ? ld_v2(ids + k1) : make_uint2(~0u, ~0u);
+            wt[d][0] = on && have0 ? (ws ? ld_b32(ws + k0) : __float_as_uint(1.0f)) : 0u;
+            wt[d][1] = on && have1 ? (ws ? ld_b32(ws + k1) : __float_as_uint(1.0f)) : 0u;
+          }
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            if (l0 + 2 * d >= L) break;
+            const bool good0 = id[d][0].y == 0u && id[d][0].x < (uint32_t)a.num_experts, good1 = id[d][1].y == 0u && id[d][1].x < (uint32_t)a.num_experts;
+            if (have0 && !good0) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)s.t, id[d][0].x);
+            if (have1 && !good1) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)s.t, id[d][1].x);
+            if (!__any_sync(0xffffffffu, good0 || good1) || !mine) continue;
+            const uint32_t stamp = layer_base + (uint32_t)(l0 + 2 * d) + 1u;
+            st_v4(meta, lane ? make_uint4(id[d][0].x, wt[d][0], id[d][1].x, wt[d][1]) : make_uint4(stamp, (uint32_t)s.t, id[d][0].x, wt[d][0]));
           }
         }
       }
