@@ -47,6 +47,8 @@
 // instead of being invisible because consecutive layers carry identical bytes.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "mcb_barrier.cuh"
 #include "mcb_dense.cuh"
 #include "mcb_fp8.cuh"
@@ -402,13 +404,105 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
   }
 }
 
-// `nact`: blocks that a layer fills, if the layers keep their order.
-template <bool FP8>
+// A step of up to this many layers has too few of one group of packs to keep loads in flight: there a warp takes all layers of 8 / D groups
+// at a time, D = 1, 2, 4 or 8 the layers that it may have.  The groups go round the warps, so no warp divides.  Kernels of their own:
+// with both ways in one, the large steps of many layers were 3 to 7 % slower and every step 0.5 to 1 us.
+// One B200, a step of 1 / 2 / 4 / 8 layers in a row of steps, dealt in runs -> this way:
+//   hidden 1024 and top-22, 512 rows    bf16 5.0 / 5.5 / 5.9 / 6.5 -> 4.2 / 3.9 / 4.4 / 5.5     e4m3 5.9 / 6.7 / 8.2 / 8.9 -> 5.2 / 5.9 / 6.0 / 7.5 us
+//                          8192 rows    bf16 34.9 / 35.7 / 37 / 41 -> 11.9 / 17.0 / 25.8 / 39.2  e4m3 30.5 / 33.7 / 39 / 54 -> 13.7 / 19.2 / 28.7 / 50
+//   hidden 7168 and top-8, 2048 rows    bf16 56 / 61 / 62 / 66 -> 20.4 / 31.3 / 41.5 / 61        e4m3 51 / 56 / 65 / 89 -> 20.6 / 31.5 / 47.6 / 81
+// (layer after layer, 8192 rows of 1024: bf16 12.0 / 19.8 / 34.9 / 63, e4m3 17.1 / 27.9 / 52 / 96).  Nine to sixteen layers by rounds of eight:
+// up to 25 % slower than runs with bf16 rows, 10 % faster to 10 % slower with e4m3 rows, so the line is at one round.
+constexpr int kFewLayers = 8;
+
+template <bool FP8, int D>
+__device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, uint32_t layer_base) {
+  constexpr int S = 8 / D, Q = D < 4 ? 4 : D, SQ = Q / D;
+  if (a.num_layers < 1) return;
+  const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5)), L = a.num_layers;
+  const long long packs = r.end[LocalRanges::R - 1], groups = (packs + 31) >> 5;
+  const int warp = (int)(blockIdx.x + (threadIdx.x >> 5) * gridDim.x);         // the smallest steps spread over the chip
+  auto parity = [&](int l) { return (layer_base + (uint32_t)l) & 1u; };
+  int from = warp;
+  if (FP8) {
+    // Rows to quantise: two packs (16 values) per lane, eight lanes a block of 128 values.  Rows follow one another in the input and where
+    // they go: lane i of all reads at 32 i and stores at 16 i.
+    const long long halves = (long long)n * (a.fp8_hidden / 16), quants = (halves + 31) >> 5;
+    const uint8_t* rows = reinterpret_cast<const uint8_t*>(a.src[0]);
+    uint8_t *q_dst = c.heap_local + a.dst_off[0], *s_dst = c.heap_local + a.dst_off[3];
+    for (long long g = warp; g < quants; g += (long long)warps * SQ) {
+      uint4 v[Q][2];
+      long long i[Q];
+#pragma unroll
+      for (int d = 0; d < Q; ++d) {
+        i[d] = (g + d / D * warps) * 32 + lane;
+        const bool on = i[d] < halves && d % D < L;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) v[d][k] = on ? ld_v4_stream(rows + i[d] * 32 + k * 16) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int d = 0; d < Q; d += 2) {
+        if (g + d / D * warps >= quants || d % D >= L) break;
+        quant_wide_pair(v[d], v[d + 1], [&](int k, uint4 q, float scale) {
+          const int at = d + k, l = at % D;
+          if (i[at] >= halves || l >= L) return;
+          st_v4(q_dst + i[at] * 16 + (parity(l) ? a.dst_par_stride[0] : 0), q);
+          if ((lane & 7) == 0) st_b32(s_dst + (i[at] >> 3) * 4 + (parity(l) ? a.dst_par_stride[3] : 0), __float_as_uint(scale));
+        });
+      }
+    }
+    from = (warp + warps - (int)(quants % warps)) % warps;      // those that quantise one group more come last
+  }
+  if constexpr (D == 1) {
+    copy_ranges(r, parity(0), (long long)from * 32 + lane, (long long)warps * 32);
+    return;
+  }
+  for (long long g = from; g < groups; g += (long long)warps * S) {
+    uint4 v[S][D];
+    uint8_t* dst[S];
+    uint64_t par_off[S];
+#pragma unroll
+    for (int u = 0; u < S; ++u) {
+      const long long i = (g + u * warps) * 32 + lane;
+      dst[u] = nullptr;
+      if (i < packs) {
+        long long off;
+        const int t = r.find(i, off);
+        dst[u] = r.dst[t] + off;
+        par_off[u] = r.par[t];
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+          if (d < L) v[u][d] = ld_v4_stream(r.src[t] + off);
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+#pragma unroll
+      for (int u = 0; u < S; ++u)
+        if (d < L && dst[u]) st_v4(dst[u] + (parity(d) ? par_off[u] : 0), v[u][d]);
+  }
+  // The words behind the last whole pack of each range.
+  if (warp == warps - 1) {
+    uint32_t w[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) w[d] = d < L ? r.load_word(lane, 0) : 0u;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+      if (d < L) r.store_word(parity(d), w[d], lane, 0);
+  }
+}
+
+// D: as in local_few, 0 for steps of more layers.  `nact`: blocks that a layer fills, if the layers keep their order.
+template <bool FP8, int D>
 __device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
   if (n <= 0) return;
   __shared__ LocalRanges r;
   local_ranges<FP8>(r, c, a, n);
-  if (!a.in_order) { local_dealt<FP8>(c, a, r, n, layer_base); return; }
+  if (!a.in_order) {
+    if constexpr (D > 0) local_few<FP8, D>(c, a, r, n, layer_base);
+    else local_dealt<FP8>(c, a, r, n, layer_base);
+    return;
+  }
   if ((int)blockIdx.x >= nact) return;
   const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)nact * blockDim.x;
   for (int l = 0; l < a.num_layers; ++l) {
@@ -502,7 +596,7 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
     }
   } else if (EMU && W == 1 && !CHECK) {      // else dense_alone_kernel
     const int nloc = active_blocks((int)gridDim.x, n, bytes_per_row + a.rsv_row_bytes, (int)blockDim.x);
-    local_layers<FP8>(c, a, n, nloc, layer_base);
+    local_layers<FP8, 0>(c, a, n, nloc, layer_base);
   } else if (grp >= 0 && lb < nact) {
     // ---- barrier mode ----------------------------------------------------------------------------
     uint32_t ep = *epoch_ptr(c, MCB_SITE_STEP, bid);
@@ -591,7 +685,7 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
 
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.
-template <bool FP8>
+template <bool FP8, int D>
 __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   pdl_wait();                 // the previous kernel of this rank (the previous step) has finished
@@ -614,7 +708,7 @@ __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant_
   for (int t = 0; t < MCB_MAX_TENSORS; ++t)
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
   const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
-  local_layers<FP8>(c, a, n, nact, layer_base);
+  local_layers<FP8, D>(c, a, n, nact, layer_base);
   step_close(a.state, step_seq, layer_base + (uint32_t)L);
 }
 
@@ -670,9 +764,17 @@ int mcb_launch_dense_step(const McbCtx* ctx, const McbDenseStepArgs* args, int g
   const bool coop = args->groups > 1;
   McbDenseStepArgs a = *args;
   a.in_order = mcb_dense_step_in_order(ctx, args);
-  if (ctx->world == 1 && !args->check)
-    return a.fp8_hidden ? launch_kernel(dense_alone_kernel<true>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a)
-                        : launch_kernel(dense_alone_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
+  if (ctx->world == 1 && !args->check) {
+    auto alone = [&](auto layers) {
+      constexpr int D = decltype(layers)::value;
+      return launch_kernel(a.fp8_hidden ? dense_alone_kernel<true, D> : dense_alone_kernel<false, D>, dim3(grid), dim3(threads), 0, stream, pdl, false,
+                           *ctx, a);
+    };
+    if (a.num_layers > kFewLayers) return alone(std::integral_constant<int, 0>{});
+    if (a.num_layers > 4) return alone(std::integral_constant<int, kFewLayers>{});
+    if (a.num_layers > 2) return alone(std::integral_constant<int, 4>{});
+    return a.num_layers > 1 ? alone(std::integral_constant<int, 2>{}) : alone(std::integral_constant<int, 1>{});
+  }
   if (args->check)
     return launch_kernel(dense_step_kernel<false, true, false>, dim3(grid), dim3(threads), 0, stream, pdl, coop, *ctx,
                          a, (const McbCtx*)nullptr, (const McbDenseStepArgs*)nullptr);

@@ -85,6 +85,21 @@ __device__ __forceinline__ float e4m3_scale(float amax) {
   return amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f;
 }
 
+// Two times two neighbouring packs per lane, eight lanes a block: put(k, the sixteen values of packs k in e4m3, their block's scale).
+// All 32 lanes.
+template <class Put>
+__device__ __forceinline__ void quant_wide_pair(const uint4* p0, const uint4* p1, Put put) {
+  float m[2];
+  block_absmax_wide(p0, p1, m[0], m[1]);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint4* p = k ? p1 : p0;
+    const float scale = e4m3_scale(m[k]);
+    const uint2 q0 = quant_pack_e4m3(p[0], scale), q1 = quant_pack_e4m3(p[1], scale);
+    put(k, make_uint4(q0.x, q0.y, q1.x, q1.y), scale);
+  }
+}
+
 // Largest magnitude of the 128-value block that starts at `block` (16 packs of 16 bytes), read by
 // ONE thread (for the packet mode, where the threads that share a block are not neighbours).
 __device__ __forceinline__ float block_absmax_serial(const uint8_t* block) {

@@ -373,3 +373,16 @@ def test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads):
             want = [(q.view(torch.uint8) if fp8 else x[:n]).to(DEV), ids[:n], w[:n]] + [scale.to(DEV)] * fp8
             for t, v in zip((gh, gi, gw, gs), want):
                 assert torch.equal(t.tensor[p, :n], v if there else torch.zeros_like(v)) and not t.tensor[p, n:].any()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("n,layers,grid,threads", [
+    (1, 1, 148, 512), (8, 1, 1, 64),      # one layer: a group per warp, several rounds of eight groups
+    (5, 2, 2, 32), (7, 2, 148, 512),      # four groups at a time
+    (7, 3, 1, 32), (8, 4, 3, 96),         # two, with and without a layer that is not there
+    (3, 5, 1, 64), (8, 8, 5, 32),         # one
+    (7, 9, 2, 64),                        # the first that is dealt in runs
+])
+def test_world_of_one_few_layers(lib, fp8, n, layers, grid, threads):
+    """Steps of up to eight layers, whose warps take all layers of one group of packs or more at a time."""
+    test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads)
