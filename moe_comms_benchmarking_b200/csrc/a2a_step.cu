@@ -25,6 +25,8 @@
 // Every wait is bounded and reports through the status words.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "mcb_barrier.cuh"
 #include "mcb_dense.cuh"
 #include "mcb_fp8.cuh"
@@ -775,6 +777,46 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
   }
 }
 
+// A warp takes a slice of a row and, D at a time, all its layers; steps that write nothing that they read.
+template <bool FP8, int PL, int D>
+__device__ __forceinline__ void alone_slices(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  AloneSlice<FP8, PL> s(a);
+  const long long mine = (long long)n * s.slices(), step = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long i = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x; i < mine; i += step) {
+    s.at(c, i);
+#pragma unroll 1
+    for (int l0 = 0; l0 < a.num_layers; l0 += D) {
+      uint4 v[D][PL], w[D][PL];
+      long long id[D];
+      float wt[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) s.load(l0 + d < a.num_layers, (layer_base + (uint32_t)(l0 + d)) & 1u, v[d], w[d], id[d], wt[d]);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        if (l0 + d >= a.num_layers) break;
+        s.deliver(c, (layer_base + (uint32_t)(l0 + d)) & 1u, layer_base + (uint32_t)(l0 + d) + 1u, v[d], w[d], id[d], wt[d]);
+      }
+    }
+  }
+}
+
+// A step of up to this many layers has too few of one piece to keep loads in flight: there the warps take slices, of one pack per lane
+// where that still gives every slice a warp of its own, else of four.  Kernels of their own, for one layer (D = 1) and for more (D = 2), which are
+// smaller than that of the dealt steps.  One B200, a step of 1 / 2 / 3 / 4 layers in a row of steps, dealt -> slices:
+//   hidden 1024 and top-22, 64 rows     bf16 5.0 / 4.5 / 4.6 / 4.5 -> 4.2 / 4.3 / 4.9 / 4.7      e4m3 5.2 / 5.3 / 4.8 / 4.8 -> 4.2 / 4.7 / 4.8 / 5.1 us
+//                          8192 rows    bf16 32.4 / 28.2 / 29.3 / 33.1 -> 9.8 / 15.5 / 21.0 / 26.7  e4m3 40.1 / 42.7 / 47 / 49 -> 13.0 / 20.0 / 27.6 / 33.5
+//   hidden 7168 and top-8, 2048 rows    bf16 39 / 44 / 47 / 50 -> 17.0 / 28.7 / 35.6 / 43.3      e4m3 56 / 63 / 72 / 77 -> 21.1 / 33.4 / 45.4 / 55.6
+// (layer after layer, 8192 rows of 1024: bf16 11.1 / 17.1 / 23.5 / 29.0, e4m3 15.1 / 25.0 / 34.5 / 44).  With five to eight layers the dealt steps of up
+// to 200 rows are 5 to 35 % faster than slices, and larger ones up to 30 % slower.  Four layers at a time,
+// or eight, were 3 to 40 % slower than two.
+constexpr int kFewLayers = 4;
+template <bool FP8, int D>
+__device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
+  if (n * ((packs + 31) / 32) <= warps) alone_slices<FP8, 1, D>(c, a, n, layer_base);
+  else alone_slices<FP8, 4, D>(c, a, n, layer_base);
+}
+
 // Layer after layer: steps that read what they write.
 template <bool FP8>
 __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
@@ -793,14 +835,15 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
 
 // The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.
-template <bool FP8>
+template <bool FP8, int D>
 __global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbA2AStepArgs a) {
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
-  if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
+  if constexpr (D > 0) alone_few<FP8, D>(c, a, st.n, st.layer_base);
+  else if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
   else if (a.apart) alone_dealt<FP8>(c, a, st.n, st.layer_base);
   else alone_many<FP8>(c, a, st.n, st.layer_base);
   step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
@@ -852,9 +895,14 @@ int mcb_launch_a2a_step(const McbCtx* ctx, const McbA2AStepArgs* args, int grid,
   if (check_a2a_step(ctx, args, grid, threads)) return cudaErrorInvalidValue;
   McbA2AStepArgs a = *args;
   a.apart = mcb_a2a_step_apart(ctx, args);
-  if (ctx->world == 1)
-    return a.fp8 ? launch_kernel(a2a_alone_kernel<true>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a)
-                 : launch_kernel(a2a_alone_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
+  if (ctx->world == 1) {
+    auto alone = [&](auto layers) {
+      constexpr int D = decltype(layers)::value;
+      return launch_kernel(a.fp8 ? a2a_alone_kernel<true, D> : a2a_alone_kernel<false, D>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
+    };
+    if (!a.apart || a.topk > 32 || a.num_layers > kFewLayers) return alone(std::integral_constant<int, 0>{});
+    return a.num_layers > 1 ? alone(std::integral_constant<int, 2>{}) : alone(std::integral_constant<int, 1>{});
+  }
   return launch_kernel(a2a_step_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a,
                        (const McbCtx*)nullptr, (const McbA2AStepArgs*)nullptr);
 }

@@ -369,6 +369,18 @@ def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, 
         assert int(w.status[0][0]) == int(heap.status.view(torch.int32)[0]) == (4 if step == 2 else 0)        # MCB_ERR_ROUTING
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,K,n,layers,grid,threads", [
+    (1152, 5, 6, 1, 148, 512), (2048, 32, 5, 2, 148, 512),      # a warp for every slice of one pack per lane
+    (1152, 5, 9, 1, 1, 64), (1152, 5, 9, 2, 2, 64),             # slices of four, the second of a row ragged, in several rounds
+    (256, 8, 7, 3, 3, 32), (1024, 6, 8, 4, 2, 96),              # an odd layer at the end, and none
+    (1024, 6, 8, 5, 2, 96),                                     # the first that is dealt
+])
+def test_a2a_step_alone_few_layers(lib, world1, fp8, H, K, n, layers, grid, threads):
+    """Steps of up to four layers, whose warps take slices of rows."""
+    test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads)
+
+
 @pytest.mark.parametrize("form", ["out_on_x", "out_on_ids", "echo"])
 def test_a2a_step_that_reads_what_it_writes(lib, world1, form):
     """The host tells steps whose layers may run into each other from those that write what they read."""
