@@ -817,6 +817,19 @@ __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs&
   else alone_slices<FP8, 4, D>(c, a, n, layer_base);
 }
 
+// Whether a step of the identity expert on bf16 rows goes by slices of four packs per lane, whatever its layers: where its slices fill
+// at least 5/6 of their last round of warps.  A slice writes its row part, its sums and its metadata in one go, which saves a dealt step's addresses; but a
+// slice is all layers, so a last round that is not full is waited for.  One B200, 58 layers, dealt -> slices:
+//   hidden 7168, 333 rows (0.98 of a round) 95 -> 87, 1000 (2.96 of 3) 270 -> 257, 2048 (6.05 of 7) 545 -> 529 us
+//   hidden 1024, 2048 rows (0.86) 87.5 -> 83.5, 4096 (1.73 of 2) 170 -> 157; hidden 2048, 4096 rows (3.46 of 4) 322 -> 303
+//   not full: hidden 7168, 512 rows (1.51 of 2) 140 -> 141, 700 (2.07 of 3) 190 -> 210; hidden 2048, 1400 rows (1.18 of 2) 113 -> 128
+// (before layers were dealt, 1000 rows of 7168: 265).  e4m3 rows, up to 8 layers: 1.0 to 0.9 of the dealt time, but the second way in their
+// kernel cost every step 0.7 to 1 us.
+__device__ __forceinline__ bool alone_full(const McbA2AStepArgs& a, int n) {
+  const unsigned warps = gridDim.x * (blockDim.x >> 5), items = (unsigned)n * (unsigned)((a.hidden / 8 + 127) / 128);
+  return a.y_off == a.recv_x_off && items * 6ull >= (items + warps - 1) / warps * 5ull * warps;
+}
+
 // Layer after layer: steps that read what they write.
 template <bool FP8>
 __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
@@ -842,10 +855,19 @@ __global__ void __launch_bounds__(512) a2a_alone_kernel(const __grid_constant__ 
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   const A2AStep st = a2a_step_open(c, a, s_cnt, s_prefix, &s_max);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.step_meta[6] = 0;
-  if constexpr (D > 0) alone_few<FP8, D>(c, a, st.n, st.layer_base);
-  else if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
-  else if (a.apart) alone_dealt<FP8>(c, a, st.n, st.layer_base);
-  else alone_many<FP8>(c, a, st.n, st.layer_base);
+  // The order of the ways is that of their code, and small steps feel it: slices behind dealt pieces cost them 0.1 us, before them 0.25.
+  if constexpr (D > 0) {
+    alone_few<FP8, D>(c, a, st.n, st.layer_base);
+  } else if constexpr (FP8) {
+    if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
+    else if (a.apart) alone_dealt<FP8>(c, a, st.n, st.layer_base);
+    else alone_many<FP8>(c, a, st.n, st.layer_base);
+  } else {
+    if (a.topk > 32) barrier_alone(c, a, st.n, st.layer_base);
+    else if (!a.apart) alone_many<FP8>(c, a, st.n, st.layer_base);
+    else if (!alone_full(a, st.n)) alone_dealt<FP8>(c, a, st.n, st.layer_base);
+    else alone_slices<FP8, 4, 2>(c, a, st.n, st.layer_base);
+  }
   step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
 }
 

@@ -375,9 +375,11 @@ def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, 
     (1152, 5, 9, 1, 1, 64), (1152, 5, 9, 2, 2, 64),             # slices of four, the second of a row ragged, in several rounds
     (256, 8, 7, 3, 3, 32), (1024, 6, 8, 4, 2, 96),              # an odd layer at the end, and none
     (1024, 6, 8, 5, 2, 96),                                     # the first that is dealt
+    (1152, 5, 3, 7, 1, 192), (1152, 5, 5, 8, 2, 192),           # bf16 rows: a full round of slices; ten of twelve
+    (1152, 5, 4, 9, 1, 192), (128, 1, 29, 6, 3, 320),           # eight of twelve, dealt; 29 of 30
 ])
 def test_a2a_step_alone_few_layers(lib, world1, fp8, H, K, n, layers, grid, threads):
-    """Steps of up to four layers, whose warps take slices of rows."""
+    """Steps of up to four layers, and larger ones whose slices fill their rounds: the warps take slices of rows."""
     test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads)
 
 
