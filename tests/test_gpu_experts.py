@@ -297,7 +297,7 @@ def test_layer_kernel_phase_trace_world1(world1):
     ([129, 1], 256, 128, 148),                           # one column block per stage; more CTAs than units
     ([256, 257, 0, 513, 5], 256, 384, 148),              # one, two and three chunks of an expert
     ([40] * 200, 512, 256, 2),                           # more units than one list holds
-    ([2600, 300, 1, 900, 2400, 700], 256, 2048, 148),    # activations beyond the L2 bound: down units follow at a distance
+    ([2600, 300, 1, 900, 2400, 700], 256, 2048, 148),    # activations beyond the L2 bound, but too few experts for a distance
 ])
 def test_expert_ffn_chunk_edges(world1, rows, H, I, grid):
     """expert_ffn_kernel where the token count of an expert meets the edges of its chunks, its token path and
@@ -335,6 +335,28 @@ def test_expert_ffn_chunk_edges(world1, rows, H, I, grid):
             assert float((act[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} gate/up"
             want = act[sl].float() @ wd[e].t() * route.pair_prob[sl].unsqueeze(1)
             assert float((y[sl].float() - want).abs().max()) < 2 ** -7 * float(want.abs().max()), f"expert {e} down"
+
+
+def _down_distance(rows, H, I, grid):
+    """The numbering of the kernels (ffn_plan in mcb_ffn.cuh): experts with tokens, and how many of them the down units of one
+    come behind its gate/up units."""
+    active, chunks, grid = sum(r > 0 for r in rows), sum((r + 255) // 256 for r in rows), max(grid & ~1, 2)
+    beyond = sum(rows) * I * 2 > 24 << 20                # bytes of activations that stay within L2
+    return active, min(active, grid * active // (H // 256 * chunks) + 2) if beyond else active
+
+
+@pytest.mark.parametrize("rows,H,I,grid", [
+    ([700, 300, 1, 900, 0, 600, 256, 257, 500, 1200], 1024, 2816, 14),     # seven CTA pairs, chunked, tiny and idle experts
+    ([700, 300, 1, 900, 0, 600, 256, 257, 500, 1200], 1024, 2816, 15),
+    ([96 + 5 * i for i in range(20)] + [0] + [110] * 40, 1024, 2048, 148), # one chunk each; the whole chip
+    ([257] * 30, 2560, 1664, 6),                                           # a second chunk of one row, long distance in units
+])
+def test_expert_ffn_down_units_at_a_distance(world1, rows, H, I, grid):
+    """Beyond the activations that stay within L2, down units follow the gate/up units of their expert at a distance of fewer
+    experts than there are.  Tolerance as in the test of the chunks."""
+    active, distance = _down_distance(rows, H, I, grid)
+    assert 2 <= distance < active
+    test_expert_ffn_chunk_edges(world1, rows, H, I, grid)
 
 
 @pytest.mark.parametrize("rows", [
@@ -577,6 +599,15 @@ def test_step_of_several_layers(world1, E, K, H, I, T, layers, sets, grid):
             assert torch.equal(d.out, want), f"{n} tokens, rep {rep}"
             assert torch.equal(d.agv_h.tensor[:n], x[:n]) and torch.equal(d.agv_r.tensor[:n], idx[:n]) and torch.equal(d.agv_p.tensor[:n], w[:n])
     d.destroy()
+
+
+@pytest.mark.parametrize("E,K,H,I,T,grid", [(24, 4, 1024, 512, 7000, 148), (24, 4, 1024, 512, 7000, 11)])
+def test_step_with_down_units_at_a_distance(world1, E, K, H, I, T, grid):
+    """A step of several layers whose down units follow at a distance of fewer experts than there are, against its layers."""
+    rows = torch.bincount(_case(T, E, K, H, I, T + 31)[1].flatten(), minlength=E).tolist()
+    active, distance = _down_distance(rows, H, I, grid)
+    assert 2 <= distance < active
+    test_step_of_several_layers(world1, E, K, H, I, T, 4, 2, grid)
 
 
 def test_step_on_its_own_output_goes_layer_by_layer(world1):
