@@ -737,7 +737,8 @@ static int check_step_args(const McbDenseStepArgs* a, int grid, int threads) {
 }
 
 // Whether a step in a world of one writes rows that it reads, or writes rows twice: an output on a source (a step in
-// place), partial sums that are gathered rows (the identity expert).  Its copies then keep the order of the layers.
+// place), partial sums that are gathered rows (the identity expert), tensors gathered to one place.  Its copies then keep the order of the
+// layers, and within a layer that of the tensors.
 int mcb_dense_step_in_order(const McbCtx* ctx, const McbDenseStepArgs* a) {
   if (ctx->world != 1) return 0;
   struct Range { uint64_t at, bytes; };
@@ -751,6 +752,11 @@ int mcb_dense_step_in_order(const McbCtx* ctx, const McbDenseStepArgs* a) {
     for (int u = 0; u < a->num_tensors; ++u) {
       const Range src{reinterpret_cast<uint64_t>(a->src[u]), cap * (a->fp8_hidden && u == 0 ? 2u * a->fp8_hidden : a->row_bytes[u])};
       hit = hit || meet(src, rows) || meet(src, out);
+      for (int k = 0; k < 4 && u < t; ++k) {             // gathered rows of either parity of two tensors
+        const Range one{heap + a->dst_off[t] + (k & 1) * a->dst_par_stride[t], cap * a->row_bytes[t]};
+        const Range two{heap + a->dst_off[u] + (k >> 1) * a->dst_par_stride[u], cap * a->row_bytes[u]};
+        hit = hit || meet(one, two);
+      }
     }
   }
   return hit;

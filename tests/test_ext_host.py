@@ -297,6 +297,27 @@ def test_step_on_its_own_rows_keeps_its_order(lib):
     assert marked(both[cap:], gh) == 1 and marked(gh.tensor[1]) == 1 and marked(rsv.tensor) == 1
 
 
+def test_step_that_gathers_twice_to_one_place_keeps_its_order(lib):
+    """Gathered tensors that share rows, in either parity, are written in turn; ones whose parities lie between one another's are apart."""
+    from moe_comms_benchmarking_b200.ops.dense import DenseStepPlan
+    h = _heap(4 << 20)
+    cap, H = 8, 256
+    rows = cap * H * 2
+    n_local, meta = torch.zeros(1, dtype=torch.int32), torch.zeros(8, dtype=torch.int32)
+    a, b, rsv = h.alloc("a", [2, cap, H], torch.bfloat16), h.alloc("b", [2, cap, H], torch.bfloat16), h.alloc("r", [cap, H], torch.bfloat16)
+    x, out = torch.zeros(cap, H, dtype=torch.bfloat16), torch.zeros(cap, H, dtype=torch.bfloat16)
+    plan = DenseStepPlan(h, [a, b], [x, torch.zeros_like(x)], out, rsv, n_local, meta, cap, 4)
+
+    def marked(off_a, stride_a, off_b, stride_b):
+        for t, (off, stride) in enumerate(((off_a, stride_a), (off_b, stride_b))):
+            plan.args.dst_off[t], plan.args.dst_par_stride[t] = a.offset + off, stride
+        return lib.mcb_dense_step_in_order(C.byref(h.ctx()), C.byref(plan.args))
+
+    assert marked(0, rows, 2 * rows, rows) == 0 and marked(0, 2 * rows, rows, 2 * rows) == 0
+    assert marked(0, rows, 0, rows) == 1 and marked(0, rows, rows, rows) == 1 and marked(rows, rows, 0, rows) == 1
+    assert marked(0, rows, 2 * rows - 16, rows) == 1
+
+
 def test_weight_tile_packing_round_trip():
     """The pre-packed weight layout: tile (row block, column block) is 16 KB of contiguous memory in the
     swizzled K-major shared-memory image; packing and unpacking are inverse, and chunk c of row r of a
