@@ -24,6 +24,7 @@
 #include "mcb_barrier.cuh"
 #include "mcb_fp8.cuh"
 #include "mcb_launch.h"
+#include "mcb_launchers.h"
 #include "mcb_noalloc.h"
 
 namespace mcb {

@@ -31,6 +31,7 @@
 #include "mcb_dense.cuh"
 #include "mcb_fp8.cuh"
 #include "mcb_launch.h"
+#include "mcb_launchers.h"
 #include "mcb_step.cuh"
 
 namespace mcb {

@@ -2,18 +2,9 @@
 // small device-memory utilities.
 #include <cuda_runtime.h>
 
-#include "mcb_gemm.h"
+#include "mcb_launchers.h"
 
 extern "C" {
-
-int mcb_launch_metadata(const McbCtx*, const McbMetaArgs*, int, cudaStream_t);
-int mcb_launch_agv(const McbCtx*, const McbAgvArgs*, int, int, int, cudaStream_t);
-int mcb_launch_rsv(const McbCtx*, const McbRsvArgs*, int, int, int, cudaStream_t);
-int mcb_launch_dense_step(const McbCtx*, const McbDenseStepArgs*, int, int, int, cudaStream_t);
-int mcb_launch_a2a_dispatch(const McbCtx*, const McbA2ADispatchArgs*, int, int, int, cudaStream_t);
-int mcb_launch_a2a_combine(const McbCtx*, const McbA2ACombineArgs*, int, int, int, cudaStream_t);
-int mcb_launch_a2a_step(const McbCtx*, const McbA2AStepArgs*, int, int, int, cudaStream_t);
-int mcb_launch_combine(const McbCtx*, const McbCombineArgs*, int, int, int, cudaStream_t);
 
 int mcb_sizeof_launch() { return (int)sizeof(McbLaunch); }
 
@@ -31,6 +22,21 @@ int mcb_launch(const McbLaunch* l, cudaStream_t stream) {
     case MCB_OP_COMBINE:      return mcb_launch_combine(l->ctx, static_cast<const McbCombineArgs*>(l->args), g, t, pdl, stream);
   }
   return (int)cudaErrorInvalidValue;
+}
+
+// Name of an operation, null behind the last one: a caller that numbers them too compares.
+const char* mcb_op_name(int op) {
+  switch (op) {
+    case MCB_OP_METADATA:     return "metadata";
+    case MCB_OP_AGV:          return "all_gather_v";
+    case MCB_OP_RSV:          return "reduce_scatter_v";
+    case MCB_OP_DENSE_STEP:   return "dense_step";
+    case MCB_OP_A2A_DISPATCH: return "a2a_dispatch";
+    case MCB_OP_A2A_COMBINE:  return "a2a_combine";
+    case MCB_OP_A2A_STEP:     return "a2a_step";
+    case MCB_OP_COMBINE:      return "expert_combine";
+  }
+  return nullptr;
 }
 
 int mcb_sizeof_ctx() { return (int)sizeof(McbCtx); }

@@ -25,6 +25,7 @@
 #include "mcb_barrier.cuh"
 #include "mcb_dense.cuh"
 #include "mcb_launch.h"
+#include "mcb_launchers.h"
 
 namespace mcb {
 

@@ -25,6 +25,7 @@
 #include "mcb_ffn.cuh"
 #include "mcb_gemm.h"
 #include "mcb_launch.h"
+#include "mcb_launchers.h"
 #include "mcb_route.cuh"
 #include "mcb_tmap.h"
 
@@ -178,7 +179,6 @@ int mcb_launch_moe_layer(const McbLayerArgs* p, int grid, int pdl, cudaStream_t 
 // One decode step with real experts, issued natively: the count exchange, then num_layers layers; layer l uses the argument
 // block (weight set) l % num_sets.  With `step` (mcb_prepare_moe_step, over the same argument blocks) several layers share a
 // launch, without it each is a layer kernel.
-int mcb_launch_metadata(const McbCtx* ctx, const McbMetaArgs* args, int pdl, cudaStream_t stream);   // dense.cu
 int mcb_launch_moe_step(const McbMoeStepArgs* p, const McbLayerArgs* sets, int num_sets, int first, int num_layers, int grid, int pdl,
                         cudaStream_t stream);                                                        // moe_step.cu
 

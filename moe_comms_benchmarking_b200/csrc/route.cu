@@ -13,6 +13,7 @@
 #include "mcb_gemm.h"
 #include "mcb_route.cuh"
 #include "mcb_launch.h"
+#include "mcb_launchers.h"
 
 namespace mcb {
 

@@ -182,7 +182,9 @@ class McbLaunch(C.Structure):
     _fields_ = [("ctx", _vp), ("args", _vp), ("op", _i32), ("grid", _i32), ("threads", _i32), ("pdl", _i32)]
 
 
-OP_METADATA, OP_AGV, OP_RSV, OP_DENSE_STEP, OP_A2A_DISPATCH, OP_A2A_COMBINE, OP_A2A_STEP, OP_COMBINE = range(8)
+# Operations of mcb_launch by number; load() compares them with the library's.
+OPS = ("metadata", "all_gather_v", "reduce_scatter_v", "dense_step", "a2a_dispatch", "a2a_combine", "a2a_step", "expert_combine")
+OP_METADATA, OP_AGV, OP_RSV, OP_DENSE_STEP, OP_A2A_DISPATCH, OP_A2A_COMBINE, OP_A2A_STEP, OP_COMBINE = range(len(OPS))
 
 
 _STRUCTS = {
@@ -195,11 +197,8 @@ _STRUCTS = {
 # by table instead of asking each value what it is.
 _ARG = {"p": C.c_void_p, "i": C.c_int}
 _LAUNCHERS = {
-    "mcb_launch_load_batch": "pip", "mcb_launch_metadata": "ppip", "mcb_launch_agv": "ppiiip", "mcb_launch_rsv": "ppiiip",
-    "mcb_launch_dense_step": "ppiiip", "mcb_launch_a2a_dispatch": "ppiiip", "mcb_launch_a2a_combine": "ppiiip",
-    "mcb_launch_a2a_step": "ppiiip", "mcb_launch_route": "piip", "mcb_launch_expert_ffn": "piip",
-    "mcb_launch_combine": "ppiiip", "mcb_launch_moe_layer": "piip", "mcb_moe_decode_step": "pppiiiipp",
-    "mcb_moe_step_joins": "pip", "mcb_prepare_moe_step": "ppip" + "p" * 8 + "i", "mcb_launch": "pp",
+    "mcb_launch_load_batch": "pip", "mcb_launch_route": "piip", "mcb_launch_expert_ffn": "piip", "mcb_launch_moe_layer": "piip",
+    "mcb_moe_decode_step": "pppiiiipp", "mcb_moe_step_joins": "pip", "mcb_prepare_moe_step": "ppip" + "p" * 8 + "i", "mcb_launch": "pp",
 }
 
 LIB_PATH = Path(__file__).resolve().parent.parent / "lib" / "libmcb.so"
@@ -219,7 +218,7 @@ def available() -> bool:
 
 
 def load():
-    """Load the library once and verify the struct layouts."""
+    """Load the library once and verify the struct layouts and operation numbers."""
     global _lib
     if _lib is not None:
         return _lib
@@ -249,6 +248,11 @@ def load():
     if lib.mcb_sizeof_layer_args() != layer_args_size():
         raise ExtensionMissing(f"layout drift: sizeof(layer_args) is {lib.mcb_sizeof_layer_args()} in libmcb.so, "
                                f"{layer_args_size()} in ctypes")
+    lib.mcb_op_name.restype = C.c_char_p
+    lib.mcb_op_name.argtypes = [C.c_int]
+    names = [lib.mcb_op_name(op) for op in range(len(OPS) + 1)]
+    if names != [op.encode() for op in OPS] + [None]:
+        raise ExtensionMissing(f"operation drift: {names} in libmcb.so, {OPS} in ctypes")
     lib.mcb_error_string.restype = C.c_char_p
     lib.mcb_error_string.argtypes = [C.c_int]
     for name, sig in _LAUNCHERS.items():

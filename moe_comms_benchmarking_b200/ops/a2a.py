@@ -80,7 +80,7 @@ class A2ADispatchPlan:
         a.n_local = n_local.data_ptr()
         a.hidden, a.topk, a.num_experts, a.cap = bufs.hidden, bufs.topk, int(num_experts), bufs.cap
         a.fp8 = 1 if bufs.fp8 else 0
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_A2A_DISPATCH, a, "a2a_dispatch")
 
     def launch(self, pdl: bool = False, stream=None):
@@ -100,7 +100,7 @@ class A2ACombinePlan:
         a.out, a.y_off = out.data_ptr(), bufs.y.offset
         a.slot_map, a.n_local = bufs.slot_map.data_ptr(), n_local.data_ptr()
         a.hidden, a.cap = bufs.hidden, bufs.cap
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_A2A_COMBINE, a, "a2a_combine")
 
     def launch(self, pdl: bool = False, stream=None):

@@ -74,7 +74,7 @@ class MetadataPlan:
         a.counts_off = heap.counts_off
         a.step_meta = step_meta.data_ptr()
         a.cap = int(cap)
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_METADATA, a, "metadata")
 
     def launch(self, pdl: bool = False, stream=None):
@@ -121,7 +121,7 @@ class AllGatherVPlan:
                 raise ValueError(f"low-latency staging holds {ll_stage.nbytes} bytes, {need} needed")
             a.ll_off, a.ll_rows = ll_stage.offset, int(ll_rows)
             self._keep += (ll_stage,)
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_AGV, a, "all_gather_v")
 
     def launch(self, pdl: bool = False, stream=None):
@@ -162,7 +162,7 @@ class ReduceScatterVPlan:
             a.ll_off, a.ll_rows, a.counts_off = ll_stage.offset, int(ll_rows), heap.counts_off
             a.ll_src_rows = min(int(cap), int(ll_rows))
             self._keep += (ll_stage,)
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_RSV, a, "reduce_scatter_v")
 
     def launch(self, pdl: bool = False, stream=None):
@@ -288,7 +288,7 @@ class DenseStepPlan:
             a.check_errors, a.check = check_errors.data_ptr(), 1
             a.delay_ns, a.delay_every = int(delay_ns), max(1, int(delay_every))
             self._keep += (check_errors,)
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_DENSE_STEP, a, "dense_step")
 
     def launch(self, pdl: bool = False, stream=None):

@@ -244,7 +244,7 @@ class ExpertCombinePlan:
         a.n_local, a.step_meta = n_local.data_ptr(), step_meta.data_ptr()
         a.hidden, a.topk, a.cap, a.site = hidden, route.topk, int(cap), int(site)
         a.partial_par_stride = partial.nbytes // 2 if two else 0
-        self.args, self._ref = a, C.byref(a)
+        self.args = a
         self._launch = _ext.Launcher(_ext.OP_COMBINE, a, "expert_combine")
 
     def launch(self, pdl: bool = False, stream=None):

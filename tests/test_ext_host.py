@@ -404,3 +404,19 @@ def test_launcher_follows_context_grid_and_stream(monkeypatch):
     err = 1
     with pytest.raises(_ext.CudaLaunchError, match="all_gather_v"):
         go(heap, 16, 64, True)
+
+
+def test_operation_numbers_are_the_librarys(lib, monkeypatch):
+    """Loading refuses a library that numbers the operations otherwise, and a launch of none of them is an error."""
+    from moe_comms_benchmarking_b200.ops import _ext
+    assert [lib.mcb_op_name(op).decode() for op in range(len(_ext.OPS))] == list(_ext.OPS)
+    for op in (-1, len(_ext.OPS)):
+        assert lib.mcb_op_name(op) is None
+        assert lib.mcb_launch(C.addressof(_ext.McbLaunch(op=op, grid=1, threads=32)), 0) != 0
+    for ops in (_ext.OPS[:-1], _ext.OPS[1::-1] + _ext.OPS[2:]):         # one less than in the library; two the other way round
+        with monkeypatch.context() as m:
+            m.setattr(_ext, "_lib", None)
+            m.setattr(_ext, "OPS", ops)
+            with pytest.raises(_ext.ExtensionMissing, match="operation drift"):
+                _ext.load()
+    assert _ext.load() is lib
