@@ -275,16 +275,19 @@ __device__ __forceinline__ void load_packs(uint4 (&v)[4], const uint8_t* row, in
   }
 }
 
-// Chunk j of the metadata row: 0 = {stamp, token, id 0, weight 0}, j = {id 2j-1, weight 2j-1, id 2j, weight 2j}.
+// Chunk j of the metadata row: 0 = {stamp, token, id 0, weight 0}, j = {id 2j-1, weight 2j-1, id 2j, weight 2j}; behind the last id
+// {-1, 0}.  Its first id is that of slot meta_slot(j), its second, of a chunk behind the first, the next one.
+__device__ __forceinline__ int meta_slot(int j) { return j == 0 ? 0 : 2 * j - 1; }
+__device__ __forceinline__ uint4 meta_chunk_of(int j, uint32_t stamp, int t, uint2 first, uint2 second) {
+  return j == 0 ? make_uint4(stamp, (uint32_t)t, first.x, first.y) : make_uint4(first.x, first.y, second.x, second.y);
+}
 __device__ __forceinline__ uint4 meta_chunk(const McbA2AStepArgs& a, int t, int j, uint32_t stamp) {
-  const int k0 = j == 0 ? 0 : 2 * j - 1, k1 = 2 * j;
   const long long tb = (long long)t * a.topk;
-  const uint32_t id0 = k0 < a.topk ? (uint32_t)a.topk_idx[tb + k0] : 0xffffffffu;
-  const uint32_t w0 = k0 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k0] : 1.0f) : 0u;
-  if (j == 0) return make_uint4(stamp, (uint32_t)t, id0, w0);
-  const uint32_t id1 = k1 < a.topk ? (uint32_t)a.topk_idx[tb + k1] : 0xffffffffu;
-  const uint32_t w1 = k1 < a.topk ? __float_as_uint(a.topk_w ? a.topk_w[tb + k1] : 1.0f) : 0u;
-  return make_uint4(id0, w0, id1, w1);
+  auto slot = [&](int k) {
+    if (k >= a.topk) return make_uint2(0xffffffffu, 0u);
+    return make_uint2((uint32_t)a.topk_idx[tb + k], __float_as_uint(a.topk_w ? a.topk_w[tb + k] : 1.0f));
+  };
+  return meta_chunk_of(j, stamp, t, slot(meta_slot(j)), j == 0 ? make_uint2(0u, 0u) : slot(2 * j));
 }
 
 // Slice of a row (and, with the first slice, the metadata row) to every destination in the mask.
@@ -575,16 +578,15 @@ struct AloneSlice {
     if (has_id && !good) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)t, (uint32_t)id);
     return __any_sync(0xffffffffu, good);
   }
-  // Chunk j of the metadata row, as in meta_chunk, from the lanes that hold its ids and weights.
+  // The metadata row, chunk by chunk from the lanes that hold its ids and weights.
   __device__ __forceinline__ void deliver_meta(uint64_t par, uint32_t stamp, long long id, float wt) const {
-    const int k0 = lane == 0 ? 0 : 2 * lane - 1, k1 = 2 * lane;
-    const uint32_t my_id = has_id ? (uint32_t)id : 0xffffffffu, my_w = __float_as_uint(wt);
-    const uint32_t id0 = __shfl_sync(0xffffffffu, my_id, k0), w0 = __shfl_sync(0xffffffffu, my_w, k0);
-    const uint32_t id1 = __shfl_sync(0xffffffffu, my_id, k1), w1 = __shfl_sync(0xffffffffu, my_w, k1);
-    const bool have0 = k0 < a.topk, have1 = k1 < a.topk;
-    uint4 m = make_uint4(have0 ? id0 : 0xffffffffu, have0 ? w0 : 0u, have1 ? id1 : 0xffffffffu, have1 ? w1 : 0u);
-    if (lane == 0) m = make_uint4(stamp, (uint32_t)t, id0, w0);
-    if (lane < (int)(a.meta_row_bytes >> 4)) st_v4(meta + par * a.meta_par_stride, m);
+    const uint32_t my_id = has_id ? (uint32_t)id : 0xffffffffu, my_w = has_id ? __float_as_uint(wt) : 0u;
+    auto slot = [&](int k) {                 // k up to 63: lanes wrap around
+      const uint2 v = make_uint2(__shfl_sync(0xffffffffu, my_id, k), __shfl_sync(0xffffffffu, my_w, k));
+      return k < a.topk ? v : make_uint2(0xffffffffu, 0u);
+    };
+    const uint2 first = slot(meta_slot(lane)), second = slot(2 * lane);
+    if (lane < (int)(a.meta_row_bytes >> 4)) st_v4(meta + par * a.meta_par_stride, meta_chunk_of(lane, stamp, t, first, second));
   }
   __device__ __forceinline__ void load(bool on, uint64_t par, uint4 (&v)[PL], uint4 (&w)[PL], long long& id, float& wt) const {
 #pragma unroll
@@ -634,13 +636,9 @@ struct AloneSlice {
 
 // The sum over one destination's row, as the fp32 accumulation from zero rounds it: 0 + v, which drops the sign of a zero.  bf16 adds two
 // values exactly where one of them is zero, so it takes one instruction for two values.
-__device__ __forceinline__ uint32_t plus_zero_bf16x2(uint32_t v) {
-  uint32_t r;
-  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
-  return r;
-}
 __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
-  return sent ? make_uint4(plus_zero_bf16x2(v.x), plus_zero_bf16x2(v.y), plus_zero_bf16x2(v.z), plus_zero_bf16x2(v.w)) : make_uint4(0, 0, 0, 0);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  return sent ? add_bf16x8(v, zero) : zero;
 }
 
 // The layers of a step that writes nothing that it reads (a.apart), dealt to the warps; topk at most 32.
@@ -690,9 +688,9 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
             if (live && l0 + d < L) st_v4(s.out, alone_sum(sent, v[d]));
         }
       } else {
-        // Chunk j of the row (meta_chunk) by lane j, which reads the two ids and weights in it itself.
+        // A chunk of the row by each lane, which reads the two ids and weights in it itself.
         const uint32_t par = (uint32_t)(k - sums) & 1u;
-        const int k0 = lane ? 2 * lane - 1 : 0, k1 = 2 * lane;
+        const int k0 = meta_slot(lane), k1 = 2 * lane;
         const bool have0 = k0 < a.topk, have1 = k1 < a.topk, mine = lane < (int)(a.meta_row_bytes >> 4);
         const int64_t* ids = a.topk_idx + (int64_t)s.t * a.topk;
         const float* ws = a.topk_w ? a.topk_w + (int64_t)s.t * a.topk : nullptr;
@@ -717,7 +715,7 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
             if (have1 && !good1) report_error(c, MCB_ERR_ROUTING, MCB_SITE_A2A_STEP, blockIdx.x, (uint32_t)s.t, id[d][1].x);
             if (!__any_sync(0xffffffffu, good0 || good1) || !mine) continue;
             const uint32_t stamp = layer_base + (uint32_t)(l0 + 2 * d) + 1u;
-            st_v4(meta, lane ? make_uint4(id[d][0].x, wt[d][0], id[d][1].x, wt[d][1]) : make_uint4(stamp, (uint32_t)s.t, id[d][0].x, wt[d][0]));
+            st_v4(meta, meta_chunk_of(lane, stamp, s.t, make_uint2(id[d][0].x, wt[d][0]), make_uint2(id[d][1].x, wt[d][1])));
           }
         }
       }
@@ -749,24 +747,18 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
           for (int k = 0; k < K; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int d = 0; d < D; d += 2) {
-          float m[2];
-          if constexpr (FP8) block_absmax_wide(v[d], v[d + 1], m[0], m[1]);
+          auto at = [&](uint8_t* base, uint64_t par_stride, int k) { return base + ((layer_base + (uint32_t)(l0 + d + k)) & 1u ? par_stride : 0); };
+          if constexpr (FP8) {
+            quant_wide_pair(v[d], v[d + 1], [&](int k) { return l0 + d + k < last && sent && live; }, [&](int k, uint4 q, float scale) {
+              st_v4(at(recv, a.x_par_stride, k), q);
+              if ((lane & 7) == 0) st_b32(at(scales, a.scale_par_stride, k), __float_as_uint(scale));
+            });
+          } else {
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (l0 + d + e >= last) break;
-            const uint32_t par = (layer_base + (uint32_t)(l0 + d + e)) & 1u;
-            const uint4* r = v[d + e];
-            uint8_t* dst = recv + (par ? a.x_par_stride : 0);
-            if constexpr (FP8) {
-              const float scale = e4m3_scale(m[e]);
-              if (sent && live) {
-                const uint2 q0 = quant_pack_e4m3(r[0], scale), q1 = quant_pack_e4m3(r[1], scale);
-                st_v4(dst, make_uint4(q0.x, q0.y, q1.x, q1.y));
-                if ((lane & 7) == 0) st_b32(scales + (par ? a.scale_par_stride : 0), __float_as_uint(scale));
-              }
-            } else {
-              if (sent && live) st_v4(dst, r[0]);
-              if (s.echo && live) st_v4(out, alone_sum(sent, r[0]));
+            for (int k = 0; k < 2; ++k) {
+              if (l0 + d + k >= last || !live) break;
+              if (sent) st_v4(at(recv, a.x_par_stride, k), v[d + k][0]);
+              if (s.echo) st_v4(out, alone_sum(sent, v[d + k][0]));
             }
           }
         }

@@ -349,19 +349,12 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
 #pragma unroll
           for (int k = 0; k < 2; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int d = 0; d < D; d += 2) {
-          float m[2];
-          block_absmax_wide(v[d], v[d + 1], m[0], m[1]);
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            if (!live || l0 + d + k >= last) continue;
+        for (int d = 0; d < D; d += 2)
+          quant_wide_pair(v[d], v[d + 1], [&](int k) { return live && l0 + d + k < last; }, [&](int k, uint4 q, float scale) {
             const uint32_t par = (layer_base + (uint32_t)(l0 + d + k)) & 1u;
-            const float sc = e4m3_scale(m[k]);
-            const uint2 q0 = quant_pack_e4m3(v[d + k][0], sc), q1 = quant_pack_e4m3(v[d + k][1], sc);
-            st_v4(q_dst + (par ? a.dst_par_stride[0] : 0), make_uint4(q0.x, q0.y, q1.x, q1.y));
-            if ((lane & 7) == 0) st_b32(s_dst + (par ? a.dst_par_stride[3] : 0), __float_as_uint(sc));
-          }
-        }
+            st_v4(q_dst + (par ? a.dst_par_stride[0] : 0), q);
+            if ((lane & 7) == 0) st_b32(s_dst + (par ? a.dst_par_stride[3] : 0), __float_as_uint(scale));
+          });
       }
     });
   };
@@ -444,9 +437,8 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
 #pragma unroll
       for (int d = 0; d < Q; d += 2) {
         if (g + d / D * warps >= quants || d % D >= L) break;
-        quant_wide_pair(v[d], v[d + 1], [&](int k, uint4 q, float scale) {
+        quant_wide_pair(v[d], v[d + 1], [&](int k) { return i[d + k] < halves && (d + k) % D < L; }, [&](int k, uint4 q, float scale) {
           const int at = d + k, l = at % D;
-          if (i[at] >= halves || l >= L) return;
           st_v4(q_dst + i[at] * 16 + (parity(l) ? a.dst_par_stride[0] : 0), q);
           if ((lane & 7) == 0) st_b32(s_dst + (i[at] >> 3) * 4 + (parity(l) ? a.dst_par_stride[3] : 0), __float_as_uint(scale));
         });
