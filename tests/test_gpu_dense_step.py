@@ -221,8 +221,7 @@ def test_step_kernel_check_payload_depends_on_the_layer(lib):
 @pytest.mark.parametrize("K,grid,threads", [(22, 148, 512), (5, 2, 64), (3, 1, 32)])
 def test_world_of_one_copies(lib, dtype, K, grid, threads):
     """A world of one: the layers of a step are flat copies of all ranges of a layer at once.  Rows of 8, 12, 20,
-    24 or 40 bytes leave words behind the last whole 16-byte pack, and the small grids reach both sides of the line
-    between the packs a thread keeps for all layers and those it works out layer by layer."""
+    24 or 40 bytes leave words behind the last whole 16-byte pack, and the small grids take several rounds of packs."""
     cap, H = 132, 264
     rig = _Rig(1, cap, H, K, 0, dtype)
     for step, (n, layers) in enumerate([(1, 3), (3, 2), (132, 2), (0, 1), (7, 4)]):
@@ -233,8 +232,8 @@ def test_world_of_one_copies(lib, dtype, K, grid, threads):
     rig.w.check_status()
 
 
-@pytest.mark.parametrize("n", [1, 2, 4, 5, 9, 16])          # 17.5 packs a row on 64 threads: up to 1, 2, 4 packs per thread and more
-@pytest.mark.parametrize("layers", [1, 2, 7, 8, 9, 17])     # on both sides of the layers whose loads go out together
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 9, 16])          # 17.5 packs a row on two warps: a ragged group of packs, words behind the last one
+@pytest.mark.parametrize("layers", [1, 2, 7, 8, 9, 17])     # every number of groups at a time, one less, and steps dealt in runs
 def test_world_of_one_layers_in_flight(lib, n, layers):
     rig = _Rig(1, 16, 64, 2, 0)
     rig.new_inputs()
@@ -298,7 +297,7 @@ def test_world_of_one_step_on_its_own_rows(lib, form, n, layers):
             assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 17])          # 32 packs to quantise a row on 96 threads: up to 1, 2, 4 per thread and more
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 17])          # 32 packs to quantise a row on three warps: fewer groups of 64 than warps, and more
 @pytest.mark.parametrize("layers", [1, 3, 8, 9])
 @pytest.mark.parametrize("out_cols", [256, 64])             # as many packs of expert outputs, and fewer than are quantised
 def test_world_of_one_quantised_layers_in_flight(lib, n, layers, out_cols):

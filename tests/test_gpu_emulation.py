@@ -321,10 +321,10 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
 @pytest.mark.parametrize("H,K,n,layers,grid,threads", [
     (128, 1, 1, 1, 148, 512),            # half a slice of one pack per lane, one id
     (1024, 32, 5, 17, 148, 512),         # 17 metadata chunks; a remainder of layers
-    (1152, 5, 8, 9, 2, 320),             # 20 warps: two packs per lane, 16 packs in the last slice
-    (1152, 5, 9, 3, 2, 320),             # four packs per lane
-    (2048, 8, 5, 2, 10, 64),             # as many slices as warps
-    (2048, 8, 6, 4, 5, 64),              # more slices than warps
+    (1152, 5, 8, 9, 2, 320),             # 20 warps: pieces of 16 packs at the end of a row, a chain each for 16 warps
+    (1152, 5, 9, 3, 2, 320),             # three layers: slices of four packs per lane, a ragged one a row
+    (2048, 8, 5, 2, 10, 64),             # two: more slices of one pack per lane than warps, so of four
+    (2048, 8, 6, 4, 5, 64),              # four: more slices of four than warps
     (7168, 33, 3, 4, 148, 512),          # more ids than lanes
     (1152, 5, 3, 9, 6, 256),             # 48 warps: a chain each for some, runs that begin and end inside a piece's layers
     (256, 2, 2, 33, 8, 64),              # more layers than a chain has in flight
@@ -569,3 +569,64 @@ def test_a2a_step_alone_metadata(world1, fp8, K):
             assert torch.equal(bufs.recv_x.tensor[par, 0].cpu(), q.view(torch.uint8)) and torch.equal(bufs.recv_scale.tensor[par, 0].cpu(), scale)
         else:
             assert torch.equal(bufs.recv_x.tensor[par, 0], x)
+
+
+@pytest.mark.parametrize("n,layers,grid,threads", [(3, 1, 148, 512), (5, 8, 148, 512), (40, 3, 2, 320)])
+def test_a2a_step_in_place_bf16(world1, n, layers, grid, threads):
+    """A step whose output is its input, identity expert on bf16 rows: the rows stay as they are but for the sign of zeros, which the
+    first layer's sum drops, and the row for no expert, which is zero."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, K, H, cap = 16, 4, 1152, n + 1
+    heap = SymmetricHeap(world1, 16 << 20, DEV)
+    bufs = A2AStepBuffers(heap, cap, H, K, False)
+    g = torch.Generator(device=DEV).manual_seed(59)
+    x = torch.randn(cap, H, device=DEV, generator=g).to(torch.bfloat16)
+    x[0, :2] = torch.tensor([0.0, -0.0])
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(cap)])
+    idx[n - 1] = -1
+    meta = torch.zeros(8, dtype=torch.int32, device=DEV)
+    bufs.recv_x.tensor.zero_()
+    before = x.clone()
+    A2AStepPlan(heap, bufs, x, idx, torch.rand(cap, K, device=DEV), x, torch.tensor([n], dtype=torch.int32, device=DEV), meta, E, layers,
+                grid=grid, threads=threads).launch()
+    torch.cuda.synchronize()
+    with pytest.raises(DeviceStatusError):
+        heap.check_status()
+    bits = lambda t: t.contiguous().view(torch.int16)
+    plain = before + 0.0                                # -0 + 0 = +0
+    assert torch.equal(bits(x[:n - 1]), bits(plain[:n - 1])) and not bits(x[n - 1]).any() and torch.equal(bits(x[n:]), bits(before[n:]))
+    last = int(meta[5])
+    for age, par in enumerate((last, 1 - last)[:layers]):
+        sent = before if layers - 1 - age == 0 else plain
+        assert torch.equal(bits(bufs.recv_x.tensor[par, 0, :n - 1]), bits(sent[:n - 1])) and not bits(bufs.recv_x.tensor[par, 0, n - 1:]).any()
+        words = bufs.recv_meta.tensor[par, 0, :n - 1].view(torch.int32).view(n - 1, -1)
+        assert bool((words[:, 0] == int(meta[7]) - age).all())
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("K,layers", [(5, 1), (5, 3), (5, 9), (32, 9), (33, 9)])
+def test_a2a_step_alone_without_weights(world1, fp8, K, layers):
+    """Without weights a step delivers weight 1: every received byte as with a tensor of ones, by slices, pieces and beyond one id per lane."""
+    from moe_comms_benchmarking_b200.ops.a2a import A2AStepBuffers, A2AStepPlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    E, H, n = 40, 1152, 7
+    g = torch.Generator(device=DEV).manual_seed(K + layers)
+    x, y = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((n, H), (2, 1, n, H)))
+    idx = torch.stack([torch.randperm(E, device=DEV, generator=g)[:K] for _ in range(n)])
+    got = []
+    for wt in (None, torch.ones(n, K, device=DEV)):
+        heap = SymmetricHeap(world1, 16 << 20, DEV)
+        bufs = A2AStepBuffers(heap, n, H, K, fp8)
+        if fp8:
+            bufs.y.tensor.copy_(y)
+        out, meta = torch.zeros(n, H, dtype=torch.bfloat16, device=DEV), torch.zeros(8, dtype=torch.int32, device=DEV)
+        for t in (bufs.recv_x, bufs.recv_meta):
+            t.tensor.zero_()
+        A2AStepPlan(heap, bufs, x, idx, wt, out, torch.tensor([n], dtype=torch.int32, device=DEV), meta, E, layers).launch()
+        torch.cuda.synchronize()
+        heap.check_status()
+        got.append([t.contiguous().view(torch.uint8).clone() for t in (out, meta, bufs.recv_x.tensor, bufs.recv_meta.tensor)])
+        words = bufs.recv_meta.tensor[int(meta[5]), 0].view(torch.int32).view(n, -1)
+        assert torch.equal(words[:, 2:2 + 2 * K:2].long(), idx) and bool((words[:, 3:3 + 2 * K:2].contiguous().view(torch.float32) == 1).all())
+    assert all(torch.equal(a, b) for a, b in zip(*got))
