@@ -647,16 +647,18 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 //   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token and parity, which
 //            carries the number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
-// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 (6 TB/s with bf16 rows); the
-// loads of a piece's layers hit L1.  One B200, against layers one after the other, in slices of up to 128 packs a warp:
-//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows
-//     bf16   35 -> 10.6 / 37 -> 12.6 / 41 -> 33 / 77 -> 72 / 271 -> 265 us
-//     e4m3   45 -> 10.8 / 45 -> 12.6 / 56 -> 37 / 91 -> 76 / 404 -> 272 us
-//   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 4096 rows
-//     bf16   25 -> 8.5 / 27 -> 18 / 99 -> 93 / 263 -> 268 (265 -> 283 on another) / 1690 -> 1088 us
-//     e4m3   31 -> 10.5 / 35 -> 19 / 112 -> 100 / 407 -> 283 / 2211 -> 1120 us
+// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 (6 TB/s with bf16 rows), which also
+// serves the loads: of 10.8 million sectors of 24 layers of 333 e4m3 rows of 7168 48 thousand hit L1.  One B200, against up to four packs per
+// lane with up to eight layers in flight where the slices fit the warps, else slices of four packs layer after layer:
+//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows (* by slices, alone_full)
+//     bf16   35 -> 10.5 / 35 -> 12.5 / 40 -> 33 / 76 -> 68 / 272 -> 249 * us
+//     e4m3   43 -> 10.5 / 45 -> 12.5 / 56 -> 29 / 91 -> 73 / 398 -> 268 us
+//   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 2048 rows
+//     bf16   25 -> 8.5 / 27 -> 18 / 101 -> 96 * / 262 -> 253 * / 786 -> 533 * us
+//     e4m3   31 -> 10.2 / 35 -> 19 / 112 -> 99 / 402 -> 280 / 969 -> 563 us
 // With one chain for both parities of a metadata row, its chunks put together by shuffles, the smallest steps took 16.7 and 14.6 us.
-// The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.
+// The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.  Slower than slices
+// remain e4m3 steps of five to seven layers, by up to 15 % at some sizes.
 template <bool FP8>
 __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   constexpr int K = FP8 ? 2 : 1;             // packs per lane of a piece

@@ -317,14 +317,17 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 
 // Nothing that a layer reads is written in the step (else: a.in_order), and all layers of a parity deliver the same rows, so the layers
 // need no order: a warp takes all layers of a few packs, and every warp gets the same number of (pack, layer) whatever the batch.  Large
-// steps are bound by the stores into L2 (7.6 TB/s at 8192 rows): the chip works on a few MB at a time, and what a warp loads in one layer
-// after the other it finds in L1.  Layer after layer over all rows, large steps went through up to 90 MB of L2 in every layer, small ones
+// steps are bound by the stores into L2 (7.6 TB/s at 8192 rows), which also serves every load: the loads' hint keeps them out of L1 (of 6.7
+// million sectors of 24 layers of 2048 rows two thousand hit there).  But the chip works on a few MB at a time; layer after layer over
+// all rows, large steps went through up to 90 MB of L2 in every layer, small ones
 // left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
-// One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against layers one after the other:
-//   bf16   29 -> 6.4 / 35 -> 8.5 / 25 -> 12.6 / 49 -> 33 / 41 -> 34 / 169 -> 112 / 655 -> 411 us
-//   e4m3   45 -> 8.5 / 53 -> 10.5 / 41 -> 14.5 / 52 -> 33 / 41 -> 37 / 154 -> 121 / 923 -> 451 us
+// One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against up to four packs per thread with up to eight
+// layers in flight where a step fits, else layer after layer:
+//   bf16   29 -> 6.4 / 35 -> 8.4 / 25 -> 12.5 / 48 -> 35 / 39 -> 35 / 169 -> 111 / 651 -> 411 us
+//   e4m3   45 -> 8.4 / 53 -> 10.4 / 41 -> 14.5 / 53 -> 33 / 42 -> 37 / 150 -> 121 / 956 -> 450 us
 // and 58 layers of hidden 7168 and top-8, 1 / 64 / 512 / 2048 rows, bf16 19 -> 6.5 / 29 -> 21 / 178 -> 116 / 961 -> 425, e4m3 with 512 / 2048
-// rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.
+// rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.  One size was
+// slower than before, e4m3 steps of 9 to 16 layers of about 512 rows of 1024, by up to 7 %.
 template <bool FP8>
 __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, uint32_t layer_base) {
   const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
