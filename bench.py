@@ -205,6 +205,8 @@ def run_native(args):
             "metric": "ms per 88-layer MoE decode step (device-timed, max over ranks)",
             "value": round(value_ms, 4), "unit": "ms", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": round(value_ms, 4), "higher_is_better": False, "scaling": "strong",
+            "layer_order": "any: in a world of one the layers of this workload do not depend on one another, so value is not the time of "
+                           "dependent layers" if world == 1 and not args.no_persistent else "one after the other",
             "vs_baseline": round(value_ms / pub[0], 4) if pub else None,
             "vs_baseline_note": "published figure is the reference's NVLS curve at EP=4 on 4xB200, digitised from "
                                 "results.png; EP differs when n_gpus != 4",
