@@ -329,6 +329,8 @@ def test_a2a_step_kernel_row_slices(lib, W, fp8, H, grid, threads):
     (1152, 5, 3, 9, 6, 256),             # 48 warps: a chain each for some, runs that begin and end inside a piece's layers
     (256, 2, 2, 33, 8, 64),              # more layers than a chain has in flight
     (1152, 5, 7, 5, 1, 64),              # two warps: many chains each, one of them one more
+    (256, 3, 7, 6, 3, 160), (256, 3, 9, 33, 3, 160),      # 15 warps, 14 with a chain more: runs that the others alone take, and all
+    (128, 2, 8, 7, 1, 96), (2048, 4, 4, 5, 16, 512),      # most warps with a chain more; fewer items than warps without
 ])
 def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads):
     """A step in a world of one whose layers run into each other, against the kernel of the emulated ranks, which takes
