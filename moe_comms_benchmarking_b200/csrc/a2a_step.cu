@@ -805,7 +805,7 @@ __device__ __forceinline__ void alone_slices(const McbCtx& c, const McbA2AStepAr
 }
 
 // A step of up to this many layers has too few of one piece to keep loads in flight: there the warps take slices, of one pack per lane
-// where that still gives every slice a warp of its own, else of four.  Kernels of their own, for one layer (D = 1) and for more (D = 2), which are
+// or two where that still gives every slice a warp of its own, else of four (four instead of two: 811 e4m3 rows of 1024 15 to 25 % slower).  Kernels of their own, for one layer (D = 1) and for more (D = 2), which are
 // smaller than that of the dealt steps.  One B200, a step of 1 / 2 / 3 / 4 layers in a row of steps, dealt -> slices:
 //   hidden 1024 and top-22, 64 rows     bf16 5.0 / 4.5 / 4.6 / 4.5 -> 4.2 / 4.3 / 4.9 / 4.7      e4m3 5.2 / 5.3 / 4.8 / 4.8 -> 4.2 / 4.7 / 4.8 / 5.1 us
 //                          8192 rows    bf16 32.4 / 28.2 / 29.3 / 33.1 -> 9.8 / 15.5 / 21.0 / 26.7  e4m3 40.1 / 42.7 / 47 / 49 -> 13.0 / 20.0 / 27.6 / 33.5
@@ -818,6 +818,7 @@ template <bool FP8, int D>
 __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5), packs = a.hidden / 8;
   if (n * ((packs + 31) / 32) <= warps) alone_slices<FP8, 1, D>(c, a, n, layer_base);
+  else if (n * ((packs + 63) / 64) <= warps) alone_slices<FP8, 2, D>(c, a, n, layer_base);
   else alone_slices<FP8, 4, D>(c, a, n, layer_base);
 }
 

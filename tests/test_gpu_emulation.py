@@ -374,6 +374,7 @@ def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, 
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("H,K,n,layers,grid,threads", [
     (1152, 5, 6, 1, 148, 512), (2048, 32, 5, 2, 148, 512),      # a warp for every slice of one pack per lane
+    (1152, 5, 9, 1, 2, 512), (1152, 5, 10, 3, 2, 512),          # for every slice of two, the third of a row of 16 packs
     (1152, 5, 9, 1, 1, 64), (1152, 5, 9, 2, 2, 64),             # slices of four, the second of a row ragged, in several rounds
     (256, 8, 7, 3, 3, 32), (1024, 6, 8, 4, 2, 96),              # an odd layer at the end, and none
     (1024, 6, 8, 5, 2, 96),                                     # the first that is dealt
