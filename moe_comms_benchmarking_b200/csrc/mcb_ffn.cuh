@@ -223,14 +223,21 @@ __device__ __forceinline__ void ffn_plan(FfnPlanS& plan, const McbFfnArgs& a, in
     // So many slots, of average size, that their down units alone make two rounds of the grid: that is how far the last slot's are from
     // its gate/up units.  With three rounds of all units (which are one of down units where n1 = 2 n2) they waited there: 8191 tokens with
     // Zipf routing, an eighth of 512 experts of 1024 x 1024, 129.6 -> 127.2 us (three rounds of down units 126.5, all gate/up units first
-    // 126.9); 4096 tokens of all experts the same (three rounds of down units 0.3 % slower).
+    // 126.9); 4096 tokens of all experts the same (three rounds of down units 0.3 % slower).  Where down units are more than twice as many as gate/up
+    // units three rounds of all units are the longer distance and stay: 48 experts of 3072 x 256 with 1100 tokens 394 us by two rounds of
+    // down units, 377 so, 64 of 7168 x 512 with 700 1180 and 1152, 32 of 4096 x 512 with 1100 508 and 520.
     // In slots the distance grows with n1 / n2.  Three rounds of all units -> this, warm clocks, us a launch, with the activations between the two:
     //   n1 = 8 n2   200 experts of 512 x 2048 with 250 tokens 464 -> 460 (14 -> 78 MB), 64 with 256 168.0 -> 165.6 (all first, 67 MB), 48 with 512
     //               218.8 -> 216.5, 16 with 1500 188.5 -> 185.7, 24 of 1024 x 4096 with 400 313.8 -> 314.2
+    //   n1 = 6 n2   64 of 512 x 1536 with 256, Zipf 130.8 -> 125.4, with 180 103.5 -> 100.5
     //   n1 = 4 n2   128 of 1024 x 2048 with 200 413.5 -> 424.5 (431 -> 432 on another), Zipf 458 -> 461, 100 of 512 x 1024 with 300 157.6 -> 155.7
-    //   n2 > n1     64 of 4096 x 512 with 512 530 -> 530
-    // so nothing asks for a bound in bytes: one of 24 MB gave between -4 and +2.5 % over these, with no trend in the shape.
-    const int lag = (int)((long long)gridDim.x * active / (plan.n2 * plan.cum[active])) + 2;
+    //   n1 = 3 n2   64 of 1536 x 2048 with 300 488 -> 494, 32 of 1024 x 1536 with 300 127 -> 124
+    //   n1 = n2     32 of 3072 x 1536 with 700 649 -> 658, 32 of 7168 x 1024 (0.6 n2) with 700 1036 -> 1015
+    // so nothing asks for a bound in bytes: one of 24 MB gave between -4 and +2.5 % over shapes up to n1 = 8 n2, with no trend in the shape.
+    const long long chunks = plan.cum[active];
+    const int down = (int)((long long)gridDim.x * active / (plan.n2 * chunks)) + 2;
+    const int all = (int)((long long)gridDim.x * 3 / 2 * active / ((plan.n1 + plan.n2) * chunks)) + 2;
+    const int lag = down > all ? down : all;
     if (lag < plan.lag) plan.lag = lag;
   }
 }

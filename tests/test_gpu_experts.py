@@ -342,13 +342,15 @@ def _down_distance(rows, H, I, grid):
     come behind its gate/up units."""
     active, chunks, grid = sum(r > 0 for r in rows), sum((r + 255) // 256 for r in rows), max(grid & ~1, 2)
     beyond = sum(rows) * I * 2 > 24 << 20                # bytes of activations that stay within L2
-    return active, min(active, grid * active // (H // 256 * chunks) + 2) if beyond else active
+    down, both = H // 256 * chunks, (H + 2 * I) // 256 * chunks
+    return active, min(active, max(grid * active // down, grid * 3 // 2 * active // both) + 2) if beyond else active
 
 
 @pytest.mark.parametrize("rows,H,I,grid", [
     ([700, 300, 1, 900, 0, 600, 256, 257, 500, 1200], 1024, 2816, 14),     # seven CTA pairs, chunked, tiny and idle experts
     ([700, 300, 1, 900, 0, 600, 256, 257, 500, 1200], 1024, 2816, 15),
     ([96 + 5 * i for i in range(20)] + [0] + [110] * 40, 1024, 2048, 148), # one chunk each; the whole chip
+    ([300, 40, 700] * 16, 4096, 896, 148),                                 # more down units than twice the gate/up units
     ([257] * 30, 2560, 1664, 6),                                           # a second chunk of one row, long distance in units
 ])
 def test_expert_ffn_down_units_at_a_distance(world1, rows, H, I, grid):
