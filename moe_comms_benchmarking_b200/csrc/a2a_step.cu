@@ -537,8 +537,8 @@ __global__ void __launch_bounds__(512) a2a_step_kernel(const __grid_constant__ M
 // ---- a world of one -----------------------------------------------------------------------------------
 // Nobody to wait for: a slice is delivered and combined in one go, with every load of it in flight at once.  The identity expert on
 // bf16 rows returns the row just delivered, which is still in registers.  PL = packs per lane; a lane holds one expert id (topk at most 32, others take
-// barrier_alone).
-template <bool FP8, int PL>
+// barrier_alone).  KEEP: loads may stay in L1 for the next layer of the slice (steps that write nothing that they read).
+template <bool FP8, int PL, bool KEEP = false>
 struct AloneSlice {
   const McbA2AStepArgs& a;
   const int lane, row_packs;
@@ -592,8 +592,9 @@ struct AloneSlice {
 #pragma unroll
     for (int u = 0; u < PL; ++u) {
       const bool live = on && p0 + u * 32 < row_packs;
-      v[u] = live ? ld_v4_stream(x + u * 512) : make_uint4(0, 0, 0, 0);
-      if (!echo) w[u] = live ? ld_v4_stream(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
+      auto ld = [](const uint8_t* p) { return KEEP ? ld_v4(p) : ld_v4_stream(p); };
+      v[u] = live ? ld(x + u * 512) : make_uint4(0, 0, 0, 0);
+      if (!echo) w[u] = live ? ld(y + par * a.y_par_stride + u * 512) : make_uint4(0, 0, 0, 0);
     }
     id = load_id(on);
     wt = load_weight(on && head);
@@ -647,8 +648,10 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 //   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token and parity, which
 //            carries the number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
-// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 (6 TB/s with bf16 rows), which also
-// serves the loads: of 10.8 million sectors of 24 layers of 333 e4m3 rows of 7168 48 thousand hit L1.  One B200, against up to four packs per
+// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 and, with e4m3 rows, by the integer
+// instructions of the quantisation; the loads may stay in L1, where 95 % of their sectors hit (24 layers of 333 e4m3 rows of 7168).  From L2, which the
+// hint against L1 made of every load: 58 layers of 333 / 1000 / 2048 e4m3 rows of 7168 98.9 / 283 / 559 -> 85.9 / 236 / 466 us, 88 layers of 333 / 2048 / 8192 of
+// 1024 29.9 / 141 / 527 -> 24.9 / 121 / 446, bf16 rows 33.3 / 124 * / 465 * -> 31.1 / 116 * / 427 *.  One B200, loads from L2, against up to four packs per
 // lane with up to eight layers in flight where the slices fit the warps, else slices of four packs layer after layer:
 //   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows (* by slices, alone_full)
 //     bf16   35 -> 10.5 / 35 -> 12.5 / 40 -> 33 / 76 -> 68 / 272 -> 249 * us
@@ -684,7 +687,7 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
           uint4 v[D];
 #pragma unroll
           for (int d = 0; d < D; ++d)
-            v[d] = live && l0 + d < L ? ld_v4_stream(s.y + ((layer_base + (uint32_t)(l0 + d)) & 1u ? a.y_par_stride : 0)) : make_uint4(0, 0, 0, 0);
+            v[d] = live && l0 + d < L ? ld_v4(s.y + ((layer_base + (uint32_t)(l0 + d)) & 1u ? a.y_par_stride : 0)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
           for (int d = 0; d < D; ++d)
             if (live && l0 + d < L) st_v4(s.out, alone_sum(sent, v[d]));
@@ -751,7 +754,7 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
 #pragma unroll
         for (int d = 0; d < D; ++d)
 #pragma unroll
-          for (int k = 0; k < K; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
+          for (int k = 0; k < K; ++k) v[d][k] = live && l0 + d < last ? ld_v4(src + k * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int d = 0; d < D; d += 2) {
           auto at = [&](uint8_t* base, uint64_t par_stride, int k) { return base + ((layer_base + (uint32_t)(l0 + d + k)) & 1u ? par_stride : 0); };
@@ -784,7 +787,7 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
 // A warp takes a slice of a row and, D at a time, all its layers; steps that write nothing that they read.
 template <bool FP8, int PL, int D>
 __device__ __forceinline__ void alone_slices(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
-  AloneSlice<FP8, PL> s(a);
+  AloneSlice<FP8, PL, !FP8> s(a);       // e4m3 rows kept in L1: one or two layers of 2048 rows of 7168 3 to 6 % slower
   const long long mine = (long long)n * s.slices(), step = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long i = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x; i < mine; i += step) {
     s.at(c, i);

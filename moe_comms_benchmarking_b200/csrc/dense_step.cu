@@ -316,11 +316,13 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 }
 
 // Nothing that a layer reads is written in the step (else: a.in_order), and all layers of a parity deliver the same rows, so the layers
-// need no order: a warp takes all layers of a few packs, and every warp gets the same number of (pack, layer) whatever the batch.  Large
-// steps are bound by the stores into L2 (7.6 TB/s at 8192 rows), which also serves every load: the loads' hint keeps them out of L1 (of 6.7
-// million sectors of 24 layers of 2048 rows two thousand hit there).  But the chip works on a few MB at a time; layer after layer over
-// all rows, large steps went through up to 90 MB of L2 in every layer, small ones
+// need no order: a warp takes all layers of a few packs, and every warp gets the same number of (pack, layer) whatever the batch.  The
+// chip works on a few MB at a time; layer after layer over all rows, large steps went through up to 90 MB of L2 in every layer, small ones
 // left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
+// The loads may stay in L1, where 95 % of their sectors hit (24 layers of 2048 rows): large steps are bound by the stores into L2, and loads with the
+// hint that keeps them out of L1 took a third of its time.  88 layers of 1000 / 2048 / 8192 rows of 1024 60.7 / 107.8 / 417 -> 50.3 / 88.1 / 335 us
+// (9.4 TB/s of stores), e4m3 65.9 / 121 / 451 -> 55.8 / 103 / 382; 58 layers of 333 / 2048 rows of 7168 83 / 416 -> 69.5 / 327, e4m3 93 / 502 ->
+// 78 / 438.  The figures below are of loads from L2.
 // One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against up to four packs per thread with up to eight
 // layers in flight where a step fits, else layer after layer:
 //   bf16   29 -> 6.4 / 35 -> 8.4 / 25 -> 12.5 / 48 -> 35 / 39 -> 35 / 169 -> 111 / 651 -> 411 us
@@ -350,7 +352,7 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
 #pragma unroll
         for (int d = 0; d < D; ++d)
 #pragma unroll
-          for (int k = 0; k < 2; ++k) v[d][k] = live && l0 + d < last ? ld_v4_stream(src + k * 16) : make_uint4(0, 0, 0, 0);
+          for (int k = 0; k < 2; ++k) v[d][k] = live && l0 + d < last ? ld_v4(src + k * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int d = 0; d < D; d += 2)
           quant_wide_pair(v[d], v[d + 1], [&](int k) { return live && l0 + d + k < last; }, [&](int k, uint4 q, float scale) {
@@ -383,7 +385,7 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
       const uint8_t* src = r.src[t] + off;
       uint8_t* dst = r.dst[t] + off;
       const uint64_t par_off = r.par[t];
-      local_layers_of(first, last, [&] { return live ? ld_v4_stream(src) : make_uint4(0, 0, 0, 0); },
+      local_layers_of(first, last, [&] { return live ? ld_v4(src) : make_uint4(0, 0, 0, 0); },
                       [&](uint4 v0, uint4 v1, bool on0, bool on1, int l) {
         const uint32_t par = (layer_base + (uint32_t)l) & 1u;
         if (live && on0) st_v4(dst + (par ? par_off : 0), v0);
@@ -409,7 +411,9 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
 //                          8192 rows    bf16 34.9 / 35.7 / 37 / 41 -> 11.9 / 17.0 / 25.8 / 39.2  e4m3 30.5 / 33.7 / 39 / 54 -> 13.7 / 19.2 / 28.7 / 50
 //   hidden 7168 and top-8, 2048 rows    bf16 56 / 61 / 62 / 66 -> 20.4 / 31.3 / 41.5 / 61        e4m3 51 / 56 / 65 / 89 -> 20.6 / 31.5 / 47.6 / 81
 // (layer after layer, 8192 rows of 1024: bf16 12.0 / 19.8 / 34.9 / 63, e4m3 17.1 / 27.9 / 52 / 96).  Nine to sixteen layers by rounds of eight:
-// up to 25 % slower than runs with bf16 rows, 10 % faster to 10 % slower with e4m3 rows, so the line is at one round.
+// up to 25 % slower than runs with bf16 rows, 10 % faster to 10 % slower with e4m3 rows, so the line is at one round.  Loads of the layers of a pack
+// after the first hit L1 here too: 4 / 8 layers of 2048 rows of 7168 41.4 / 61.8 -> 38.3 / 50.6 us, e4m3 46.3 / 81 -> 44.4 / 75.9 (the figures above are of
+// loads from L2).
 constexpr int kFewLayers = 8;
 
 template <bool FP8, int D>
@@ -435,7 +439,7 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
         i[d] = (g + d / D * warps) * 32 + lane;
         const bool on = i[d] < halves && d % D < L;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) v[d][k] = on ? ld_v4_stream(rows + i[d] * 32 + k * 16) : make_uint4(0, 0, 0, 0);
+        for (int k = 0; k < 2; ++k) v[d][k] = on ? ld_v4(rows + i[d] * 32 + k * 16) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int d = 0; d < Q; d += 2) {
@@ -468,7 +472,7 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
         par_off[u] = r.par[t];
 #pragma unroll
         for (int d = 0; d < D; ++d)
-          if (d < L) v[u][d] = ld_v4_stream(r.src[t] + off);
+          if (d < L) v[u][d] = ld_v4(r.src[t] + off);
       }
     }
 #pragma unroll
