@@ -42,7 +42,13 @@ __device__ __forceinline__ uint2 quant_pack_e4m3(uint4 v, float scale) {
       q[i] = __nv_cvt_float2_to_fp8x2(make_float2(__fdiv_rn(bf16_lo(w[i]), scale), __fdiv_rn(bf16_hi(w[i]), scale)), __NV_SATFINITE,
                                       __NV_E4M3);
   }
-  return make_uint2(__byte_perm(q[0], q[1], 0x5410), __byte_perm(q[2], q[3], 0x5410));
+  // By a move of halves, which the conversion can do itself; as byte permutations the steps with e4m3 rows were 1 to 4 % slower.
+  auto join = [](uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mov.b32 %0, {%1, %2};" : "=r"(r) : "h"((uint16_t)a), "h"((uint16_t)b));
+    return r;
+  };
+  return make_uint2(join(q[0], q[1]), join(q[2], q[3]));
 }
 
 // Largest magnitudes of the even and of the odd values of a pack, as bf16x2 (NaNs are passed over).
@@ -52,8 +58,13 @@ __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
   return r;
 }
 __device__ __forceinline__ uint32_t pack_absmax2(uint4 v) {
-  constexpr uint32_t kAbs = 0x7fff7fffu;
-  return max_bf16x2(max_bf16x2(v.x & kAbs, v.y & kAbs), max_bf16x2(v.z & kAbs, v.w & kAbs));
+  // Of magnitudes, with a sign that is cleared once (cleared on the way in, 1 to 2 % of the steps with e4m3 rows, which are bound by the ALU pipe).
+  auto absmax = [](uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  };
+  return absmax(absmax(v.x, v.y), absmax(v.z, v.w)) & 0x7fff7fffu;
 }
 __device__ __forceinline__ float pack_absmax(uint4 v) {
   const uint32_t m = pack_absmax2(v);

@@ -433,6 +433,36 @@ def test_fp8_quantisation_bytes(lib, exponent):
     w.check_status()
 
 
+def test_fp8_scale_passes_over_nan(lib):
+    """A block's scale comes from the largest magnitude of its values that are numbers, wherever that stands and whatever its sign; from
+    infinities too; and is 1 where there are none."""
+    nan, inf = float("nan"), float("inf")
+    x = torch.ones(128 * 4, 128)
+    for i in range(128):
+        x[i, i] = -3.0                                                    # the largest in every place of a block, negative
+        x[128 + i, i], x[128 + i, (i + 1) % 128] = nan, -5.0              # behind a NaN
+        x[256 + i] = -nan if i % 2 else nan                               # only NaNs, but for one number in half of the blocks
+        if i % 4 > 1:
+            x[256 + i, i] = -0.25
+        x[384 + i, i], x[384 + i, i ^ 1] = (inf if i % 2 else -inf), nan
+    x = x.view(-1, 1024).to(torch.bfloat16)
+    w = EmuWorld(1, 32 << 20, DEV)
+    cap, H = x.shape
+    b = w.a2a_step_buffers(cap, H, 1, True)
+    meta, out = torch.zeros(8, dtype=torch.int32, device=DEV), torch.zeros(cap, H, dtype=torch.bfloat16, device=DEV)
+    idx, wt = torch.zeros(cap, 1, dtype=torch.int64, device=DEV), torch.ones(cap, 1, device=DEV)
+    w.a2a_step(b, [x.to(DEV)], [idx], [wt], [out], _scalars([cap]), [meta], 4, 1)
+    xb = x.float().view(-1, 128)
+    amax = torch.where(xb.isnan(), torch.zeros_like(xb), xb.abs()).amax(dim=1, keepdim=True)
+    scale = torch.where(amax > 0, amax / 448.0, torch.ones_like(amax))
+    q = (xb / scale).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).view(torch.uint8)
+    par = int(meta[5])
+    assert torch.equal(b["recv_scale"][0].tensor[par, 0].cpu().view(-1, 1), scale)
+    got, undefined = b["recv_x"][0].tensor[par, 0].cpu().view(-1, 128), (xb / scale).isnan()
+    assert torch.equal(got[~undefined], q[~undefined]) and (got[undefined] & 0x7f == 0x7f).all()
+    w.check_status()
+
+
 def test_a2a_fp8_dispatch(lib):
     W, E, K, H, counts = 2, 16, 4, 512, [6, 3]
     w, b, xs, idxs, ws, n_locals, cap = _a2a_case(W, E, K, H, counts, True, 13)
