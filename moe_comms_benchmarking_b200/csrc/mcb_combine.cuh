@@ -13,11 +13,13 @@
 // now 9).  With four packs every warp has an item and memory is the limit; what is best there depends on the kernel around:
 //   combine_kernel (ALONE)  one row at a time, with ordinary loads.  4096 rows of 1024 values, 8 pairs each: 9.5 us (18.4 with
 //                           four rows in flight and streaming loads, 28 with two, 11.4 with four and ordinary loads); 22 pairs
-//                           each, 184 MB of them: 39.6 (53, 90, 61);
+//                           each, 184 MB of them: 39.6 (53, 90, 61).  A world of one comes here only with rows that are no multiple of 32 bytes;
 //   behind the experts      two rows, with streaming loads.  The combine of the layer kernel at 4096 / 2048 tokens of 22 pairs:
 //                           41 / 24 us (44 / 26 with four rows, 59 / 37 with one and ordinary loads, 53 / 32 with one).
 // Call from all threads of the block (any size that is a multiple of 32), or in a world of one from `nwarps` of its warps.
 #pragma once
+#include <type_traits>
+
 #include "mcb_barrier.cuh"
 #include "mcb_gemm.h"
 
@@ -124,6 +126,59 @@ __device__ __forceinline__ void combine_items(const McbCtx& c, const McbCombineA
 #pragma unroll
     for (int u = 0; u < PL; ++u)
       if (p0 + u * 32 < s.packs) st_v4(out + (uint64_t)(t - s.offset) * s.row_bytes + (uint64_t)(p0 + u * 32) * 16, v[u]);
+  }
+}
+
+// The sums of a launch of its own in a world of one (combine_alone_kernel), where rows allow packs of 32 bytes: a warp takes 32 packs of BYTES of
+// a row, R pair rows in flight.  As long as every slice of 512 bytes has a warp of its own, latency is the limit: packs of 16 bytes, eight rows.
+// Beyond that the rate of loads from L2 is, which for 32 bytes per lane is twice that for 16 (copies of 16 MB, 16.4 against 8.2 TB/s), and the warps:
+// without the buffers of the sums over ranks the kernel has two blocks per SM.  One B200, us a launch in a row of them, before (one block per SM,
+// slices of 512, 1024 and 2048 bytes of 16 per lane) -> now, an eighth of 512 experts, rows of 1024 values:
+//   64 / 1024 / 2048 / 4096 / 8191 tokens of top-22, 2.75 pairs each   2.7 / 4.4 / 5.0 / 7.1 / 10.9 -> 2.3 / 3.7 / 4.1 / 5.6 / 8.9
+//   half of the experts, 512 / 2000 / 4096 tokens, 11 pairs each       4.5 / 10.6 / 20.8 -> 3.7 / 6.4 / 14.1
+//   8 of 64 experts, rows of 7168, 64 / 512 / 4096 tokens of top-8     3.9 / 6.4 / 29.2 -> 3.2 / 4.8 / 24.3
+// One row in flight instead of two 5.6 -> 6.5 (4096 tokens), three the same, four 6.0; three blocks per SM 6.8; 16 bytes per lane throughout 7.5.
+template <int BYTES, int R>
+__device__ __forceinline__ void combine_alone_items(const McbCombineArgs& a, int begin, int end, int offset) {
+  static_assert(BYTES == 16 || BYTES == 32, "a pack");
+  using Pack = typename std::conditional<BYTES == 32, Pack32, uint4>::type;
+  const int lane = threadIdx.x & 31, row_bytes = a.hidden * 2, slices = (row_bytes + 32 * BYTES - 1) / (32 * BYTES);
+  const long long items = (long long)(end - begin) * slices, step = (long long)gridDim.x * (blockDim.x >> 5);
+  const uint8_t* y = reinterpret_cast<const uint8_t*>(a.y);
+  uint8_t* out = reinterpret_cast<uint8_t*>(a.out);
+  for (long long i = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x; i < items; i += step) {
+    const int t = (int)(i / slices), at = ((int)(i - (long long)t * slices) * 32 + lane) * BYTES;
+    const bool live = at < row_bytes;
+    float acc[BYTES / 16][8] = {};
+    for (int k0 = 0; k0 < a.topk; k0 += 32) {
+      const int k = k0 + lane;
+      const int my_pos = k < a.topk ? a.pair_pos[(long long)(begin + t) * a.topk + k] : -1;
+      uint32_t have = __ballot_sync(0xffffffffu, my_pos >= 0);
+      while (have) {
+        Pack v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const bool row = have != 0;
+          const int pos = __shfl_sync(0xffffffffu, my_pos, row ? __ffs(have) - 1 : 0);
+          have &= have - 1;
+          const uint8_t* p = y + (long long)pos * row_bytes + at;
+          if constexpr (BYTES == 32) v[r] = row && live ? ld_v8_stream(p) : Pack32{};
+          else v[r] = row && live ? ld_v4_stream(p) : uint4{};
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if constexpr (BYTES == 32) { acc_row(acc[0], v[r].lo); acc_row(acc[1], v[r].hi); }
+          else acc_row(acc[0], v[r]);
+        }
+      }
+    }
+    if (!live) continue;
+    uint8_t* dst = out + (long long)(begin + t - offset) * row_bytes + at;
+    auto packed = [](const float (&s)[8]) {
+      return make_uint4(pack_bf16x2(s[0], s[1]), pack_bf16x2(s[2], s[3]), pack_bf16x2(s[4], s[5]), pack_bf16x2(s[6], s[7]));
+    };
+    if constexpr (BYTES == 32) st_v8(dst, Pack32{packed(acc[0]), packed(acc[1])});
+    else st_v4(dst, packed(acc[0]));
   }
 }
 

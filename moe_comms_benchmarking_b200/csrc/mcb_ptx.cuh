@@ -47,6 +47,23 @@ __device__ __forceinline__ void st_b32(void* p, uint32_t v) {
   asm volatile("st.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
+// 32 bytes, 32-byte aligned.
+struct Pack32 {
+  uint4 lo, hi;
+};
+__device__ __forceinline__ Pack32 ld_v8_stream(const void* p) {
+  Pack32 v;
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w)
+               : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_v8(void* p, Pack32 v) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               :: "l"(p), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z), "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y), "r"(v.hi.z), "r"(v.hi.w)
+               : "memory");
+}
+
 // Volatile 16-byte read used to poll flagged packets that a peer writes.
 __device__ __forceinline__ uint4 ld_v4_volatile(const void* p) {
   uint4 v;

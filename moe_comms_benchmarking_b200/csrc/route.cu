@@ -40,6 +40,20 @@ __global__ void __launch_bounds__(512) combine_kernel(const __grid_constant__ Mc
   combine_body<true>(c, a);
 }
 
+// The same in a world of one where rows allow packs of 32 bytes.
+__global__ void __launch_bounds__(512, 2) combine_alone_kernel(const __grid_constant__ McbCombineArgs a) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int offset = a.step_meta[1], T = a.step_meta[0];
+  int n = *a.n_local;
+  n = n < 0 ? 0 : n > a.cap ? a.cap : n;
+  const int begin = offset < 0 ? 0 : offset, end = T - offset < n ? T : offset + n;
+  if (begin >= end) return;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  if ((long long)(end - begin) * ((a.hidden + 255) / 256) <= warps) combine_alone_items<16, 8>(a, begin, end, offset);
+  else combine_alone_items<32, 2>(a, begin, end, offset);
+}
+
 }  // namespace mcb
 
 using namespace mcb;
@@ -59,6 +73,8 @@ int mcb_launch_combine(const McbCtx* ctx, const McbCombineArgs* args, int grid, 
                        cudaStream_t stream) {
   if (grid < 1 || grid > MCB_MAX_BLOCKS || threads < 32 || threads > 512 || (threads & 31) || args->hidden % 8)
     return cudaErrorInvalidValue;
+  if (ctx->world == 1 && args->hidden % 16 == 0 && !((reinterpret_cast<uintptr_t>(args->y) | reinterpret_cast<uintptr_t>(args->out)) & 31))
+    return launch_kernel(combine_alone_kernel, dim3(2 * grid), dim3(threads), 0, stream, pdl, false, *args);
   return launch_kernel(combine_kernel<false>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, *args,
                        (const McbCtx*)nullptr, (const McbCombineArgs*)nullptr);
 }

@@ -404,6 +404,40 @@ def test_expert_combine_slices(world1, T, K, H):
     assert torch.allclose(out.float(), ref, rtol=2 ** -8, atol=1e-5)      # fp32 sums in another order, rounded once
 
 
+@pytest.mark.parametrize("T,K,H,shift,own", [
+    (4, 5, 512, 0, None), (5, 5, 512, 0, None),          # 8 warps: a slice of 512 bytes each, more of them: slices of 1024 bytes
+    (9, 33, 528, 0, None), (3, 2, 16, 0, None),          # a ragged last slice of either, more ids than lanes, half a pack
+    (9, 5, 520, 0, None), (9, 5, 512, 8, None),          # no packs of 32 bytes: by the length of a row, by where the rows lie
+    (40, 4, 768, 0, (7, 21)), (40, 4, 768, 0, (30, 25)), (40, 4, 768, 0, (3, 0)),      # own rows inside, past the end, none
+])
+def test_expert_combine_alone(world1, T, K, H, shift, own):
+    """The sums of a world of one add a token's rows in the order of its ids, in fp32 from zero, and round once, whichever way they go;
+    rows of others keep what they held."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertCombinePlan, RouteBuffers
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    g = torch.Generator(device=DEV).manual_seed(T * K + H)
+    heap = SymmetricHeap(world1, T * H * 2 + (1 << 20), DEV)
+    route = RouteBuffers(T, K, K, DEV)
+    y = torch.randn(route.max_pairs * H + shift, device=DEV, generator=g).to(torch.bfloat16)[shift:].view(-1, H)
+    pos = torch.randint(0, route.max_pairs, (T, K), device=DEV, generator=g, dtype=torch.int32)
+    pos[torch.rand(T, K, device=DEV, generator=g) < 0.4] = -1
+    pos[0] = -1
+    route.pair_pos.copy_(pos)
+    first, rows = own or (0, T)
+    out = torch.full((T, H), 7.0, dtype=torch.bfloat16, device=DEV)
+    n, meta = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([rows], [T, first, rows, 1]))
+    ExpertCombinePlan(heap, y, route, heap.alloc("partial", [T, H], torch.bfloat16), out, n, meta, T, grid=2, threads=64).launch()
+    torch.cuda.synchronize()
+    heap.check_status()
+    ref = torch.zeros(T, H, device=DEV)
+    for k in range(K):
+        ref += torch.where((pos[:, k] >= 0).unsqueeze(1), y[pos[:, k].clamp(min=0).long()].float(), torch.zeros(1, device=DEV))
+    want = torch.full_like(out, 7.0)
+    mine = ref[first:first + rows].to(torch.bfloat16)
+    want[:mine.shape[0]] = mine
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("form", ["gathered", "no_weights", "own", "own_weights", "hidden_only", "order"])
 def test_layer_plan_follows_its_routing_plan(world1, form):
     """The layer kernel of a world of one routes by the ids and weights of its RoutePlan: the gathered ones, tensors of
