@@ -492,17 +492,9 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
   }
 }
 
-// D: as in local_few, 0 for steps of more layers.  `nact`: blocks that a layer fills, if the layers keep their order.
-template <bool FP8, int D>
-__device__ __forceinline__ void local_layers(const McbCtx& c, const McbDenseStepArgs& a, int n, int nact, uint32_t layer_base) {
-  if (n <= 0) return;
-  __shared__ LocalRanges r;
-  local_ranges<FP8>(r, c, a, n);
-  if (!a.in_order) {
-    if constexpr (D > 0) local_few<FP8, D>(c, a, r, n, layer_base);
-    else local_dealt<FP8>(c, a, r, n, layer_base);
-    return;
-  }
+// Layer after layer: steps that read what they write.  `nact`: blocks that a layer fills.
+template <bool FP8>
+__device__ __forceinline__ void local_in_order(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, int nact, uint32_t layer_base) {
   if ((int)blockIdx.x >= nact) return;
   const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)nact * blockDim.x;
   for (int l = 0; l < a.num_layers; ++l) {
@@ -595,8 +587,11 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
       if (tid == 0) *epoch_ptr(c, MCB_SITE_STEP_CREDIT, bid) = cb + (uint32_t)L;
     }
   } else if (EMU && W == 1 && !CHECK) {      // else dense_alone_kernel
+    __shared__ LocalRanges r;
+    local_ranges<FP8>(r, c, a, n);
     const int nloc = active_blocks((int)gridDim.x, n, bytes_per_row + a.rsv_row_bytes, (int)blockDim.x);
-    local_layers<FP8, 0>(c, a, n, nloc, layer_base);
+    if (n > 0 && a.in_order) local_in_order<FP8>(c, a, r, n, nloc, layer_base);
+    else if (n > 0) local_dealt<FP8>(c, a, r, n, layer_base);
   } else if (grp >= 0 && lb < nact) {
     // ---- barrier mode ----------------------------------------------------------------------------
     uint32_t ep = *epoch_ptr(c, MCB_SITE_STEP, bid);
@@ -683,10 +678,15 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
   }
 }
 
-// The step of a world of one, a kernel of its own: everything is inline, so the arguments are read from the constant bank and not
-// through pointers after every store.
+// The step of a world of one, a kernel of its own for each way: everything is inline, so the arguments are read from the constant bank and not
+// through pointers after every store.  D: as in local_few; kDealt: more layers; kInOrder: steps that read what they write.  With the last way in
+// each of the kernels, dealt steps were slower and so was one layer of e4m3 rows: 8192 rows of 1024, 88 layers 336 -> 298 us, 100 rows 9.5 -> 8.5; e4m3
+// 365 -> 344, one layer of 37 rows 4.8 -> 3.8.  Few layers of bf16 rows keep it: without it steps of 3.5 us took 0.1 to 0.3 us more.
+// Dealt e4m3 steps have 20 warps per block where others have 16: the quantisation waits for its own instructions, 344 -> 333 us, 58 layers of 2048 rows of
+// 7168 394 -> 375, small ones the same.  Copies do not gain from more warps: 640 threads 342 us where 512 took 331, 768 383.
+constexpr int kInOrder = 0, kDealt = -1;
 template <bool FP8, int D>
-__global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
+__global__ void __launch_bounds__(FP8 && D == kDealt ? 640 : 512, 1) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   pdl_wait();                 // the previous kernel of this rank (the previous step) has finished
   pdl_launch_dependents();
@@ -707,8 +707,20 @@ __global__ void __launch_bounds__(512) dense_alone_kernel(const __grid_constant_
 #pragma unroll
   for (int t = 0; t < MCB_MAX_TENSORS; ++t)
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
-  const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
-  local_layers<FP8, D>(c, a, n, nact, layer_base);
+  __shared__ LocalRanges r;
+  if (n > 0) {
+    local_ranges<FP8>(r, c, a, n);
+    if constexpr (D == kDealt) {
+      local_dealt<FP8>(c, a, r, n, layer_base);
+    } else {
+      bool in_order = D == kInOrder;
+      if constexpr (D > 0) {
+        if (!FP8) in_order = a.in_order;
+        if (!in_order) local_few<FP8, D>(c, a, r, n, layer_base);
+      }
+      if (in_order) local_in_order<FP8>(c, a, r, n, active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x), layer_base);
+    }
+  }
   step_close(a.state, step_seq, layer_base + (uint32_t)L);
 }
 
@@ -773,10 +785,12 @@ int mcb_launch_dense_step(const McbCtx* ctx, const McbDenseStepArgs* args, int g
   if (ctx->world == 1 && !args->check) {
     auto alone = [&](auto layers) {
       constexpr int D = decltype(layers)::value;
-      return launch_kernel(a.fp8_hidden ? dense_alone_kernel<true, D> : dense_alone_kernel<false, D>, dim3(grid), dim3(threads), 0, stream, pdl, false,
+      const int block = D == kDealt && a.fp8_hidden ? threads / 32 * 20 / 16 * 32 : threads;
+      return launch_kernel(a.fp8_hidden ? dense_alone_kernel<true, D> : dense_alone_kernel<false, D>, dim3(grid), dim3(block), 0, stream, pdl, false,
                            *ctx, a);
     };
-    if (a.num_layers > kFewLayers) return alone(std::integral_constant<int, 0>{});
+    if (a.in_order && (a.fp8_hidden || a.num_layers > kFewLayers)) return alone(std::integral_constant<int, kInOrder>{});
+    if (a.num_layers > kFewLayers) return alone(std::integral_constant<int, kDealt>{});
     if (a.num_layers > 4) return alone(std::integral_constant<int, kFewLayers>{});
     if (a.num_layers > 2) return alone(std::integral_constant<int, 4>{});
     return a.num_layers > 1 ? alone(std::integral_constant<int, 2>{}) : alone(std::integral_constant<int, 1>{});
