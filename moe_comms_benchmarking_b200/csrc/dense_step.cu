@@ -330,11 +330,24 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 // and 58 layers of hidden 7168 and top-8, 1 / 64 / 512 / 2048 rows, bf16 19 -> 6.5 / 29 -> 21 / 178 -> 116 / 961 -> 425, e4m3 with 512 / 2048
 // rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.  One size was
 // slower than before, e4m3 steps of 9 to 16 layers of about 512 rows of 1024, by up to 7 %.
+// Large copies of many layers go by half of the warps.  A layer's stores merge in L1 with those of the layer before the last to the same rows, if these are
+// still there: of 26.8 million sectors stored by 24 layers of 8192 rows 14.2 million went on to L2 with 16 warps per block and 10.8 million with 8.  With fewer
+// layers or fewer items per warp the time until a run's first load is there counts for more.  16 -> 8 warps, us (12 warps):
+//   88 layers  1024 values, 60 rows (13 items a warp) 6.4 -> 7.1 (6.6), 150 (47) 11.3 -> 13.9 (12.3), 400 (126) 22.6 -> 21.9 (22.3), 8192 292 -> 259 (267)
+//   58 layers  7168 values, 20 rows (28) 7.2 -> 8.7 (7.8), 60 (83) 15.4 -> 14.5 (14.8), 400 66.3 -> 60.5 (63.6), 2048 301 -> 289 (287)
+//   40 layers  7168 values, 60 rows (57) 11.5 -> 11.0 (11.3), 400 45.9 -> 42.1 (44.6), 2048 206 -> 207 (203); 1024 values, 8192 rows 128.5 -> 125.6 (122.8)
+//   26 layers  768 values, 400 rows (27) 7.3 -> 7.5 (7.3), 8192 62.8 -> 65.6 (61.2); 7168 values, 2048 rows 138 -> 158 (142)
+// Six warps: 1 to 14 % slower than eight.
+constexpr int kHalfLayers = 40, kHalfItems = 64;
+
 template <bool FP8>
 __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, uint32_t layer_base) {
-  const int lane = threadIdx.x & 31, warps = (int)(gridDim.x * (blockDim.x >> 5));
-  const int warp = (int)(blockIdx.x + (threadIdx.x >> 5) * gridDim.x);         // the smallest steps spread over the chip
   const long long packs = r.end[LocalRanges::R - 1], groups = (packs + 31) >> 5;
+  int used = (int)(blockDim.x >> 5);                                            // warps of a block that take part
+  if (!FP8 && a.num_layers >= kHalfLayers && (groups + 1) * a.num_layers >= (long long)kHalfItems * used * gridDim.x) used = (used + 1) / 2;
+  if ((int)(threadIdx.x >> 5) >= used) return;
+  const int lane = threadIdx.x & 31, warps = (int)gridDim.x * used;
+  const int warp = (int)(blockIdx.x + (threadIdx.x >> 5) * gridDim.x);         // the smallest steps spread over the chip
   auto quantise = [&] {
     // Two packs (16 values) per lane, so eight lanes hold a block of 128 values and a lane stores 16 bytes: 13 to 18 % faster than one.
     const int H = (int)a.fp8_hidden, ppr = H / 16, nblk = H / 128;

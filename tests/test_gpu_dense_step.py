@@ -385,3 +385,13 @@ def test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads):
 def test_world_of_one_few_layers(lib, fp8, n, layers, grid, threads):
     """Steps of up to eight layers, whose warps take all layers of one group of packs or more at a time."""
     test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads)
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("n,layers,grid,threads", [
+    (8, 40, 1, 96), (8, 41, 2, 64), (7, 88, 1, 32),       # half of three warps, of two, one
+    (8, 39, 1, 96), (1, 40, 2, 96),                       # too few layers, too few items per warp
+])
+def test_world_of_one_half_of_the_warps(lib, fp8, n, layers, grid, threads):
+    """Large copies of many layers go by half of the warps of a block."""
+    test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads)
