@@ -19,7 +19,6 @@
 
 namespace mcb {
 
-constexpr int kRouteThreads = 1024;
 constexpr int kMaxLocalExperts = 1024;
 // Shared memory of a routing block: counts, own begins (later cursors), offsets, scan scratch.
 constexpr int kRouteSmemWords = 3 * kMaxLocalExperts + 1 + 3 * 32;
@@ -53,8 +52,8 @@ __device__ __forceinline__ RouteShare route_share(const McbRouteArgs& a, int blo
   return s;
 }
 template <class Group>
-__device__ __forceinline__ bool route_counts_all(const Group& g, const RouteShare& s) {
-  return s.entries <= (long long)kRouteAllPerThread * g.size();
+__device__ __forceinline__ bool route_counts_all(const Group& g, const RouteShare& s, int per_thread = kRouteAllPerThread) {
+  return s.entries <= (long long)per_thread * g.size();
 }
 
 // Counts the entries [lo, hi) into m.cnt and, with SPLIT, those before `split` into m.begin too.  All threads of the group.
@@ -206,17 +205,26 @@ __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& 
 // experts, now 5.8; 8.5 and 4.2 at 1408; 3.0 and 3.8 at 128 of 32, where the wider scan shows); with many the blocks wait for one
 // another on a counter that only grows (the grid must be co-resident).  There a thread keeps its first kRouteKept entries from the
 // counting to the placing, and the last block to have read the counters is found while the others place: 22528 / 45056 / 90112
-// entries, 64 of 512 experts local, 10.4 -> 8.5 / 10.5 -> 8.5 / 10.6 -> 9.3 us.
+// entries, 64 of 512 experts local, 10.4 -> 8.5 / 10.5 -> 8.5 / 10.6 -> 9.3 us (32 blocks of 1024 threads).
 // Shares are runs of entries: with entries dealt to the blocks in turn, an expert's rows come in another order, and FFN and
 // combine of 8191 tokens with Zipf routing were 2 % slower; asked for before the number of tokens is known, few entries took
 // 8.4 us (7.2).  Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.
 constexpr int kRouteKept = 4;
+// Blocks of a launch of its own.  Blocks of 512 threads cost less to start and at each of their barriers than as many threads in blocks of 1024; three of them
+// for every one that the caller asked for (32) read and place large batches sooner.  One B200, us a launch in a row of them, 64 of 512 experts local:
+//   entries                       352   1408   5632   8800   11264   15400   45056   90112   180202
+//   32 blocks of 1024 threads     4.0    4.2    4.9    5.5     5.7     6.3     6.9     7.7      9.7
+//   96 of 512                     3.3    3.5    4.6    5.4     5.9     5.9     6.0     6.7      6.5
+//   64 of 512                     3.5    3.5    4.5    5.4     5.9     5.7     6.0     6.8      8.1
+//   128 of 256 / of 512    3.2 / 3.3  3.7 / 3.6  5.3 / 4.6  5.5 / 5.8  5.7 / 6.1  5.7 / 6.0  6.0 / 6.2  6.7 / 6.8  7.8 / 6.5
+// There every block counts all of up to 24 entries per thread: 8800 entries 5.4 us (5.7 through the counters), 11264 5.9 (6.0), 15400 6.8 (5.9).
+constexpr int kRouteThreads = 512, kRouteBlocks = 3, kRouteAllAlone = 24;
 __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
   const RouteSmem m(smem);
   const int tid = threadIdx.x, E = a.num_local_experts;
   const RouteShare s = route_share(a, (int)blockIdx.x, (int)gridDim.x);
   const BlockGroup g;
-  if (route_counts_all(g, s)) {
+  if (route_counts_all(g, s, kRouteAllAlone)) {
     if (s.lo >= s.hi && blockIdx.x != 0) return;
     route_count<true>(g, a, a.topk_idx, m, 0, s.entries, s.lo);
     route_offsets(g, a, m, blockIdx.x == 0);

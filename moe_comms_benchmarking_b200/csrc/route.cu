@@ -66,7 +66,8 @@ int mcb_sizeof_combine_args() { return (int)sizeof(McbCombineArgs); }
 int mcb_launch_route(const McbRouteArgs* args, int grid, int pdl, cudaStream_t stream) {
   if (grid < 1 || grid > 128 || args->num_local_experts > kMaxLocalExperts || args->num_local_experts < 1)
     return cudaErrorInvalidValue;
-  return launch_kernel(route_kernel, dim3(grid), dim3(kRouteThreads), 0, stream, pdl, false, *args);
+  const int blocks = kRouteBlocks * grid < 128 ? kRouteBlocks * grid : 128;            // they wait for one another: no more than there are SMs
+  return launch_kernel(route_kernel, dim3(blocks), dim3(kRouteThreads), 0, stream, pdl, false, *args);
 }
 
 int mcb_launch_combine(const McbCtx* ctx, const McbCombineArgs* args, int grid, int threads, int pdl,

@@ -596,6 +596,12 @@ def test_route_many_entries(world1, T, grid):
         assert bool((route.pair_pos[T:] == -7).all()) and int(route.max_rows) == int(counts.max())
 
 
+@pytest.mark.parametrize("T,grid", [(2457, 1), (2457, 32), (2458, 1), (2458, 32), (2458, 43), (3, 32)])
+def test_route_around_the_line(world1, T, grid):
+    """The last size whose entries every block counts, the first that is shared out, over three and 96 blocks and as many as there may be."""
+    test_route_many_entries(world1, T, grid)
+
+
 @pytest.mark.parametrize("E,K,H,I,T,layers,sets,grid", [
     (8, 2, 256, 128, 3, 2, 1, 148),          # two layers; fewer units than CTA pairs
     (8, 2, 256, 128, 90, 40, 20, 148),       # more weight sets than one launch takes, buffers used many times over
