@@ -302,7 +302,10 @@ __device__ __forceinline__ void local_ranges(LocalRanges& r, const McbCtx& c, co
   __syncthreads();
 }
 
-// Layers [first, last) of one pack per lane, the loads of eight of them in flight together.
+// Layers [first, last) of one pack per lane, the loads of eight of them in flight together, and the stores of one parity before those of the other: they
+// go to the same place, and more of them merge in L1 than in the order of the layers.  One B200, us a step: 88 layers of 1000 / 6000 rows of 1024 42.8 / 212 ->
+// 38.6 / 180, 58 layers of 333 / 1000 rows of 7168 57.0 / 144 -> 51.2 / 133, 60 rows or fewer up to 5 % faster or the same.  (One parity of a whole run before the
+// other: large steps another 0 to 3 % faster, those of up to 60 rows 2 to 10 % slower.  e4m3 rows, which alternate, and all-to-all pieces did not gain.)
 template <class Load, class Store>
 __device__ __forceinline__ void local_layers_of(int first, int last, Load load, Store store) {
   constexpr int D = 8;
@@ -311,7 +314,9 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 #pragma unroll
     for (int d = 0; d < D; ++d) v[d] = l0 + d < last ? load() : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int d = 0; d < D; d += 2) store(v[d], v[d + 1], l0 + d < last, l0 + d + 1 < last, l0 + d);
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+      for (int d = p; d < D; d += 2) store(v[d], l0 + d < last, l0 + p);
   }
 }
 
@@ -399,10 +404,9 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
       uint8_t* dst = r.dst[t] + off;
       const uint64_t par_off = r.par[t];
       local_layers_of(first, last, [&] { return live ? ld_v4(src) : make_uint4(0, 0, 0, 0); },
-                      [&](uint4 v0, uint4 v1, bool on0, bool on1, int l) {
+                      [&](uint4 v, bool on, int l) {
         const uint32_t par = (layer_base + (uint32_t)l) & 1u;
-        if (live && on0) st_v4(dst + (par ? par_off : 0), v0);
-        if (live && on1) st_v4(dst + (par ? 0 : par_off), v1);
+        if (live && on) st_v4(dst + (par ? par_off : 0), v);
       });
     });
   };
