@@ -662,6 +662,15 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 // With one chain for both parities of a metadata row, its chunks put together by shuffles, the smallest steps took 16.7 and 14.6 us.
 // The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.  Slower than slices
 // remain e4m3 steps of five layers, by up to 14 % at some sizes.
+// Steps of bf16 rows are bound by the stores that leave L1, where stores to the same rows merge.  So of eight layers of a piece in flight those to the received rows
+// of one parity come first, then those of the other, then the sums; and from kHalfLayers layers on half of the warps take part, whose rows are still in L1
+// more often.  In the order of the layers (large steps by slices) -> so, us a step:
+//   hidden 1024, 88 layers of 20 / 150 / 1000 / 6000 rows   9.0 -> 8.1, 13.9 -> 10.8, 61.4 -> 37.3, 328 -> 191 (16 warps 8.4 / 11.4 / 44.1 / 241)
+//   hidden 7168, 58 layers of 20 / 333 / 2048 rows          9.7 -> 7.3, 83.4 -> 48.5, 490 -> 258 (7.7 / 59.4 / 335)
+//   26 layers, 333 and 2048 rows                            39.0 -> 27.4, 219 -> 132 (8 warps 26.8, 151); hidden 768 8.8 -> 7.2, 28.5 -> 20.5 (8.1, 24.3)
+//   40 layers, hidden 768 and 1024, 2048 rows               41.8 -> 28.7, 53.5 -> 37.9 (30.2, 36.9); 48 layers 49.3 -> 33.1, 64.4 -> 45.5 (33.9, 42.3)
+// (e4m3 rows, bound by their instructions, take their layers as they come.)
+constexpr int kHalfLayers = 48;
 template <bool FP8>
 __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
   constexpr int K = FP8 ? 2 : 1;             // packs per lane of a piece
@@ -672,7 +681,12 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
   constexpr int kCost = FP8 ? 5 : 2;
   AloneSlice<FP8, 1> s(a);
   const int lane = s.lane, L = a.num_layers, per_row = (s.row_packs + 32 * K - 1) / (32 * K);
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5), warp = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x;
+  unsigned used = blockDim.x >> 5;                       // warps of a block that take part
+  if constexpr (!FP8) {
+    if (L >= kHalfLayers) used = (used + 1) / 2;
+    if (threadIdx.x >> 5 >= used) return;
+  }
+  const long long warps = (long long)gridDim.x * used, warp = blockIdx.x + (long long)(threadIdx.x >> 5) * gridDim.x;
   const long long sums = s.echo ? 0 : (long long)n * s.slices(), chains = sums + 2ll * n, items = (long long)n * per_row * L;
   const uint64_t row_bytes = (uint64_t)a.hidden * 2;
 
@@ -755,22 +769,26 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
         for (int d = 0; d < D; ++d)
 #pragma unroll
           for (int k = 0; k < K; ++k) v[d][k] = live && l0 + d < last ? ld_v4(src + k * 16) : make_uint4(0, 0, 0, 0);
+        if constexpr (FP8) {
 #pragma unroll
-        for (int d = 0; d < D; d += 2) {
-          auto at = [&](uint8_t* base, uint64_t par_stride, int k) { return base + ((layer_base + (uint32_t)(l0 + d + k)) & 1u ? par_stride : 0); };
-          if constexpr (FP8) {
+          for (int d = 0; d < D; d += 2) {
+            auto at = [&](uint8_t* base, uint64_t par_stride, int k) { return base + ((layer_base + (uint32_t)(l0 + d + k)) & 1u ? par_stride : 0); };
             quant_wide_pair(v[d], v[d + 1], [&](int k) { return l0 + d + k < last && sent && live; }, [&](int k, uint4 q, float scale) {
               st_v4(at(recv, a.x_par_stride, k), q);
               if ((lane & 7) == 0) st_b32(at(scales, a.scale_par_stride, k), __float_as_uint(scale));
             });
-          } else {
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              if (l0 + d + k >= last || !live) break;
-              if (sent) st_v4(at(recv, a.x_par_stride, k), v[d + k][0]);
-              if (s.echo) st_v4(out, alone_sum(sent, v[d + k][0]));
-            }
           }
+        } else {
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            uint8_t* dst = recv + ((layer_base + (uint32_t)(l0 + p)) & 1u ? a.x_par_stride : 0);
+#pragma unroll
+            for (int d = p; d < D; d += 2)
+              if (l0 + d < last && live && sent) st_v4(dst, v[d][0]);
+          }
+#pragma unroll
+          for (int d = 0; d < D; ++d)
+            if (l0 + d < last && live && s.echo) st_v4(out, alone_sum(sent, v[d][0]));
         }
       }
     });
@@ -825,14 +843,13 @@ __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs&
   else alone_slices<FP8, 4, D>(c, a, n, layer_base);
 }
 
-// Whether a step of the identity expert on bf16 rows goes by slices of four packs per lane, whatever its layers: where its slices fill
-// at least 5/6 of their last round of warps.  A slice writes its row part, its sums and its metadata in one go, which saves a dealt step's addresses; but a
-// slice is all layers, so a last round that is not full is waited for.  One B200, 58 layers, dealt -> slices:
-//   hidden 7168, 333 rows (0.98 of a round) 95 -> 87, 1000 (2.96 of 3) 270 -> 257, 2048 (6.05 of 7) 545 -> 529 us
-//   hidden 1024, 2048 rows (0.86) 87.5 -> 83.5, 4096 (1.73 of 2) 170 -> 157; hidden 2048, 4096 rows (3.46 of 4) 322 -> 303
-//   not full: hidden 7168, 512 rows (1.51 of 2) 140 -> 141, 700 (2.07 of 3) 190 -> 210; hidden 2048, 1400 rows (1.18 of 2) 113 -> 128
-// (before layers were dealt, 1000 rows of 7168: 265).  e4m3 rows, up to 8 layers: 1.0 to 0.9 of the dealt time, but the second way in their
-// kernel cost every step 0.7 to 1 us.
+// Whether a step of the identity expert on bf16 rows with five or six layers goes by slices of four packs per lane: where its slices fill at least 5/6 of their
+// last round of warps.  A slice writes its row part, its sums and its metadata in one go, which saves a dealt step's addresses; but a
+// slice is all layers, so a last round that is not full is waited for.  One B200, dealt -> slices, us a step:
+//   5 layers, hidden 1024 / 768, 2048 rows (0.86 and 0.86 of a round) 11.1 -> 9.7, 9.9 -> 8.3, hidden 7168, 333 rows (0.98) 10.2 -> 10.2, 1000 (2.96 of 3) 20.4 -> 24.1
+//   6 layers 11.2 -> 11.1, 10.3 -> 9.1, 10.5 -> 11.6, 21.4 -> 27.7; 7 layers 12.2 -> 12.2, 10.8 -> 10.5, 10.9 -> 12.7, 22.5 -> 31.8
+// (before the stores of dealt bf16 pieces were put in order, slices were faster with any number of layers where they filled their rounds).
+constexpr int kSliceLayers = 6;
 __device__ __forceinline__ bool alone_full(const McbA2AStepArgs& a, int n) {
   const unsigned warps = gridDim.x * (blockDim.x >> 5), items = (unsigned)n * (unsigned)((a.hidden / 8 + 127) / 128);
   return a.y_off == a.recv_x_off && items * 6ull >= (items + warps - 1) / warps * 5ull * warps;
@@ -855,10 +872,10 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
 }
 
 // The step of a world of one, a kernel of its own for each way: everything is inline, so the arguments are read from the constant bank and not
-// through pointers after every store.  D: as in alone_few; kDealt: more layers; kInOrder: steps that read what they write, more than 32 ids.  With the
+// through pointers after every store.  D: as in alone_few; kDealt: more layers; kDealtOrSlices: alone_full; kInOrder: steps that read what they write, more than 32 ids.  With the
 // last in the kernel of dealt steps, these had 24 bytes of stack and e4m3 ones were slower: 58 layers of 333 rows of 7168 82.2 -> 78.1 us, 88 layers of
 // one / 37 / 2048 rows of 1024 7.9 / 9.5 / 115 -> 7.2 / 8.7 / 110.  (More or fewer than 16 warps per block: 3 to 10 % slower with e4m3 rows.)
-constexpr int kInOrder = 0, kDealt = -1;
+constexpr int kInOrder = 0, kDealt = -1, kDealtOrSlices = -2;
 template <bool FP8, int D>
 __global__ void __launch_bounds__(512, 1) a2a_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbA2AStepArgs a) {
   pdl_wait();
@@ -873,8 +890,8 @@ __global__ void __launch_bounds__(512, 1) a2a_alone_kernel(const __grid_constant
   } else if constexpr (D > 0) {
     alone_few<FP8, D>(c, a, st.n, st.layer_base);
   } else {
-    if (FP8 || !alone_full(a, st.n)) alone_dealt<FP8>(c, a, st.n, st.layer_base);
-    else alone_slices<FP8, 4, 2>(c, a, st.n, st.layer_base);
+    if (D == kDealt || !alone_full(a, st.n)) alone_dealt<FP8>(c, a, st.n, st.layer_base);
+    else if constexpr (D != kDealt) alone_slices<FP8, 4, 2>(c, a, st.n, st.layer_base);
   }
   step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
 }
@@ -928,9 +945,13 @@ int mcb_launch_a2a_step(const McbCtx* ctx, const McbA2AStepArgs* args, int grid,
   if (ctx->world == 1) {
     auto alone = [&](auto layers) {
       constexpr int D = decltype(layers)::value;
-      return launch_kernel(a.fp8 ? a2a_alone_kernel<true, D> : a2a_alone_kernel<false, D>, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
+      auto kernel = a2a_alone_kernel<false, D>;
+      if constexpr (D != kDealtOrSlices)
+        if (a.fp8) kernel = a2a_alone_kernel<true, D>;
+      return launch_kernel(kernel, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
     };
     if (!a.apart || a.topk > 32) return alone(std::integral_constant<int, kInOrder>{});
+    if (a.num_layers > kFewLayers && a.num_layers <= kSliceLayers && !a.fp8) return alone(std::integral_constant<int, kDealtOrSlices>{});
     if (a.num_layers > kFewLayers) return alone(std::integral_constant<int, kDealt>{});
     return a.num_layers > 1 ? alone(std::integral_constant<int, 2>{}) : alone(std::integral_constant<int, 1>{});
   }

@@ -386,6 +386,17 @@ def test_a2a_step_alone_few_layers(lib, world1, fp8, H, K, n, layers, grid, thre
     test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads)
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("H,K,n,layers,grid,threads", [
+    (1152, 5, 3, 5, 1, 192), (1152, 5, 5, 6, 2, 192), (1152, 5, 4, 6, 1, 192),      # bf16 rows: slices, a full round and ten of twelve; eight, dealt
+    (256, 3, 7, 47, 3, 160), (256, 3, 7, 48, 3, 160), (1152, 5, 3, 49, 2, 64),      # bf16 rows: all warps, half of them
+    (128, 1, 2, 60, 1, 32), (1024, 6, 5, 51, 1, 96),                                # one warp, two of three
+])
+def test_a2a_step_alone_ways_of_bf16_rows(lib, world1, fp8, H, K, n, layers, grid, threads):
+    """Where bf16 steps go by slices or half of the warps."""
+    test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads)
+
+
 @pytest.mark.parametrize("form", ["out_on_x", "out_on_ids", "echo"])
 def test_a2a_step_that_reads_what_it_writes(lib, world1, form):
     """The host tells steps whose layers may run into each other from those that write what they read."""
