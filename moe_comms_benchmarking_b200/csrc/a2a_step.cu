@@ -648,12 +648,12 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 //   chains   what a layer leaves behind of its own, layer after layer by one warp: the metadata row of a token and parity, which
 //            carries the number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
-// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores into L2 and, with e4m3 rows, by the integer
+// A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores that leave L1 (below) or, with e4m3 rows, by the
 // instructions of the quantisation; the loads may stay in L1, where 95 % of their sectors hit (24 layers of 333 e4m3 rows of 7168).  From L2, which the
 // hint against L1 made of every load: 58 layers of 333 / 1000 / 2048 e4m3 rows of 7168 98.9 / 283 / 559 -> 85.9 / 236 / 466 us, 88 layers of 333 / 2048 / 8192 of
 // 1024 29.9 / 141 / 527 -> 24.9 / 121 / 446, bf16 rows 33.3 / 124 * / 465 * -> 31.1 / 116 * / 427 *.  One B200, loads from L2, against up to four packs per
 // lane with up to eight layers in flight where the slices fit the warps, else slices of four packs layer after layer:
-//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows (* by slices, alone_full)
+//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows (* by slices, as these bf16 steps went then)
 //     bf16   35 -> 10.5 / 35 -> 12.5 / 40 -> 33 / 76 -> 68 / 272 -> 249 * us
 //     e4m3   43 -> 10.5 / 45 -> 12.5 / 56 -> 29 / 91 -> 73 / 398 -> 268 us
 //   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 2048 rows

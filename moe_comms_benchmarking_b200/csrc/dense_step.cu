@@ -324,9 +324,9 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 // need no order: a warp takes all layers of a few packs, and every warp gets the same number of (pack, layer) whatever the batch.  The
 // chip works on a few MB at a time; layer after layer over all rows, large steps went through up to 90 MB of L2 in every layer, small ones
 // left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
-// The loads may stay in L1, where 95 % of their sectors hit (24 layers of 2048 rows): large steps are bound by the stores into L2, and loads with the
-// hint that keeps them out of L1 took a third of its time.  88 layers of 1000 / 2048 / 8192 rows of 1024 60.7 / 107.8 / 417 -> 50.3 / 88.1 / 335 us
-// (9.4 TB/s of stores), e4m3 65.9 / 121 / 451 -> 55.8 / 103 / 382; 58 layers of 333 / 2048 rows of 7168 83 / 416 -> 69.5 / 327, e4m3 93 / 502 ->
+// The loads may stay in L1, where 95 % of their sectors hit (24 layers of 2048 rows): large steps are bound by the stores that L1 has to
+// take and pass on, and loads with the hint that keeps them out of L1 took a third of L2's time.  88 layers of 1000 / 2048 / 8192 rows of 1024 60.7 / 107.8 / 417 -> 50.3 / 88.1 / 335 us
+// with all warps and stores in the order of the layers, e4m3 65.9 / 121 / 451 -> 55.8 / 103 / 382; 58 layers of 333 / 2048 rows of 7168 83 / 416 -> 69.5 / 327, e4m3 93 / 502 ->
 // 78 / 438.  The figures below are of loads from L2.
 // One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against up to four packs per thread with up to eight
 // layers in flight where a step fits, else layer after layer:
