@@ -780,15 +780,19 @@ __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArg
           }
         } else {
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            uint8_t* dst = recv + ((layer_base + (uint32_t)(l0 + p)) & 1u ? a.x_par_stride : 0);
+          for (int odd_layer = 0; odd_layer < 2; ++odd_layer) {
+            uint8_t* dst = recv + ((layer_base + (uint32_t)(l0 + odd_layer)) & 1u ? a.x_par_stride : 0);
 #pragma unroll
-            for (int d = p; d < D; d += 2)
+            for (int d = odd_layer; d < D; d += 2)
               if (l0 + d < last && live && sent) st_v4(dst, v[d][0]);
           }
+          // Left at the first that is not there: with eight predicated sums small steps of five layers and more took 0.2 us more (8 layers of
+          // 20 / 150 rows of 1024 4.9 / 6.0 -> 4.7 / 5.7 us), 150 rows of 7168 5 % more (7.8 -> 7.4).
 #pragma unroll
-          for (int d = 0; d < D; ++d)
-            if (l0 + d < last && live && s.echo) st_v4(out, alone_sum(sent, v[d][0]));
+          for (int d = 0; d < D; ++d) {
+            if (l0 + d >= last || !live || !s.echo) break;
+            st_v4(out, alone_sum(sent, v[d][0]));
+          }
         }
       }
     });
