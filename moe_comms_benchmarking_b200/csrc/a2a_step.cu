@@ -847,16 +847,23 @@ __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs&
   else alone_slices<FP8, 4, D>(c, a, n, layer_base);
 }
 
-// Whether a step of the identity expert on bf16 rows with five or six layers goes by slices of four packs per lane: where its slices fill at least 5/6 of their
-// last round of warps.  A slice writes its row part, its sums and its metadata in one go, which saves a dealt step's addresses; but a
-// slice is all layers, so a last round that is not full is waited for.  One B200, dealt -> slices, us a step:
-//   5 layers, hidden 1024 / 768, 2048 rows (0.86 and 0.86 of a round) 11.1 -> 9.7, 9.9 -> 8.3, hidden 7168, 333 rows (0.98) 10.2 -> 10.2, 1000 (2.96 of 3) 20.4 -> 24.1
-//   6 layers 11.2 -> 11.1, 10.3 -> 9.1, 10.5 -> 11.6, 21.4 -> 27.7; 7 layers 12.2 -> 12.2, 10.8 -> 10.5, 10.9 -> 12.7, 22.5 -> 31.8
-// (before the stores of dealt bf16 pieces were put in order, slices were faster with any number of layers where they filled their rounds).
-constexpr int kSliceLayers = 6;
-__device__ __forceinline__ bool alone_full(const McbA2AStepArgs& a, int n) {
+// Whether a step of the identity expert on bf16 rows with five or six layers goes by slices of four packs per lane, where a slice is a whole row.  It writes its
+// row, its sums and its metadata in one go, which saves a dealt step's addresses, but it is all layers of a row: a last round of warps that is less than 5/6
+// full is waited for, and where rows are longer, or a warp gets more of them, dealt pieces keep more loads in flight and more of their stores merge.
+// One B200, us a step, dealt -> slices, one / two / three rounds of warps (0.96 full):
+//   five layers   256 values 7.3 -> 5.8 / 10.3 -> 8.6 / 13.6 -> 11.9        512 values 8.9 -> 7.8 / 12.9 -> 11.8 / 16.4 -> 15.7
+//                 768 values 10.1 -> 9.2 / 15.2 -> 14.9 / 19.6 -> 20.0      1024 values 11.2 -> 10.7 / 17.3 -> 17.7 / 23.0 -> 24.5
+//   six layers    256 values 7.8 -> 6.7 / 10.5 -> 9.2 / 13.5 -> 12.4        512 values 8.6 -> 8.4 / 13.2 -> 13.2 / 17.3 -> 18.1
+//                 768 values 9.9 -> 10.0 / 15.5 -> 16.9 / 20.0 -> 23.2      1024 values 11.1 -> 11.7 / 17.6 -> 20.2 / 23.7 -> 29.0
+// Two slices to a row and more: 2048 values, five layers 9.8 -> 10.1 / 15.4 -> 17.3; 7168 values, 324 / 974 rows 9.5 -> 10.3 / 18.3 -> 23.3; six layers
+// 15 to 45 % slower; only where the rows in and out no longer stay in L2 (93 MB, five layers) 0 to 3 % faster.  Seven layers: dealt everywhere.
+// The line is at so many values for a warp; the host takes the rest out (kSliceLayers), so that the kernel's other way stays as it is.
+constexpr int kSliceLayers = 6, kSliceValuesFive = 1536, kSliceValuesSix = 512;
+__device__ __forceinline__ bool alone_by_slices(const McbA2AStepArgs& a, int n) {
   const unsigned warps = gridDim.x * (blockDim.x >> 5), items = (unsigned)n * (unsigned)((a.hidden / 8 + 127) / 128);
-  return a.y_off == a.recv_x_off && items * 6ull >= (items + warps - 1) / warps * 5ull * warps;
+  const bool full = a.y_off == a.recv_x_off && items * 6ull >= (items + warps - 1) / warps * 5ull * warps;
+  return full && (unsigned long long)items * (unsigned)a.hidden <=
+                     (unsigned long long)warps * (a.num_layers < kSliceLayers || a.hidden <= 256 ? kSliceValuesFive : kSliceValuesSix);
 }
 
 // Layer after layer: steps that read what they write.
@@ -876,8 +883,8 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
 }
 
 // The step of a world of one, a kernel of its own for each way: everything is inline, so the arguments are read from the constant bank and not
-// through pointers after every store.  D: as in alone_few; kDealt: more layers; kDealtOrSlices: alone_full; kInOrder: steps that read what they write, more than 32 ids.  With the
-// last in the kernel of dealt steps, these had 24 bytes of stack and e4m3 ones were slower: 58 layers of 333 rows of 7168 82.2 -> 78.1 us, 88 layers of
+// through pointers after every store.  D: as in alone_few; kDealt: more layers; kDealtOrSlices: alone_by_slices; kInOrder: steps that read what they write,
+// more than 32 ids.  With the last in the kernel of dealt steps, these had 24 bytes of stack and e4m3 ones were slower: 58 layers of 333 rows of 7168 82.2 -> 78.1 us, 88 layers of
 // one / 37 / 2048 rows of 1024 7.9 / 9.5 / 115 -> 7.2 / 8.7 / 110.  (More or fewer than 16 warps per block: 3 to 10 % slower with e4m3 rows.)
 constexpr int kInOrder = 0, kDealt = -1, kDealtOrSlices = -2;
 template <bool FP8, int D>
@@ -894,7 +901,7 @@ __global__ void __launch_bounds__(512, 1) a2a_alone_kernel(const __grid_constant
   } else if constexpr (D > 0) {
     alone_few<FP8, D>(c, a, st.n, st.layer_base);
   } else {
-    if (D == kDealt || !alone_full(a, st.n)) alone_dealt<FP8>(c, a, st.n, st.layer_base);
+    if (D == kDealt || !alone_by_slices(a, st.n)) alone_dealt<FP8>(c, a, st.n, st.layer_base);
     else if constexpr (D != kDealt) alone_slices<FP8, 4, 2>(c, a, st.n, st.layer_base);
   }
   step_close(a.state, st.step_seq, st.layer_base + (uint32_t)a.num_layers);
@@ -955,7 +962,8 @@ int mcb_launch_a2a_step(const McbCtx* ctx, const McbA2AStepArgs* args, int grid,
       return launch_kernel(kernel, dim3(grid), dim3(threads), 0, stream, pdl, false, *ctx, a);
     };
     if (!a.apart || a.topk > 32) return alone(std::integral_constant<int, kInOrder>{});
-    if (a.num_layers > kFewLayers && a.num_layers <= kSliceLayers && !a.fp8) return alone(std::integral_constant<int, kDealtOrSlices>{});
+    if (a.num_layers > kFewLayers && a.num_layers <= kSliceLayers && !a.fp8 && a.hidden <= (a.num_layers < kSliceLayers ? 1024 : 512))
+      return alone(std::integral_constant<int, kDealtOrSlices>{});
     if (a.num_layers > kFewLayers) return alone(std::integral_constant<int, kDealt>{});
     return a.num_layers > 1 ? alone(std::integral_constant<int, 2>{}) : alone(std::integral_constant<int, 1>{});
   }

@@ -378,17 +378,21 @@ def test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, 
     (1152, 5, 9, 1, 1, 64), (1152, 5, 9, 2, 2, 64),             # slices of four, the second of a row ragged, in several rounds
     (256, 8, 7, 3, 3, 32), (1024, 6, 8, 4, 2, 96),              # an odd layer at the end, and none
     (1024, 6, 8, 5, 2, 96),                                     # the first that is dealt
-    (1152, 5, 3, 7, 1, 192), (1152, 5, 5, 8, 2, 192),           # bf16 rows: a full round of slices; ten of twelve
-    (1152, 5, 4, 9, 1, 192), (128, 1, 29, 6, 3, 320),           # eight of twelve, dealt; 29 of 30
+    (1152, 5, 3, 7, 1, 192), (1152, 5, 5, 8, 2, 192),           # more layers, dealt: three and five rows of two slices each for six and twelve warps
+    (1152, 5, 4, 9, 1, 192), (128, 1, 29, 6, 3, 320),           # four rows; bf16: 29 slices for 30 warps
 ])
 def test_a2a_step_alone_few_layers(lib, world1, fp8, H, K, n, layers, grid, threads):
-    """Steps of up to four layers, and larger ones whose slices fill their rounds: the warps take slices of rows."""
+    """Steps of up to four layers, whose warps take slices of rows, and somewhat more."""
     test_a2a_step_alone_like_the_ranks(lib, world1, fp8, H, K, n, layers, grid, threads)
 
 
 @pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("H,K,n,layers,grid,threads", [
-    (1152, 5, 3, 5, 1, 192), (1152, 5, 5, 6, 2, 192), (1152, 5, 4, 6, 1, 192),      # bf16 rows: slices, a full round and ten of twelve; eight, dealt
+    (1152, 5, 3, 5, 1, 192), (1152, 5, 5, 6, 2, 192), (1152, 5, 4, 6, 1, 192),      # bf16 rows of two slices: dealt
+    (1024, 5, 6, 5, 1, 192), (1024, 5, 5, 5, 1, 192), (1024, 5, 4, 5, 1, 192),      # of one: a full round of six warps, five of six; four, dealt
+    (1024, 5, 12, 5, 1, 192), (512, 5, 18, 5, 1, 192), (512, 5, 23, 5, 1, 192),     # two rounds, dealt; three of half the length; four, dealt
+    (512, 5, 6, 6, 1, 192), (512, 5, 12, 6, 1, 192), (896, 5, 6, 6, 1, 192),        # six layers: slices; two rounds and longer rows, dealt
+    (256, 3, 29, 5, 1, 192), (256, 3, 30, 6, 1, 192), (128, 1, 11, 6, 1, 192),      # short rows, any number of rounds
     (256, 3, 7, 47, 3, 160), (256, 3, 7, 48, 3, 160), (1152, 5, 3, 49, 2, 64),      # bf16 rows: all warps, half of them
     (128, 1, 2, 60, 1, 32), (1024, 6, 5, 51, 1, 96),                                # one warp, two of three
 ])
