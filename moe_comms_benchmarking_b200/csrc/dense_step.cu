@@ -702,12 +702,15 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
 // The step of a world of one, a kernel of its own for each way: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.  D: as in local_few; kDealt: more layers; kInOrder: steps that read what they write.  With the last way in
 // each of the kernels, dealt steps were slower and so was one layer of e4m3 rows: 8192 rows of 1024, 88 layers 336 -> 298 us, 100 rows 9.5 -> 8.5; e4m3
-// 365 -> 344, one layer of 37 rows 4.8 -> 3.8.  Few layers of bf16 rows keep it: without it steps of 3.5 us took 0.1 to 0.3 us more.
+// 365 -> 344, one layer of 37 rows 4.8 -> 3.8.  Few layers of bf16 rows keep it, and are compiled for no number of blocks per SM (93 to 95 registers instead of
+// 121 to 128): without either, steps of 3.5 us took 0.1 to 0.5 us more.  2 / 3 / 4 layers of 20 rows of 1024 3.79 / 3.68 / 3.62 -> 3.56 / 3.48 / 3.38 us, of 150 rows
+// 3.79 / 3.87 / 3.84 -> 3.58 / 3.52 / 3.46; large steps of two layers would be faster with more (1000 rows of 7168 11.5 and 12.4).
 // Dealt e4m3 steps have 20 warps per block where others have 16: the quantisation waits for its own instructions, 344 -> 333 us, 58 layers of 2048 rows of
 // 7168 394 -> 375, small ones the same.  Copies do not gain from more warps: 640 threads 342 us where 512 took 331, 768 383.
 constexpr int kInOrder = 0, kDealt = -1;
 template <bool FP8, int D>
-__global__ void __launch_bounds__(FP8 && D == kDealt ? 640 : 512, 1) dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
+__global__ void __launch_bounds__(FP8 && D == kDealt ? 640 : 512, FP8 || D <= 0 ? 1 : 0)
+dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbDenseStepArgs a) {
   __shared__ int s_prefix[2], s_cnt[1], s_max;
   pdl_wait();                 // the previous kernel of this rank (the previous step) has finished
   pdl_launch_dependents();
@@ -728,18 +731,17 @@ __global__ void __launch_bounds__(FP8 && D == kDealt ? 640 : 512, 1) dense_alone
 #pragma unroll
   for (int t = 0; t < MCB_MAX_TENSORS; ++t)
     if (t < a.num_tensors) bytes_per_row += a.row_bytes[t];
-  __shared__ LocalRanges r;
+  const int nact = active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x);
   if (n > 0) {
+    __shared__ LocalRanges r;
     local_ranges<FP8>(r, c, a, n);
     if constexpr (D == kDealt) {
       local_dealt<FP8>(c, a, r, n, layer_base);
+    } else if constexpr (D == kInOrder) {
+      local_in_order<FP8>(c, a, r, n, nact, layer_base);
     } else {
-      bool in_order = D == kInOrder;
-      if constexpr (D > 0) {
-        if (!FP8) in_order = a.in_order;
-        if (!in_order) local_few<FP8, D>(c, a, r, n, layer_base);
-      }
-      if (in_order) local_in_order<FP8>(c, a, r, n, active_blocks((int)gridDim.x, n, bytes_per_row, (int)blockDim.x), layer_base);
+      if (FP8 || !a.in_order) local_few<FP8, D>(c, a, r, n, layer_base);
+      else local_in_order<FP8>(c, a, r, n, nact, layer_base);
     }
   }
   step_close(a.state, step_seq, layer_base + (uint32_t)L);
