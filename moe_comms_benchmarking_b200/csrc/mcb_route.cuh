@@ -200,7 +200,7 @@ __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& 
   }
 }
 
-// The whole routing by the blocks of a launch that has nothing else to share a barrier with.  With few entries nobody waits
+// The whole routing by the blocks of a launch: one of its own, or the fused dispatch + FC1 kernel's.  With few entries nobody waits
 // for another block: all count all entries and place their own (one block alone: 21.9 us a launch at 11264 entries of 512
 // experts, now 5.8; 8.5 and 4.2 at 1408; 3.0 and 3.8 at 128 of 32, where the wider scan shows); with many the blocks wait for one
 // another on a counter that only grows (the grid must be co-resident).  There a thread keeps its first kRouteKept entries from the
@@ -210,21 +210,25 @@ __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& 
 // combine of 8191 tokens with Zipf routing were 2 % slower; asked for before the number of tokens is known, few entries took
 // 8.4 us (7.2).  Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.
 constexpr int kRouteKept = 4;
-// Blocks of a launch of its own.  Blocks of 512 threads cost less to start and at each of their barriers than as many threads in blocks of 1024; three of them
-// for every one that the caller asked for (32) read and place large batches sooner.  One B200, us a launch in a row of them, 64 of 512 experts local:
+// Blocks of a launch of its own (ROUTE_GRID of the plan).  Blocks of 512 threads cost less to start and at each of their barriers than as many threads in blocks
+// of 1024, and 96 of them read and place large batches sooner than 32.  One B200, us a launch in a row of them, 64 of 512 experts local:
 //   entries                       352   1408   5632   8800   11264   15400   45056   90112   180202
 //   32 blocks of 1024 threads     4.0    4.2    4.9    5.5     5.7     6.3     6.9     7.7      9.7
 //   96 of 512                     3.3    3.5    4.6    5.4     5.9     5.9     6.0     6.7      6.5
 //   64 of 512                     3.5    3.5    4.5    5.4     5.9     5.7     6.0     6.8      8.1
 //   128 of 256 / of 512    3.2 / 3.3  3.7 / 3.6  5.3 / 4.6  5.5 / 5.8  5.7 / 6.1  5.7 / 6.0  6.0 / 6.2  6.7 / 6.8  7.8 / 6.5
-// There every block counts all of up to 24 entries per thread: 8800 entries 5.4 us (5.7 through the counters), 11264 5.9 (6.0), 15400 6.8 (5.9).
-constexpr int kRouteThreads = 512, kRouteBlocks = 3, kRouteAllAlone = 24;
-__device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem) {
+// Blocks of 512 threads count all of up to 24 entries per thread: 8800 entries 5.4 us (5.7 through the counters), 11264 5.9 (6.0), 15400 6.8 (5.9).
+// Callers that ask for fewer than 96 blocks get blocks of 1024 threads where the buffers hold more entries than 512 threads keep: 32 blocks of 512 / 1024 with
+// 45056, 90112, 180202 entries 6.4 / 7.0, 8.2 / 7.5, 11.1 / 9.8 us; 8 blocks with 11264, 22528, 90112 6.1 / 6.8, 8.1 / 7.4, 16.1 / 12.9.
+// The fused dispatch + FC1 kernel (blocks of 320 threads) counts all of as many: a layer of 512 / 64 / 16 experts of 512 x 256 with 5632 entries 102.0 -> 98.7,
+// 40.9 -> 40.4, 40.2 -> 39.8 us (16 per thread -> 24), with 7168 entries 102.7 -> 99.6, 43.3 -> 43.0, 41.9 -> 42.1.
+constexpr int kRouteThreads = 512, kRouteWideThreads = 1024, kRouteBlocks = 96, kRouteAllAlone = 24;
+__device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem, int all_per_thread = kRouteAllAlone) {
   const RouteSmem m(smem);
   const int tid = threadIdx.x, E = a.num_local_experts;
   const RouteShare s = route_share(a, (int)blockIdx.x, (int)gridDim.x);
   const BlockGroup g;
-  if (route_counts_all(g, s, kRouteAllAlone)) {
+  if (route_counts_all(g, s, all_per_thread)) {
     if (s.lo >= s.hi && blockIdx.x != 0) return;
     route_count<true>(g, a, a.topk_idx, m, 0, s.entries, s.lo);
     route_offsets(g, a, m, blockIdx.x == 0);

@@ -21,6 +21,7 @@ from ..parallel.symm_heap import HeapTensor, SymmetricHeap
 
 NUM_SMS = 148
 BLOCK_M = 128
+ROUTE_GRID = 96          # blocks of a routing launch: the number measured best over all batch sizes (csrc/mcb_route.cuh)
 # Activations (or expert outputs) of a layer up to which the layers of a step alternate between two buffers of them: nobody then waits
 # for the slowest CTA of the layer before, but twice the memory is written, which leaves L2 from some size on.  512 experts of
 # 1024 x 1024, one / 64 / 128 / 256 tokens (11.5 MB) 23.8 / 409 / 448 / 459 us a layer (26.1 / 411 / 452 / 459 with one buffer); 300 tokens
@@ -163,8 +164,11 @@ class RouteBuffers:
 
 
 class RoutePlan:
+    """Routing as a launch of its own.  ``grid`` is the most blocks that it takes (they wait on one another, so on a device
+    that holds fewer at once it takes those); the results do not depend on it."""
+
     def __init__(self, bufs: RouteBuffers, topk_idx: torch.Tensor, topk_w: torch.Tensor | None, num_tokens: torch.Tensor,
-                 expert_begin: int, status: torch.Tensor | None = None, grid: int = 32, timeout_s: float = 2.0):
+                 expert_begin: int, status: torch.Tensor | None = None, grid: int = ROUTE_GRID, timeout_s: float = 2.0):
         if topk_idx.dtype != torch.int64 or topk_idx.dim() != 2 or topk_idx.shape[1] != bufs.topk:
             raise ValueError("topk_idx must be int64 [tokens, topk]")
         if topk_idx.shape[0] < bufs.max_tokens:
@@ -172,7 +176,7 @@ class RoutePlan:
         if num_tokens.dtype != torch.int32:
             raise ValueError("num_tokens must be an int32 device scalar")
         if not (1 <= grid <= 128):
-            raise ValueError("routing grid must be in [1, 128] (its blocks wait on one another)")
+            raise ValueError("routing grid must be in [1, 128] blocks (they wait on one another)")
         self.bufs, self.grid = bufs, grid
         self._keep = (topk_idx, topk_w, num_tokens, status)
         a = _ext.McbRouteArgs()
@@ -226,8 +230,11 @@ class GroupedGemmPlan:
 
 
 class ExpertCombinePlan:
+    """The sums of every token's pair rows, and over the ranks, as a launch of its own of ``grid`` blocks: by default one per SM, and
+    two in a world of one whose rows are whole packs of 32 bytes, which then has a kernel of its own (``combine_alone_kernel``)."""
+
     def __init__(self, heap: SymmetricHeap, y: torch.Tensor, route: RouteBuffers, partial: HeapTensor, out: torch.Tensor,
-                 n_local: torch.Tensor, step_meta: torch.Tensor, cap: int, grid: int = NUM_SMS, threads: int = 512,
+                 n_local: torch.Tensor, step_meta: torch.Tensor, cap: int, grid: int | None = None, threads: int = 512,
                  site: int = _ext.SITE_FUSED_FC2):
         hidden = y.shape[-1]
         if y.dtype != torch.bfloat16 or out.dtype != torch.bfloat16 or hidden % 8:
@@ -237,6 +244,9 @@ class ExpertCombinePlan:
         two = partial.tensor.dim() == 3         # [2, cap * world, hidden]: alternate copies, layer by layer
         if (two and (partial.tensor.shape[0] != 2 or partial.tensor.shape[1] < rows)) or partial.nbytes < rows * hidden * 2:
             raise ValueError("partial-sum buffer must be [cap * world, hidden] or [2, cap * world, hidden]")
+        if grid is None:
+            alone = heap.world == 1 and hidden % 16 == 0 and (y.data_ptr() | out.data_ptr()) % 32 == 0
+            grid = 2 * NUM_SMS if alone else NUM_SMS
         self.heap, self.grid, self.threads = heap, grid, threads
         self._keep = (y, route, partial, out, n_local, step_meta)
         a = _ext.McbCombineArgs()

@@ -32,7 +32,7 @@ from ..config import Config
 from ..ops import _ext, oracle
 from ..ops.dense import AllGatherVPlan, MetadataPlan, DEFAULT_GRID, DEFAULT_THREADS, agv_ll_stage_bytes
 from ..ops.experts import (DispatchRouteFc1Plan, ExpertCombinePlan, ExpertFfnPlan, ExpertWeights, Fc2CombinePlan,
-                           GroupedGemmPlan, MoeLayerPlan, RouteBuffers, RoutePlan, NUM_SMS)
+                           GroupedGemmPlan, MoeLayerPlan, RouteBuffers, RoutePlan)
 from .base import Dispatcher
 from .dense import resolve_ll_rows
 from .symm_heap import SymmetricHeap, required_bytes
@@ -106,7 +106,7 @@ class FusedExpertDispatcher(Dispatcher):
         self.route_plan = RoutePlan(self.route, self.agv_r.tensor, self.agv_p.tensor, self.step_metadata[0:1],
                                     expert_begin=cfg.rank * E, status=st)
         self.combine_plan = ExpertCombinePlan(h, self.y, self.route, self.partial, self.out_buf, self.n_local,
-                                              self.step_metadata, cap, grid=NUM_SMS)
+                                              self.step_metadata, cap)
         if self.layer_kernel:
             self.ffn = [ExpertFfnPlan(w, self.route, self.agv_h.tensor, self.act, self.y, st) for w in self.weights]
             self.layer_plan = MoeLayerPlan(h, self.agv_plan, self.route_plan, self.ffn, self.combine_plan, self.meta_plan,

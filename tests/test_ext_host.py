@@ -420,3 +420,14 @@ def test_operation_numbers_are_the_librarys(lib, monkeypatch):
             with pytest.raises(_ext.ExtensionMissing, match="operation drift"):
                 _ext.load()
     assert _ext.load() is lib
+
+
+def test_route_grid_is_the_most_blocks():
+    """A routing launch takes as many blocks as the caller asks for, fewer only where the device holds fewer at once; wider blocks where few have many entries."""
+    lib = _ext.load()
+    assert [lib.mcb_route_blocks(g, 592) for g in (1, 2, 32, 96, 128)] == [1, 2, 32, 96, 128]
+    assert [lib.mcb_route_blocks(g, 72) for g in (1, 72, 73, 128)] == [1, 72, 72, 72]
+    assert [lib.mcb_route_blocks(g, 592) for g in (-1, 0, 129)] == [0, 0, 0]
+    threads = lambda entries, g: lib.mcb_route_threads(C.byref(_ext.McbRouteArgs(max_tokens=entries, topk=1)), g)
+    assert [threads(n, 2) for n in (1, 4096, 4097)] == [512, 512, 1024]
+    assert threads(1 << 20, 95) == 1024 and threads(1 << 20, 96) == threads(1 << 20, 128) == 512

@@ -405,16 +405,18 @@ def test_expert_combine_slices(world1, T, K, H):
 
 
 @pytest.mark.parametrize("T,K,H,shift,own", [
-    (4, 5, 512, 0, None), (5, 5, 512, 0, None),          # 8 warps: a slice of 512 bytes each, more of them: slices of 1024 bytes
-    (9, 33, 528, 0, None), (3, 2, 16, 0, None),          # a ragged last slice of either, more ids than lanes, half a pack
+    (4, 5, 512, 0, None), (148, 5, 512, 0, None), (149, 5, 512, 0, None),      # 296 warps: a slice of 512 bytes each, more of them: slices of 1024 bytes
+    (150, 33, 528, 0, None), (3, 2, 16, 0, None),        # a ragged last slice of either, more ids than lanes, half a pack
     (9, 5, 520, 0, None), (9, 5, 512, 8, None),          # no packs of 32 bytes: by the length of a row, by where the rows lie
-    (40, 4, 768, 0, (7, 21)), (40, 4, 768, 0, (30, 25)), (40, 4, 768, 0, (3, 0)),      # own rows inside, past the end, none
+    (400, 4, 768, 0, (7, 210)), (400, 4, 768, 0, (300, 250)), (400, 4, 768, 0, (3, 0)),      # own rows inside, past the end, none
+    (9, 5, 512, -1, None), (40, 4, 768, -1, (7, 21)),    # two blocks: the kernel of any world
 ])
 def test_expert_combine_alone(world1, T, K, H, shift, own):
     """The sums of a world of one add a token's rows in the order of its ids, in fp32 from zero, and round once, whichever way they go;
     rows of others keep what they held."""
     from moe_comms_benchmarking_b200.ops.experts import ExpertCombinePlan, RouteBuffers
     from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    grid, shift = (2, 0) if shift < 0 else (None, shift)
     g = torch.Generator(device=DEV).manual_seed(T * K + H)
     heap = SymmetricHeap(world1, T * H * 2 + (1 << 20), DEV)
     route = RouteBuffers(T, K, K, DEV)
@@ -426,7 +428,9 @@ def test_expert_combine_alone(world1, T, K, H, shift, own):
     first, rows = own or (0, T)
     out = torch.full((T, H), 7.0, dtype=torch.bfloat16, device=DEV)
     n, meta = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([rows], [T, first, rows, 1]))
-    ExpertCombinePlan(heap, y, route, heap.alloc("partial", [T, H], torch.bfloat16), out, n, meta, T, grid=2, threads=64).launch()
+    plan = ExpertCombinePlan(heap, y, route, heap.alloc("partial", [T, H], torch.bfloat16), out, n, meta, T, grid=grid, threads=32)
+    assert plan.grid == (2 if grid else 148 if H % 16 or shift else 296)
+    plan.launch()
     torch.cuda.synchronize()
     heap.check_status()
     ref = torch.zeros(T, H, device=DEV)
@@ -596,9 +600,11 @@ def test_route_many_entries(world1, T, grid):
         assert bool((route.pair_pos[T:] == -7).all()) and int(route.max_rows) == int(counts.max())
 
 
-@pytest.mark.parametrize("T,grid", [(2457, 1), (2457, 32), (2458, 1), (2458, 32), (2458, 43), (3, 32)])
+@pytest.mark.parametrize("T,grid", [(2457, 96), (2458, 96), (2458, 128), (3, 96), (3, 1),      # blocks of 512 threads
+                                    (816, 2), (817, 2), (3276, 3), (3277, 3)])                 # two wider ones and not, three of 1024
 def test_route_around_the_line(world1, T, grid):
-    """The last size whose entries every block counts, the first that is shared out, over three and 96 blocks and as many as there may be."""
+    """The last size whose entries every block counts, the first that is shared out; the last buffers that fewer blocks take with 512 threads, the first
+    with 1024."""
     test_route_many_entries(world1, T, grid)
 
 
