@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(THREADS, 1) route_kernel(const __grid_constant
   pdl_wait();
   pdl_launch_dependents();
   __shared__ int s_route[kRouteSmemWords];
-  route_device(a, s_route, THREADS == kRouteThreads ? kRouteAllAlone : kRouteAllPerThread);
+  route_device(a, s_route, THREADS != kRouteThreads ? kRouteAllPerThread : a.num_local_experts > 512 ? kRouteAllMany : kRouteAllAlone);
 }
 
 // ------------------------------------------------------------------------------------------------

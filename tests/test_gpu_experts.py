@@ -571,12 +571,12 @@ def test_expert_ffn_token_rows_of_any_shape(world1, shape):
 
 
 @pytest.mark.parametrize("T,grid", [(4097, 1), (4097, 3), (3277, 1), (5000, 128), (12300, 3)])
-def test_route_many_entries(world1, T, grid):
+def test_route_many_entries(world1, T, grid, E=24):
     """Routing whose entries are shared out over waiting blocks: all of a thread's kept until they are placed, more than that,
     and blocks without any; every entry of a local expert in its expert's rows once, the others marked, twice."""
     from moe_comms_benchmarking_b200.ops.experts import RouteBuffers, RoutePlan
-    E, K, first = 24, 5, 7
-    _, idx, w = _case(T, 40, K, 8, 8, 41)
+    K, first = 5, 7
+    _, idx, w = _case(T, E + 16, K, 8, 8, 41)
     route = RouteBuffers(T + 3, K, E, DEV)
     pad = lambda t: torch.cat([t, t[:3]]).contiguous()
     status = torch.zeros(8, dtype=torch.int32, device=DEV)
@@ -606,6 +606,12 @@ def test_route_around_the_line(world1, T, grid):
     """The last size whose entries every block counts, the first that is shared out; the last buffers that fewer blocks take with 512 threads, the first
     with 1024."""
     test_route_many_entries(world1, T, grid)
+
+
+@pytest.mark.parametrize("T,E", [(2458, 512), (2457, 513), (3276, 1024), (3277, 1024)])
+def test_route_around_the_line_many_experts(world1, T, E):
+    """From 513 local experts on every block counts more entries before they are shared out."""
+    test_route_many_entries(world1, T, 96, E)
 
 
 @pytest.mark.parametrize("E,K,H,I,T,layers,sets,grid", [
