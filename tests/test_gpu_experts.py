@@ -139,6 +139,46 @@ def test_expert_ffn_weights_as_m_against_oracle(world1, T, E, K, H, I, grid):
         assert float((out - ref).abs().max()) < 0.03 * float(ref.abs().max()) + 1e-3, "layer"
 
 
+@pytest.mark.parametrize("E,used", [(1024, 1024), (1024, 1023), (700, 640)])
+def test_expert_ffn_many_experts(world1, E, used):
+    """Up to as many experts as there may be, most with a token or two, some with two and three chunks, the last one empty or not: every pair's output against
+    fp32 with the same weights."""
+    from moe_comms_benchmarking_b200.ops.experts import ExpertFfnPlan, ExpertWeights, RouteBuffers, RoutePlan
+    from moe_comms_benchmarking_b200.parallel.symm_heap import SymmetricHeap
+    T, K, H, I = 1900, 2, 256, 128
+    x, _, w = _case(T, 8, K, H, I, 47)
+    t = torch.arange(T, device=DEV)
+    large = torch.tensor([3, 300, used - 1], device=DEV)                       # 600, 300 and 257 tokens, and one to three more
+    second = torch.cat([large[0].expand(600), large[1].expand(300), large[2].expand(257), t[1157:] * 7 % used])
+    idx = torch.stack([t % used, second], dim=1)
+    idx[:, 1] = torch.where(idx[:, 0] == idx[:, 1], (idx[:, 1] + 1) % used, idx[:, 1])
+    counts = torch.bincount(idx.flatten(), minlength=E)
+    assert bool((counts[:used] > 0).all()) and int(counts.max()) > 512 and int((counts > 256).sum()) == 3
+    heap = SymmetricHeap(world1, 1 << 20, DEV)
+    route = RouteBuffers(T, K, E, DEV)
+    weights = ExpertWeights(E, H, I, DEV, seed=5, std=0.05)
+    act = torch.full((route.max_pairs, I), float("nan"), dtype=torch.bfloat16, device=DEV)
+    y = torch.full((route.max_pairs, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+    RoutePlan(route, idx, w, torch.tensor([T], dtype=torch.int32, device=DEV), 0, heap.status).launch()
+    ExpertFfnPlan(weights, route, x, act, y, heap.status).launch()
+    torch.cuda.synchronize()
+    heap.check_status()
+    off, token = route.expert_offset.tolist(), route.pair_token.long()
+    w1, w2 = weights.w_gate_up, weights.w_down
+    # Rounded to bf16 once (2^-9, and as much again where that falls on the other side) from fp32 sums: 256 products whose magnitudes add up to about 10,
+    # each partial sum within 2^-23, 3e-4.
+    close = lambda got, want: bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 3e-4).all())
+    assert off[E] == T * K and torch.equal(route.expert_offset[1:].long() - route.expert_offset[:-1].long(), counts)
+    for e in range(E):
+        lo, hi = off[e], off[e + 1]
+        if lo == hi:
+            continue
+        gu = x[token[lo:hi]].double() @ w1[e].double().t()
+        assert close(act[lo:hi], torch.nn.functional.silu(gu[:, :I]) * gu[:, I:]), f"activations of expert {e}"
+        down = act[lo:hi].double() @ w2[e].double().t()                         # of the kernel's own activations
+        assert close(y[lo:hi], down * route.pair_prob[lo:hi].double().unsqueeze(1)), f"outputs of expert {e}"
+
+
 @pytest.mark.parametrize("W,B,ll_rows", [(2, 96, 0), (4, 40, 0), (2, 7, 16), (4, 1, 16)])
 def test_moe_layer_kernel_emulated_ranks(lib, W, B, ll_rows):
     """The whole-layer kernel (dispatch, routing, experts, combine in one cooperative launch) with W
