@@ -387,11 +387,20 @@ def test_world_of_one_few_layers(lib, fp8, n, layers, grid, threads):
     test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads)
 
 
-@pytest.mark.parametrize("fp8", [False, True])
 @pytest.mark.parametrize("n,layers,grid,threads", [
     (8, 40, 1, 96), (8, 41, 2, 64), (7, 88, 1, 32),       # half of three warps, of two, one
     (8, 39, 1, 96), (1, 40, 2, 96),                       # too few layers, too few items per warp
 ])
-def test_world_of_one_half_of_the_warps(lib, fp8, n, layers, grid, threads):
-    """Large copies of many layers go by half of the warps of a block."""
-    test_world_of_one_layers_dealt(lib, fp8, n, layers, grid, threads)
+def test_world_of_one_half_of_the_warps(lib, n, layers, grid, threads):
+    """Large bf16 copies of many layers go by half of the warps of a block."""
+    test_world_of_one_layers_dealt(lib, False, n, layers, grid, threads)
+
+
+@pytest.mark.parametrize("n,layers,grid,threads", [
+    (8, 88, 1, 512), (8, 41, 2, 384), (7, 17, 1, 128),    # 20 warps for 16, 15 for 12, five for four: several runs a warp, which begin inside a group's layers
+    (3, 60, 1, 96), (8, 39, 1, 32),                       # none more for three and for one
+    (5, 9, 148, 512),                                     # fewer items than warps
+])
+def test_world_of_one_more_warps(lib, n, layers, grid, threads):
+    """Dealt e4m3 steps have five warps for every four that the caller asked for."""
+    test_world_of_one_layers_dealt(lib, True, n, layers, grid, threads)
