@@ -513,15 +513,18 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
   }
 }
 
-// Layer after layer: steps that read what they write.  `nact`: blocks that a layer fills.
-template <bool FP8>
+// Layer after layer: steps that read what they write.  `nact`: blocks that a layer fills.  FEW: as in copy_ranges_in_order.  In a kernel of its own a layer of few
+// rows is a chain of a load and a store for each range, and what stands between them counts: 58 layers of 1 / 37 / 333 rows of 1024 in the kernel of dealt steps 97 / 115 /
+// 120 us, on their own 95 / 121 / 127, with FEW 92 / 109 / 110; e4m3 130 / 155 / 161, 126 / 147 / 152, 114 / 128 / 130.  2048 rows of 7168 952, 955, 956 (with FEW there
+// too 976).  The line: three packs of the expert outputs for a thread.
+template <bool FP8, bool FEW = false>
 __device__ __forceinline__ void local_in_order(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, int nact, uint32_t layer_base) {
   if ((int)blockIdx.x >= nact) return;
   const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)nact * blockDim.x;
   for (int l = 0; l < a.num_layers; ++l) {
     const uint32_t par = (layer_base + (uint32_t)l) & 1u;
     if (FP8) fp8_push<true>(c, a, par, 0, 0, n, start, stride);
-    copy_ranges_in_order(r, par, start, stride);
+    copy_ranges_in_order<FEW>(r, par, start, stride);
   }
 }
 
@@ -738,7 +741,8 @@ dense_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ Mcb
     if constexpr (D == kDealt) {
       local_dealt<FP8>(c, a, r, n, layer_base);
     } else if constexpr (D == kInOrder) {
-      local_in_order<FP8>(c, a, r, n, nact, layer_base);
+      if ((long long)n * a.rsv_row_bytes < 48ll * nact * blockDim.x) local_in_order<FP8, true>(c, a, r, n, nact, layer_base);
+      else local_in_order<FP8>(c, a, r, n, nact, layer_base);
     } else {
       if (FP8 || !a.in_order) local_few<FP8, D>(c, a, r, n, layer_base);
       else local_in_order<FP8>(c, a, r, n, nact, layer_base);

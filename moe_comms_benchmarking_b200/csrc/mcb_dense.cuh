@@ -144,6 +144,8 @@ __device__ __forceinline__ void copy_ranges(const LocalRanges& r, uint32_t parit
 
 // The same range by range, each dealt from the first thread on: pack i of every range belongs to the same thread, so what
 // a range reads of an earlier one's rows, in the same place, it reads after that one's store.
+// FEW: for threads that have one or two packs of a range; they leave the loops behind the last one.
+template <bool FEW = false>
 __device__ __forceinline__ void copy_ranges_in_order(const LocalRanges& r, uint32_t parity, long long start, long long stride) {
   constexpr int U = 8;
   const uint32_t word = r.load_word();
@@ -154,11 +156,15 @@ __device__ __forceinline__ void copy_ranges_in_order(const LocalRanges& r, uint3
     for (long long i0 = start; i0 < packs; i0 += stride * U) {
       uint4 v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u) {
+        if (FEW && i0 + u * stride >= packs) break;
         if (i0 + u * stride < packs) v[u] = ld_v4_stream(src + (i0 + u * stride) * 16);
+      }
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u) {
+        if (FEW && i0 + u * stride >= packs) break;
         if (i0 + u * stride < packs) st_v4(dst + (i0 + u * stride) * 16, v[u]);
+      }
     }
   }
   r.store_word(parity, word);

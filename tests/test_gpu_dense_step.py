@@ -297,6 +297,12 @@ def test_world_of_one_step_on_its_own_rows(lib, form, n, layers):
             assert torch.equal(gi.tensor[p, :n], ids[:n]) and torch.equal(gw.tensor[p, :n], w[:n])
 
 
+@pytest.mark.parametrize("form", ["in_place", "in_place_fp8", "identity"])
+@pytest.mark.parametrize("n,layers", [(11, 9), (12, 9), (130, 10)])      # fewer than three packs of the outputs for each of 128 threads, three, 33
+def test_world_of_one_step_on_its_own_rows_many_layers(lib, form, n, layers):
+    test_world_of_one_step_on_its_own_rows(lib, form, n, layers)
+
+
 @pytest.mark.parametrize("n", [1, 2, 3, 5, 9, 17])          # 32 packs to quantise a row on three warps: fewer groups of 64 than warps, and more
 @pytest.mark.parametrize("layers", [1, 3, 8, 9])
 @pytest.mark.parametrize("out_cols", [256, 64])             # as many packs of expert outputs, and fewer than are quantised
