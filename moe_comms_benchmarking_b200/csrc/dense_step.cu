@@ -47,6 +47,7 @@
 // instead of being invisible because consecutive layers carry identical bytes.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <type_traits>
 
 #include "mcb_barrier.cuh"
@@ -304,8 +305,9 @@ __device__ __forceinline__ void local_ranges(LocalRanges& r, const McbCtx& c, co
 
 // Layers [first, last) of one pack per lane, the loads of eight of them in flight together, and the stores of one parity before those of the other: they
 // go to the same place, and more of them merge in L1 than in the order of the layers.  One B200, us a step: 88 layers of 1000 / 6000 rows of 1024 42.8 / 212 ->
-// 38.6 / 180, 58 layers of 333 / 1000 rows of 7168 57.0 / 144 -> 51.2 / 133, 60 rows or fewer up to 5 % faster or the same.  (One parity of a whole run before the
-// other: large steps another 0 to 3 % faster, those of up to 60 rows 2 to 10 % slower.  e4m3 rows, which alternate, and all-to-all pieces did not gain.)
+// 38.6 / 180, 58 layers of 333 / 1000 rows of 7168 57.0 / 144 -> 51.2 / 133, 60 rows or fewer up to 5 % faster or the same.  (One parity of a whole run
+// before the other: large steps another 0 to 3 % faster, those of up to 60 rows 2 to 10 % slower.  e4m3 rows, which alternate, and all-to-all pieces did not
+// gain.)
 template <class Load, class Store>
 __device__ __forceinline__ void local_layers_of(int first, int last, Load load, Store store) {
   constexpr int D = 8;
@@ -325,31 +327,29 @@ __device__ __forceinline__ void local_layers_of(int first, int last, Load load, 
 // chip works on a few MB at a time; layer after layer over all rows, large steps went through up to 90 MB of L2 in every layer, small ones
 // left most of the chip idle, and sizes just above a whole number of packs per thread paid for the next one.
 // The loads may stay in L1, where 95 % of their sectors hit (24 layers of 2048 rows): large steps are bound by the stores that L1 has to
-// take and pass on, and loads with the hint that keeps them out of L1 took a third of L2's time.  88 layers of 1000 / 2048 / 8192 rows of 1024 60.7 / 107.8 / 417 -> 50.3 / 88.1 / 335 us
-// with all warps and stores in the order of the layers, e4m3 65.9 / 121 / 451 -> 55.8 / 103 / 382; 58 layers of 333 / 2048 rows of 7168 83 / 416 -> 69.5 / 327, e4m3 93 / 502 ->
-// 78 / 438.  The figures below are of loads from L2.
-// One B200, 88 layers of hidden 1024 and top-22, 1 / 37 / 100 / 333 / 512 / 2048 / 8192 rows, against up to four packs per thread with up to eight
-// layers in flight where a step fits, else layer after layer:
-//   bf16   29 -> 6.4 / 35 -> 8.4 / 25 -> 12.5 / 48 -> 35 / 39 -> 35 / 169 -> 111 / 651 -> 411 us
-//   e4m3   45 -> 8.4 / 53 -> 10.4 / 41 -> 14.5 / 53 -> 33 / 42 -> 37 / 150 -> 121 / 956 -> 450 us
-// and 58 layers of hidden 7168 and top-8, 1 / 64 / 512 / 2048 rows, bf16 19 -> 6.5 / 29 -> 21 / 178 -> 116 / 961 -> 425, e4m3 with 512 / 2048
-// rows 284 -> 133 / 1175 -> 501.  Sixteen layers in flight, or the loads of the next eight ahead of the stores: 6 to 15 % slower.  One size was
-// slower than before, e4m3 steps of 9 to 16 layers of about 512 rows of 1024, by up to 7 %.
-// Large copies of many layers go by half of the warps.  A layer's stores merge in L1 with those of the layer before the last to the same rows, if these are
-// still there: of 26.8 million sectors stored by 24 layers of 8192 rows 14.2 million went on to L2 with 16 warps per block and 10.8 million with 8.  With fewer
-// layers or fewer items per warp the time until a run's first load is there counts for more.  16 -> 8 warps, us (12 warps):
-//   88 layers  1024 values, 60 rows (13 items a warp) 6.4 -> 7.1 (6.6), 150 (47) 11.3 -> 13.9 (12.3), 400 (126) 22.6 -> 21.9 (22.3), 8192 292 -> 259 (267)
-//   58 layers  7168 values, 20 rows (28) 7.2 -> 8.7 (7.8), 60 (83) 15.4 -> 14.5 (14.8), 400 66.3 -> 60.5 (63.6), 2048 301 -> 289 (287)
-//   40 layers  7168 values, 60 rows (57) 11.5 -> 11.0 (11.3), 400 45.9 -> 42.1 (44.6), 2048 206 -> 207 (203); 1024 values, 8192 rows 128.5 -> 125.6 (122.8)
-//   26 layers  768 values, 400 rows (27) 7.3 -> 7.5 (7.3), 8192 62.8 -> 65.6 (61.2); 7168 values, 2048 rows 138 -> 158 (142)
-// Six warps: 1 to 14 % slower than eight.
-constexpr int kHalfLayers = 40, kHalfItems = 64;
+// take and pass on, and loads with the hint that keeps them out of L1 made 88 layers of 1000 to 8192 rows of 1024 20 to 25 % slower.
+// One B200, 58 layers, layer after layer (local_in_order) -> dealt, 1 / 37 / 333 / 2048 rows, us a step:
+//   1024 values  bf16 92 -> 4.2 / 109 -> 5.4 / 110 -> 20 / 131 -> 47     e4m3 114 -> 5.3 / 128 -> 7.3 / 130 -> 17.6 / 199 -> 61
+//   7168 values  bf16 98 -> 4.3 / 100 -> 11.5 / 128 -> 51 / 956 -> 274   e4m3 120 -> 5.6 / 121 -> 12.2 / 197 -> 67 / 1085 -> 373
+// Sixteen layers in flight, or the loads of the next eight ahead of the stores, were 6 to 15 % slower.
+// Copies of many layers with enough for every warp go by half of the warps: a layer's stores merge in L1 with earlier ones to the same rows, if these are still
+// there (of 26.8 million sectors stored by 24 layers of 8192 rows in the order of the layers 14.2 million went on to L2 with 16 warps per block and 10.8 million
+// with 8).  With fewer items a warp the time until a run's first load is there counts for more, and with many groups and fewer layers the rate of the warps.
+// One B200, all warps -> half of them, us a step (in brackets: (group, layer) items, groups for each of all warps):
+//   88 layers  1024 values, 60 rows (19) 6.0 -> 7.0, 150 (48) 10.7 -> 13.6, 1000 (317) 40.9 -> 38.9, 8192 (2593) 243 -> 238;  7168 values, 60 (125) 20.2 -> 19.7,
+//              2048 (4276) 393 -> 388
+//   58 layers  1024 values, 150 (31) 7.8 -> 9.8, 1000 (209) 28.0 -> 27.2, 8192 (1709, 29) 163 -> 166;  7168 values, 60 (83) 15.0 -> 14.6, 400 (551, 9) 58.6 -> 56.9,
+//              1000 (1376, 24) 133.8 -> 133.6, 2048 (2819, 49) 264 -> 275
+//   40 layers  7168 values, 60 (57) 10.5 -> 10.3, 400 (380, 9) 40.7 -> 39.9, 1000 (949, 24) 92.1 -> 94.8;  2048 values, 2048 rows (560, 14) 56.4 -> 56.3, 8192 (56) 211 -> 228
+//   32 layers  1024 values, 1000 rows (115) 16.2 -> 16.0, 2048 (236) 26.6 -> 27.0;  26 layers 23.3 -> 24.5
+constexpr int kHalfLayers = 40, kHalfItems = 64, kHalfAlways = 64, kHalfGroups = 20;
 
 template <bool FP8>
 __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, uint32_t layer_base) {
   const long long packs = r.end[LocalRanges::R - 1], groups = (packs + 31) >> 5;
   int used = (int)(blockDim.x >> 5);                                            // warps of a block that take part
-  if (!FP8 && a.num_layers >= kHalfLayers && (groups + 1) * a.num_layers >= (long long)kHalfItems * used * gridDim.x) used = (used + 1) / 2;
+  const int most = a.num_layers >= kHalfAlways ? INT_MAX : kHalfGroups * used * (int)gridDim.x;
+  if (!FP8 && a.num_layers >= kHalfLayers && (groups + 1) * a.num_layers >= (long long)kHalfItems * used * gridDim.x && groups <= most) used = (used + 1) / 2;
   if ((int)(threadIdx.x >> 5) >= used) return;
   const int lane = threadIdx.x & 31, warps = (int)gridDim.x * used;
   const int warp = (int)(blockIdx.x + (threadIdx.x >> 5) * gridDim.x);         // the smallest steps spread over the chip
@@ -424,14 +424,12 @@ __device__ __forceinline__ void local_dealt(const McbCtx& c, const McbDenseStepA
 // at a time, D = 1, 2, 4 or 8 the layers that it may have.  The groups go round the warps, so no warp divides.  Kernels of their own:
 // with both ways in one, the large steps of many layers were 3 to 7 % slower and every step 0.5 to 1 us.
 // One B200, a step of 1 / 2 / 4 / 8 layers in a row of steps, dealt in runs -> this way:
-//   hidden 1024 and top-22, 512 rows    bf16 5.0 / 5.5 / 5.9 / 6.5 -> 4.2 / 3.9 / 4.4 / 5.5     e4m3 5.9 / 6.7 / 8.2 / 8.9 -> 5.2 / 5.9 / 6.0 / 7.5 us
-//                          8192 rows    bf16 34.9 / 35.7 / 37 / 41 -> 11.9 / 17.0 / 25.8 / 39.2  e4m3 30.5 / 33.7 / 39 / 54 -> 13.7 / 19.2 / 28.7 / 50
-//   hidden 7168 and top-8, 2048 rows    bf16 56 / 61 / 62 / 66 -> 20.4 / 31.3 / 41.5 / 61        e4m3 51 / 56 / 65 / 89 -> 20.6 / 31.5 / 47.6 / 81
-// (layer after layer, 8192 rows of 1024: bf16 12.0 / 19.8 / 34.9 / 63, e4m3 17.1 / 27.9 / 52 / 96).  Nine to sixteen layers by rounds of eight:
-// up to 25 % slower than runs with bf16 rows, 10 % faster to 10 % slower with e4m3 rows, so the line is at one round.  Loads of the layers of a pack
-// after the first hit L1 here too: 4 / 8 layers of 2048 rows of 7168 41.4 / 61.8 -> 38.3 / 50.6 us, e4m3 46.3 / 81 -> 44.4 / 75.9 (the figures above are of
-// loads from L2).  With the stores to one place one after the other instead of layer by layer, 2 / 4 / 8 layers of 6000 rows of 1024 11.6 / 16.9 / 22.9 ->
-// 10.7 / 13.4 / 19.8, of 333 rows of 7168 6.7 / 8.8 / 10.4 -> 6.1 / 7.3 / 9.4.
+//   hidden 1024 and top-22, 64 rows     bf16 4.0 / 4.0 / 3.9 / 4.6 -> 3.8 / 3.6 / 3.3 / 3.6          e4m3 5.6 / 5.8 / 6.0 / 6.1 -> 4.2 / 4.3 / 4.6 / 5.7 us
+//                          512 rows     bf16 4.8 / 5.3 / 5.3 / 5.6 -> 4.1 / 4.0 / 4.1 / 4.8          e4m3 5.9 / 6.9 / 7.8 / 8.2 -> 4.6 / 4.9 / 5.3 / 6.4
+//                          8192 rows    bf16 29.9 / 33.2 / 33.2 / 35.2 -> 11.8 / 16.1 / 19.5 / 28.5  e4m3 23.6 / 26.4 / 30.5 / 41.9 -> 11.0 / 14.6 / 22.5 / 38.3
+//   hidden 7168 and top-8, 2048 rows    bf16 54 / 57 / 57 / 59 -> 20.3 / 29.5 / 35.2 / 49.7          e4m3 41.5 / 46.3 / 52.7 / 70.7 -> 17.6 / 28.6 / 42.0 / 68.4
+// Nine to sixteen layers by rounds of eight were up to 25 % slower than runs with bf16 rows and 10 % either way with e4m3 rows, so the line is at one round.
+// Stores to one place one after the other instead of layer by layer: 2 / 4 / 8 layers of 333 rows of 7168 6.7 / 8.8 / 10.4 -> 6.1 / 7.3 / 9.4.
 constexpr int kFewLayers = 8;
 
 template <bool FP8, int D>
@@ -513,10 +511,10 @@ __device__ __forceinline__ void local_few(const McbCtx& c, const McbDenseStepArg
   }
 }
 
-// Layer after layer: steps that read what they write.  `nact`: blocks that a layer fills.  FEW: as in copy_ranges_in_order.  In a kernel of its own a layer of few
-// rows is a chain of a load and a store for each range, and what stands between them counts: 58 layers of 1 / 37 / 333 rows of 1024 in the kernel of dealt steps 97 / 115 /
-// 120 us, on their own 95 / 121 / 127, with FEW 92 / 109 / 110; e4m3 130 / 155 / 161, 126 / 147 / 152, 114 / 128 / 130.  2048 rows of 7168 952, 955, 956 (with FEW there
-// too 976).  The line: three packs of the expert outputs for a thread.
+// Layer after layer: steps that read what they write.  `nact`: blocks that a layer fills.  FEW: as in copy_ranges_in_order.  In a kernel of its own a layer
+// of few rows is a chain of a load and a store for each range, and what stands between them counts: 58 layers of 1 / 37 / 333 rows of 1024 in the kernel of
+// dealt steps 97 / 115 / 120 us, on their own 95 / 121 / 127, with FEW 92 / 109 / 110; e4m3 130 / 155 / 161, 126 / 147 / 152, 114 / 128 / 130.  2048 rows of
+// 7168 952, 955, 956 (with FEW there too 976).  The line: three packs of the expert outputs for a thread.
 template <bool FP8, bool FEW = false>
 __device__ __forceinline__ void local_in_order(const McbCtx& c, const McbDenseStepArgs& a, const LocalRanges& r, int n, int nact, uint32_t layer_base) {
   if ((int)blockIdx.x >= nact) return;
@@ -706,10 +704,10 @@ __global__ void __launch_bounds__(512) dense_step_kernel(const __grid_constant__
 // through pointers after every store.  D: as in local_few; kDealt: more layers; kInOrder: steps that read what they write.  With the last way in
 // each of the kernels, dealt steps were slower and so was one layer of e4m3 rows: 8192 rows of 1024, 88 layers 336 -> 298 us, 100 rows 9.5 -> 8.5; e4m3
 // 365 -> 344, one layer of 37 rows 4.8 -> 3.8.  Few layers of bf16 rows keep it, and are compiled for no number of blocks per SM (93 to 95 registers instead of
-// 121 to 128): without either, steps of 3.5 us took 0.1 to 0.5 us more.  2 / 3 / 4 layers of 20 rows of 1024 3.79 / 3.68 / 3.62 -> 3.56 / 3.48 / 3.38 us, of 150 rows
-// 3.79 / 3.87 / 3.84 -> 3.58 / 3.52 / 3.46; large steps of two layers would be faster with more (1000 rows of 7168 11.5 and 12.4).
-// Dealt e4m3 steps have 20 warps per block where others have 16: the quantisation waits for its own instructions, 344 -> 333 us, 58 layers of 2048 rows of
-// 7168 394 -> 375, small ones the same.  Copies do not gain from more warps: 640 threads 342 us where 512 took 331, 768 383.
+// 121 to 128): without either, steps of 3.5 us took 0.1 to 0.5 us more.  2 / 3 / 4 layers of 20 rows of 1024 3.79 / 3.68 / 3.62 -> 3.56 / 3.48 / 3.38 us, of
+// 150 rows 3.79 / 3.87 / 3.84 -> 3.58 / 3.52 / 3.46; large steps of two layers would be faster with more (1000 rows of 7168 11.5 and 12.4). Dealt e4m3 steps
+// have 20 warps per block where others have 16: the quantisation waits for its own instructions, 344 -> 333 us, 58 layers of 2048 rows of 7168 394 -> 375,
+// small ones the same.  Copies do not gain from more warps: 640 threads 342 us where 512 took 331, 768 383.
 constexpr int kInOrder = 0, kDealt = -1;
 template <bool FP8, int D>
 __global__ void __launch_bounds__(FP8 && D == kDealt ? 640 : 512, FP8 || D <= 0 ? 1 : 0)

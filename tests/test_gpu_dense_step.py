@@ -396,6 +396,7 @@ def test_world_of_one_few_layers(lib, fp8, n, layers, grid, threads):
 @pytest.mark.parametrize("n,layers,grid,threads", [
     (8, 40, 1, 96), (8, 41, 2, 64), (7, 88, 1, 32),       # half of three warps, of two, one
     (8, 39, 1, 96), (1, 40, 2, 96),                       # too few layers, too few items per warp
+    (8, 63, 1, 32), (5, 63, 1, 32), (8, 64, 1, 32),       # one warp: more groups than go by half with 63 layers, as many; more with 64
 ])
 def test_world_of_one_half_of_the_warps(lib, n, layers, grid, threads):
     """Large bf16 copies of many layers go by half of the warps of a block."""
