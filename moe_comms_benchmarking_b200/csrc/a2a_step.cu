@@ -649,27 +649,27 @@ __device__ __forceinline__ uint4 alone_sum(bool sent, uint4 v) {
 //            carries the number of its layer, and 32 packs of a row of sums over expert outputs, which alternate between two buffers.  (The identity
 //            expert on bf16 rows returns the row: its sums are the pieces' own.)
 // A warp with one chain more than others takes fewer pieces.  Large steps are bound by the stores that leave L1 (below) or, with e4m3 rows, by the
-// instructions of the quantisation; the loads may stay in L1, where 95 % of their sectors hit (24 layers of 333 e4m3 rows of 7168).  From L2, which the
-// hint against L1 made of every load: 58 layers of 333 / 1000 / 2048 e4m3 rows of 7168 98.9 / 283 / 559 -> 85.9 / 236 / 466 us, 88 layers of 333 / 2048 / 8192 of
-// 1024 29.9 / 141 / 527 -> 24.9 / 121 / 446, bf16 rows 33.3 / 124 * / 465 * -> 31.1 / 116 * / 427 *.  One B200, loads from L2, against up to four packs per
-// lane with up to eight layers in flight where the slices fit the warps, else slices of four packs layer after layer:
-//   88 layers of hidden 1024 and top-22, 1 / 37 / 333 / 1000 / 4096 rows (* by slices, as these bf16 steps went then)
-//     bf16   35 -> 10.5 / 35 -> 12.5 / 40 -> 33 / 76 -> 68 / 272 -> 249 * us
-//     e4m3   43 -> 10.5 / 45 -> 12.5 / 56 -> 29 / 91 -> 73 / 398 -> 268 us
-//   58 layers of hidden 7168 and top-8, 1 / 37 / 333 / 1000 / 2048 rows
-//     bf16   25 -> 8.5 / 27 -> 18 / 101 -> 96 * / 262 -> 253 * / 786 -> 533 * us
-//     e4m3   31 -> 10.2 / 35 -> 19 / 112 -> 99 / 402 -> 280 / 969 -> 563 us
+// instructions of the quantisation; the loads may stay in L1, where 95 % of their sectors hit (24 layers of 333 e4m3 rows of 7168).  With the hint that
+// keeps them out, e4m3 steps of 333 to 2048 rows of 7168 were 15 to 20 % slower.
+// One B200, 58 layers, layer after layer (alone_many) -> dealt, 1 / 37 / 333 / 2048 rows, us a step:
+//   1024 values  bf16 55 -> 5.5 / 57 -> 6.8 / 58 -> 12.1 / 87 -> 48     e4m3 84 -> 6.2 / 86 -> 7.2 / 87 -> 15.6 / 132 -> 73
+//   7168 values  bf16 54 -> 5.5 / 57 -> 9.2 / 93 -> 46 / 752 -> 245     e4m3 84 -> 6.2 / 86 -> 12.7 / 125 -> 75 / 911 -> 427
 // With one chain for both parities of a metadata row, its chunks put together by shuffles, the smallest steps took 16.7 and 14.6 us.
 // The ids asked for in every layer again, or more layers in flight than here, were 10 to 25 % slower with e4m3 rows.  Slower than slices
 // remain e4m3 steps of five layers, by up to 14 % at some sizes.
-// Steps of bf16 rows are bound by the stores that leave L1, where stores to the same rows merge.  So of eight layers of a piece in flight those to the received rows
-// of one parity come first, then those of the other, then the sums; and from kHalfLayers layers on half of the warps take part, whose rows are still in L1
-// more often.  In the order of the layers (large steps by slices) -> so, us a step:
-//   hidden 1024, 88 layers of 20 / 150 / 1000 / 6000 rows   9.0 -> 8.1, 13.9 -> 10.8, 61.4 -> 37.3, 328 -> 191 (16 warps 8.4 / 11.4 / 44.1 / 241)
-//   hidden 7168, 58 layers of 20 / 333 / 2048 rows          9.7 -> 7.3, 83.4 -> 48.5, 490 -> 258 (7.7 / 59.4 / 335)
-//   26 layers, 333 and 2048 rows                            39.0 -> 27.4, 219 -> 132 (8 warps 26.8, 151); hidden 768 8.8 -> 7.2, 28.5 -> 20.5 (8.1, 24.3)
-//   40 layers, hidden 768 and 1024, 2048 rows               41.8 -> 28.7, 53.5 -> 37.9 (30.2, 36.9); 48 layers 49.3 -> 33.1, 64.4 -> 45.5 (33.9, 42.3)
-// (e4m3 rows, bound by their instructions, take their layers as they come.)
+// Steps of bf16 rows are bound by the stores that leave L1, where stores to the same rows merge.  So of eight layers of a piece in flight those to the
+// received rows of one parity come first, then those of the other, then the sums; and from kHalfLayers layers on half of the warps take part, whose rows are
+// still in L1 more often.  All warps -> half of them, us a step (in brackets: (piece, layer) items for each of all warps):
+//   58 layers   1024 values, 1 / 150 (15) / 333 (33) / 2048 rows 6.3 -> 6.1, 8.6 -> 9.1, 13.2 -> 12.1, 56.6 -> 47.8;  7168 values, 20 (14) / 2048 7.5 -> 7.2, 331 -> 246
+//   48 layers   1024 values, the same rows 5.5 -> 5.2, 7.5 -> 7.9, 11.5 -> 10.8, 47.2 -> 40.8;  2048 values, 20 / 150 (24) / 2048 6.4 -> 6.0, 9.9 -> 9.9, 83.6 -> 66.7
+//               768 values, 333 (20) / 2048 9.6 -> 9.8, 34.1 -> 32.1;  7168 values, 20 / 2048 6.8 -> 6.5, 270 -> 206
+//   40 layers   768 values, 333 (17) / 1000 (51) / 2048 (104) 8.4 -> 8.9, 15.9 -> 16.3, 28.8 -> 28.3;  1024 values, 150 (10) / 1000 (68) 6.8 -> 7.2, 21.0 -> 20.0
+//               7168 values, 20 (9) / 150 (71) / 2048 6.4 -> 6.2, 20.3 -> 17.8, 221 -> 177
+//   26 layers   768 values, 333 / 2048 6.9 -> 7.6, 20.2 -> 22.0;  1024 values, 150 / 2048 6.3 -> 7.3, 26.2 -> 26.4;  7168 values, 333 / 2048 27.9 -> 24.3, 139 -> 133
+// From 48 layers on half is better but for some 10 to 25 items a warp, by up to 6 %.  Below, large steps of long rows would gain too, but a line that depends
+// on the number of rows costs every small step 0.1 us.  With expert outputs of their own, whose sums are chains, half is up to 17 % slower at 10 to 35 items
+// a warp (48 layers of 150 rows of 1024 8.2 -> 9.6) and up to 25 % faster beyond (88 layers of 333 rows of 7168 108 -> 80). (e4m3 rows, bound by their
+// instructions, take their layers as they come.)
 constexpr int kHalfLayers = 48;
 template <bool FP8>
 __device__ __forceinline__ void alone_dealt(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
@@ -830,14 +830,14 @@ __device__ __forceinline__ void alone_slices(const McbCtx& c, const McbA2AStepAr
 }
 
 // A step of up to this many layers has too few of one piece to keep loads in flight: there the warps take slices, of one pack per lane
-// or two where that still gives every slice a warp of its own, else of four (four instead of two: 811 e4m3 rows of 1024 15 to 25 % slower).  Kernels of their own, for one layer (D = 1) and for more (D = 2), which are
-// smaller than that of the dealt steps.  One B200, a step of 1 / 2 / 3 / 4 layers in a row of steps, dealt -> slices:
-//   hidden 1024 and top-22, 64 rows     bf16 5.0 / 4.5 / 4.6 / 4.5 -> 4.2 / 4.3 / 4.9 / 4.7      e4m3 5.2 / 5.3 / 4.8 / 4.8 -> 4.2 / 4.7 / 4.8 / 5.1 us
-//                          8192 rows    bf16 32.4 / 28.2 / 29.3 / 33.1 -> 9.8 / 15.5 / 21.0 / 26.7  e4m3 40.1 / 42.7 / 47 / 49 -> 13.0 / 20.0 / 27.6 / 33.5
-//   hidden 7168 and top-8, 2048 rows    bf16 39 / 44 / 47 / 50 -> 17.0 / 28.7 / 35.6 / 43.3      e4m3 56 / 63 / 72 / 77 -> 21.1 / 33.4 / 45.4 / 55.6
-// (layer after layer, 8192 rows of 1024: bf16 11.1 / 17.1 / 23.5 / 29.0, e4m3 15.1 / 25.0 / 34.5 / 44).  With five to eight layers the dealt steps of up
-// to 200 rows are 5 to 35 % faster than slices, and larger ones up to 30 % slower.  Four layers at a time,
-// or eight, were 3 to 40 % slower than two.
+// or two where that still gives every slice a warp of its own, else of four (four instead of two: 811 e4m3 rows of 1024 15 to 25 % slower).  Kernels of their
+// own, for one layer (D = 1) and for more (D = 2), which are smaller than that of the dealt steps.  One B200, a step of 1 / 2 / 3 / 4 layers in a row of
+// steps, dealt -> slices:
+//   hidden 1024 and top-22, 64 rows     bf16 4.7 / 4.7 / 4.8 / 4.7 -> 4.2 / 4.3 / 4.7 / 4.6          e4m3 4.9 / 5.0 / 4.9 / 5.0 -> 4.1 / 4.5 / 5.1 / 5.5 us
+//                          512 rows     bf16 5.7 / 5.7 / 5.9 / 5.9 -> 4.3 / 4.3 / 4.8 / 5.0          e4m3 6.1 / 6.4 / 7.2 / 7.4 -> 4.3 / 4.8 / 5.5 / 6.0
+//                          8192 rows    bf16 23.4 / 25.4 / 27.2 / 28.5 -> 9.9 / 14.7 / 20.0 / 24.9   e4m3 36.2 / 39.9 / 44.0 / 46.4 -> 12.8 / 19.9 / 26.7 / 32.1
+//   hidden 7168 and top-8, 2048 rows    bf16 37.0 / 42.5 / 43.8 / 44.6 -> 16.1 / 24.1 / 31.1 / 38.9  e4m3 56.9 / 62.9 / 68.7 / 72.7 -> 20.6 / 32.6 / 44.2 / 53.4
+// Four layers at a time, or eight, were 3 to 40 % slower than two.
 constexpr int kFewLayers = 4;
 template <bool FP8, int D>
 __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs& a, int n, uint32_t layer_base) {
@@ -847,10 +847,10 @@ __device__ __forceinline__ void alone_few(const McbCtx& c, const McbA2AStepArgs&
   else alone_slices<FP8, 4, D>(c, a, n, layer_base);
 }
 
-// Whether a step of the identity expert on bf16 rows with five or six layers goes by slices of four packs per lane, where a slice is a whole row.  It writes its
-// row, its sums and its metadata in one go, which saves a dealt step's addresses, but it is all layers of a row: a last round of warps that is less than 5/6
-// full is waited for, and where rows are longer, or a warp gets more of them, dealt pieces keep more loads in flight and more of their stores merge.
-// One B200, us a step, dealt -> slices, one / two / three rounds of warps (0.96 full):
+// Whether a step of the identity expert on bf16 rows with five or six layers goes by slices of four packs per lane, where a slice is a whole row.  It writes
+// its row, its sums and its metadata in one go, which saves a dealt step's addresses, but it is all layers of a row: a last round of warps that is less than
+// 5/6 full is waited for, and where rows are longer, or a warp gets more of them, dealt pieces keep more loads in flight and more of their stores merge. One
+// B200, us a step, dealt -> slices, one / two / three rounds of warps (0.96 full):
 //   five layers   256 values 7.3 -> 5.8 / 10.3 -> 8.6 / 13.6 -> 11.9        512 values 8.9 -> 7.8 / 12.9 -> 11.8 / 16.4 -> 15.7
 //                 768 values 10.1 -> 9.2 / 15.2 -> 14.9 / 19.6 -> 20.0      1024 values 11.2 -> 10.7 / 17.3 -> 17.7 / 23.0 -> 24.5
 //   six layers    256 values 7.8 -> 6.7 / 10.5 -> 9.2 / 13.5 -> 12.4        512 values 8.6 -> 8.4 / 13.2 -> 13.2 / 17.3 -> 18.1
@@ -884,8 +884,9 @@ __device__ __forceinline__ void alone_many(const McbCtx& c, const McbA2AStepArgs
 
 // The step of a world of one, a kernel of its own for each way: everything is inline, so the arguments are read from the constant bank and not
 // through pointers after every store.  D: as in alone_few; kDealt: more layers; kDealtOrSlices: alone_by_slices; kInOrder: steps that read what they write,
-// more than 32 ids.  With the last in the kernel of dealt steps, these had 24 bytes of stack and e4m3 ones were slower: 58 layers of 333 rows of 7168 82.2 -> 78.1 us, 88 layers of
-// one / 37 / 2048 rows of 1024 7.9 / 9.5 / 115 -> 7.2 / 8.7 / 110.  (More or fewer than 16 warps per block: 3 to 10 % slower with e4m3 rows.)
+// more than 32 ids.  With the last in the kernel of dealt steps, these had 24 bytes of stack and e4m3 ones were slower: 58 layers of 333 rows of 7168 82.2 ->
+// 78.1 us, 88 layers of one / 37 / 2048 rows of 1024 7.9 / 9.5 / 115 -> 7.2 / 8.7 / 110.  (More or fewer than 16 warps per block: 3 to 10 % slower with e4m3
+// rows.)
 constexpr int kInOrder = 0, kDealt = -1, kDealtOrSlices = -2;
 template <bool FP8, int D>
 __global__ void __launch_bounds__(512, 1) a2a_alone_kernel(const __grid_constant__ McbCtx c, const __grid_constant__ McbA2AStepArgs a) {

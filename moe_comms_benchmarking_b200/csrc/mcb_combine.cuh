@@ -13,7 +13,8 @@
 // now 9).  With four packs every warp has an item and memory is the limit; what is best there depends on the kernel around:
 //   combine_kernel (ALONE)  one row at a time, with ordinary loads.  4096 rows of 1024 values, 8 pairs each: 9.5 us (18.4 with
 //                           four rows in flight and streaming loads, 28 with two, 11.4 with four and ordinary loads); 22 pairs
-//                           each, 184 MB of them: 39.6 (53, 90, 61).  A world of one comes here only with rows that are no multiple of 32 bytes;
+//                           each, 184 MB of them: 39.6 (53, 90, 61).  A world of one comes here with rows that are no multiple of 32 bytes,
+//                           with y or out off a 32-byte boundary, and with fewer blocks than combine_alone_kernel takes;
 //   behind the experts      two rows, with streaming loads.  The combine of the layer kernel at 4096 / 2048 tokens of 22 pairs:
 //                           41 / 24 us (44 / 26 with four rows, 59 / 37 with one and ordinary loads, 53 / 32 with one).
 // Call from all threads of the block (any size that is a multiple of 32), or in a world of one from `nwarps` of its warps.

@@ -197,7 +197,8 @@ __device__ __forceinline__ int ffn_slots(const Group& g, const int* off, int E, 
   const int e0 = tid * per, e1 = e0 + per < E ? e0 + per : E;
   // Experts with tokens in the low kFfnSlotBits, chunks above: one scan for both, and one of the warps' sums by every warp for itself.  Nothing streams
   // before the units are listed: with a scan each, the warps' sums added up one by one and every unit searched for through both of its bounds (unit), the
-  // smallest launches took 14.5 us (14.0 so; 8 tokens of 16 experts of 512 x 256), 64 experts of 1024 x 1024 with 174 / 2800 / 11000 pairs 61.9 / 70.3 / 86.4 (61.2 / 69.6 / 85.2).
+  // smallest launches took 14.5 us (14.0 so; 8 tokens of 16 experts of 512 x 256), 64 experts of 1024 x 1024 with 174 / 2800 / 11000 pairs 61.9 / 70.3 / 86.4
+  // (61.2 / 69.6 / 85.2).
   uint32_t mine = 0;
   for (int e = e0; e < e1; ++e) {
     const int rows = off[e + 1] - off[e];

@@ -210,21 +210,21 @@ __device__ __forceinline__ void route_place(const Group& g, const McbRouteArgs& 
 // combine of 8191 tokens with Zipf routing were 2 % slower; asked for before the number of tokens is known, few entries took
 // 8.4 us (7.2).  Call from all threads of every block; `smem` is kRouteSmemWords words of shared memory.
 constexpr int kRouteKept = 4;
-// Blocks of a launch of its own (ROUTE_GRID of the plan).  Blocks of 512 threads cost less to start and at each of their barriers than as many threads in blocks
-// of 1024, and 96 of them read and place large batches sooner than 32.  One B200, us a launch in a row of them, 64 of 512 experts local:
+// Blocks of a launch of its own (ROUTE_GRID of the plan).  Blocks of 512 threads cost less to start and at each of their barriers than as many threads in
+// blocks of 1024, and 96 of them read and place large batches sooner than 32.  One B200, us a launch in a row of them, 64 of 512 experts local:
 //   entries                       352   1408   5632   8800   11264   15400   45056   90112   180202
 //   32 blocks of 1024 threads     4.0    4.2    4.9    5.5     5.7     6.3     6.9     7.7      9.7
 //   96 of 512                     3.3    3.5    4.6    5.4     5.9     5.9     6.0     6.7      6.5
 //   64 of 512                     3.5    3.5    4.5    5.4     5.9     5.7     6.0     6.8      8.1
 //   128 of 256 / of 512    3.2 / 3.3  3.7 / 3.6  5.3 / 4.6  5.5 / 5.8  5.7 / 6.1  5.7 / 6.0  6.0 / 6.2  6.7 / 6.8  7.8 / 6.5
 // Blocks of 512 threads count all of up to 24 entries per thread, of up to 32 with more than 512 local experts, whose counters cost more.  All counted by
-// every block (through the counters), us: 64 local experts 8800 entries 5.4 (5.7), 11264 5.9 (6.0), 15400 6.8 (5.9); 512 of them 11264 5.7 (6.2), 12200 5.8 (6.7),
-// 15400 6.5 (6.5); 1024 of them 12200 6.1 (7.1), 15400 6.8 (7.3).  (32 blocks of 1024 threads took 5.6 to 6.0 with 11264; asking for eight entries at a time instead of four
-// brings these to 5.6 and everything below 9000 entries 5 to 8 % up, as a second loop for more than 10240 entries 0 to 2 %.)
-// Callers that ask for fewer than 96 blocks get blocks of 1024 threads where the buffers hold more entries than 512 threads keep: 32 blocks of 512 / 1024 with
-// 45056, 90112, 180202 entries 6.4 / 7.0, 8.2 / 7.5, 11.1 / 9.8 us; 8 blocks with 11264, 22528, 90112 6.1 / 6.8, 8.1 / 7.4, 16.1 / 12.9.
-// The fused dispatch + FC1 kernel (blocks of 320 threads) counts all of as many: a layer of 512 / 64 / 16 experts of 512 x 256 with 5632 entries 102.0 -> 98.7,
-// 40.9 -> 40.4, 40.2 -> 39.8 us (16 per thread -> 24), with 7168 entries 102.7 -> 99.6, 43.3 -> 43.0, 41.9 -> 42.1.
+// every block (through the counters), us: 64 local experts 8800 entries 5.4 (5.7), 11264 5.9 (6.0), 15400 6.8 (5.9); 512 of them 11264 5.7 (6.2), 12200 5.8
+// (6.7), 15400 6.5 (6.5); 1024 of them 12200 6.1 (7.1), 15400 6.8 (7.3).  (32 blocks of 1024 threads took 5.6 to 6.0 with 11264; asking for eight entries at
+// a time instead of four brings these to 5.6 and everything below 9000 entries 5 to 8 % up, as a second loop for more than 10240 entries 0 to 2 %.) Callers
+// that ask for fewer than 96 blocks get blocks of 1024 threads where the buffers hold more entries than 512 threads keep: 32 blocks of 512 / 1024 with 45056,
+// 90112, 180202 entries 6.4 / 7.0, 8.2 / 7.5, 11.1 / 9.8 us; 8 blocks with 11264, 22528, 90112 6.1 / 6.8, 8.1 / 7.4, 16.1 / 12.9. The fused dispatch + FC1
+// kernel (blocks of 320 threads) counts all of as many: a layer of 512 / 64 / 16 experts of 512 x 256 with 5632 entries 102.0 -> 98.7, 40.9 -> 40.4, 40.2 ->
+// 39.8 us (16 per thread -> 24), with 7168 entries 102.7 -> 99.6, 43.3 -> 43.0, 41.9 -> 42.1.
 constexpr int kRouteThreads = 512, kRouteWideThreads = 1024, kRouteBlocks = 96, kRouteAllAlone = 24, kRouteAllMany = 32;
 __device__ __forceinline__ void route_device(const McbRouteArgs& a, int* smem, int all_per_thread = kRouteAllAlone) {
   const RouteSmem m(smem);

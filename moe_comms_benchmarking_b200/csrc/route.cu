@@ -43,9 +43,9 @@ __global__ void __launch_bounds__(512) combine_kernel(const __grid_constant__ Mc
   combine_body<true>(c, a);
 }
 
-// The same in a world of one where rows allow packs of 32 bytes, by two blocks for each of the chip's 148 SMs.  With fewer blocks it is slower than the kernel above at
-// large batches: 4096 tokens of 22 ids, an eighth local, by 148 / 64 / 16 blocks 7.1 / 11.7 / 36.7 us (7.2 / 10.9 / 30.5 above, 5.8 by 296), 8 ids and rows of
-// 7168 34.8 / 63.3 / 207 (29.9 / 49.5 / 149, 24.1); so callers that ask for fewer get that one.
+// The same in a world of one where rows allow packs of 32 bytes, by two blocks for each of the chip's 148 SMs.  With fewer blocks it is slower than the
+// kernel above at large batches: 4096 tokens of 22 ids, an eighth local, by 148 / 64 / 16 blocks 7.1 / 11.7 / 36.7 us (7.2 / 10.9 / 30.5 above, 5.8 by 296),
+// 8 ids and rows of 7168 34.8 / 63.3 / 207 (29.9 / 49.5 / 149, 24.1); so callers that ask for fewer get that one.
 constexpr int kCombineAloneBlocks = 2 * 148;
 __global__ void __launch_bounds__(512, 2) combine_alone_kernel(const __grid_constant__ McbCombineArgs a) {
   pdl_wait();
